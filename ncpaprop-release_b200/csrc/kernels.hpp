@@ -32,11 +32,14 @@ struct ProblemInfo {
     int c_lo, c_hi;        // Sturm counts at lo, hi
     int M, off;            // number of modes and offset into the mode arrays
     int used_wkb;
+    int wkb_trial;         // first WKB trial that ends the walk (kWkbNone before it is taken)
     int n_scan;            // shifts of the isolation scan (<= kScanMax)
     int n_scan_raw;        // the size estimated from the problem alone (before the batch-wide trim)
     float m_est;           // estimated mode count in [lo, hi] (-1: not estimated)
     double g0;             // wide-angle rows: ground term of row 0, 1 / (dz admittance + 1)
 };
+
+constexpr int kWkbNone = 1 << 30;
 
 struct WorkItem {
     int problem;  // problem index
@@ -92,7 +95,7 @@ int launch_attn_weight(cudaStream_t st, int nk, const double* zk, const double* 
 int launch_build_matrix(cudaStream_t st, int nk, const double* zk, const double* ceffk, const double* ceffcoef,
                         int n_az, int P, ProblemInfo* pinfo, int nz, int nz_pad, double z_min, double dz_grid,
                         double dz, double admittance, double* s, double* kz2, double* g);
-// WKB window and scaled bounds (K2)
+// WKB window and scaled bounds (K2); the records carry wkb_trial = kWkbNone
 int launch_window(cudaStream_t st, int P, ProblemInfo* pinfo, const double* kz2, int wkb, int wvnum,
                   double c_min, double c_max, unsigned* err);
 // isolation scan (K3a): sizes each problem's scan (ProblemInfo::n_scan) from

@@ -856,6 +856,7 @@ void layout_groups(ncpa_modes* M, std::vector<Group>& groups, long long& s_tot, 
                 pi.az = g.az[a];
                 pi.ceffmin_bits = 0x7ff0000000000000ull;
                 pi.ceffmax_bits = 0ull;
+                pi.wkb_trial = ncpa::kWkbNone;
                 pi.dz = g.geo.dz;
                 pi.nz = g.nz;
                 pi.isrc = g.geo.isrc;
