@@ -53,6 +53,13 @@ __device__ __forceinline__ double spline_deriv(int n, const double* __restrict__
     return c[2] + t * (2.0 * c[1] + t * 3.0 * c[0]);
 }
 
+// shift t of an isolation scan of n points on an even grid of [lo, hi]
+__device__ __forceinline__ double scan_x(double lo, double hi, int t, int n) {
+    if (t == 0) return lo;
+    if (t == n - 1) return hi;
+    return lo + (hi - lo) * ((double)t / (double)(n - 1));
+}
+
 // ---------------------------------------------------------------------------
 // power-of-two rescaling (exact)
 // ---------------------------------------------------------------------------

@@ -15,6 +15,7 @@
 //  K6  ModBB transfer function + pulse synthesis
 //      (ModalBroadbandPropagator.cpp:245-277, BroadbandPropagator.cpp:327-662)
 #include "device_common.cuh"
+#include "item_sched.cuh"
 #include "kernels.hpp"
 
 #include <cuda/std/complex>
@@ -530,10 +531,11 @@ __global__ void k_window(int P, ProblemInfo* __restrict__ pinfo, int wkb, int wv
         k_max = 2 * kPi * pi.freq / c_min;
     }
     const double h2 = dz * dz;
+    const double lo = (k_min * k_min) * h2, hi = (k_max * k_max) * h2;
     pinfo[p].k_min = k_min;
     pinfo[p].k_max = k_max;
-    pinfo[p].lo = (k_min * k_min) * h2;
-    pinfo[p].hi = (k_max * k_max) * h2;
+    pinfo[p].lo = lo;
+    pinfo[p].hi = hi;
     pinfo[p].used_wkb = wkb ? 1 : 0;
     pinfo[p].n_scan = kScanDefault;
     pinfo[p].n_scan_raw = kScanDefault;
@@ -554,13 +556,6 @@ int launch_window(cudaStream_t st, int P, ProblemInfo* pinfo, const double* kz2,
     return n;
 }
 
-// shift t of an isolation scan of n points on an even grid of [lo, hi]
-__device__ __forceinline__ double scan_x(double lo, double hi, int t, int n) {
-    if (t == 0) return lo;
-    if (t == n - 1) return hi;
-    return lo + (hi - lo) * ((double)t / (double)(n - 1));
-}
-
 // K3a-1: the size of each problem's isolation scan.  The number of
 // eigenvalues of S (diagonal s_i, unit off-diagonals) below x is close to the
 // sum over the rows of theta_i / pi with cos theta_i = (s_i - x) / 2 clipped
@@ -570,7 +565,6 @@ __device__ __forceinline__ double scan_x(double lo, double hi, int t, int n) {
 // unit), between 64 and kScanMax: problems with many close
 // eigenvalues start their bisection better isolated, those with few stop
 // paying for shifts that isolate nothing.
-constexpr int kScanStep = 64;  // shifts per scan unit (one warp, two per lane)
 constexpr int kSizeThreads = 256;
 __global__ void __launch_bounds__(kSizeThreads) k_scan_size(ProblemInfo* __restrict__ pinfo,
                                                            const double* __restrict__ s) {
@@ -1043,56 +1037,6 @@ __device__ __forceinline__ bool scan_trimmable(const ProblemInfo& q) {
     const int u = q.n_scan_raw / kScanStep;
     return u >= 2 && q.m_est >= 0.f && (float)((u - 1) * kScanStep) >= 1.75f * q.m_est;
 }
-
-// Item scheduler of the bisection (and of the isolation scan's units, all of
-// equal cost).  The bisection's item list is cost-ordered, heaviest first
-// (k_make_items with order 1).  On each warp scheduler (SM and sub-partition)
-// the first warp to arrive takes items from the heavy end of the list and the
-// next workers - 1 from the light end, so a scheduler runs a heavy and a
-// light item side by side; later warps run no bisection (in the fused launch
-// they exit, or take eigenvector items when ev_workers_only is off).  A worker first draws a ticket
-// (n tickets for n items) and then an index from its end of the list: front
-// and back indices never meet, so every item runs exactly once.  Where the
-// CTAs land only decides the balance: the first warp on every scheduler is a
-// worker.  sched: kSchedInts ints zeroed before the launch; null keeps plain
-// round-robin (item q to warp q mod (grid x kWarpsPerCta)).
-struct ItemSched {
-    int* S;
-    int role;     // 0: none, 1: heavy end, 2: light end
-    bool worker;  // the warp runs bisection items (every warp without sched)
-    __device__ ItemSched(int* sched, int workers) : S(sched), role(0), worker(true) {
-        if (!S) return;
-        const int lane = threadIdx.x & 31;
-        if (lane == 0) {
-            // the warp's SM and its sub-partition (hardware warp slot mod 4; a
-            // CTA's warp index does not determine it)
-            unsigned smid, slot;
-            asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-            asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
-            const int key = smid < (unsigned)kSchedSms ? (int)(smid * 4 + (slot & 3u)) : -1;
-            const int k = key >= 0 ? atomicAdd(S + 3 + key, 1) : 0;
-            role = k == 0 ? 1 : (k < workers ? 2 : 0);
-        }
-        role = __shfl_sync(0xffffffffu, role, 0);
-        worker = role != 0;
-    }
-    // next item of this warp (-1: none left); walk = plain round-robin position
-    __device__ long long next(int n, long long& walk, long long stride) {
-        if (!S) {
-            const long long it = walk;
-            walk += stride;
-            return it < n ? it : -1;
-        }
-        if (!role) return -1;
-        int it = -1;
-        if ((threadIdx.x & 31) == 0) {
-            if (atomicAdd(S, 1) < n) it = role == 1 ? atomicAdd(S + 1, 1) : n - 1 - atomicAdd(S + 2, 1);
-        }
-        it = __shfl_sync(0xffffffffu, it, 0);
-        if (it < 0) role = 0;
-        return it;
-    }
-};
 
 // unit u of the (trimmed) scan: its problem p, first shift tb and the
 // problem's scan size n; p = -1 past the last unit.  Every warp lane takes

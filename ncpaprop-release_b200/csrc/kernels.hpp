@@ -36,6 +36,11 @@ struct ProblemInfo {
     int n_scan;            // shifts of the isolation scan (<= kScanMax)
     int n_scan_raw;        // the size estimated from the problem alone (before the batch-wide trim)
     float m_est;           // estimated mode count in [lo, hi] (-1: not estimated)
+    int upp, sp_blk;       // the scan's panels (panel.cu): scan units per panel and rows per block (0: raw rows)
+    int item0;             // first work item
+    int grp_off, grp_cap;  // panel descriptors reserved for the work items
+    int blk_cap;           // block records reserved (the scan's panels, then the work items')
+    long long blk_off;     // the first of them
     double g0;             // wide-angle rows: ground term of row 0, 1 / (dz admittance + 1)
 };
 
@@ -45,10 +50,27 @@ struct WorkItem {
     int problem;  // problem index
     int j0;       // first eigen-index inside the problem (0 = lowest k)
     int m;        // eigenvalues in this item (<= kWItem for bisection)
-    int pad;
+    int pad;      // its panel (panel.cu; -1: none)
+};
+
+// Panel expansions (panel.cu): degrees of the block matrices and of their
+// derivatives with respect to a weight, record sizes in doubles, records per
+// shared-memory chunk, block sizes and the bound on r B^2
+constexpr int kPD = 14, kPW = 11;
+constexpr int kRecT = 4 * (kPD + 1) + 2, kRecW = 4 * (kPW + 1);
+constexpr int kPanelChunk = 4;
+constexpr int kPanelMaxBlk = 128, kPanelMinBlk = 8;
+constexpr double kRhoMax = 10.0;
+
+struct PanelDesc {
+    double xc, r;   // shifts within r of xc
+    long long rec;  // first block record
+    int blk;        // rows per block
+    int problem;    // -1: unused
 };
 
 constexpr int kScanMax = 512;      // count slots per problem of the isolation scan
+constexpr int kScanStep = 64;      // shifts per scan unit (one warp, two per lane)
 constexpr int kScanDefault = 256;  // shifts per problem unless the scan sizes them (wide-angle rows)
 constexpr int kChunk = 1024;      // doubles per TMA chunk of the diagonal
 constexpr int kBlk = 16;          // eigenvector checkpoint interval
@@ -60,6 +82,8 @@ inline long long ck_slot_elems(long long nz) {
     const long long a = (nz + kBlk - 1) / kBlk, b = 3 * ((nz + kCkRows - 1) / kCkRows);
     return (a > b ? a : b) * 32;
 }
+// elements per warp slot of the coarse rows of grids of up to nz points
+inline long long coarse_slot_elems(long long nz) { return (nz + kCkRows - 1) / kCkRows * 32; }
 constexpr int kThreads = 256;     // threads of the scan CTAs
 constexpr int kWItem = 32;        // eigenvalues per warp work item of the bisection
 constexpr int kEvItem = 32;       // eigenvalues per warp work item of the eigenvector kernel
@@ -189,6 +213,48 @@ int fused_wmod_ctas_per_sm();
 int launch_make_items(cudaStream_t st, int P, ProblemInfo* pinfo, const int* counts, int max_modes, int bis_item,
                       WorkItem* bis_items, int bis_cap, WorkItem* ev_items, int ev_cap, int* tot, unsigned* err,
                       int* pstat = nullptr, int order = 0);
+// The eigen-solve on panel expansions (panel.cu; ESS rows).  T: block
+// transfer matrices (kRecT doubles a record), W0, W1: their derivatives for the
+// weights w and, for group speeds, g (kRecW doubles).
+// Isolation scan: sizes, batch-wide trim (slots: warp schedulers of the device,
+// 0 for none; done: a zeroed counter), expansions and Sturm counts at
+// pinfo[p].n_scan points, counts[p kScanMax + t]
+int launch_panel_scan(cudaStream_t st, int P, int nz_max, ProblemInfo* pinfo, const double* s, double* T, int* counts,
+                      int slots, unsigned* done, unsigned* err);
+// c_lo, c_hi, M and off of every problem, the work items (at most bis_item
+// eigenvalues, their panel in WorkItem::pad or -1) and the panels; tot =
+// {items, items, modes}; kErrTooMany above max_modes or cap
+int launch_panel_items(cudaStream_t st, int P, ProblemInfo* pinfo, const int* counts, int max_modes, int bis_item,
+                       WorkItem* items, int cap, PanelDesc* desc, int* tot, unsigned* err, int order);
+// expansions of the work items' panels
+int launch_panel_expand(cudaStream_t st, int n_desc, int nz_max, const ProblemInfo* pinfo, const PanelDesc* desc,
+                        const double* s, const double* w, const double* g, double* T, double* W0, double* W1);
+constexpr int kPanelSlots = 4;  // two pairs of warps, two directions each
+constexpr int kCkVals = 4;  // doubles of a coarse row's checkpoint, at most
+struct ModesArgs {
+    const ProblemInfo* pinfo;
+    const double* rows;
+    const double* w;
+    const double* g;  // null: no group speeds
+    const double *T, *W0, *W1;
+    const PanelDesc* desc;
+    const int* counts;
+    const WorkItem* items;
+    const int* n_items_dev;
+    double tol;
+    double* mu;
+    double *kr, *ki, *vs, *vr, *vg;
+    double* ck_u;  // per CTA: kPanelSlots x kCkVals ck_stride doubles, kPanelSlots x ck_stride ints
+    int* ck_e;
+    long long ck_stride;
+    int* sched;  // item counter (zeroed) or null: round-robin
+    unsigned* err;
+    unsigned long long* steps;  // optional counter of row steps
+};
+// what: 1 eigenvalues, 2 mode values of the eigenvalues in mu, 3 both
+int launch_panel_modes(cudaStream_t st, int grid, const ModesArgs& a, int what);
+int panel_ctas_per_sm();
+
 // resident eigenvector CTAs per SM for the variant selected by a
 int eigvec_ctas_per_sm(const EigvecArgs& a);
 // modal sums

@@ -111,6 +111,7 @@ struct ncpa_ctx {
     int num_sms = 148;
     DevBuf d_err;                  // device status word
     DevBuf ck1, ck2, cke;          // eigenvector checkpoint scratch
+    DevBuf ex;                     // panel expansions
     std::map<int, DevBuf> twiddle; // per nfft
     DevBuf bb_out;                 // waveforms kept in HBM (NULL host buffer)
     DevBuf ms_img, ms_q, ms_tab, ms_raw, ms_vz, ms_idx, ms_re, ms_im;  // modal-sum scratch (grow-only)
@@ -152,7 +153,7 @@ struct ncpa_ctx {
     bool stats = false;            // ncpa_ctx_set_timing: accumulate per phase
     bool stats_fused = false;      // ncpa_ctx_set_timing(ctx, 2): ... keeping the fused launch
     std::map<std::string, std::pair<double, long long>> phase;
-    std::map<std::string, std::array<int, 3>> tune_cache;  // plan shape -> tuned launch shapes
+    std::map<std::string, std::array<int, 2>> tune_cache;  // plan shape -> tuned launch shapes
     void count(int n) { launches += n; }
 };
 
@@ -196,6 +197,7 @@ struct ncpa_profile {
     double z0 = 0.0;
     int has_z0 = 0;
     double z_lo = 0.0, z_hi = 0.0;
+    std::vector<double> h_c0, h_u, h_v;  // host copies: bounds of c_eff size the panel expansions
     int plan_refs = 0;  // plans whose graphs read this profile's arrays
 };
 
@@ -209,6 +211,8 @@ struct ncpa_modes {
     bool multi_job = false;                     // built by ncpa_ess_solve_jobs (one profile per job)
     bool plan_owned = false;                    // the arrays are a plan's graph buffers
     std::vector<ProblemInfo> info;
+    long long n_blocks = 0;  // block records of the panel expansions
+    int n_desc = 0;          // panels of the work items
     int Mtot = 0;
     DevBuf d_pinfo, d_kr, d_ki, d_vs, d_vr, d_vg, d_vfull, d_vfull_off;
     mutable DevBuf tl_re, tl_im, tl_inc;  // 1-D TL kept in HBM
@@ -467,182 +471,136 @@ void enqueue_group(ncpa_ctx* ctx, PhaseTimer& tm, const Group& g, GroupBufs& b, 
 
 // Launch shapes of the device-driven eigen-solve (the autotuner's knobs).
 struct Tuning {
-    int bis_item = ncpa::kWItem;  // eigenvalues per bisection work item (<= 32)
-    int bis_ctas = 0;             // bisection CTAs per SM (0: as many as fit)
-    int ev_ctas = 0;              // eigenvector CTAs per SM (0: as many as fit)
+    int bis_item = ncpa::kWItem;  // eigenvalues per work item (<= 32)
+    int bis_ctas = 0;             // CTAs per SM (0: as many as fit)
 };
 
-// Buffers of the device-driven eigen-solve.  The eigenvector checkpoint
-// scratch is the context's (grown on demand) unless own_ck is set (a
-// captured graph must keep its addresses for good).
+// Buffers of the device-driven eigen-solve.  The panel expansions and the
+// eigenvector checkpoints are the context's (grown on demand: as per-solve
+// allocations of some hundred MB they cost the host 350 us a solve) unless
+// own_ck is set (a captured graph must keep its addresses for good).
 struct SolveBufs {
-    DevBuf counts, bis, ev, tot, mu, counter, sched;
-    DevBuf pstat, fq;  // fused launch: per-problem readiness; ready queue, done flags, queue counters
-    DevBuf ck1, ck2, cke;
+    DevBuf counts, items, tot, mu, sched;
+    DevBuf desc;
+    DevBuf ex, ck1, cke;  // own_ck: panel expansions and checkpoints (else the context's)
+    double *T = nullptr, *W0 = nullptr, *W1 = nullptr;
     bool own_ck = false;
-    int bis_cap = 0, ev_cap = 0;
+    int item_cap = 0;
 };
 
-ncpa::EigvecArgs eigvec_args(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, double* s, double* w,
-                             double* gs, SolveBufs& b) {
-    ncpa::EigvecArgs ea{};
-    ea.pinfo = M->d_pinfo.as<ProblemInfo>();
-    ea.s = s;
-    ea.w = w;
-    ea.g = prm->want_group_speed ? gs : nullptr;
-    ea.items = b.ev.as<WorkItem>();
-    ea.n_items = 0;
-    ea.n_items_dev = b.tot.as<int>() + 1;
-    ea.counter = b.counter.as<int>() + 1;
-    ea.mu = b.mu.as<double>();
-    ea.kr = M->d_kr.as<double>();
-    ea.ki = M->d_ki.as<double>();
-    ea.vs = M->d_vs.as<double>();
-    ea.vr = M->d_vr.as<double>();
-    ea.vg = M->d_vg.as<double>();
-    ea.err = ctx->d_err.as<unsigned>();
-    return ea;
-}
-
-int eigvec_grid(ncpa_ctx* ctx, const ncpa::EigvecArgs& ea, int ev_cap, int ctas_per_sm) {
-    const int fit = ncpa::eigvec_ctas_per_sm(ea);
-    const int per_sm = ctas_per_sm > 0 ? std::min(ctas_per_sm, fit) : fit;
-    return std::max(1, std::min(ev_cap / ncpa::kEvWarpsPerCta + 1, ctx->num_sms * per_sm));
+int modes_grid(const ncpa_ctx* ctx, int ctas_per_sm) {
+    const int fit = ncpa::panel_ctas_per_sm();
+    return ctx->num_sms * (ctas_per_sm > 0 ? std::min(ctas_per_sm, fit) : fit);
 }
 
 // Allocates the eigen-solve's buffers and the mode arrays (max_modes per
-// problem) and sizes the eigenvector checkpoint scratch for the largest grid
-// any of the given tunings launches.  min_bis_item sizes the bisection item
-// list for the smallest item size that will run.
-void prepare_solve(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, int min_bis_item, SolveBufs& b,
-                   double* s, double* w, double* gs) {
+// problem) and sizes the checkpoint scratch for the largest grid any of the
+// given tunings launches.  min_bis_item sizes the item list for the smallest
+// item size that will run.
+void prepare_solve(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, int min_bis_item, SolveBufs& b) {
     cudaStream_t st = ctx->stream;
     const int P = M->P;
     const int cap_modes = M->prm.max_modes;
     const size_t mcap = (size_t)P * cap_modes;
     b.counts.alloc((size_t)P * ncpa::kScanMax * 4, st);
-    b.bis_cap = P * ((cap_modes + min_bis_item - 1) / min_bis_item);
-    b.ev_cap = P * ((cap_modes + ncpa::kEvItem - 1) / ncpa::kEvItem);
-    b.bis.alloc((size_t)b.bis_cap * sizeof(WorkItem), st);
-    b.ev.alloc((size_t)b.ev_cap * sizeof(WorkItem), st);
+    b.item_cap = P * ((cap_modes + min_bis_item - 1) / min_bis_item);
+    b.desc.alloc((size_t)M->n_desc * sizeof(ncpa::PanelDesc), st);
+    b.items.alloc((size_t)b.item_cap * sizeof(WorkItem), st);
     b.tot.alloc(4 * sizeof(int), st);
-    b.pstat.alloc((size_t)3 * P * sizeof(int), st);
-    b.fq.alloc(((size_t)2 * b.ev_cap + 2) * sizeof(int), st);
     b.mu.alloc(mcap * 8, st);
-    b.counter.alloc(2 * sizeof(int), st);
-    b.sched.alloc(ncpa::kSchedInts * sizeof(int), st);
+    b.sched.alloc(4 * sizeof(int), st);
+    const size_t nT = (size_t)M->n_blocks * ncpa::kRecT, nW = (size_t)M->n_blocks * ncpa::kRecW;
+    DevBuf& ex = b.own_ck ? b.ex : ctx->ex;
+    const size_t n_ex = (nT + (prm->want_group_speed ? 2 : 1) * nW) * 8;
+    // a quarter more than asked when it grows: other atmospheres need a little more or less
+    if (ex.bytes < n_ex) ex.alloc(b.own_ck ? n_ex : n_ex + n_ex / 4, st);
+    b.T = ex.as<double>();
+    b.W0 = b.T + nT;
+    b.W1 = prm->want_group_speed ? b.W0 + nW : nullptr;
     M->d_kr.alloc(mcap * 8, st);
     M->d_ki.alloc(mcap * 8, st);
     M->d_vs.alloc(mcap * 8, st);
     M->d_vr.alloc(mcap * 8, st);
     M->d_vg.alloc(mcap * 8, st);
-    const ncpa::EigvecArgs ea = eigvec_args(ctx, M, prm, s, w, gs, b);
-    const int grid_e = eigvec_grid(ctx, ea, b.ev_cap, 0);  // the largest grid
-    const long long slot = ncpa::ck_slot_elems(M->nz_max);
-    const size_t need = (size_t)grid_e * ncpa::kEvWarpsPerCta * slot;
+    const size_t need = (size_t)modes_grid(ctx, 0) * ncpa::kPanelSlots * ncpa::coarse_slot_elems(M->nz_max);
     DevBuf& c1 = b.own_ck ? b.ck1 : ctx->ck1;
-    DevBuf& c2 = b.own_ck ? b.ck2 : ctx->ck2;
     DevBuf& ce = b.own_ck ? b.cke : ctx->cke;
-    if (c1.bytes < need * 8) {
-        c1.alloc(need * 8, st);
-        c2.alloc(need * 8, st);
-        ce.alloc(need * 4, st);
-    }
+    c1.alloc(need * ncpa::kCkVals * 8, st);
+    ce.alloc(need * 4, st);
 }
 
-// Window, Sturm scan, device-built work items, bisection and eigenvectors
-// over all problems of M, then copies of the item/mode totals, the problem
 // warp schedulers of the device for the scan trim (0: no trim)
 int scan_slots(const ncpa_ctx* ctx) { return ctx->scan_trim ? 4 * ctx->num_sms : 0; }
 
-// records and the device status word to tot_dst, info_dst and err_dst.  No
-// host synchronisation: the whole sequence can be captured in a CUDA graph.
+// Window, panel expansions, Sturm scan, device-built work items, eigenvalues
+// and mode values over all problems of M, then copies of the item/mode
+// totals, the problem records and the device status word to tot_dst, info_dst
+// and err_dst.  No host synchronisation: the whole sequence can be captured
+// in a CUDA graph.
 void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_params* prm, bool wkb, double* s,
                    double* w, double* gs, double* kz2, SolveBufs& b, const Tuning& t, bool count_steps,
                    int* tot_dst, ProblemInfo* info_dst, unsigned* err_dst) {
     cudaStream_t st = ctx->stream;
     const int P = M->P;
     ProblemInfo* d_pinfo = M->d_pinfo.as<ProblemInfo>();
+    ncpa::PanelDesc* desc = b.desc.as<ncpa::PanelDesc>();
     unsigned* err = ctx->d_err.as<unsigned>();
+    const double* g = prm->want_group_speed ? gs : nullptr;
     // ---- K2 window ----
     check_launch(ctx, ncpa::launch_window(st, P, d_pinfo, wkb ? kz2 : nullptr, wkb ? 1 : 0, prm->wvnum_filter,
                                           prm->c_min, prm->c_max, err));
     tm.mark("window");
-    // ---- K3a scan ----
-    // the scan's units claimed per warp scheduler through the item scheduler's
-    // state (zeroed again below before the bisection uses it)
-    int* scan_sched = nullptr;
-    if (scan_slots(ctx) > 0) {
-        scan_sched = b.sched.as<int>();
-        CK(cudaMemsetAsync(scan_sched, 0, ncpa::kSchedInts * sizeof(int), st));
-    }
-    check_launch(ctx, ncpa::launch_scan(st, P, d_pinfo, s, b.counts.as<int>(), err, scan_slots(ctx), scan_sched));
+    // ---- isolation scan ----
+    // item counters of the launches below and the scan's block counter
+    CK(cudaMemsetAsync(b.sched.p, 0, 4 * sizeof(int), st));
+    check_launch(ctx, ncpa::launch_panel_scan(st, P, M->nz_max, d_pinfo, s, b.T, b.counts.as<int>(),
+                                              scan_slots(ctx), b.sched.as<unsigned>() + 2, err));
     tm.mark("scan");
-    // fused bisection + eigenvectors (one launch, eigenvectors of finished
-    // problems overlapping the others' bisection), unless per-phase timing or
-    // step counts ask for the kernels alone, or group speeds are wanted
-    const bool fuse = ctx->fuse_solve && !ctx->timing && (!ctx->stats || ctx->stats_fused) && !count_steps &&
-                      !prm->want_group_speed;
-    check_launch(ctx, ncpa::launch_make_items(st, P, d_pinfo, b.counts.as<int>(), M->prm.max_modes, t.bis_item,
-                                              b.bis.as<WorkItem>(), b.bis_cap, b.ev.as<WorkItem>(), b.ev_cap,
-                                              b.tot.as<int>(), err, fuse ? b.pstat.as<int>() : nullptr,
-                                              ctx->bis_order ? 1 : 0));
-    CK(cudaMemsetAsync(b.counter.p, 0, 2 * sizeof(int), st));
-    int* sched = nullptr;
-    if (ctx->bis_order) {
-        sched = b.sched.as<int>();
-        CK(cudaMemsetAsync(sched, 0, ncpa::kSchedInts * sizeof(int), st));
-    }
+    // one launch for eigenvalues and mode values, unless per-phase timing or
+    // step counts ask for the two apart
+    const bool fuse = ctx->fuse_solve && !ctx->timing && (!ctx->stats || ctx->stats_fused) && !count_steps;
+    check_launch(ctx, ncpa::launch_panel_items(st, P, d_pinfo, b.counts.as<int>(), M->prm.max_modes, t.bis_item,
+                                               b.items.as<WorkItem>(), b.item_cap, desc, b.tot.as<int>(), err,
+                                               ctx->bis_order ? 1 : 0));
     tm.mark("host-items");
-    const int fit_b = ncpa::bisect_ctas_per_sm();
-    const int grid_b = ctx->num_sms * (t.bis_ctas > 0 ? std::min(t.bis_ctas, fit_b) : fit_b);
-    ncpa::EigvecArgs ea = eigvec_args(ctx, M, prm, s, w, gs, b);
-    const int grid_e = eigvec_grid(ctx, ea, b.ev_cap, t.ev_ctas);
-    ea.ck_q1 = (b.own_ck ? b.ck1 : ctx->ck1).as<double>();
-    ea.ck_q2 = (b.own_ck ? b.ck2 : ctx->ck2).as<double>();
-    ea.ck_e = (b.own_ck ? b.cke : ctx->cke).as<int>();
-    ea.ck_slot_stride = ncpa::ck_slot_elems(M->nz_max);
+    // ---- panel expansions ----
+    check_launch(ctx, ncpa::launch_panel_expand(st, M->n_desc, M->nz_max, d_pinfo, desc, s, w, g, b.T,
+                                                b.W0, b.W1));
+    tm.mark("expand");
+    ncpa::ModesArgs a{};
+    a.pinfo = d_pinfo;
+    a.rows = s;
+    a.w = w;
+    a.g = g;
+    a.T = b.T;
+    a.W0 = b.W0;
+    a.W1 = b.W1;
+    a.desc = desc;
+    a.counts = b.counts.as<int>();
+    a.items = b.items.as<WorkItem>();
+    a.n_items_dev = b.tot.as<int>();
+    a.tol = kBisectTol;
+    a.mu = b.mu.as<double>();
+    a.kr = M->d_kr.as<double>();
+    a.ki = M->d_ki.as<double>();
+    a.vs = M->d_vs.as<double>();
+    a.vr = M->d_vr.as<double>();
+    a.vg = M->d_vg.as<double>();
+    a.ck_u = (b.own_ck ? b.ck1 : ctx->ck1).as<double>();
+    a.ck_e = (b.own_ck ? b.cke : ctx->cke).as<int>();
+    a.ck_stride = ncpa::coarse_slot_elems(M->nz_max);
+    a.sched = ctx->bis_order ? b.sched.as<int>() : nullptr;
+    a.err = err;
     if (fuse) {
-        int* fq = b.fq.as<int>();
-        CK(cudaMemsetAsync(fq, 0, ((size_t)2 * b.ev_cap + 2) * sizeof(int), st));
-        ncpa::FusedArgs fa{};
-        fa.P = P;
-        fa.pinfo = d_pinfo;
-        fa.s = s;
-        fa.counts = b.counts.as<int>();
-        fa.bis = b.bis.as<WorkItem>();
-        fa.n_bis_dev = b.tot.as<int>();
-        fa.tol = kBisectTol;
-        fa.mu = b.mu.as<double>();
-        fa.err = err;
-        fa.pstat = b.pstat.as<int>();
-        fa.queue = fq;
-        fa.ev_done = fq + b.ev_cap;
-        fa.wait_ns = ctx->fuse_wait_ns;
-        fa.sched = sched;
-        fa.workers = ctx->bis_workers;
-        fa.ev_workers_only = ctx->fuse_ev_workers && sched ? 1 : 0;
-        fa.q_head = fq + 2 * b.ev_cap;
-        fa.q_tail = fq + 2 * b.ev_cap + 1;
-        fa.ea = ea;
-        // no more warps than the checkpoint scratch has slots (sized for grid_e)
-        const int fit_f = ncpa::fused_ctas_per_sm();
-        const int grid_f =
-            std::min(grid_e, ctx->num_sms * (t.bis_ctas > 0 ? std::min(t.bis_ctas, fit_f) : fit_f));
-        check_launch(ctx, ncpa::launch_bisect_eigvec(st, grid_f, fa));
+        check_launch(ctx, ncpa::launch_panel_modes(st, modes_grid(ctx, t.bis_ctas), a, 3));
         tm.mark("bisect+eigvec");
-        ea.ev_done = fa.ev_done;  // the items the fused launch did not finish
-        check_launch(ctx, ncpa::launch_eigvec(st, grid_e, ea));
-        tm.mark("eigvec-rest");
     } else {
-        // ---- K3 bisection ----
-        check_launch(ctx, ncpa::launch_bisect(st, grid_b, d_pinfo, s, b.counts.as<int>(), b.bis.as<WorkItem>(), 0,
-                                              b.counter.as<int>(), kBisectTol, b.mu.as<double>(), err,
-                                              count_steps ? ctx->d_stats.as<unsigned long long>() : nullptr,
-                                              b.tot.as<int>(), sched, ctx->bis_workers));
+        a.steps = count_steps ? ctx->d_stats.as<unsigned long long>() : nullptr;
+        check_launch(ctx, ncpa::launch_panel_modes(st, modes_grid(ctx, t.bis_ctas), a, 1));
         tm.mark("bisect");
-        // ---- K4 eigenvectors ----
-        check_launch(ctx, ncpa::launch_eigvec(st, grid_e, ea));
+        a.steps = nullptr;
+        if (a.sched) ++a.sched;
+        check_launch(ctx, ncpa::launch_panel_modes(st, modes_grid(ctx, t.bis_ctas), a, 2));
         tm.mark("eigvec");
     }
     CK(cudaMemcpyAsync(tot_dst, b.tot.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -686,7 +644,7 @@ void solve_core(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_par
         Tuning t;
         if (ctx->item_override > 0) t.bis_item = std::min(ctx->item_override, ncpa::kWItem);
         SolveBufs b;
-        prepare_solve(ctx, M, prm, t.bis_item, b, s.as<double>(), w.as<double>(), g.as<double>());
+        prepare_solve(ctx, M, prm, t.bis_item, b);
         unsigned h_err = 0;
         enqueue_solve(ctx, tm, M, prm, wkb, s.as<double>(), w.as<double>(), g.as<double>(), kz2.as<double>(), b, t,
                       ctx->stats && !ctx->stats_fused, ctx->h_tot, M->info.data(), &h_err);
@@ -803,11 +761,10 @@ void solve_core(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_par
         const int grid_e = std::min((n_ev + ewpc - 1) / ewpc, ctx->num_sms * ncpa::eigvec_ctas_per_sm(ea));
         const long long slot = ncpa::ck_slot_elems(M->nz_max);
         const size_t need = (size_t)grid_e * ewpc * slot;
-        if (ctx->ck1.bytes < need * 8) {
-            ctx->ck1.alloc(need * 8, st);
-            ctx->ck2.alloc(need * 8, st);
-            ctx->cke.alloc(need * 4, st);
-        }
+        // (alloc keeps a buffer that is large enough)
+        ctx->ck1.alloc(need * 8, st);
+        ctx->ck2.alloc(need * 8, st);
+        ctx->cke.alloc(need * 4, st);
         ea.ck_q1 = ctx->ck1.as<double>();
         ea.ck_q2 = ctx->ck2.as<double>();
         ea.ck_e = ctx->cke.as<int>();
@@ -870,12 +827,83 @@ void layout_groups(ncpa_modes* M, std::vector<Group>& groups, long long& s_tot, 
     }
 }
 
+// extremes of c_eff = c0 + u sin(az) + v cos(az) at the knots
+std::pair<double, double> ceff_bounds(const ncpa_profile* prof, double az_deg) {
+    const double s = std::sin(az_deg * kPi / 180.0), c = std::cos(az_deg * kPi / 180.0);
+    const double *c0 = prof->h_c0.data(), *u = prof->h_u.data(), *v = prof->h_v.data();
+    double lo[4] = {INFINITY, INFINITY, INFINITY, INFINITY}, hi[4] = {0.0, 0.0, 0.0, 0.0};
+    const int n = prof->n;
+    for (int i = 0; i < n; i += 4)
+        for (int k = 0; k < 4; ++k) {  // four independent chains
+            const int j = std::min(i + k, n - 1);
+            const double x = c0[j] + (u[j] * s + v[j] * c);
+            lo[k] = x < lo[k] ? x : lo[k];
+            hi[k] = x > hi[k] ? x : hi[k];
+        }
+    return {std::min(std::min(lo[0], lo[1]), std::min(lo[2], lo[3])),
+            std::max(std::max(hi[0], hi[1]), std::max(hi[2], hi[3]))};
+}
+
+// Reserves the panels and block records of every problem (panel.cu).  With
+// the extremes c_lo, c_hi of c_eff at the knots (or the wavenumber filter's),
+// the window of h^2 k^2 has a half-width of at most R = h^2 omega^2 (1 / c_lo^2 -
+// 1 / c_hi^2) / 2, and a column of height H at most about 2 f H sqrt(1 / c_lo^2
+// - 1 / c_hi^2) modes.  At the largest block B two neighbouring panels span
+// more than 2 kRhoMax / B^2, and an item that needs a smaller block of b rows is
+// itself wider than kRhoMax / (2 b)^2; over disjoint panels that makes at most
+// 2 nz R B / kRhoMax records, or 2 nz sqrt(n R / kRhoMax) for n items.  slack
+// widens R for plans, whose profiles may change between replays.  A problem
+// that needs more after all sweeps its raw rows.
+void layout_panels(ncpa_modes* M, const std::vector<Group>& groups, const ncpa_ess_params* prm, double slack) {
+    M->n_blocks = 0;
+    M->n_desc = 0;
+    const double rho = ncpa::kRhoMax, B = ncpa::kPanelMaxBlk;
+    const double n_s = ncpa::kScanMax / ncpa::kScanStep;  // scan panels
+    std::map<std::pair<const ncpa_profile*, double>, std::pair<double, double>> seen;
+    for (const Group& g : groups)
+        for (int a = 0; a < g.n_az; ++a) {
+            double c_lo, c_hi;
+            if (prm->wvnum_filter) {
+                c_lo = std::min(prm->c_min, prm->c_max);
+                c_hi = std::max(prm->c_min, prm->c_max);
+            } else {
+                // jobs of a sweep share their profile and azimuths
+                auto [it, fresh] = seen.try_emplace({g.prof, g.az[a]});
+                if (fresh) it->second = ceff_bounds(g.prof, g.az[a]);
+                c_lo = it->second.first;
+                c_hi = it->second.second;
+            }
+            c_lo = std::max(c_lo, 50.0);
+            c_hi = std::max(c_hi, 1.001 * c_lo);
+            const double dk = 1.0 / (c_lo * c_lo) - 1.0 / (c_hi * c_hi);
+            for (int f = 0; f < g.n_freq; ++f) {
+                ProblemInfo& pi = M->info[g.p0 + f * g.n_az + a];
+                const double kh = pi.omega * pi.dz, nz = pi.nz;
+                const double R = std::min(1.05 * slack * 0.5 * kh * kh * dk, 8.0);
+                // items of 16 modes, the smallest a plan tries
+                const double n_it = std::min((2.0 * pi.freq * pi.dz * nz * std::sqrt(dk * slack) + 32.0) / 16.0, 4096.0);
+                const double n = std::max(n_it, n_s);
+                const double n_g = std::ceil(std::min(2.0 * R * B * B / rho + 2.0, n_it));
+                const double blocks = std::min(2.0 * nz * R * B / rho, 2.0 * nz * std::sqrt(n * R / rho)) +
+                                      2.0 * std::ceil(nz / B);
+                pi.grp_off = M->n_desc;
+                pi.grp_cap = (int)n_g;
+                M->n_desc += pi.grp_cap;
+                pi.blk_off = M->n_blocks;
+                // every panel's records are padded to whole chunks
+                pi.blk_cap = (int)blocks + (int)(std::max(n_g, n_s) + 1.0) * ncpa::kPanelChunk;
+                M->n_blocks += pi.blk_cap;
+            }
+        }
+}
+
 void solve_groups(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, std::vector<Group>& groups) {
     cudaStream_t st = ctx->stream;
     PhaseTimer tm(ctx);
     tm.mark("start");
     long long s_tot = 0, w_tot = 0;
     layout_groups(M, groups, s_tot, w_tot);
+    layout_panels(M, groups, prm, 1.0);
     upload(M->d_pinfo, M->info, st);
     const bool wkb = wants_wkb(prm);
     DevBuf s, w, gs, kz2;
@@ -1089,7 +1117,7 @@ void solve_wmod(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, std::v
     const int grid_f = fused ? ctx->num_sms * ncpa::fused_wmod_ctas_per_sm() : 0;
     const long long slot = ncpa::ck_slot_elems(M->nz_max);
     const size_t need = (size_t)std::max(grid_e, grid_f) * ncpa::kEvWarpsPerCta * slot;
-    if (n_ev > 0 && ctx->ck1.bytes < need * 8) {
+    if (n_ev > 0) {  // alloc keeps a buffer that is large enough
         ctx->ck1.alloc(need * 8, st);
         ctx->ck2.alloc(need * 8, st);
         ctx->cke.alloc(need * 4, st);
@@ -1176,7 +1204,6 @@ struct PlanData {
     double* h_rho = nullptr;
     cudaGraphExec_t exec = nullptr;
     long long kernels = 0;  // kernel launches in one replay
-    int fit_e = 1;          // eigenvector CTAs per SM that fit
     double tuned_ms = 0.0;
 };
 
@@ -1468,6 +1495,7 @@ ncpa_status ncpa_ctx_destroy(ncpa_ctx* ctx) {
     ctx->twiddle.clear();
     ctx->bb_out.release();
     ctx->d_stats.release();
+    ctx->ex.release();
     ctx->ck1.release();
     ctx->ck2.release();
     ctx->cke.release();
@@ -1503,6 +1531,10 @@ namespace {
 void fill_profile(ncpa_ctx* ctx, ncpa_profile* P, const ncpa_profile_desc* d) {
     cudaStream_t st = ctx->stream;
     const int n = P->n;
+    P->h_c0.resize(n);
+    for (int i = 0; i < n; ++i) P->h_c0[i] = d->c0 ? d->c0[i] : std::sqrt(1.4 * d->p[i] / d->rho[i]);
+    P->h_u.assign(d->u, d->u + n);
+    P->h_v.assign(d->v, d->v + n);
     const std::pair<DevBuf*, const double*> cols[] = {{&P->z, d->z}, {&P->u, d->u}, {&P->v, d->v},
                                                       {&P->t, d->t}, {&P->p, d->p}, {&P->rho, d->rho}};
     for (const auto& c : cols) CK(cudaMemcpyAsync(c.first->p, c.second, n * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -2526,6 +2558,7 @@ ncpa_status ncpa_ess_plan_create(ncpa_ctx* ctx, const ncpa_ess_job* jobs, int n_
         M->az.assign(1, pl.groups[0].az[0]);
         long long s_tot = 0, w_tot = 0;
         layout_groups(M, pl.groups, s_tot, w_tot);
+        layout_panels(M, pl.groups, prm, 2.0);
         upload(pl.pinfo_init, M->info, st);
         M->d_pinfo.alloc((size_t)P * sizeof(ProblemInfo), st);
         pl.wkb = wants_wkb(prm);
@@ -2540,10 +2573,8 @@ ncpa_status ncpa_ess_plan_create(ncpa_ctx* ctx, const ncpa_ess_job* jobs, int n_
         pl.gb.resize(pl.groups.size());
         for (size_t gi = 0; gi < pl.groups.size(); ++gi) prepare_group(ctx, prm, pl.groups[gi], pl.gb[gi]);
         const int kMinItem = 16;  // smallest bisection item the tuner tries
-        double* gsp = prm->want_group_speed ? pl.gs.as<double>() : nullptr;
         pl.sb.own_ck = true;
-        prepare_solve(ctx, M, &pl.prm, tune ? kMinItem : ncpa::kWItem, pl.sb, pl.s.as<double>(), pl.w.as<double>(),
-                      gsp);
+        prepare_solve(ctx, M, &pl.prm, tune ? kMinItem : ncpa::kWItem, pl.sb);
         if (tl) {
             pl.with_tl = true;
             pl.tp = *tl;
@@ -2552,10 +2583,6 @@ ncpa_status ncpa_ess_plan_create(ncpa_ctx* ctx, const ncpa_ess_job* jobs, int n_
             M->tl_im.alloc(n, st);
             M->tl_inc.alloc(n, st);
         }
-        ncpa::bisect_ctas_per_sm();  // sets the kernels' shared-memory attributes before any capture
-        const int fit_e = ncpa::eigvec_ctas_per_sm(eigvec_args(ctx, M, &pl.prm, pl.s.as<double>(), pl.w.as<double>(),
-                                                               gsp, pl.sb));
-        pl.fit_e = fit_e;
         CK(cudaStreamSynchronize(st));
         char key[160];
         std::snprintf(key, sizeof key, "P%d s%lld w%lld nz%d m%d g%d t%d", P, s_tot, w_tot, M->nz_max,
@@ -2565,10 +2592,9 @@ ncpa_status ncpa_ess_plan_create(ncpa_ctx* ctx, const ncpa_ess_job* jobs, int n_
             if (hit != ctx->tune_cache.end()) {
                 pl.tuning.bis_item = hit->second[0];
                 pl.tuning.bis_ctas = hit->second[1];
-                pl.tuning.ev_ctas = hit->second[2];
             } else {
-                // coordinate search: item size, then bisection CTAs per SM, then
-                // eigenvector CTAs per SM, each timed on its captured graph
+                // coordinate search: item size, then CTAs per SM, each timed on
+                // its captured graph
                 Tuning best;
                 double best_ms = 1e300;
                 auto consider = [&](const Tuning& t) {
@@ -2593,19 +2619,13 @@ ncpa_status ncpa_ess_plan_create(ncpa_ctx* ctx, const ncpa_ess_job* jobs, int n_
                     consider(t);
                 }
                 const Tuning after_item = best;
-                for (int c = 1; c < ncpa::bisect_ctas_per_sm(); ++c) {
+                for (int c = 1; c < ncpa::panel_ctas_per_sm(); ++c) {
                     Tuning t = after_item;
                     t.bis_ctas = c;
                     consider(t);
                 }
-                const Tuning after_bis = best;
-                for (int c = 1; c < fit_e; ++c) {
-                    Tuning t = after_bis;
-                    t.ev_ctas = c;
-                    consider(t);
-                }
                 pl.tuning = best;
-                ctx->tune_cache[key] = {best.bis_item, best.bis_ctas, best.ev_ctas};
+                ctx->tune_cache[key] = {best.bis_item, best.bis_ctas};
             }
         }
         pl.exec = capture_plan(pl, pl.tuning);
@@ -2655,8 +2675,10 @@ ncpa_status ncpa_ess_plan_tuning(const ncpa_plan* plan, int* bis_item, int* bis_
     if (!plan) return NCPA_EINVAL;
     const PlanData& pl = plan->d;
     if (bis_item) *bis_item = pl.tuning.bis_item;
-    if (bis_ctas_per_sm) *bis_ctas_per_sm = pl.tuning.bis_ctas > 0 ? pl.tuning.bis_ctas : ncpa::bisect_ctas_per_sm();
-    if (ev_ctas_per_sm) *ev_ctas_per_sm = pl.tuning.ev_ctas > 0 ? pl.tuning.ev_ctas : pl.fit_e;
+    // eigenvalues and mode values run in one launch: one shape for both
+    const int ctas = pl.tuning.bis_ctas > 0 ? pl.tuning.bis_ctas : ncpa::panel_ctas_per_sm();
+    if (bis_ctas_per_sm) *bis_ctas_per_sm = ctas;
+    if (ev_ctas_per_sm) *ev_ctas_per_sm = ctas;
     if (ms) *ms = pl.tuned_ms;
     return NCPA_OK;
 }

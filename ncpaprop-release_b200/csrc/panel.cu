@@ -1,0 +1,1557 @@
+// The eigen-solve on panel expansions of the tridiagonal rows.
+//
+// The rows S = h^2 A - x (unit off-diagonals) act on the state (u_i, e_i),
+// u_i = (-1)^{i+1} p_i of the Sturm recurrence and e_i = u_i - u_{i-1}, as
+//   e_i = e_{i-1} - sigma_i u_{i-1},   u_i = u_{i-1} + e_i,
+//   sigma_i = s_i + 2 - x:
+// a discrete u'' = -sigma u.  The 2 x 2 transfer matrix of a block of B
+// consecutive rows is a smooth function of x: with x = x_c + r t, |t| <= 1, its
+// entries behave like cos and sin of B sqrt(sigma), whose Taylor series in t
+// falls like rho^k / (2k)!, rho = r B^2.  So the shifts of a solve are grouped
+// into panels (of scan points, then of work items), as wide as rho <= kRhoMax =
+// 10 allows at B = 128 rows a block, or one unit or item each at smaller
+// blocks; per panel and block the four entries are expanded once to degree kPD
+// (a thread per column, so the work is parallel over the rows), and every sweep
+// of the scan, the multisection, Laguerre's iteration and the eigenvector
+// passes advances B rows with four Horner evaluations.  The first term left
+// out, rho^15 / 30!, is 4e-18.
+//
+// What it buys (the row recurrence is bound by FP64 issue, 2 instructions a row
+// for a count and 6 with two derivatives, plus one for the sign): at B = 128
+// a count costs 60 instructions a block (0.47 a row) and a Laguerre chain 180
+// (1.4 a row), and the serial chain is two FMAs a block instead of one a row.
+// Accuracy: the rounding of a block perturbs sigma by about 1e-16 on one row
+// in B, and errors relative to u are harmless; eigenvalues agree with a
+// 128-bit evaluation of the row recurrence to 1e-18 (units of h^2 A; the row
+// recurrence itself: 1e-17), mode values to 1e-12.
+//
+// Counts.  The number of negative pivots is nz minus the sign changes of u.
+// In a block, the solution that starts with u = 0 changes sign n2(x) times, and
+// any other solution n2 or n2 + 1 times (Sturm separation), so the parity of
+// the sign change between the block's ends decides.  n2 is counted at the
+// panel's centre; elsewhere in the panel it differs by at most one (the phase
+// over half a panel is at most sqrt(rho) ~ 3.2 rad), downwards in t, which the
+// sign of the entry T12 tells.
+//
+// Eigenvectors.  u runs up from the ground and b, the solution that meets the
+// upper boundary, runs down; they are joined at the twist row r where |u b| is
+// largest.  The norm sum z^2, the attenuation integral sum z^2 w and the
+// group-speed integral need no sums over rows: for a perturbation sigma_i +
+// eps W_i the derivatives (u_eps, e_eps) satisfy
+//   u e_eps - e u_eps = - sum over the rows so far of W_i u_{i-1}^2
+// (and with the other sign downwards for b), so the derivative chains of the
+// same block matrices give them: d/dx (W = -1) from the Horner steps, d/deps
+// expanded to degree kPW.  Both directions stop at the twist, where neither
+// solution is contaminated by the growing one.  (A single chain carried to the
+// far boundary would do at half the cost, but its error is first order in the
+// eigenvalue's: 1e-6 of Im k for ducted modes, whose weights aloft are 1e9
+// times those in the duct.)
+#include <algorithm>
+#include <cmath>
+
+#include "device_common.cuh"
+#include "kernels.hpp"
+
+namespace ncpa {
+
+namespace {
+
+constexpr int kTD = kPanelChunk * kRecT;  // doubles of a chunk of T records
+constexpr int kWD = kPanelChunk * kRecW;  // doubles of a chunk of one weight's records
+constexpr int kPBuf = 3;                  // ring slots per warp
+constexpr int kPWarps = 4;                // warps per CTA (two pairs)
+constexpr int kPanelCtas = 3;             // CTAs per SM
+constexpr int kRecZeros = 4 * (kPD + 1), kRecSplit = kRecZeros + 1;
+static_assert(kRecT == kRecSplit + 1 && kRecT % 2 == 0, "T record: coefficients, zero count, split, 16-byte size");
+static_assert(kRecW == 4 * (kPW + 1), "W record: coefficients");
+
+// ---------------------------------------------------------------------------
+// row formats
+// ---------------------------------------------------------------------------
+// sigma at centre xc and its linear and quadratic coefficients in t
+struct EssPanel {
+    static constexpr int kW = 1;
+    static constexpr bool kUnitNorm = true;  // the norm is -dg/dx: no weight of ones
+    // around the panel's centre, for the expansion
+    __device__ static __forceinline__ double centre(const double* __restrict__ row, int i, double xc) {
+        return (__ldg(row + i) + 2.0) - xc;
+    }
+    // of the row itself at a shift (s_i - x in doubles)
+    __device__ static __forceinline__ double sigma(const double* __restrict__ row, int i, double x) {
+        return (__ldg(row + i) - x) + 2.0;
+    }
+    // -d sigma / dx
+    __device__ static __forceinline__ double slope(const double* __restrict__, int, double) { return 1.0; }
+    __device__ static __forceinline__ double e_init(const ProblemInfo&) { return 1.0; }  // p_{-2} = 0
+    __device__ static __forceinline__ double lo(const ProblemInfo& pi) { return pi.lo; }
+    __device__ static __forceinline__ double hi(const ProblemInfo& pi) { return pi.hi; }
+    __device__ static __forceinline__ double tol_scale(const ProblemInfo&) { return 1.0; }
+    // The shift that a row sees.  The stored rows are multiples of 2^-52 in (-2,
+    // -1] (but for the ground row and very coarse grids).  So in doubles s_i - x
+    // is s_i less x rounded to that grid where it lies above -2, and below,
+    // where doubles are 2^-51 apart, s_i less the grid point under or over x as
+    // s_i is even or odd: halfway, on average.  The block sweeps take their
+    // shifts there too (a block counts as below by its middle row), so they see
+    // the matrix that an evaluation of the rows sees to about 1e-18, and pairs
+    // of modes closer than 1e-8 or phases k r at 1000 km come out alike
+    // whichever way they are computed.
+    struct Shift {
+        double above, below;
+    };
+    __device__ static __forceinline__ Shift shift(double x) {
+        return {(1.0 + x) - 1.0, (floor(x * 4503599627370496.0) + 0.5) * 2.220446049250313e-16};
+    }
+    // rows below this are on the coarser side
+    __device__ static __forceinline__ double split(const double* __restrict__ row, int i) {
+        return __ldg(row + i) + 2.0;
+    }
+};
+
+// ---------------------------------------------------------------------------
+// panels
+// ---------------------------------------------------------------------------
+struct Panel {
+    double xc, r;
+    const double* rows;  // raw rows of the problem
+    long long rec;       // first block record
+    int nblk, blk, nz;   // blk = 0: no records, the sweeps run on the raw rows
+    double e0;
+};
+
+template <class Row>
+__device__ __forceinline__ Panel panel_of(const ProblemInfo& pi, const PanelDesc& d, const double* rows) {
+    Panel P;
+    P.xc = d.xc;
+    P.r = d.blk ? d.r : 1.0;  // raw rows: derivatives in x itself
+    P.blk = d.blk;
+    P.rows = rows + (size_t)pi.s_off * Row::kW;
+    P.nz = pi.nz;
+    P.nblk = d.blk ? (pi.nz + d.blk - 1) / d.blk : 0;
+    P.rec = d.rec;
+    P.e0 = Row::e_init(pi);
+    return P;
+}
+
+__device__ __forceinline__ int padded(int nblk) { return (nblk + kPanelChunk - 1) / kPanelChunk * kPanelChunk; }
+
+// rows per block for shifts within r of the centre: the most that keep r B^2
+// within kRhoMax (0: not even kPanelMinBlk)
+__device__ __forceinline__ int block_rows(double r) {
+    for (int B = kPanelMaxBlk; B >= kPanelMinBlk; B >>= 1)
+        if (r * (double)B * (double)B <= kRhoMax) return B;
+    return 0;
+}
+
+// panel q of a problem's isolation scan: pi.upp units of kScanStep points
+template <class Row>
+__device__ __forceinline__ PanelDesc scan_panel(const ProblemInfo& pi, int q) {
+    const int n = pi.n_scan, t0 = q * pi.upp * kScanStep, t1 = min(n, t0 + pi.upp * kScanStep) - 1;
+    PanelDesc d;
+    const double a = scan_x(Row::lo(pi), Row::hi(pi), t0, n), b = scan_x(Row::lo(pi), Row::hi(pi), t1, n);
+    d.xc = 0.5 * (a + b);
+    d.r = fmax(0.5 * fabs(b - a), 1e-300);
+    d.blk = pi.upp ? pi.sp_blk : 0;
+    d.rec = pi.blk_off + (long long)q * padded(d.blk ? (pi.nz + d.blk - 1) / d.blk : 0);
+    d.problem = 0;
+    return d;
+}
+
+// The scan's panels of a problem whose scan size is final: as many units per
+// panel as kRhoMax allows at the largest block, or one unit and a smaller one
+template <class Row>
+__device__ void plan_scan_panels(ProblemInfo& pi, int n) {
+    const int units = n / kScanStep;
+    const double d = fabs(Row::hi(pi) - Row::lo(pi)) / (double)(n - 1);
+    int upp = units, B = 0;
+    for (; upp >= 1; --upp) {
+        const double r = 0.5 * d * (double)(upp * kScanStep - 1);
+        if (r * (double)kPanelMaxBlk * (double)kPanelMaxBlk <= kRhoMax) {
+            B = kPanelMaxBlk;
+            break;
+        }
+    }
+    if (!B) {
+        upp = 1;
+        B = block_rows(0.5 * d * (double)(kScanStep - 1));
+    }
+    const long long need = B ? (long long)((units + upp - 1) / upp) * padded((pi.nz + B - 1) / B) : 0;
+    const bool fits = B != 0 && need <= pi.blk_cap;
+    pi.upp = fits ? upp : 0;
+    pi.sp_blk = fits ? B : 0;
+}
+
+// ---------------------------------------------------------------------------
+// expansion
+// ---------------------------------------------------------------------------
+constexpr int kExpThreads = 64;
+
+// One thread per (panel, block, column of the transfer matrix): it runs the
+// block's rows with the power series of u and e in t, and of their derivatives
+// with respect to a perturbation eps W_i of sigma.  Bound by FP64 issue: 3
+// instructions per row and coefficient (4 for the W series); the B rows of a
+// thread are consecutive, so a warp touches 16 lines at a time, each used for
+// 16 rows out of L1.
+template <class Row, int NW>
+__device__ __forceinline__ void expand_block(const Panel& P, int b, int col, const double* __restrict__ wp,
+                                             const double* __restrict__ gp, double* __restrict__ T,
+                                             double* __restrict__ W0, double* __restrict__ W1) {
+    const int a = b * P.blk, end = min(P.nz, a + P.blk);
+    constexpr int kNW0 = NW > 0 ? kPW + 1 : 1;
+    double u[kPD + 1], e[kPD + 1], v0[kNW0], f0[kNW0];
+    double v1[NW > 1 ? kPW + 1 : 1], f1[NW > 1 ? kPW + 1 : 1];
+#pragma unroll
+    for (int k = 0; k <= kPD; ++k) u[k] = e[k] = 0.0;
+#pragma unroll
+    for (int k = 0; k < kNW0; ++k) v0[k] = f0[k] = 0.0;
+    if (NW > 1) {
+#pragma unroll
+        for (int k = 0; k <= kPW; ++k) v1[k] = f1[k] = 0.0;
+    }
+    if (col == 0) u[0] = 1.0;
+    else e[0] = 1.0;
+    const double r = P.r;
+    unsigned prev = 0u;
+    int n2 = 0;
+    for (int i = a; i < end; ++i) {
+        const double sg = -Row::centre(P.rows, i, P.xc);
+        const double wi = NW > 0 ? -__ldg(wp + i) : 0.0;
+        const double gi = NW > 1 ? (gp ? -__ldg(gp + i) : -1.0) : 0.0;
+#pragma unroll
+        for (int k = 0; NW > 0 && k <= kPW; ++k) {
+            double x = fma(sg, v0[k], f0[k]);
+            if (k > 0) x = fma(r, v0[k - 1], x);
+            f0[k] = fma(wi, u[k], x);
+            if (NW > 1) {
+                double y = fma(sg, v1[k], f1[k]);
+                if (k > 0) y = fma(r, v1[k - 1], y);
+                f1[k] = fma(gi, u[k], y);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k <= kPD; ++k) {
+            e[k] = fma(sg, u[k], e[k]);
+            if (k > 0) e[k] = fma(r, u[k - 1], e[k]);
+        }
+#pragma unroll
+        for (int k = 0; k <= kPD; ++k) u[k] += e[k];
+#pragma unroll
+        for (int k = 0; NW > 0 && k <= kPW; ++k) {
+            v0[k] += f0[k];
+            if (NW > 1) v1[k] += f1[k];
+        }
+        // zeros of the solution that starts with u = 0 (column 1), at t = 0
+        const unsigned s = static_cast<unsigned>(__double2hiint(u[0])) >> 31;
+        n2 += static_cast<int>(s ^ prev);
+        prev = s;
+    }
+    const size_t rec = (size_t)(P.rec + b);
+    double* o = T + rec * kRecT + col;
+#pragma unroll
+    for (int k = 0; k <= kPD; ++k) {
+        o[4 * k] = u[k];
+        o[4 * k + 2] = e[k];
+    }
+    if (col == 1) {
+        T[rec * kRecT + kRecZeros] = __hiloint2double(0, n2);
+        T[rec * kRecT + kRecSplit] = Row::split(P.rows, min(P.nz - 1, a + P.blk / 2));
+    }
+    if (NW > 0) {
+        o = W0 + rec * kRecW + col;
+#pragma unroll
+        for (int k = 0; k <= kPW; ++k) {
+            o[4 * k] = v0[k];
+            o[4 * k + 2] = f0[k];
+        }
+    }
+    if (NW > 1) {
+        o = W1 + rec * kRecW + col;
+#pragma unroll
+        for (int k = 0; k <= kPW; ++k) {
+            o[4 * k] = v1[k];
+            o[4 * k + 2] = f1[k];
+        }
+    }
+}
+
+// the panels of the work items, one per blockIdx.y
+template <class Row, int NW>
+__global__ void __launch_bounds__(kExpThreads) k_expand_items(const ProblemInfo* __restrict__ pinfo,
+                                                              const PanelDesc* __restrict__ desc, int d0,
+                                                              const double* __restrict__ rows,
+                                                              const double* __restrict__ w,
+                                                              const double* __restrict__ g, double* __restrict__ T,
+                                                              double* __restrict__ W0, double* __restrict__ W1) {
+    const PanelDesc d = desc[d0 + blockIdx.y];
+    if (d.problem < 0 || !d.blk) return;
+    const ProblemInfo& pi = pinfo[d.problem];
+    const Panel P = panel_of<Row>(pi, d, rows);
+    const double* gp = NW > 1 && g ? g + pi.s_off : nullptr;
+    for (int t = blockIdx.x * kExpThreads + threadIdx.x; t < 2 * P.nblk; t += gridDim.x * kExpThreads)
+        expand_block<Row, NW>(P, t >> 1, t & 1, w + pi.w_off, gp, T, W0, W1);
+}
+
+// the scan's panels: kScanMax / kScanStep slots per problem on blockIdx.y
+constexpr int kScanSlots = kScanMax / kScanStep;
+template <class Row>
+__global__ void __launch_bounds__(kExpThreads) k_expand_scan(const ProblemInfo* __restrict__ pinfo, int p0,
+                                                             const double* __restrict__ rows,
+                                                             double* __restrict__ T) {
+    const ProblemInfo& pi = pinfo[p0 + blockIdx.y / kScanSlots];
+    const int q = blockIdx.y % kScanSlots;
+    if (!pi.upp || q * pi.upp * kScanStep >= pi.n_scan) return;
+    const Panel P = panel_of<Row>(pi, scan_panel<Row>(pi, q), rows);
+    for (int t = blockIdx.x * kExpThreads + threadIdx.x; t < 2 * P.nblk; t += gridDim.x * kExpThreads)
+        expand_block<Row, 0>(P, t >> 1, t & 1, nullptr, nullptr, T, nullptr, nullptr);
+}
+
+// ---------------------------------------------------------------------------
+// sweeps
+// ---------------------------------------------------------------------------
+// A warp's ring of chunks in shared memory (1-D bulk copies), sl doubles per
+// slot: T records, then the weights' (eigenvector passes), or raw rows
+struct PRing {
+    double* buf;
+    uint64_t* bars;
+    unsigned loads;  // identical in all lanes
+    int sl;
+};
+
+__device__ __forceinline__ PRing make_ring(unsigned char* smem, int wid, int sl) {
+    PRing R;
+    R.sl = sl;
+    R.buf = reinterpret_cast<double*>(smem) + (size_t)wid * kPBuf * sl;
+    R.bars = reinterpret_cast<uint64_t*>(smem + (size_t)kPWarps * kPBuf * sl * 8) + wid * kPBuf;
+    R.loads = 0;
+    if ((threadIdx.x & 31) == 0) {
+        for (int k = 0; k < kPBuf; ++k) mbar_init(&R.bars[k], 1);
+        fence_mbar_init();
+    }
+    __syncwarp();
+    return R;
+}
+template <int kSl>
+constexpr size_t kRingBytes = (size_t)kPWarps * kPBuf * (kSl * 8 + 8);
+
+// Streams n chunks through the ring: issue(slot buffer, barrier, c) starts the
+// copies of chunk c, use(slot buffer, c) consumes it (all lanes).
+template <class Issue, class Use>
+__device__ __forceinline__ void ring_stream(PRing& R, int n, unsigned* err, Issue issue, Use use) {
+    const int lane = threadIdx.x & 31;
+    const unsigned base = R.loads;
+    auto start = [&](int c) {
+        const int slot = (base + c) % kPBuf;
+        issue(R.buf + slot * R.sl, &R.bars[slot], c);
+    };
+    if (lane == 0) {
+        fence_proxy_async();
+        for (int c = 0; c < n && c < kPBuf; ++c) start(c);
+    }
+    __syncwarp();
+    for (int c = 0; c < n; ++c) {
+        const unsigned k = base + c;
+        const int slot = k % kPBuf;
+        mbar_wait_bounded(&R.bars[slot], (k / kPBuf) & 1u, err);
+        use(R.buf + slot * R.sl, c);
+        __syncwarp();
+        if (lane == 0 && c + kPBuf < n) {
+            fence_proxy_async();
+            start(c + kPBuf);
+        }
+    }
+    R.loads = base + n;
+}
+
+// t of a shift x in the blocks of a panel
+template <class Row>
+struct BlockShift {
+    double x, t0, t1;
+    __device__ __forceinline__ BlockShift() {}
+    __device__ __forceinline__ BlockShift(const Panel& P, double x_) : x(x_) {
+        const typename Row::Shift s = Row::shift(x_);
+        const double rinv = 1.0 / P.r;
+        t0 = (s.above - P.xc) * rinv;
+        t1 = (s.below - P.xc) * rinv;
+    }
+    __device__ __forceinline__ double at(const double* rec) const { return x > rec[kRecSplit] ? t1 : t0; }
+};
+
+__device__ __forceinline__ unsigned neg(double v) { return static_cast<unsigned>(__double2hiint(v)) >> 31; }
+
+// sign changes of a chain across a block: u before, un after, T12 at the
+// chain's t, n2 at the panel's centre
+__device__ __forceinline__ int block_zeros(double u, double un, double T12, double t, int n2) {
+    if (neg(T12) != static_cast<unsigned>(n2 & 1)) n2 += t > 0.0 ? -1 : 1;
+    return n2 + static_cast<int>((neg(u) ^ neg(un)) ^ static_cast<unsigned>(n2 & 1));
+}
+
+__device__ __forceinline__ void scale2(double& a, double& b) {
+    const int sh = rescale_shift(a, b);
+    if (sh) {
+        const double sc = pow2(-sh);
+        a *= sc;
+        b *= sc;
+    }
+}
+
+// the four entries of two blocks at NC shifts per lane: 8 NC independent Horner
+// chains, so a lone warp keeps the FP64 pipe busy over their latency
+template <int NC>
+__device__ __forceinline__ void horner_blocks(const double* __restrict__ c0, const double* __restrict__ c1,
+                                              const double (&t)[2][NC], double (&p)[2][NC][4]) {
+    const double2* q[2] = {reinterpret_cast<const double2*>(c0), reinterpret_cast<const double2*>(c1)};
+#pragma unroll
+    for (int k = kPD; k >= 0; --k)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const double2 v = q[b][2 * k], w = q[b][2 * k + 1];
+            const double cf[4] = {v.x, v.y, w.x, w.y};
+#pragma unroll
+            for (int n = 0; n < NC; ++n)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) p[b][n][j] = k == kPD ? cf[j] : fma(p[b][n][j], t[b][n], cf[j]);
+        }
+}
+
+// Sturm counts at NC shifts per lane
+template <class Row, int NC>
+__device__ __forceinline__ void count_sweep(const Panel& P, const double* __restrict__ Trec, const double (&x)[NC],
+                                            PRing& R, unsigned* err, int (&cnt)[NC]) {
+    double u[NC], e[NC];
+    BlockShift<Row> sh[NC];
+    int zeros[NC];
+#pragma unroll
+    for (int n = 0; n < NC; ++n) {
+        u[n] = 1.0;
+        e[n] = P.e0;
+        zeros[n] = 0;
+        sh[n] = BlockShift<Row>(P, x[n]);
+    }
+    if (P.blk) {
+        const double* src = Trec + (size_t)P.rec * kRecT;
+        ring_stream(
+            R, (P.nblk + kPanelChunk - 1) / kPanelChunk, err,
+            [&](double* dst, uint64_t* bar, int c) {
+                mbar_expect_tx(bar, kTD * 8);
+                tma_load_1d(dst, src + (size_t)c * kTD, kTD * 8, bar);
+            },
+            [&](const double* rec, int c) {
+                const int nb = min(kPanelChunk, P.nblk - c * kPanelChunk);
+                for (int q = 0; q < nb; q += 2, rec += 2 * kRecT) {
+                    double p[2][NC][4], t[2][NC];
+#pragma unroll
+                    for (int n = 0; n < NC; ++n) {
+                        t[0][n] = sh[n].at(rec);
+                        t[1][n] = sh[n].at(rec + kRecT);
+                    }
+                    horner_blocks<NC>(rec, rec + kRecT, t, p);
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        if (q + b >= nb) break;
+                        const int n2 = __double2loint(rec[b * kRecT + kRecZeros]);
+#pragma unroll
+                        for (int n = 0; n < NC; ++n) {
+                            const double(&m)[4] = p[b][n];
+                            const double un = fma(m[0], u[n], m[1] * e[n]);
+                            e[n] = fma(m[2], u[n], m[3] * e[n]);
+                            zeros[n] += block_zeros(u[n], un, m[1], t[b][n], n2);
+                            u[n] = un;
+                        }
+                    }
+                }
+#pragma unroll
+                for (int n = 0; n < NC; ++n) scale2(u[n], e[n]);
+            });
+    } else {
+        // no records (a window so wide against the grid that blocks of 8 rows
+        // have no short expansion, or beyond the reserved records): row by row
+        for (int i = 0; i < P.nz; ++i) {
+#pragma unroll
+            for (int n = 0; n < NC; ++n) {
+                e[n] = fma(-Row::sigma(P.rows, i, x[n]), u[n], e[n]);
+                const double un = u[n] + e[n];
+                zeros[n] += static_cast<int>(neg(un) ^ neg(u[n]));
+                u[n] = un;
+                if ((i & 15) == 15) scale2(u[n], e[n]);
+            }
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < NC; ++n) cnt[n] = P.nz - zeros[n];
+}
+
+// ---------------------------------------------------------------------------
+// Laguerre sweeps.  The lower half of the blocks runs upwards (u), the upper
+// half downwards (b), one warp each, both with their first and half second
+// derivatives in t; at the block between, W = u e^b - e u^b is -u_{nz-1}, the
+// determinant up to sign, and its derivatives follow by the product rule.  An
+// isolated eigenvalue needs no counts: the sign of the determinant is the
+// parity of the count.
+// ---------------------------------------------------------------------------
+struct LagChain {
+    double u, e, u1, e1, u2, e2;
+    __device__ __forceinline__ void rescale() {
+        const int sh = rescale_shift(fmax(fmax(fabs(u), fabs(u1)), fabs(u2)), fmax(fmax(fabs(e), fabs(e1)), fabs(e2)));
+        if (sh) {
+            const double sc = pow2(-sh);
+            u *= sc;
+            e *= sc;
+            u1 *= sc;
+            e1 *= sc;
+            u2 *= sc;
+            e2 *= sc;
+        }
+    }
+};
+
+// entries at t with first (d) and half second (s) derivatives
+__device__ __forceinline__ void horner_der2(const double* __restrict__ c, double t, double (&p)[4], double (&d)[4],
+                                            double (&s)[4]) {
+    const double2* q = reinterpret_cast<const double2*>(c);
+#pragma unroll
+    for (int k = kPD; k >= 0; --k) {
+        const double2 v = q[2 * k], w = q[2 * k + 1];
+        const double cf[4] = {v.x, v.y, w.x, w.y};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (k < kPD - 1) s[j] = k == kPD - 2 ? d[j] : fma(s[j], t, d[j]);
+            if (k < kPD) d[j] = k == kPD - 1 ? p[j] : fma(d[j], t, p[j]);
+            p[j] = k == kPD ? cf[j] : fma(p[j], t, cf[j]);
+        }
+    }
+}
+
+template <class Row>
+__device__ __forceinline__ void laguerre_half(const Panel& P, const double* __restrict__ Trec, double x, int half,
+                                              PRing& R, unsigned* err, LagChain& C) {
+    C = half ? LagChain{0.0, -1.0, 0.0, 0.0, 0.0, 0.0} : LagChain{1.0, P.e0, 0.0, 0.0, 0.0, 0.0};
+    if (P.blk) {
+        const BlockShift<Row> sh(P, x);
+        const double* src = Trec + (size_t)P.rec * kRecT;
+        const int nch = (P.nblk + kPanelChunk - 1) / kPanelChunk, nu = (nch + 1) / 2;  // chunks; those of u
+        ring_stream(
+            R, half ? nch - nu : nu, err,
+            [&](double* dst, uint64_t* bar, int o) {
+                const size_t c = half ? nch - 1 - o : o;
+                mbar_expect_tx(bar, kTD * 8);
+                tma_load_1d(dst, src + c * kTD, kTD * 8, bar);
+            },
+            [&](const double* buf, int o) {
+                const int c = half ? nch - 1 - o : o, nb = min(kPanelChunk, P.nblk - c * kPanelChunk);
+                for (int i = 0; i < nb; ++i) {
+                    const double* rec = buf + (half ? nb - 1 - i : i) * kRecT;
+                    double p[4], d[4], s[4];
+                    horner_der2(rec, sh.at(rec), p, d, s);
+                    if (half) {  // the inverses: (u, e) -> (p3 u - p1 e, p0 e - p2 u)
+                        const double m[4] = {p[3], -p[1], -p[2], p[0]}, f[4] = {d[3], -d[1], -d[2], d[0]},
+                                     g[4] = {s[3], -s[1], -s[2], s[0]};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            p[j] = m[j];
+                            d[j] = f[j];
+                            s[j] = g[j];
+                        }
+                    }
+                    const double u2 = fma(p[0], C.u2, p[1] * C.e2) + fma(d[0], C.u1, d[1] * C.e1) +
+                                      fma(s[0], C.u, s[1] * C.e);
+                    const double e2 = fma(p[2], C.u2, p[3] * C.e2) + fma(d[2], C.u1, d[3] * C.e1) +
+                                      fma(s[2], C.u, s[3] * C.e);
+                    const double u1 = fma(p[0], C.u1, p[1] * C.e1) + fma(d[0], C.u, d[1] * C.e);
+                    const double e1 = fma(p[2], C.u1, p[3] * C.e1) + fma(d[2], C.u, d[3] * C.e);
+                    const double u = fma(p[0], C.u, p[1] * C.e), e = fma(p[2], C.u, p[3] * C.e);
+                    C = LagChain{u, e, u1, e1, u2, e2};
+                }
+                C.rescale();
+            });
+    } else {
+        const int h = P.nz / 2, n = half ? P.nz - h : h;
+        for (int j = 0; j < n; ++j) {
+            const int i = half ? P.nz - 1 - j : j;
+            const double sg = Row::sigma(P.rows, i, x), sl = Row::slope(P.rows, i, x);
+            if (half) {
+                C.u -= C.e;
+                C.u1 -= C.e1;
+                C.u2 -= C.e2;
+                C.e2 = fma(sg, C.u2, fma(-sl, C.u1, C.e2));
+                C.e1 = fma(sg, C.u1, fma(-sl, C.u, C.e1));
+                C.e = fma(sg, C.u, C.e);
+            } else {
+                C.e2 = fma(-sg, C.u2, fma(sl, C.u1, C.e2));
+                C.e1 = fma(-sg, C.u1, fma(sl, C.u, C.e1));
+                C.e = fma(-sg, C.u, C.e);
+                C.u += C.e;
+                C.u1 += C.e1;
+                C.u2 += C.e2;
+            }
+            if ((j & 15) == 15) C.rescale();
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// isolation scan: units of kScanStep shifts, one warp each
+// ---------------------------------------------------------------------------
+template <class Row>
+__global__ void __launch_bounds__(kPWarps * 32) k_panel_scan(const ProblemInfo* __restrict__ pinfo,
+                                                             const double* __restrict__ rows,
+                                                             const double* __restrict__ T, int* __restrict__ counts,
+                                                             unsigned* err) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int slot = blockIdx.x * kPWarps + wid, p = slot / kScanSlots, unit = slot % kScanSlots;
+    const ProblemInfo& pi = pinfo[p];
+    const int n = pi.n_scan;
+    if (unit * kScanStep >= n) return;
+    PRing R = make_ring(smem_raw, wid, kTD);
+    const Panel P = panel_of<Row>(pi, scan_panel<Row>(pi, pi.upp ? unit / pi.upp : 0), rows);
+    const int t0 = unit * kScanStep + 2 * lane;
+    const double lo = Row::lo(pi), hi = Row::hi(pi);
+    const double x[2] = {scan_x(lo, hi, t0, n), scan_x(lo, hi, t0 + 1, n)};
+    int c[2];
+    count_sweep<Row, 2>(P, T, x, R, err, c);
+    *reinterpret_cast<int2*>(counts + (size_t)p * kScanMax + t0) = make_int2(c[0], c[1]);
+}
+
+// ---------------------------------------------------------------------------
+// work items
+// ---------------------------------------------------------------------------
+constexpr int kItemThreads = 1024;
+
+__device__ int block_scan(int v, int* sh, int* total) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += a;
+    }
+    __syncthreads();  // sh free
+    if (lane == 31) sh[wid] = incl;
+    __syncthreads();
+    if (wid == 0) {
+        int w = sh[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int a = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += a;
+        }
+        sh[lane] = w;
+    }
+    __syncthreads();
+    *total = sh[31];
+    return incl - v + (wid ? sh[wid - 1] : 0);
+}
+
+// One CTA: per problem the mode number, the CSR offset and the place of its
+// items in the list.  With order set and P <= kRankMax the problems are listed
+// by the cost of an item, nz x m x (1 + M / 512) (m eigenvalues of a problem
+// with M: denser windows need more rounds), heaviest first; the item scheduler
+// then takes items from both ends.
+constexpr int kRankMax = 4096;
+
+__global__ void __launch_bounds__(kItemThreads) k_panel_items(int P, ProblemInfo* __restrict__ pinfo,
+                                                              const int* __restrict__ counts, int max_modes,
+                                                              int bis_item, int cap, int* __restrict__ tot,
+                                                              unsigned* __restrict__ err, int order) {
+    __shared__ int sh[32];
+    __shared__ float skey[kRankMax];
+    __shared__ int sperm[kRankMax];
+    const bool ranked = order != 0 && P <= kRankMax;
+    int base_m = 0;
+    for (int p0 = 0; p0 < P; p0 += kItemThreads) {
+        const int p = p0 + threadIdx.x;
+        int M = 0;
+        if (p < P) {
+            const ProblemInfo& pi = pinfo[p];
+            const int c_lo = counts[(size_t)p * kScanMax], c_hi = counts[(size_t)p * kScanMax + pi.n_scan - 1];
+            M = max(0, c_hi - c_lo);
+            if (M > max_modes) {
+                atomicOr(err, kErrTooMany);
+                M = max_modes;
+            }
+            pinfo[p].c_lo = c_lo;
+            pinfo[p].c_hi = c_hi;
+            pinfo[p].M = M;
+            const int nb = (M + bis_item - 1) / bis_item;
+            if (ranked)
+                skey[p] = nb > 0 ? (float)pi.nz * ((float)M / (float)nb) * (1.0f + (float)M * (1.0f / 512.0f)) : 0.f;
+        }
+        int tm;
+        const int om = block_scan(M, sh, &tm);
+        if (p < P) pinfo[p].off = base_m + om;
+        base_m += tm;
+    }
+    __syncthreads();
+    if (ranked) {
+        for (int p = threadIdx.x; p < P; p += kItemThreads) {
+            const float kp = skey[p];
+            int r = 0;
+            for (int q = 0; q < P; ++q) {
+                const float kq = skey[q];
+                r += (kq > kp || (kq == kp && q < p)) ? 1 : 0;
+            }
+            sperm[r] = p;
+        }
+        __syncthreads();
+    }
+    int base = 0;
+    for (int r0 = 0; r0 < P; r0 += kItemThreads) {
+        const int r = r0 + threadIdx.x;
+        const int p = r < P ? (ranked ? sperm[r] : r) : 0;
+        const int nb = r < P ? (pinfo[p].M + bis_item - 1) / bis_item : 0;
+        int tb;
+        const int ob = block_scan(nb, sh, &tb);
+        if (r < P) pinfo[p].item0 = base + ob;
+        base += tb;
+    }
+    if (threadIdx.x == 0) {
+        if (base > cap) atomicOr(err, kErrTooMany);
+        tot[0] = min(base, cap);
+        tot[1] = min(base, cap);
+        tot[2] = base_m;
+    }
+}
+
+// index of the last scan point with a count <= J (counts are monotone; a
+// rounding slip between neighbours still ends at a valid bracket)
+__device__ __forceinline__ int scan_bracket(const int* __restrict__ cnt, int n, int J) {
+    int t0 = 0, t1 = n - 1;
+    while (t1 - t0 > 1) {
+        const int t = (t0 + t1) >> 1;
+        if (cnt[t] <= J) t0 = t;
+        else t1 = t;
+    }
+    return t0;
+}
+
+// One warp per problem: its items (at most bis_item consecutive eigenvalues,
+// balanced) and their panels.  Consecutive items share a panel while their
+// brackets fit kRhoMax at the largest block; an item too wide for that gets
+// its own panel and a smaller block.  Items beyond the problem's panels or
+// records (sized by the host from the profile's sound speeds) keep none and
+// sweep the raw rows.
+constexpr int kPlanWarps = 2, kPlanItems = 256;
+template <class Row>
+__global__ void __launch_bounds__(kPlanWarps * 32) k_panel_groups(int P, const ProblemInfo* __restrict__ pinfo,
+                                                                  const int* __restrict__ counts, int bis_item,
+                                                                  WorkItem* __restrict__ items, int cap,
+                                                                  PanelDesc* __restrict__ desc) {
+    __shared__ double xa[kPlanWarps][kPlanItems], xb[kPlanWarps][kPlanItems];
+    __shared__ int grp[kPlanWarps][kPlanItems];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int p = blockIdx.x * kPlanWarps + wid;
+    if (p >= P) return;
+    const ProblemInfo& pi = pinfo[p];
+    const int* cnt = counts + (size_t)p * kScanMax;
+    const double lo = Row::lo(pi), hi = Row::hi(pi);
+    const int M = pi.M, n = pi.n_scan, nb = (M + bis_item - 1) / bis_item;
+    int ng = 0, used = 0;  // panels and records taken so far (warp-uniform)
+    for (int k0 = 0; k0 < nb; k0 += kPlanItems) {
+        const int m = min(kPlanItems, nb - k0);
+        for (int i = lane; i < m; i += 32) {
+            const int k = k0 + i;
+            const int j0 = (int)((long long)M * k / nb), j1 = (int)((long long)M * (k + 1) / nb);
+            const double a = scan_x(lo, hi, scan_bracket(cnt, n, pi.c_lo + j0), n);
+            const double b = scan_x(lo, hi, scan_bracket(cnt, n, pi.c_lo + j1 - 1) + 1, n);
+            xa[wid][i] = fmin(a, b);
+            xb[wid][i] = fmax(a, b);
+        }
+        __syncwarp();
+        if (lane == 0) {
+            for (int i = 0; i < m;) {
+                const double a = xa[wid][i];
+                double b = xb[wid][i];
+                int e = i + 1;
+                auto wide = [&](double c) {
+                    return !(0.5 * (c - a) * (double)kPanelMaxBlk * (double)kPanelMaxBlk <= kRhoMax);
+                };
+                if (!wide(b))
+                    while (e < m && !wide(fmax(b, xb[wid][e]))) b = fmax(b, xb[wid][e++]);
+                PanelDesc d;
+                d.xc = 0.5 * (a + b);
+                d.r = fmax(0.5 * (b - a), 1e-300);
+                d.blk = block_rows(d.r);
+                d.problem = p;
+                d.rec = pi.blk_off + used;
+                const int need = d.blk ? padded((pi.nz + d.blk - 1) / d.blk) : 0;
+                int id = -1;
+                if (d.blk && ng < pi.grp_cap && used + need <= pi.blk_cap) {
+                    id = pi.grp_off + ng++;
+                    desc[id] = d;
+                    used += need;
+                }
+                for (; i < e; ++i) grp[wid][i] = id;
+            }
+        }
+        __syncwarp();
+        for (int i = lane; i < m; i += 32) {
+            const int k = k0 + i, q = pi.item0 + k;
+            const int j0 = (int)((long long)M * k / nb), j1 = (int)((long long)M * (k + 1) / nb);
+            if (q < cap) items[q] = WorkItem{p, j0, j1 - j0, grp[wid][i]};
+        }
+        __syncwarp();
+        ng = __shfl_sync(0xffffffffu, ng, 0);
+        used = __shfl_sync(0xffffffffu, used, 0);
+    }
+    for (int i = ng + lane; i < pi.grp_cap; i += 32) {
+        PanelDesc d{};
+        d.problem = -1;
+        desc[pi.grp_off + i] = d;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// A work item runs on a pair of warps: of a Laguerre sweep they take the front
+// and the back rows, of a counting sweep 32 shifts each, of the eigenvectors the
+// upward and the downward pass.  Both keep the state of every slot and take the
+// same decisions from what they exchange, one barrier a round.
+// ---------------------------------------------------------------------------
+struct PairBox {
+    double v[2][2][6][32];  // [round parity][half][value][lane]
+    int c[2][2][32];        // counts
+    int err[2][2];
+    int item[2];
+};
+
+struct Pair {
+    PairBox* box;
+    int id, half;
+    int turn;  // buffer of the next exchange
+    __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, 64;" ::"r"(1 + id) : "memory"); }
+};
+
+// position of the n-th (0-based) set bit of m
+__device__ __forceinline__ int nth_set(unsigned m, int n) {
+    int pos = 0;
+#pragma unroll
+    for (int sh = 16; sh >= 1; sh >>= 1) {
+        const unsigned low = m & ((1u << sh) - 1u);
+        const int c = __popc(low);
+        if (n >= c) {
+            n -= c;
+            m >>= sh;
+            pos += sh;
+        } else {
+            m = low;
+        }
+    }
+    return pos;
+}
+
+// Eigenvalues of a work item (<= 32), lane l owning slot l, to x.  Every round:
+// slots isolated in their bracket (Sturm counts J and J + 1 at its ends) take a
+// safeguarded Laguerre step; the other virtual lanes (v = lane + 32 half) are
+// dealt over the slots not yet isolated and cut their brackets.  A slot is final
+// when the correction is below tol, or when the last two steps stayed inside
+// the bracket and the cubic model predicts the next one below tol.
+template <class Row>
+__device__ __forceinline__ double panel_bisect(const ProblemInfo& pi, const Panel& P, const WorkItem& w,
+                                               const double* __restrict__ Trec, const int* __restrict__ counts,
+                                               double tol_in, unsigned* err, unsigned long long* steps, PRing& R,
+                                               Pair& pr) {
+    const int lane = threadIdx.x & 31;
+    const double lo = Row::lo(pi), hi = Row::hi(pi);
+    const int nz = pi.nz, n = pi.n_scan;
+    const int* cnt = counts + (size_t)w.problem * kScanMax;
+    const double tol = tol_in * Row::tol_scale(pi);
+    const int J = pi.c_lo + w.j0 + lane;
+    double a = P.xc, b = P.xc, x = P.xc;
+    double dprev = 0.0;  // size of the previous accepted correction (0: none yet)
+    int ca = 0, cb = 0, mode = 2;
+    if (lane < w.m) {  // bracket from the scan
+        const int t0 = scan_bracket(cnt, n, J);
+        ca = cnt[t0];
+        cb = cnt[t0 + 1];
+        if (!(ca <= J && cb > J)) atomicOr(err, kErrBracket);
+        a = scan_x(lo, hi, t0, n);
+        b = scan_x(lo, hi, t0 + 1, n);
+        x = 0.5 * (a + b);
+        mode = !(b - a > tol) ? 2 : ((ca == J && cb == J + 1) ? 1 : 0);
+    }
+    for (int round = 0; round < 512; ++round) {
+        const unsigned nm = __ballot_sync(0xffffffffu, mode == 1);
+        const unsigned bm = __ballot_sync(0xffffffffu, mode == 0);
+        const int nN = __popc(nm), nB = __popc(bm);
+        if (nN + nB == 0) break;
+        const int nlB = 64 - nN;
+        PairBox& X = *pr.box;
+        const int tb = pr.turn;
+        pr.turn ^= 1;
+        if (nB > 0) {  // counts: this half's virtual lanes
+            const int v = lane + 32 * pr.half;
+            const bool on = v >= nN;
+            const int t = on ? v - nN : 0, k = t % nB, g = t / nB, G = (nlB - 1 - k) / nB + 1;
+            const int e = nth_set(bm, k);
+            const double ae = __shfl_sync(0xffffffffu, a, e);
+            const double be = __shfl_sync(0xffffffffu, b, e);
+            const double xs[1] = {ae + (be - ae) * ((double)(g + 1) / (double)(G + 1))};
+            int c[1];
+            count_sweep<Row, 1>(P, Trec, xs, R, err, c);
+            X.c[tb][pr.half][lane] = c[0];
+        }
+        if (nN > 0) {  // Laguerre chains of slots nth_set(nm, lane)
+            const double xe = __shfl_sync(0xffffffffu, x, lane < nN ? nth_set(nm, lane) : 0);
+            LagChain C;
+            laguerre_half<Row>(P, Trec, xe, pr.half, R, err, C);
+            double(&o)[6][32] = X.v[tb][pr.half];
+            o[0][lane] = C.u;
+            o[1][lane] = C.e;
+            o[2][lane] = C.u1;
+            o[3][lane] = C.e1;
+            o[4][lane] = C.u2;
+            o[5][lane] = C.e2;
+        }
+        if (steps && lane == 0 && pr.half == 0) {
+            atomicAdd(steps, (unsigned long long)((nB > 0 ? 64 : 0) + (nN > 0 ? 32 : 0)) * (unsigned long long)nz);
+            if (nN > 0) atomicAdd(steps + 1, 32ull * (unsigned long long)nz);
+        }
+        if (lane == 0) X.err[tb][pr.half] = (*((volatile unsigned*)err) & kErrTimeout) != 0u;
+        pr.sync();
+        if (mode == 1) {
+            const int v = __popc(nm & ((1u << lane) - 1u));
+            const double(&F)[6][32] = X.v[tb][0];
+            const double(&B)[6][32] = X.v[tb][1];
+            const double u = F[0][v], e = F[1][v], u1 = F[2][v], e1 = F[3][v], u2 = F[4][v], e2 = F[5][v];
+            const double y = B[0][v], z = B[1][v], y1 = B[2][v], z1 = B[3][v], y2 = B[4][v], z2 = B[5][v];
+            const double W = u * z - e * y;
+            const double W1 = u1 * z + u * z1 - (e1 * y + e * y1);
+            const double W2 = u2 * z + u1 * z1 + u * z2 - (e2 * y + e1 * y1 + e * y2);  // half W''
+            const double rinv = 1.0 / P.r, g = W1 / W * rinv, h = fma(g, g, -(2.0 * (W2 / W) * rinv * rinv));
+            // below the eigenvalue the count nz - (sign changes of u) is J, above
+            // it J + 1; W = -u_{nz-1}
+            const bool below = ((neg(W) ^ 1u) ^ static_cast<unsigned>(nz & 1)) == static_cast<unsigned>(J & 1);
+            const double xo = x;
+            if (below) a = xo;
+            else b = xo;
+            const double corr = laguerre_step(g, h, (double)nz, below);
+            const double ad = fabs(corr);
+            if (ad <= tol) {
+                x = fmin(fmax(xo - corr, a), b);
+                mode = 2;
+            } else {
+                const double xn = xo - corr;
+                const bool ok = isfinite(xn) && xn > a && xn < b;
+                x = ok ? xn : 0.5 * (a + b);
+                const double ad2 = ad * ad, dp2 = dprev * dprev;
+                if (!(b - a > tol)) mode = 2;
+                // cubic convergence: the next correction would be about ad^4 / dprev^3
+                else if (ok && dprev > 0.0 && ad <= 0.25 * dprev && ad2 * ad2 <= tol * dp2 * dprev) mode = 2;
+                dprev = ok ? ad : 0.0;
+            }
+        } else if (mode == 0) {
+            const int k = __popc(bm & ((1u << lane) - 1u));
+            const int G = (nlB - 1 - k) / nB + 1;
+            int gb = -1, cg = ca;
+            for (int g = 0; g < G; ++g) {
+                const int v = nN + k + g * nB, c = X.c[tb][v >> 5][v & 31];
+                if (c <= J) {
+                    gb = g;
+                    cg = c;
+                }
+            }
+            const double A0 = a, B0 = b;
+            const int g1 = gb + 1, v1 = nN + k + g1 * nB;
+            if (gb >= 0) {
+                ca = cg;
+                a = A0 + (B0 - A0) * ((double)(gb + 1) / (double)(G + 1));
+            }
+            if (g1 < G) {
+                cb = X.c[tb][v1 >> 5][v1 & 31];
+                b = A0 + (B0 - A0) * ((double)(gb + 2) / (double)(G + 1));
+            }
+            x = 0.5 * (a + b);
+            if (!(b - a > tol) || (a == A0 && b == B0)) mode = 2;
+            else if (ca == J && cb == J + 1) mode = 1;
+        }
+        if (X.err[tb][0] | X.err[tb][1]) break;  // a ring wait gave up: abandon the item
+    }
+    return x;
+}
+
+// ---------------------------------------------------------------------------
+// one item: mode values, norm and integrals
+// ---------------------------------------------------------------------------
+// state (u, e) before row i0 advanced to before row i1 (i1 >= i0) at shift x
+template <class Row>
+__device__ __forceinline__ void rows_up(const double* __restrict__ rows, int i0, int i1, double x, double& u,
+                                        double& e) {
+    for (int i = i0; i < i1; ++i) {
+        e = fma(-Row::sigma(rows, i, x), u, e);
+        u += e;
+    }
+}
+// state after row i0 - 1 taken down to before row i1 (i1 <= i0)
+template <class Row>
+__device__ __forceinline__ void rows_down(const double* __restrict__ rows, int i0, int i1, double x, double& u,
+                                          double& e) {
+    for (int i = i0 - 1; i >= i1; --i) {
+        u -= e;
+        e = fma(Row::sigma(rows, i, x), u, e);
+    }
+}
+
+// v = m 2^E with |m| in [1, 2)
+__device__ __forceinline__ void normalize(double& v, int& E) {
+    const int e = biased_exp(v);
+    if (e == 0) return;
+    v *= pow2(1023 - e);
+    E += e - 1023;
+}
+
+// the inverse of a transfer matrix (determinant 1) applied to (u, e)
+__device__ __forceinline__ void adj_apply(const double (&p)[4], double& u, double& e) {
+    const double a = fma(p[3], u, -(p[1] * e)), b = fma(p[0], e, -(p[2] * u));
+    u = a;
+    e = b;
+}
+__device__ __forceinline__ void adj_add(const double (&d)[4], double u, double e, double& du, double& de) {
+    du += fma(d[3], u, -(d[1] * e));
+    de += fma(d[0], e, -(d[2] * u));
+}
+
+// sums an item keeps: the norm (from d/dx where -d sigma / dx = 1) and the weights
+template <class Row, int NW>
+constexpr int kSums = (Row::kUnitNorm ? 1 : 0) + NW;
+
+// a chain (u, e) with its derivatives d/dt and d/deps
+template <class Row, int NW>
+struct VecChain {
+    double u, e, u1, e1, uw[NW], ew[NW];
+    int E;  // common exponent
+    __device__ __forceinline__ void start(double u0, double e0) {
+        u = u0;
+        e = e0;
+        u1 = e1 = 0.0;
+#pragma unroll
+        for (int n = 0; n < NW; ++n) uw[n] = ew[n] = 0.0;
+        E = 0;
+    }
+    __device__ __forceinline__ void rescale() {
+        double m = fabs(u), k = fabs(e);
+        if (Row::kUnitNorm) {
+            m = fmax(m, fabs(u1));
+            k = fmax(k, fabs(e1));
+        }
+#pragma unroll
+        for (int n = 0; n < NW; ++n) {
+            m = fmax(m, fabs(uw[n]));
+            k = fmax(k, fabs(ew[n]));
+        }
+        const int x = max(biased_exp(m), biased_exp(k)), sh = x - 1023;
+        if (x != 0 && (sh > 240 || sh < -240)) {  // products of two stay finite
+            const double sc = pow2(-sh);
+            u *= sc;
+            e *= sc;
+            if (Row::kUnitNorm) {
+                u1 *= sc;
+                e1 *= sc;
+            }
+#pragma unroll
+            for (int n = 0; n < NW; ++n) {
+                uw[n] *= sc;
+                ew[n] *= sc;
+            }
+            E += sh;
+        }
+    }
+    // sum number n of the rows passed so far (sgn = 1 upwards, -1 downwards)
+    __device__ __forceinline__ double sum(int n, double rinv, double sgn) const {
+        if (Row::kUnitNorm && n == 0) return sgn * ((u * e1 - e * u1) * rinv);
+        const int k = n - (kSums<Row, NW> - NW);
+        return sgn * (e * uw[k] - u * ew[k]);
+    }
+};
+
+// matrices of two blocks at t: values, d/dt (Row::kUnitNorm) and the weights'
+template <class Row, int NW>
+struct VecMats {
+    double p[2][4], d[2][4], w[2][NW][4];
+    __device__ __forceinline__ void eval(const double* const (&T)[2], const double* const (&W)[2],
+                                         const double (&t)[2]) {
+        const double2* q[2] = {reinterpret_cast<const double2*>(T[0]), reinterpret_cast<const double2*>(T[1])};
+#pragma unroll
+        for (int k = kPD; k >= 0; --k)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const double2 v0 = q[b][2 * k], v1 = q[b][2 * k + 1];
+                const double cf[4] = {v0.x, v0.y, v1.x, v1.y};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (Row::kUnitNorm && k < kPD) d[b][j] = k == kPD - 1 ? p[b][j] : fma(d[b][j], t[b], p[b][j]);
+                    p[b][j] = k == kPD ? cf[j] : fma(p[b][j], t[b], cf[j]);
+                }
+                if (k <= kPW) {
+#pragma unroll
+                    for (int n = 0; n < NW; ++n) {
+                        const double2* r = reinterpret_cast<const double2*>(W[b] + n * kWD);
+                        const double2 w0 = r[2 * k], w1 = r[2 * k + 1];
+                        const double wf[4] = {w0.x, w0.y, w1.x, w1.y};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) w[b][n][j] = k == kPW ? wf[j] : fma(w[b][n][j], t[b], wf[j]);
+                    }
+                }
+            }
+    }
+    __device__ __forceinline__ void up(int b, VecChain<Row, NW>& C) const {
+        const double(&m)[4] = p[b];
+        if (Row::kUnitNorm) {
+            const double v = fma(m[0], C.u1, m[1] * C.e1) + fma(d[b][0], C.u, d[b][1] * C.e);
+            C.e1 = fma(m[2], C.u1, m[3] * C.e1) + fma(d[b][2], C.u, d[b][3] * C.e);
+            C.u1 = v;
+        }
+#pragma unroll
+        for (int n = 0; n < NW; ++n) {
+            const double(&g)[4] = w[b][n];
+            const double v = fma(m[0], C.uw[n], m[1] * C.ew[n]) + fma(g[0], C.u, g[1] * C.e);
+            C.ew[n] = fma(m[2], C.uw[n], m[3] * C.ew[n]) + fma(g[2], C.u, g[3] * C.e);
+            C.uw[n] = v;
+        }
+        const double un = fma(m[0], C.u, m[1] * C.e);
+        C.e = fma(m[2], C.u, m[3] * C.e);
+        C.u = un;
+    }
+    __device__ __forceinline__ void down(int b, VecChain<Row, NW>& C) const {
+        if (Row::kUnitNorm) {
+            adj_apply(p[b], C.u1, C.e1);
+            adj_add(d[b], C.u, C.e, C.u1, C.e1);
+        }
+#pragma unroll
+        for (int n = 0; n < NW; ++n) {
+            adj_apply(p[b], C.uw[n], C.ew[n]);
+            adj_add(w[b][n], C.u, C.e, C.uw[n], C.ew[n]);
+        }
+        adj_apply(p[b], C.u, C.e);
+    }
+};
+
+// Half of the eigenvector work of an item: the upward chain u (half 0) or the
+// downward chain b (half 1); at every coarse row (multiples of kCkRows) its
+// value, exponent and sums go to the checkpoints.  vs, vr: its values at the
+// source and receiver rows.
+template <class Row, int NW>
+__device__ __forceinline__ void vector_half(const ModesArgs& A, const ProblemInfo& pi, const Panel& P, double mu,
+                                            int half, PRing& R, double* __restrict__ ck, int* __restrict__ cke,
+                                            double& vs, int& Es, double& vr, int& Er) {
+    constexpr int kN = kSums<Row, NW>;
+    const int lane = threadIdx.x & 31;
+    const int nz = P.nz, isrc = pi.isrc, ircv = pi.ircv;
+    const double rinv = 1.0 / P.r;
+    const BlockShift<Row> sh(P, mu);
+    const double* wp = A.w + pi.w_off;
+    const double* gp = NW > 1 && A.g ? A.g + pi.s_off : nullptr;
+    auto weight = [&](int n, int i) { return n == 0 ? __ldg(wp + i) : (gp ? __ldg(gp + i) : 1.0); };
+    VecChain<Row, NW> C;
+    if (half == 0) C.start(1.0, P.e0);
+    else C.start(0.0, -1.0);
+    vs = vr = 0.0;
+    Es = Er = 0;
+    auto keep = [&](int a, double sgn) {  // state before row a
+        if (a % kCkRows) return;
+        const size_t c = (size_t)(a / kCkRows);
+        double* o = ck + c * (1 + kN) * 32 + lane;
+        o[0] = C.u;
+#pragma unroll
+        for (int n = 0; n < kN; ++n) o[32 * (1 + n)] = C.sum(n, rinv, sgn);
+        cke[c * 32 + lane] = C.E;
+    };
+    // the chain at row i of the block [a, end): from below (u) or above (b)
+    auto value = [&](int i, int a, int end, double& v, int& E) {
+        if (i < a || i >= end) return;
+        double f = C.e;
+        v = C.u;
+        E = C.E;
+        if (half == 0) rows_up<Row>(P.rows, a, i, mu, v, f);
+        else rows_down<Row>(P.rows, end, i, mu, v, f);
+    };
+    if (P.blk) {
+        const int nch = (P.nblk + kPanelChunk - 1) / kPanelChunk;
+        const double* src = A.T + (size_t)P.rec * kRecT;
+        const double* sw[2] = {A.W0 + (size_t)P.rec * kRecW, NW > 1 ? A.W1 + (size_t)P.rec * kRecW : nullptr};
+        ring_stream(
+            R, nch, A.err,
+            [&](double* dst, uint64_t* bar, int o) {
+                const size_t c = half ? nch - 1 - o : o;
+                mbar_expect_tx(bar, (kTD + NW * kWD) * 8);
+                tma_load_1d(dst, src + c * kTD, kTD * 8, bar);
+#pragma unroll
+                for (int n = 0; n < NW; ++n) tma_load_1d(dst + kTD + n * kWD, sw[n] + c * kWD, kWD * 8, bar);
+            },
+            [&](const double* buf, int o) {
+                const int c = half ? nch - 1 - o : o, nb = min(kPanelChunk, P.nblk - c * kPanelChunk);
+                for (int q0 = 0; q0 < kPanelChunk; q0 += 2) {
+                    const int qa = half ? kPanelChunk - 1 - q0 : q0, qb = half ? qa - 1 : qa + 1;
+                    if (min(qa, qb) >= nb) continue;
+                    VecMats<Row, NW> M;
+                    const double* const Ts[2] = {buf + qa * kRecT, buf + qb * kRecT};
+                    const double* const Ws[2] = {buf + kTD + qa * kRecW, buf + kTD + qb * kRecW};
+                    const double t[2] = {sh.at(Ts[0]), sh.at(Ts[1])};
+                    M.eval(Ts, Ws, t);
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        const int q = b ? qb : qa;
+                        if (q >= nb) continue;
+                        const int a = (c * kPanelChunk + q) * P.blk, end = min(nz, a + P.blk);
+                        if (half == 0) keep(a, 1.0);
+                        value(isrc, a, end, vs, Es);
+                        value(ircv, a, end, vr, Er);
+                        if (half == 0) {
+                            M.up(b, C);
+                        } else {
+                            M.down(b, C);
+                            keep(a, -1.0);
+                        }
+                    }
+                }
+                C.rescale();
+            });
+    } else {
+        const int nb = (nz + 15) / 16;
+        for (int o = 0; o < nb; ++o) {
+            const int a = 16 * (half ? nb - 1 - o : o), end = min(nz, a + 16);
+            if (half == 0) keep(a, 1.0);
+            value(isrc, a, end, vs, Es);
+            value(ircv, a, end, vr, Er);
+            for (int j = a; j < end; ++j) {
+                const int i = half ? a + end - 1 - j : j;
+                const double sg = Row::sigma(P.rows, i, mu), sl = Row::slope(P.rows, i, mu);
+                if (half == 0) {
+                    C.e1 = fma(-sg, C.u1, fma(sl, C.u, C.e1));
+#pragma unroll
+                    for (int n = 0; n < NW; ++n) C.ew[n] = fma(-sg, C.uw[n], fma(-weight(n, i), C.u, C.ew[n]));
+                    C.e = fma(-sg, C.u, C.e);
+                    C.u += C.e;
+                    C.u1 += C.e1;
+#pragma unroll
+                    for (int n = 0; n < NW; ++n) C.uw[n] += C.ew[n];
+                } else {
+                    C.u -= C.e;
+                    C.u1 -= C.e1;
+                    C.e1 = fma(sg, C.u1, fma(-sl, C.u, C.e1));
+#pragma unroll
+                    for (int n = 0; n < NW; ++n) {
+                        C.uw[n] -= C.ew[n];
+                        C.ew[n] = fma(sg, C.uw[n], fma(weight(n, i), C.u, C.ew[n]));
+                    }
+                    C.e = fma(sg, C.u, C.e);
+                }
+            }
+            if (half) keep(a, -1.0);
+            C.rescale();
+        }
+    }
+}
+
+// |u b| at a coarse row as m 2^E, m in [1, 2) (m = 0: none yet)
+struct TwistKey {
+    double m;
+    int E, c;
+    __device__ __forceinline__ void take(double u, int Eu, double b, int Eb, int at) {
+        double v = fabs(u * b);
+        int e = Eu + Eb;
+        normalize(v, e);
+        if (v > 0.0 && (m == 0.0 || e > E || (e == E && v > m))) {
+            m = v;
+            E = e;
+            c = at;
+        }
+    }
+};
+
+template <class Row, int NW>
+__device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemInfo& pi, const Panel& P,
+                                             const WorkItem& w, double mu, PRing& R, Pair& pr, double* __restrict__ ck,
+                                             int* __restrict__ cke) {
+    constexpr int kN = kSums<Row, NW>;
+    const int lane = threadIdx.x & 31, half = pr.half;
+    const int nc = (P.nz + kCkRows - 1) / kCkRows;
+    double* cks[2] = {ck, ck + A.ck_stride * (1 + kN)};
+    int* ckes[2] = {cke, cke + A.ck_stride};
+    double vs, vr;
+    int Es, Er;
+    vector_half<Row, NW>(A, pi, P, mu, half, R, cks[half], ckes[half], vs, Es, vr, Er);
+    PairBox& X = *pr.box;
+    const int tb = pr.turn, t2 = tb ^ 1;
+    if (half) {
+        X.v[tb][1][0][lane] = vs;
+        X.v[tb][1][1][lane] = vr;
+        X.v[tb][1][2][lane] = __hiloint2double(Es, Er);
+    }
+    pr.sync();  // checkpoints of both halves (and the box) visible to both
+    // the twist: the coarse row with the largest |u b|, the lowest of equal ones;
+    // each half looks through half of the rows
+    TwistKey K{0.0, 0, 0};
+    const int c0 = half ? nc / 2 : 0, c1 = half ? nc : nc / 2;
+#pragma unroll 4
+    for (int c = c0; c < c1; ++c) {
+        const size_t o = (size_t)c * (1 + kN) * 32 + lane, i = (size_t)c * 32 + lane;
+        K.take(__ldcg(cks[0] + o), __ldcg(ckes[0] + i), __ldcg(cks[1] + o), __ldcg(ckes[1] + i), c);
+    }
+    if (half) {
+        X.v[t2][1][0][lane] = K.m;
+        X.v[t2][1][1][lane] = __hiloint2double(K.E, K.c);
+    }
+    pr.sync();
+    if (half) return;
+    {
+        const double m = X.v[t2][1][0][lane], ec = X.v[t2][1][1][lane];
+        const int E = __double2hiint(ec);
+        if (m > 0.0 && (K.m == 0.0 || E > K.E || (E == K.E && m > K.m))) K.c = __double2loint(ec);
+    }
+    const double us = vs, ur = vr, bs = X.v[tb][1][0][lane], br = X.v[tb][1][1][lane];
+    const double eb = X.v[tb][1][2][lane];
+    const int Eus = Es, Eur = Er, Ebs = __double2hiint(eb), Ebr = __double2loint(eb);
+    const size_t o = (size_t)K.c * (1 + kN) * 32 + lane;
+    double ut = __ldcg(cks[0] + o), bt = __ldcg(cks[1] + o);
+    const int Eu0 = __ldcg(ckes[0] + (size_t)K.c * 32 + lane), Eb0 = __ldcg(ckes[1] + (size_t)K.c * 32 + lane);
+    int Eut = Eu0, Ebt = Eb0;
+    normalize(ut, Eut);
+    normalize(bt, Ebt);
+    const int eut = Eut - Eu0, ebt = Ebt - Eb0;  // exponents of u and b themselves
+    const double iu2 = 1.0 / (ut * ut), ib2 = 1.0 / (bt * bt);
+    auto total = [&](int n) {  // sum over all rows in units of z_r^2
+        double x = __ldcg(cks[0] + o + 32 * (1 + n)), y = __ldcg(cks[1] + o + 32 * (1 + n));
+        int ex = 0, ey = 0;
+        normalize(x, ex);
+        normalize(y, ey);
+        // both sums were taken at the exponents of u and b at the twist
+        return x * iu2 * pow2(ex - 2 * eut) + y * ib2 * pow2(ey - 2 * ebt);
+    };
+    const int r = K.c * kCkRows, isrc = pi.isrc, ircv = pi.ircv;
+    const int n1 = Row::kUnitNorm ? 0 : kN - 1, nw = kN - NW;
+    const double nrm = total(n1);  // sum z^2 / z_r^2
+    const double f2 = Row::kUnitNorm ? 1.0 : 1.0 / (1.0 + (mu / pi.dz) * (mu / pi.dz));
+    const double scale = Row::kUnitNorm ? 1.0 / sqrt(nrm * pi.dz) : sqrt(f2 / (nrm * pi.dz));
+    const double zs = (isrc <= r) ? (us / ut) * pow2(Eus - Eut) : (bs / bt) * pow2(Ebs - Ebt);
+    const double zr = (ircv <= r) ? (ur / ut) * pow2(Eur - Eut) : (br / bt) * pow2(Ebr - Ebt);
+    const double absorption = total(nw) / nrm * f2;
+    const double ks = Row::kUnitNorm ? sqrt(mu / (pi.dz * pi.dz)) : mu / pi.dz;
+    const auto kp = csqrt_principal(ks * ks, absorption);
+    if (lane < w.m) {
+        const int i = pi.off + w.j0 + lane;
+        A.kr[i] = kp.real();
+        A.ki[i] = kp.imag();
+        A.vs[i] = zs * scale;
+        A.vr[i] = zr * scale;
+        if (Row::kUnitNorm && NW > 1) {
+            const double vph = pi.omega / kp.real();
+            A.vg[i] = 1.0 / (vph * (total(nw + 1) / nrm));
+        } else if (A.vg) {
+            A.vg[i] = 0.0;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// eigenvalues and mode values of every item.  kDo: 1 eigenvalues to mu, 2 mode
+// values of the eigenvalues in mu, 3 both.  The pairs take items from the
+// cost-ordered list as they get free (sched: a zeroed counter), or round-robin.
+// ---------------------------------------------------------------------------
+template <class Row, int NW, int kDo>
+__global__ void __launch_bounds__(kPWarps * 32, kPanelCtas) k_panel_modes(ModesArgs A) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    constexpr int kSl = kTD + NW * kWD;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int n_items = *A.n_items_dev;
+    PRing R = make_ring(smem_raw, wid, kSl);
+    Pair pr;
+    pr.box = reinterpret_cast<PairBox*>(smem_raw + kRingBytes<kSl>) + (wid >> 1);
+    pr.id = wid >> 1;
+    pr.half = wid & 1;
+    pr.turn = 0;
+    const long long gp = (long long)blockIdx.x * (kPWarps / 2) + pr.id;
+    double* ck = A.ck_u + gp * 2 * A.ck_stride * (1 + kSums<Row, NW>);
+    int* cke = A.ck_e + gp * 2 * A.ck_stride;
+    long long walk = gp;
+    for (int turn = 0;; turn ^= 1) {
+        if (pr.half == 0 && lane == 0) {
+            long long it = walk;
+            if (A.sched) it = atomicAdd(A.sched, 1);
+            pr.box->item[turn] = it < n_items ? (int)it : -1;
+        }
+        walk += (long long)gridDim.x * (kPWarps / 2);
+        pr.sync();
+        const int it = pr.box->item[turn];
+        if (it < 0) break;
+        const WorkItem w = A.items[it];
+        const ProblemInfo& pi = A.pinfo[w.problem];
+        PanelDesc d{};
+        if (w.pad >= 0) d = A.desc[w.pad];
+        else d.xc = Row::lo(pi);
+        const Panel P = panel_of<Row>(pi, d, A.rows);
+        double x = P.xc;
+        if (kDo & 1) {
+            x = panel_bisect<Row>(pi, P, w, A.T, A.counts, A.tol, A.err, A.steps, R, pr);
+            if (pr.half == 0 && lane < w.m) A.mu[pi.off + w.j0 + lane] = x;
+        } else if (lane < w.m) {
+            x = A.mu[pi.off + w.j0 + lane];
+        }
+        if (kDo & 2) panel_vector<Row, NW>(A, pi, P, w, x, R, pr, ck, cke);
+    }
+}
+
+template <class Row, int NW>
+int modes_launch(cudaStream_t st, int grid, const ModesArgs& a, int what) {
+    const size_t sm = kRingBytes<kTD + NW * kWD> + (kPWarps / 2) * sizeof(PairBox);
+    void (*f)(ModesArgs) = what == 1   ? k_panel_modes<Row, NW, 1>
+                           : what == 2 ? k_panel_modes<Row, NW, 2>
+                                       : k_panel_modes<Row, NW, 3>;
+    cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    f<<<grid, kPWarps * 32, sm, st>>>(a);
+    return 1;
+}
+
+// CTAs per panel: enough for one thread per column of 128-row blocks, more
+// blocks go round the loop
+int expand_ctas(int nz_max) {
+    return std::max(1, (2 * ((nz_max + kPanelMaxBlk - 1) / kPanelMaxBlk) + kExpThreads - 1) / kExpThreads);
+}
+
+template <class Row, int NW>
+int expand_launch(cudaStream_t st, int n_desc, int nz_max, const ProblemInfo* pinfo, const PanelDesc* desc,
+                  const double* rows, const double* w, const double* g, double* T, double* W0, double* W1) {
+    int n = 0;
+    for (int d0 = 0; d0 < n_desc; d0 += 65535, ++n) {  // grid.y limit
+        dim3 grid(expand_ctas(nz_max), std::min(65535, n_desc - d0));
+        k_expand_items<Row, NW><<<grid, kExpThreads, 0, st>>>(pinfo, desc, d0, rows, w, g, T, W0, W1);
+    }
+    return n;
+}
+
+// Scan size of every problem, then (last block) the batch-wide trim and the
+// scan's panels.  The number of eigenvalues of S (diagonal s_i, unit
+// off-diagonals) below x is close to the sum over the rows of theta_i / pi with
+// cos theta_i = (s_i - x) / 2 clipped to [-1, 1] (each row's local band is [s_i
+// - 2, s_i + 2]); on the 20000-point grids of 0.002-0.5 Hz it gives the mode
+// count in [lo, hi] within one mode.  The scan takes about two shifts per mode
+// plus 32, in units of kScanStep.  Trim: with slots > 0 (the device's warp
+// schedulers) and U units in all, the batch drops U mod slots units when that is
+// at most a quarter of U, one each from the first problems that keep at least
+// 1.75 shifts per estimated mode.
+constexpr int kSizeThreads = 256;
+
+__device__ __forceinline__ bool scan_trimmable(int n_scan_raw, float m_est) {
+    const int u = n_scan_raw / kScanStep;
+    return u >= 2 && m_est >= 0.f && (float)((u - 1) * kScanStep) >= 1.75f * m_est;
+}
+
+__device__ int size_block_sum(int v, int* sh) {  // inclusive over the threads; sh[kSizeThreads] ints
+    const int t = threadIdx.x;
+    __syncthreads();
+    sh[t] = v;
+    __syncthreads();
+    for (int o = 1; o < kSizeThreads; o <<= 1) {
+        const int a = t >= o ? sh[t - o] : 0;
+        __syncthreads();
+        sh[t] += a;
+        __syncthreads();
+    }
+    return sh[t];
+}
+
+__global__ void __launch_bounds__(kSizeThreads) k_panel_size(int P, ProblemInfo* __restrict__ pinfo,
+                                                             const double* __restrict__ s, int slots,
+                                                             unsigned* __restrict__ done) {
+    __shared__ float part[kSizeThreads / 32];
+    __shared__ int sh[kSizeThreads];
+    __shared__ bool last;
+    {
+        const int p = blockIdx.x;
+        const double lo = pinfo[p].lo, hi = pinfo[p].hi;
+        const double* row = s + pinfo[p].s_off;
+        const int nz = pinfo[p].nz;
+        float acc = 0.f;
+        for (int i = threadIdx.x; i < nz; i += kSizeThreads) {
+            const double v = row[i];
+            const float ch = fminf(fmaxf((float)((v - hi) * 0.5), -1.f), 1.f);
+            const float cl = fminf(fmaxf((float)((v - lo) * 0.5), -1.f), 1.f);
+            acc += acosf(ch) - acosf(cl);
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float t = 0.f;
+            for (int w = 0; w < kSizeThreads / 32; ++w) t += part[w];
+            const float m_est = fmaxf(t * (float)(1.0 / kPi), 0.f);
+            const int n = ((int)(2.f * m_est) + 32 + kScanStep - 1) / kScanStep * kScanStep;
+            pinfo[p].n_scan_raw = min(max(n, kScanStep), kScanMax);
+            pinfo[p].m_est = m_est;
+            __threadfence();
+            last = atomicAdd(done, 1u) == gridDim.x - 1;
+        }
+        __syncthreads();
+    }
+    if (!last) return;
+    __threadfence();
+    // the records are read past L1: other blocks wrote them
+    auto raw = [&](int p) { return __ldcg(&pinfo[p].n_scan_raw); };
+    auto trim = [&](int p) { return scan_trimmable(raw(p), __ldcg(&pinfo[p].m_est)) ? 1 : 0; };
+    int remove = 0;
+    if (slots > 0) {
+        int u = 0;
+        for (int p = threadIdx.x; p < P; p += kSizeThreads) u += raw(p) / kScanStep;
+        size_block_sum(u, sh);
+        const int U = sh[kSizeThreads - 1];
+        const int rem = U % slots;
+        if (U >= slots && 4 * rem <= U) remove = rem;
+    }
+    int trimmed = 0;
+    for (int p0 = 0; p0 < P; p0 += kSizeThreads) {
+        const int p = p0 + threadIdx.x;
+        const int tr = remove > 0 && p < P ? trim(p) : 0;
+        const int incl = remove > 0 ? size_block_sum(tr, sh) : 0;
+        if (p < P) {
+            int n = raw(p);
+            if (tr && trimmed + incl - 1 < remove) n -= kScanStep;
+            pinfo[p].n_scan = n;
+            plan_scan_panels<EssPanel>(pinfo[p], n);
+        }
+        if (remove > 0) trimmed += sh[kSizeThreads - 1];
+        __syncthreads();
+    }
+}
+
+template <class Row>
+int scan_launch(cudaStream_t st, int P, int nz_max, const ProblemInfo* pinfo, const double* rows, double* T,
+                int* counts, unsigned* err) {
+    int n = 1;
+    const int step = 65535 / kScanSlots;
+    for (int p0 = 0; p0 < P; p0 += step, ++n) {  // grid.y limit
+        dim3 grid(expand_ctas(nz_max), kScanSlots * std::min(step, P - p0));
+        k_expand_scan<Row><<<grid, kExpThreads, 0, st>>>(pinfo, p0, rows, T);
+    }
+    static_assert(kScanSlots % kPWarps == 0, "a CTA's units belong to one problem");
+    k_panel_scan<Row><<<P * (kScanSlots / kPWarps), kPWarps * 32, kRingBytes<kTD>, st>>>(pinfo, rows, T, counts, err);
+    return n;
+}
+
+}  // namespace
+
+int launch_panel_scan(cudaStream_t st, int P, int nz_max, ProblemInfo* pinfo, const double* s, double* T, int* counts,
+                      int slots, unsigned* done, unsigned* err) {
+    k_panel_size<<<P, kSizeThreads, 0, st>>>(P, pinfo, s, slots, done);
+    return 1 + scan_launch<EssPanel>(st, P, nz_max, pinfo, s, T, counts, err);
+}
+
+int launch_panel_items(cudaStream_t st, int P, ProblemInfo* pinfo, const int* counts, int max_modes, int bis_item,
+                       WorkItem* items, int cap, PanelDesc* desc, int* tot, unsigned* err, int order) {
+    if (bis_item < 1 || bis_item > kWItem) return -1;
+    k_panel_items<<<1, kItemThreads, 0, st>>>(P, pinfo, counts, max_modes, bis_item, cap, tot, err, order);
+    k_panel_groups<EssPanel><<<(P + kPlanWarps - 1) / kPlanWarps, kPlanWarps * 32, 0, st>>>(P, pinfo, counts, bis_item,
+                                                                                          items, cap, desc);
+    return 2;
+}
+
+int launch_panel_expand(cudaStream_t st, int n_desc, int nz_max, const ProblemInfo* pinfo, const PanelDesc* desc,
+                        const double* s, const double* w, const double* g, double* T, double* W0, double* W1) {
+    return g ? expand_launch<EssPanel, 2>(st, n_desc, nz_max, pinfo, desc, s, w, g, T, W0, W1)
+             : expand_launch<EssPanel, 1>(st, n_desc, nz_max, pinfo, desc, s, w, nullptr, T, W0, nullptr);
+}
+
+int launch_panel_modes(cudaStream_t st, int grid, const ModesArgs& a, int what) {
+    return a.g ? modes_launch<EssPanel, 2>(st, grid, a, what) : modes_launch<EssPanel, 1>(st, grid, a, what);
+}
+
+int panel_ctas_per_sm() { return kPanelCtas; }
+
+}  // namespace ncpa

@@ -123,10 +123,13 @@ namespace {
 
 double estimate_bytes(const ncpa_server* s, const Request& r) {
     // per problem: matrix, weights, group speeds, WKB work row, scan counts,
-    // modes (up to 2048 of 5 doubles), 1-D TL; plus the profile and waveforms
+    // modes (up to 2048 of 5 doubles), 1-D TL; the panel expansions of the
+    // eigen-solve (about 500 bytes per row and Hz); plus the profile and waveforms
+    double hz = 0.0;
+    for (double f : r.freqs) hz += f;
     const double per_problem = 4.0 * 8.0 * s->nz_pad + 256 * 4 + 2048.0 * 5 * 8 + 3.0 * 8 * r.n_ranges;
     const double waves = (double)r.wave_ranges.size() * 8.0 * std::max(r.nfft, 4 * ((int)r.freqs.size() + 1));
-    return per_problem * (double)r.freqs.size() + 12.0 * 8 * r.n_knots + waves;
+    return per_problem * (double)r.freqs.size() + 500.0 * hz * s->nz_pad + 12.0 * 8 * r.n_knots + waves;
 }
 
 bool same_key(const CacheEntry& e, const Request& r) {
