@@ -14,6 +14,8 @@
 //  K5  modal sums for 1-D / 2-D transmission loss (ModeSolver.cpp:292-565)
 //  K6  ModBB transfer function + pulse synthesis
 //      (ModalBroadbandPropagator.cpp:245-277, BroadbandPropagator.cpp:327-662)
+#include <algorithm>
+
 #include "device_common.cuh"
 #include "item_sched.cuh"
 #include "kernels.hpp"
@@ -2554,71 +2556,237 @@ int launch_tl1d(cudaStream_t st, int P, const ProblemInfo* pinfo, const double* 
     return 1;
 }
 
-// 2-D TL on the sampled heights: P(r_i, z_j) = sum_m vz[j][m] b_m(r_i) with
-// b_m = v_m(z_s) e^{i k r}/sqrt(k); one CTA per range, threads over heights.
-__global__ void __launch_bounds__(256) k_tl2d(int M, const double* __restrict__ kr, const double* __restrict__ ki,
-                                              const double* __restrict__ vs_src, const double* __restrict__ vz,
-                                              int nzo, int nr, double dr, int lossless, long long sr,
-                                              long long sj, double* __restrict__ re, double* __restrict__ im) {
-    const int ir = blockIdx.x;
-    const double r = (ir + 1) * dr;
-    __shared__ double br[kTlTile], bi[kTlTile];
-    double accr[4] = {0, 0, 0, 0}, acci[4] = {0, 0, 0, 0};
-    for (int m0 = 0; m0 < M; m0 += kTlTile) {
-        __syncthreads();
-        for (int t = threadIdx.x; t < kTlTile && m0 + t < M; t += blockDim.x) {
-            const int m = m0 + t;
-            const double a = kr[m], b = lossless ? 0.0 : ki[m];
-            const auto sk = csqrt_principal(a, b);
-            const double den = sk.real() * sk.real() + sk.imag() * sk.imag();
-            const double isr = sk.real() / den, isi = -sk.imag() / den;
-            double sn, cs;
-            sincos(a * r, &sn, &cs);
-            const double amp = exp(-b * r) * vs_src[m];
-            const double er = amp * cs, ei = amp * sn;
-            br[t] = er * isr - ei * isi;
-            bi[t] = er * isi + ei * isr;
+// ===========================================================================
+// K5b: FP64 modal sum at many heights (2-D TL, receiver arrays):
+//   P(r_i, z_j) = C(r_i) sum_m v_m(z_j) b_m(r_i),  b_m = v_m(z_s) e^{i k r} / sqrt(k),
+// a real matrix product of [heights x modes] and [modes x 2 ranges], bound by
+// the FP64 unit: it goes through the FP64 matrix instructions, whose operand
+// traffic is a third of that of the same tile in FMAs (shared memory bound the
+// latter).  A CTA takes 64 heights x 8 NB ranges and 32 modes a step, two
+// buffers deep; its warps take 32 heights x 4 NB ranges of one half of each
+// step, the two halves added at the end: with whole steps to four warps the
+// last CTAs of a grid ran on their SM at a quarter of its rate.  b is not
+// evaluated per point: k_sum_phases tabulates b_m every 32nd tile, e^{i k dr}
+// of the 32 tiles up to there and of the ranges of one, and a CTA multiplies
+// the three (8 instructions a value instead of sine, cosine and exponential
+// each).  64 heights x 20000 ranges x 1185 modes: 3150 us with a thread per
+// range walking the modes, 476 us as a 4 x 4 tile of FMAs, 340 us as this
+// (165 us at the FP64 peak; the copies and products of a step take the rest).
+// ===========================================================================
+
+namespace {
+
+constexpr int kSumJ = 64, kSumK = 32;  // heights of a CTA, modes of a step; it takes 8 NB ranges
+constexpr int kSumMid = 32;  // tiles of a coarse phase
+constexpr int kSumThreads = 256;
+constexpr int kSumLd = 68;  // 4 mod 16 doubles: the fragments' 4 x 4 words of a half warp on different banks
+constexpr size_t kSumSmem = 2 * kSumK * 2 * kSumLd * 8;
+static_assert(kSumJ + 4 <= kSumLd && 2 * 8 * 4 + 4 <= kSumLd, "tile");
+static_assert(kSumSmem / 8 >= 32 * 128, "the partial sums reuse the buffers");
+
+// tab[row][m]: n0 coarse phases, kSumMid middle ones, n1 (ranges of a tile) fine ones
+__global__ void __launch_bounds__(128) k_sum_phases(int M, const double* __restrict__ kr,
+                                                    const double* __restrict__ ki,
+                                                    const double* __restrict__ vs_src, double dr, int lossless,
+                                                    int n0, int n1, double2* __restrict__ tab) {
+    const int m = blockIdx.y * blockDim.x + threadIdx.x, t = blockIdx.x;
+    if (m >= M) return;
+    const double a = kr[m], b = lossless ? 0.0 : ki[m];
+    double sn, cs;
+    double2 v;
+    if (t < n0) {
+        const double r = ((double)t * (kSumMid * n1) + 1.0) * dr;
+        const auto sk = csqrt_principal(a, b);
+        const double den = sk.real() * sk.real() + sk.imag() * sk.imag();
+        const double isr = sk.real() / den, isi = -sk.imag() / den;
+        sincos(a * r, &sn, &cs);
+        const double amp = exp(-b * r) * vs_src[m];
+        const double er = amp * cs, ei = amp * sn;
+        v = make_double2(er * isr - ei * isi, er * isi + ei * isr);
+    } else {
+        const double r = (double)(t < n0 + kSumMid ? (t - n0) * n1 : t - n0 - kSumMid) * dr;
+        sincos(a * r, &sn, &cs);
+        const double w = exp(-b * r);
+        v = make_double2(w * cs, w * sn);
+    }
+    tab[(size_t)t * M + m] = v;
+}
+
+// C += A B of 16 x 8 by 8 x 8 on the FP64 matrix unit
+__device__ __forceinline__ void mma_f64(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
+    return make_double2(fma(a.x, b.x, -(a.y * b.y)), fma(a.x, b.y, a.y * b.x));
+}
+
+// n bytes (8 or 16) to shared memory, zeros where off
+template <int N>
+__device__ __forceinline__ void copy_async(double* dst, const void* src, bool on) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "n"(N), "r"(on ? N : 0));
+}
+
+template <int NB>
+__global__ void __launch_bounds__(kSumThreads, 2) k_modal_sum(int M, const double2* __restrict__ tab, int n0,
+                                                              const double* __restrict__ vec,
+                                                              const int* __restrict__ rows, int nj, int nr,
+                                                              double dr, long long sr, long long sj,
+                                                              double* __restrict__ re, double* __restrict__ im) {
+    constexpr int kSumR = 8 * NB;
+    extern __shared__ __align__(16) double smem[];
+    using Buf = double[kSumK][kSumLd];
+    Buf* A = reinterpret_cast<Buf*>(smem);  // [2][mode][height]
+    Buf* B = A + 2;                         // [2][mode][range, re | im]
+    __shared__ long long roff[kSumJ];
+    const int tile = blockIdx.x, j0 = blockIdx.y * kSumJ;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q4 = lane & 3;
+    const int jw = (warp & 1) * 32, cw = ((warp >> 1) & 1) * kSumR, kw = (warp >> 2) * (kSumK / 2);
+    if (threadIdx.x < kSumJ) {
+        const int j = j0 + threadIdx.x;
+        roff[threadIdx.x] = j < nj ? (long long)rows[j] * M : -1;
+    }
+    __syncthreads();
+    double acc[2][NB][4];
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[a][b][c] = 0.0;
+    // copies: a thread 8 heights and 4 ranges of one mode; 4 modes x 4 rows a
+    // half warp, whose words fall on different banks
+    const int cm = 8 * (warp & 3) + (lane & 3) + 4 * (lane >> 4), c4 = (lane >> 2) & 3;
+    const int cj = (kSumJ / 2) * (warp >> 2) + c4, cr = (kSumR / 2) * (warp >> 2) + c4;
+    const double2* coarse = tab + (size_t)(tile / kSumMid) * M;
+    const double2* mid = tab + (size_t)(n0 + tile % kSumMid) * M;
+    const double2* fine = tab + (size_t)(n0 + kSumMid + cr) * M;
+    double2 x0 = make_double2(0.0, 0.0), x1 = x0;
+    auto issue = [&](int m0, int s) {
+        const int m = m0 + cm;
+        const bool on = m < M;
+        const int mc = on ? m : 0;
+#pragma unroll
+        for (int q = 0; q < kSumJ / 8; ++q) {
+            const long long o = roff[cj + 4 * q];
+            copy_async<8>(&A[s][cm][cj + 4 * q], vec + (o < 0 ? 0 : o) + mc, on && o >= 0);
+        }
+#pragma unroll
+        for (int q = 0; q < kSumR / 8; ++q)
+            copy_async<16>(&B[s][cm][2 * (cr + 4 * q)], fine + (size_t)(4 * q) * M + mc, on);
+        x0 = coarse[mc];
+        x1 = mid[mc];
+    };
+    if (M > 0) issue(0, 0);
+    int s = 0;
+    for (int m0 = 0; m0 < M; m0 += kSumK, s ^= 1) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        const double2 x = cmul(x0, x1);
+#pragma unroll
+        for (int q = 0; q < kSumR / 8; ++q) {  // this thread's own copies
+            double2* p = reinterpret_cast<double2*>(&B[s][cm][2 * (cr + 4 * q)]);
+            *p = cmul(x, *p);
         }
         __syncthreads();
-        const int mt = min(kTlTile, M - m0);
+        if (m0 + kSumK < M) issue(m0 + kSumK, s ^ 1);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int j = threadIdx.x + u * blockDim.x;
-            if (j < nzo) {
-                const double* row = vz + (size_t)j * M + m0;
-                for (int t = 0; t < mt; ++t) {
-                    accr[u] += row[t] * br[t];
-                    acci[u] += row[t] * bi[t];
-                }
-            }
+        for (int kk = 0; kk < kSumK / 2; kk += 8) {
+            const int k = kw + kk + q4;
+            double fa[2][4], fb[NB][2];
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) fa[a][i] = A[s][k + 4 * (i >> 1)][jw + 16 * a + g + 8 * (i & 1)];
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) fb[b][i] = B[s][k + 4 * i][cw + 8 * b + g];
+#pragma unroll
+            for (int a = 0; a < 2; ++a)
+#pragma unroll
+                for (int b = 0; b < NB; ++b) mma_f64(acc[a][b], fa[a], fb[b]);
         }
     }
-    const double c0 = 1000.0 * 4 * kPi / sqrt(8.0 * kPi) / sqrt(r);
+    // the second halves of the steps to the first warps
+    __syncthreads();
+    double* part = smem + (threadIdx.x & 127);
+    if (warp >= 4) {
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < NB; ++b)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) part[((a * NB + b) * 4 + c) * 128] = acc[a][b][c];
+    }
+    __syncthreads();
+    if (warp >= 4) return;
     const double ang = kPi * 0.25;
-    const double fr = c0 * sin(ang), fi = c0 * cos(ang);
+    const double sa = sin(ang), ca = cos(ang);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        const int j = threadIdx.x + u * blockDim.x;
-        if (j < nzo) {
-            const size_t o = (size_t)ir * sr + (size_t)j * sj;
-            re[o] = fr * accr[u] - fi * acci[u];
-            im[o] = fr * acci[u] + fi * accr[u];
+    for (int b = 0; b < NB; ++b) {
+        const int i = tile * kSumR + (cw >> 1) + 4 * b + q4;
+        if (i >= nr) continue;
+        const double c0 = 1000.0 * 4 * kPi / sqrt(8.0 * kPi) / sqrt((i + 1) * dr);
+        const double fr = c0 * sa, fi = c0 * ca;
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const int j = j0 + jw + 8 * a + g;
+            if (j >= nj) continue;
+            const int c = 2 * (a & 1), p = ((a >> 1) * NB + b) * 4 + c;
+            const double xr = acc[a >> 1][b][c] + part[p * 128], xi = acc[a >> 1][b][c + 1] + part[(p + 1) * 128];
+            const size_t o = (size_t)i * sr + (size_t)j * sj;
+            re[o] = fr * xr - fi * xi;
+            im[o] = fr * xi + fi * xr;
         }
     }
 }
 
-int launch_tl2d(cudaStream_t st, int M, const double* kr, const double* ki, const double* vs_src,
-                const double* vz, int nzo, int nr, double dr, int lossless, double* re, double* im) {
-    if (nzo > 1024) return -1;  // four heights per thread
-    k_tl2d<<<nr, 256, 0, st>>>(M, kr, ki, vs_src, vz, nzo, nr, dr, lossless, nzo, 1, re, im);
+int sum_coarse(int nr, int nb) { return (nr + kSumMid * 8 * nb - 1) / (kSumMid * 8 * nb); }
+
+template <int NB>
+int run_modal_sum(cudaStream_t st, int M, const double2* tab, const double* vec, const int* rows, int nj, int nr,
+                  double dr, long long sr, long long sj, double* re, double* im) {
+    if (cudaFuncSetAttribute(k_modal_sum<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSumSmem) !=
+        cudaSuccess)
+        return -1;
+    const dim3 grid((nr + 8 * NB - 1) / (8 * NB), (nj + kSumJ - 1) / kSumJ);
+    k_modal_sum<NB><<<grid, kSumThreads, kSumSmem, st>>>(M, tab, sum_coarse(nr, NB), vec, rows, nj, nr, dr, sr, sj,
+                                                        re, im);
     return 1;
 }
 
-int launch_tl2d_rcv_major(cudaStream_t st, int M, const double* kr, const double* ki, const double* vs_src,
-                          const double* vz, int n_rcv, int nr, double dr, int lossless, double* re, double* im) {
-    if (n_rcv > 1024) return -1;
-    k_tl2d<<<nr, 256, 0, st>>>(M, kr, ki, vs_src, vz, n_rcv, nr, dr, lossless, 1, nr, re, im);
-    return 1;
+}  // namespace
+
+size_t modal_sum_scratch(int M, int nr) {
+    return (size_t)(sum_coarse(nr, 2) + kSumMid + 32) * (size_t)std::max(M, 1) * sizeof(double2);
+}
+
+int launch_modal_sum(cudaStream_t st, int M, const double* kr, const double* ki, const double* vs_src,
+                     const double* vec, const int* rows, int nj, int nr, double dr, int lossless, bool range_major,
+                     int num_sms, void* scratch, double* re, double* im) {
+    // 32, 24 or 16 ranges a CTA: whichever keeps the last round of CTAs (2 on
+    // an SM) fullest, a round of one more tile costing as much as a full one
+    // (64 heights x 20000 ranges x 1185 modes: 24 ranges 330 us, 32 381 us)
+    int nb = 4;
+    long long best = 0;
+    for (int n = 4; n >= 2; --n) {
+        const long long ctas = (long long)((nr + 8 * n - 1) / (8 * n)) * ((nj + kSumJ - 1) / kSumJ);
+        const long long cost = (ctas + 2 * num_sms - 1) / (2 * num_sms) * (n + 1);  // + 1: the heights' copies
+        if (best == 0 || cost < best) best = cost, nb = n;
+    }
+    double2* tab = static_cast<double2*>(scratch);
+    const int n0 = sum_coarse(nr, nb), n1 = 8 * nb;
+    if (M > 0)
+        k_sum_phases<<<dim3(n0 + kSumMid + n1, (M + 127) / 128), 128, 0, st>>>(M, kr, ki, vs_src, dr, lossless, n0,
+                                                                             n1, tab);
+    const long long sr = range_major ? nj : 1, sj = range_major ? 1 : nr;
+    const int rc = nb == 4   ? run_modal_sum<4>(st, M, tab, vec, rows, nj, nr, dr, sr, sj, re, im)
+                   : nb == 3 ? run_modal_sum<3>(st, M, tab, vec, rows, nj, nr, dr, sr, sj, re, im)
+                             : run_modal_sum<2>(st, M, tab, vec, rows, nj, nr, dr, sr, sj, re, im);
+    return rc < 0 ? rc : rc + (M > 0);
 }
 
 // ===========================================================================

@@ -261,11 +261,13 @@ int eigvec_ctas_per_sm(const EigvecArgs& a);
 int launch_tl1d(cudaStream_t st, int P, const ProblemInfo* pinfo, const double* kr, const double* ki,
                 const double* vs, const double* vr, int nr, double dr, int lossless, double* re, double* im,
                 double* incoh);
-int launch_tl2d(cudaStream_t st, int M, const double* kr, const double* ki, const double* vs_src,
-                const double* vz, int nzo, int nr, double dr, int lossless, double* re, double* im);
-// same sum with [n_rcv x nr] output (receiver-major)
-int launch_tl2d_rcv_major(cudaStream_t st, int M, const double* kr, const double* ki, const double* vs_src,
-                          const double* vz, int n_rcv, int nr, double dr, int lossless, double* re, double* im);
+// FP64 modal sum at heights rows[j] (rows of vec, M values each):
+// re/im [nr x nj] with range_major, else [nj x nr]; scratch of
+// modal_sum_scratch bytes
+size_t modal_sum_scratch(int M, int nr);
+int launch_modal_sum(cudaStream_t st, int M, const double* kr, const double* ki, const double* vs_src,
+                     const double* vec, const int* rows, int nj, int nr, double dr, int lossless, bool range_major,
+                     int num_sms, void* scratch, double* re, double* im);
 // out[c][r] = in[r][c] (rows x cols doubles)
 int launch_transpose(cudaStream_t st, int rows, int cols, const double* in, double* out);
 // broadband synthesis
@@ -324,7 +326,6 @@ MsPlan ms_plan(int n_rcv, int M, int n_ranges, int num_sms);
 double ms_guard_tau(const MsPlan& p);
 // the error bound eps behind it: |P_tc - P| <= eps S
 double ms_guard_eps(const MsPlan& p);
-int launch_ms_gather(cudaStream_t st, int n_rcv, int M, const int* idx, const double* vfull, double* vz);
 // fmt: 0 = 3-term split-BF16 (kind::f16), 1 = TF32 (kind::tf32), 2 = guarded
 // 6-term split-BF16.  Buffers: a_img = A as complex FP32 per (receiver group,
 // mode chunk), q = tile phases, tab = the B' image of each mode chunk

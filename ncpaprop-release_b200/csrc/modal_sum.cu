@@ -918,15 +918,6 @@ __global__ void __launch_bounds__(256) k_ms_fix(const int* __restrict__ fix_coun
     }
 }
 
-// gather of the mode values at the receiver grid points: vz[j][m] = v[idx_j][m]
-__global__ void k_ms_gather(int n_rcv, int M, const int* __restrict__ idx, const double* __restrict__ vfull,
-                            double* __restrict__ vz) {
-    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= (long long)n_rcv * M) return;
-    const int m = (int)(id % M), j = (int)(id / M);
-    vz[id] = vfull[(size_t)idx[j] * M + m];
-}
-
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
@@ -974,13 +965,6 @@ double ms_guard_tau(const MsPlan& p) {
     // |dP| <= eps S, a point with |P_tc| >= eps S (1 + 1 / d) satisfies it
     const double d = 1.0 - std::pow(10.0, -kMsGuardTlDb / 20.0);
     return ms_guard_eps(p) * (1.0 + 1.0 / d);
-}
-
-int launch_ms_gather(cudaStream_t st, int n_rcv, int M, const int* idx, const double* vfull, double* vz) {
-    const long long n = (long long)n_rcv * M;
-    if (n == 0) return 0;
-    k_ms_gather<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n_rcv, M, idx, vfull, vz);
-    return 1;
 }
 
 // a_img receives A (complex FP32), tab the B' images, q the tile phases

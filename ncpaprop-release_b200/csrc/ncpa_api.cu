@@ -2067,13 +2067,11 @@ void modal_sum_rows(ncpa_ctx* ctx, const ncpa_modes* m, int problem, const std::
         const double* ki = m->d_ki.as<double>() + pi.off;
         const double* vs = m->d_vs.as<double>() + pi.off;
         if (method == NCPA_SUM_FP64) {
-            ctx->ms_vz.alloc((size_t)n_rcv * M * 8, st);
-            check_launch(ctx, ncpa::launch_ms_gather(st, n_rcv, M, ctx->ms_idx.as<int>(), vfull,
-                                                     ctx->ms_vz.as<double>()));
+            ctx->ms_vz.alloc(ncpa::modal_sum_scratch(M, nr), st);
             tm.mark("ms-prep");
-            check_launch(ctx, ncpa::launch_tl2d_rcv_major(st, M, kr, ki, vs, ctx->ms_vz.as<double>(), n_rcv, nr,
-                                                          tp->dr_m, tp->lossless, ctx->ms_re.as<double>(),
-                                                          ctx->ms_im.as<double>()));
+            check_launch(ctx, ncpa::launch_modal_sum(st, M, kr, ki, vs, vfull, ctx->ms_idx.as<int>(), n_rcv, nr,
+                                                     tp->dr_m, tp->lossless, false, ctx->num_sms, ctx->ms_vz.p,
+                                                     ctx->ms_re.as<double>(), ctx->ms_im.as<double>()));
             tm.mark("ms-fp64");
         } else {
             const ncpa::MsPlan pl = ncpa::ms_plan(n_rcv, M, nr, ctx->num_sms);
@@ -2196,25 +2194,22 @@ ncpa_status ncpa_tl_2d(ncpa_ctx* ctx, const ncpa_modes* m, int problem, const nc
             check_device_status(ctx);
             return NCPA_OK;
         }
-        // rows of the sampled heights and the source row (last), gathered on
-        // the device: the full vectors never leave HBM
-        std::vector<int> rows(nzo + 1);
+        std::vector<int> rows(nzo);
         for (int j = 0; j < nzo; ++j) {
             rows[j] = j * stepj;
             if (z_out) z_out[j] = (j * stepj) * pi.dz;
         }
-        rows[nzo] = pi.isrc;
-        DevBuf drows, dvz, dre, dim;
+        DevBuf drows, dre, dim;
         upload(drows, rows, st);
-        dvz.alloc((size_t)(nzo + 1) * std::max(Mm, 1) * 8, st);
-        check_launch(ctx, ncpa::launch_ms_gather(st, nzo + 1, Mm, drows.as<int>(),
-                                                 m->d_vfull.as<double>() + m->vfull_off[problem], dvz.as<double>()));
         const size_t n = (size_t)tp->n_ranges * nzo;
         dre.alloc(n * 8, st);
         dim.alloc(n * 8, st);
-        check_launch(ctx, ncpa::launch_tl2d(st, Mm, m->d_kr.as<double>() + pi.off, m->d_ki.as<double>() + pi.off,
-                                            dvz.as<double>() + (size_t)nzo * Mm, dvz.as<double>(), nzo, tp->n_ranges,
-                                            tp->dr_m, tp->lossless, dre.as<double>(), dim.as<double>()));
+        ctx->ms_vz.alloc(ncpa::modal_sum_scratch(Mm, tp->n_ranges), st);
+        const double* vec = m->d_vfull.as<double>() + m->vfull_off[problem];
+        check_launch(ctx, ncpa::launch_modal_sum(st, Mm, m->d_kr.as<double>() + pi.off, m->d_ki.as<double>() + pi.off,
+                                                 vec + (size_t)pi.isrc * Mm, vec, drows.as<int>(), nzo, tp->n_ranges,
+                                                 tp->dr_m, tp->lossless, true, ctx->num_sms, ctx->ms_vz.p,
+                                                 dre.as<double>(), dim.as<double>()));
         CK(cudaMemcpyAsync(re, dre.p, n * 8, cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(im, dim.p, n * 8, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
