@@ -231,6 +231,17 @@ int launch_panel_expand(cudaStream_t st, int n_desc, int nz_max, const ProblemIn
                         const double* s, const double* w, const double* g, double* T, double* W0, double* W1);
 constexpr int kPanelSlots = 4;  // two pairs of warps, two directions each
 constexpr int kCkVals = 4;  // doubles of a coarse row's checkpoint, at most
+// full vectors: the state of a chain before a coarse row, times 2^E
+struct VecState {
+    double u, e;
+    int E, pad;
+};
+// and per mode its shift, the factors of either chain (with exponents) that
+// make it the mode function, and the row where they meet
+struct VecTwist {
+    double mu, fu, fb;
+    int Eu, Eb, r, pad;
+};
 struct ModesArgs {
     const ProblemInfo* pinfo;
     const double* rows;
@@ -247,12 +258,23 @@ struct ModesArgs {
     double* ck_u;  // per CTA: kPanelSlots x kCkVals ck_stride doubles, kPanelSlots x ck_stride ints
     int* ck_e;
     long long ck_stride;
+    // full vectors (null: none): per problem at vstate_off the upward states
+    // [coarse row][mode], then the downward ones
+    VecState* vstate;
+    const long long* vstate_off;
+    VecTwist* vtwist;
+    unsigned long long* vpeak;  // zeroed
+    double* vfull;              // [row][mode] per problem at vfull_off
+    const long long* vfull_off;
     int* sched;  // item counter (zeroed) or null: round-robin
     unsigned* err;
     unsigned long long* steps;  // optional counter of row steps
 };
 // what: 1 eigenvalues, 2 mode values of the eigenvalues in mu, 3 both
 int launch_panel_modes(cudaStream_t st, int grid, const ModesArgs& a, int what);
+// the mode functions at every row from the states that launch_panel_modes
+// left; m_max: the most modes of a problem
+int launch_panel_fill(cudaStream_t st, int P, int nz_max, int m_max, const ModesArgs& a);
 int panel_ctas_per_sm();
 
 // resident eigenvector CTAs per SM for the variant selected by a

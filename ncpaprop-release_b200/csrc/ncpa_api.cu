@@ -532,11 +532,61 @@ void prepare_solve(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, int
 // warp schedulers of the device for the scan trim (0: no trim)
 int scan_slots(const ncpa_ctx* ctx) { return ctx->scan_trim ? 4 * ctx->num_sms : 0; }
 
+// after the work items: a problem above max_modes is an error
+void check_mode_limit(ncpa_ctx* ctx, const ncpa_modes* M, unsigned err) {
+    if (!(err & ncpa::kErrTooMany)) return;
+    CK(cudaMemsetAsync(ctx->d_err.p, 0, sizeof(unsigned), ctx->stream));
+    int worst = 0;
+    for (int p = 0; p < M->P; ++p)
+        if (M->info[p].c_hi - M->info[p].c_lo > M->info[worst].c_hi - M->info[worst].c_lo) worst = p;
+    char buf[160];
+    std::snprintf(buf, sizeof buf, "problem %d (f=%g Hz, az=%g) has %d modes > max_modes %d", worst,
+                  M->info[worst].freq, M->info[worst].az, M->info[worst].c_hi - M->info[worst].c_lo,
+                  M->prm.max_modes);
+    throw ApiError(NCPA_ETOOMANY, buf);
+}
+
+// Buffers of the full vectors, sized by the modes found: the one host wait
+// before the end of a solve.
+struct VecBufs {
+    DevBuf state, off, twist, peak;
+    int m_max = 0;
+};
+
+void prepare_vectors(ncpa_ctx* ctx, ncpa_modes* M, SolveBufs& b, VecBufs& v) {
+    cudaStream_t st = ctx->stream;
+    const int P = M->P;
+    unsigned err = 0;
+    CK(cudaMemcpyAsync(M->info.data(), M->d_pinfo.p, P * sizeof(ProblemInfo), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(&err, ctx->d_err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    check_mode_limit(ctx, M, err);
+    std::vector<long long> off(P);
+    M->vfull_off.resize(P);
+    long long acc = 0, n_state = 0, n_modes = 0;
+    for (int p = 0; p < P; ++p) {
+        const ProblemInfo& pi = M->info[p];
+        M->vfull_off[p] = acc;
+        off[p] = n_state;
+        acc += (long long)pi.M * pi.nz;
+        n_state += 2ll * pi.M * ((pi.nz + ncpa::kCkRows - 1) / ncpa::kCkRows);
+        n_modes += pi.M;
+        v.m_max = std::max(v.m_max, pi.M);
+    }
+    M->d_vfull.alloc((size_t)std::max(1LL, acc) * 8, st);
+    v.state.alloc((size_t)std::max(1LL, n_state) * sizeof(ncpa::VecState), st);
+    v.twist.alloc((size_t)std::max(1LL, n_modes) * sizeof(ncpa::VecTwist), st);
+    v.peak.alloc((size_t)std::max(1LL, n_modes) * 8, st);
+    CK(cudaMemsetAsync(v.peak.p, 0, v.peak.bytes, st));
+    upload(M->d_vfull_off, M->vfull_off, st);
+    upload(v.off, off, st);
+}
+
 // Window, panel expansions, Sturm scan, device-built work items, eigenvalues
 // and mode values over all problems of M, then copies of the item/mode
 // totals, the problem records and the device status word to tot_dst, info_dst
-// and err_dst.  No host synchronisation: the whole sequence can be captured
-// in a CUDA graph.
+// and err_dst.  No host synchronisation, except for want_vectors (which plans
+// refuse): the whole sequence can be captured in a CUDA graph.
 void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_params* prm, bool wkb, double* s,
                    double* w, double* gs, double* kz2, SolveBufs& b, const Tuning& t, bool count_steps,
                    int* tot_dst, ProblemInfo* info_dst, unsigned* err_dst) {
@@ -563,6 +613,8 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
                                                b.items.as<WorkItem>(), b.item_cap, desc, b.tot.as<int>(), err,
                                                ctx->bis_order ? 1 : 0));
     tm.mark("host-items");
+    VecBufs v;
+    if (prm->want_vectors) prepare_vectors(ctx, M, b, v);
     // ---- panel expansions ----
     check_launch(ctx, ncpa::launch_panel_expand(st, M->n_desc, M->nz_max, d_pinfo, desc, s, w, g, b.T,
                                                 b.W0, b.W1));
@@ -591,6 +643,14 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
     a.ck_stride = ncpa::coarse_slot_elems(M->nz_max);
     a.sched = ctx->bis_order ? b.sched.as<int>() : nullptr;
     a.err = err;
+    if (prm->want_vectors) {
+        a.vstate = v.state.as<ncpa::VecState>();
+        a.vstate_off = v.off.as<long long>();
+        a.vtwist = v.twist.as<ncpa::VecTwist>();
+        a.vpeak = v.peak.as<unsigned long long>();
+        a.vfull = M->d_vfull.as<double>();
+        a.vfull_off = M->d_vfull_off.as<long long>();
+    }
     if (fuse) {
         check_launch(ctx, ncpa::launch_panel_modes(st, modes_grid(ctx, t.bis_ctas), a, 3));
         tm.mark("bisect+eigvec");
@@ -603,6 +663,10 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
         check_launch(ctx, ncpa::launch_panel_modes(st, modes_grid(ctx, t.bis_ctas), a, 2));
         tm.mark("eigvec");
     }
+    if (prm->want_vectors) {
+        check_launch(ctx, ncpa::launch_panel_fill(st, P, M->nz_max, v.m_max, a));
+        tm.mark("vectors");
+    }
     CK(cudaMemcpyAsync(tot_dst, b.tot.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(info_dst, d_pinfo, P * sizeof(ProblemInfo), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(err_dst, err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
@@ -614,17 +678,7 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
 void finish_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const int* tot, const unsigned* err) {
     cudaStream_t st = ctx->stream;
     CK(cudaStreamSynchronize(st));
-    if (*err & ncpa::kErrTooMany) {
-        CK(cudaMemsetAsync(ctx->d_err.p, 0, sizeof(unsigned), st));
-        int worst = 0;
-        for (int p = 0; p < M->P; ++p)
-            if (M->info[p].c_hi - M->info[p].c_lo > M->info[worst].c_hi - M->info[worst].c_lo) worst = p;
-        char buf[160];
-        std::snprintf(buf, sizeof buf, "problem %d (f=%g Hz, az=%g) has %d modes > max_modes %d", worst,
-                      M->info[worst].freq, M->info[worst].az, M->info[worst].c_hi - M->info[worst].c_lo,
-                      M->prm.max_modes);
-        throw ApiError(NCPA_ETOOMANY, buf);
-    }
+    check_mode_limit(ctx, M, *err);
     M->Mtot = tot[2];
     M->host_valid = false;
     if (!M->prm.keep_on_device) fetch_modes(M);
@@ -637,146 +691,14 @@ void finish_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const int* tot, 
 // at the offsets in its ProblemInfo).
 void solve_core(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_params* prm, bool wkb, DevBuf& s,
                 DevBuf& w, DevBuf& g, DevBuf& kz2) {
-    cudaStream_t st = ctx->stream;
-    const int P = M->P;
-    ProblemInfo* d_pinfo = M->d_pinfo.as<ProblemInfo>();
-    if (!prm->want_vectors) {  // device-built work items, one host wait at the end
-        Tuning t;
-        if (ctx->item_override > 0) t.bis_item = std::min(ctx->item_override, ncpa::kWItem);
-        SolveBufs b;
-        prepare_solve(ctx, M, prm, t.bis_item, b);
-        unsigned h_err = 0;
-        enqueue_solve(ctx, tm, M, prm, wkb, s.as<double>(), w.as<double>(), g.as<double>(), kz2.as<double>(), b, t,
-                      ctx->stats && !ctx->stats_fused, ctx->h_tot, M->info.data(), &h_err);
-        finish_solve(ctx, tm, M, ctx->h_tot, &h_err);
-        return;
-    }
-    // ---- K2 window ----
-    check_launch(ctx, ncpa::launch_window(st, P, d_pinfo, wkb ? kz2.as<double>() : nullptr, wkb ? 1 : 0,
-                                          prm->wvnum_filter, prm->c_min, prm->c_max, ctx->d_err.as<unsigned>()));
-    tm.mark("window");
-    // ---- K3a scan ----
-    DevBuf counts;
-    counts.alloc((size_t)P * ncpa::kScanMax * 4, st);
-    check_launch(ctx, ncpa::launch_scan(st, P, d_pinfo, s.as<double>(), counts.as<int>(), ctx->d_err.as<unsigned>(),
-                                        scan_slots(ctx)));
-    tm.mark("scan");
-    std::vector<int> hcounts((size_t)P * ncpa::kScanMax);
-    CK(cudaMemcpyAsync(hcounts.data(), counts.p, hcounts.size() * 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(M->info.data(), d_pinfo, P * sizeof(ProblemInfo), cudaMemcpyDeviceToHost, st));
-    check_device_status(ctx);
-    // ---- modes per problem, offsets, work items ----
-    std::vector<WorkItem> items;
-    int off = 0;
-    for (int p = 0; p < P; ++p) {
-        ProblemInfo& pi = M->info[p];
-        pi.c_lo = hcounts[(size_t)p * ncpa::kScanMax];
-        pi.c_hi = hcounts[(size_t)p * ncpa::kScanMax + pi.n_scan - 1];
-        pi.M = std::max(0, pi.c_hi - pi.c_lo);
-        if (pi.M > M->prm.max_modes) {
-            char buf[160];
-            std::snprintf(buf, sizeof buf, "problem %d (f=%g Hz, az=%g) has %d modes > max_modes %d", p, pi.freq,
-                          pi.az, pi.M, M->prm.max_modes);
-            throw ApiError(NCPA_ETOOMANY, buf);
-        }
-        pi.off = off;
-        off += pi.M;
-    }
-    // eigenvalues per bisection item: 32 (one per lane).  Smaller items give
-    // each eigenvalue more shifts per round but cost more Sturm sequences in
-    // total, which measured slower on the 256-frequency workload (16: +26 %,
-    // 8: +100 %); NCPA_BISECT_ITEM overrides it for tuning.
-    const int item_sz = ctx->item_override > 0 ? ctx->item_override : ncpa::kWItem;
-    for (int p = 0; p < P; ++p) {
-        const ProblemInfo& pi = M->info[p];
-        const int nit = (pi.M + item_sz - 1) / item_sz;
-        for (int k = 0; k < nit; ++k) {
-            int j0 = (int)((long long)pi.M * k / nit), j1 = (int)((long long)pi.M * (k + 1) / nit);
-            items.push_back(WorkItem{p, j0, j1 - j0, 0});
-        }
-    }
-    M->Mtot = off;
-    // largest items first: they need the most multisection rounds
-    std::stable_sort(items.begin(), items.end(), [](const WorkItem& a, const WorkItem& b) { return a.m > b.m; });
-    CK(cudaMemcpyAsync(d_pinfo, M->info.data(), P * sizeof(ProblemInfo), cudaMemcpyHostToDevice, st));
-    const int Mt = std::max(1, M->Mtot);
-    DevBuf mu, d_items, d_counter;
-    mu.alloc((size_t)Mt * 8, st);
-    M->d_kr.alloc((size_t)Mt * 8, st);
-    M->d_ki.alloc((size_t)Mt * 8, st);
-    M->d_vs.alloc((size_t)Mt * 8, st);
-    M->d_vr.alloc((size_t)Mt * 8, st);
-    M->d_vg.alloc((size_t)Mt * 8, st);
-    if (prm->want_vectors) {
-        M->vfull_off.resize(P);
-        long long acc = 0;
-        for (int p = 0; p < P; ++p) {
-            M->vfull_off[p] = acc;
-            acc += (long long)M->info[p].M * M->info[p].nz;
-        }
-        M->d_vfull.alloc((size_t)std::max(1LL, acc) * 8, st);
-        upload(M->d_vfull_off, M->vfull_off, st);
-    }
-    const int n_items = (int)items.size();
-    if (n_items > 0) {
-        upload(d_items, items, st);
-        d_counter.alloc(2 * sizeof(int), st);
-        CK(cudaMemsetAsync(d_counter.p, 0, 2 * sizeof(int), st));
-        // ---- K3 bisection ----
-        const int wpc = 4;  // warps per bisection CTA
-        int grid_b = std::min((n_items + wpc - 1) / wpc, ctx->num_sms * ncpa::bisect_ctas_per_sm());
-        tm.mark("host-items");
-        check_launch(ctx, ncpa::launch_bisect(st, grid_b, d_pinfo, s.as<double>(), counts.as<int>(),
-                                              d_items.as<WorkItem>(), n_items, d_counter.as<int>(), kBisectTol,
-                                              mu.as<double>(), ctx->d_err.as<unsigned>(),
-                                              ctx->stats ? ctx->d_stats.as<unsigned long long>() : nullptr));
-        tm.mark("bisect");
-        // ---- K4 eigenvectors: items of <= kEvItem eigenvalues ----
-        std::vector<WorkItem> ev_items;
-        for (int p = 0; p < P; ++p) {
-            const int Mp = M->info[p].M;
-            for (int j0 = 0; j0 < Mp; j0 += ncpa::kEvItem)
-                ev_items.push_back(WorkItem{p, j0, std::min(ncpa::kEvItem, Mp - j0), 0});
-        }
-        DevBuf d_ev_items;
-        upload(d_ev_items, ev_items, st);
-        const int n_ev = (int)ev_items.size();
-        ncpa::EigvecArgs ea{};
-        ea.pinfo = d_pinfo;
-        ea.s = s.as<double>();
-        ea.w = w.as<double>();
-        ea.g = prm->want_group_speed ? g.as<double>() : nullptr;
-        ea.items = d_ev_items.as<WorkItem>();
-        ea.n_items = n_ev;
-        ea.counter = d_counter.as<int>() + 1;
-        ea.mu = mu.as<double>();
-        ea.kr = M->d_kr.as<double>();
-        ea.ki = M->d_ki.as<double>();
-        ea.vs = M->d_vs.as<double>();
-        ea.vr = M->d_vr.as<double>();
-        ea.vg = M->d_vg.as<double>();
-        ea.vfull = prm->want_vectors ? M->d_vfull.as<double>() : nullptr;
-        ea.vfull_off = prm->want_vectors ? M->d_vfull_off.as<long long>() : nullptr;
-        const int ewpc = ncpa::kEvWarpsPerCta;
-        const int grid_e = std::min((n_ev + ewpc - 1) / ewpc, ctx->num_sms * ncpa::eigvec_ctas_per_sm(ea));
-        const long long slot = ncpa::ck_slot_elems(M->nz_max);
-        const size_t need = (size_t)grid_e * ewpc * slot;
-        // (alloc keeps a buffer that is large enough)
-        ctx->ck1.alloc(need * 8, st);
-        ctx->ck2.alloc(need * 8, st);
-        ctx->cke.alloc(need * 4, st);
-        ea.ck_q1 = ctx->ck1.as<double>();
-        ea.ck_q2 = ctx->ck2.as<double>();
-        ea.ck_e = ctx->cke.as<int>();
-        ea.ck_slot_stride = slot;
-        ea.err = ctx->d_err.as<unsigned>();
-        check_launch(ctx, ncpa::launch_eigvec(st, grid_e, ea));
-    }
-    tm.mark("eigvec");
-    // ---- results to host ----
-    if (!prm->keep_on_device) fetch_modes(M);
-    check_device_status(ctx);
-    tm.mark("fetch");
+    Tuning t;
+    if (ctx->item_override > 0) t.bis_item = std::min(ctx->item_override, ncpa::kWItem);
+    SolveBufs b;
+    prepare_solve(ctx, M, prm, t.bis_item, b);
+    unsigned h_err = 0;
+    enqueue_solve(ctx, tm, M, prm, wkb, s.as<double>(), w.as<double>(), g.as<double>(), kz2.as<double>(), b, t,
+                  ctx->stats && !ctx->stats_fused, ctx->h_tot, M->info.data(), &h_err);
+    finish_solve(ctx, tm, M, ctx->h_tot, &h_err);
 }
 
 void init_modes(ncpa_modes* M, ncpa_ctx* ctx, const ncpa_ess_params* prm, int P) {

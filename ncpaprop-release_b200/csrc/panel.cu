@@ -1125,11 +1125,12 @@ struct VecMats {
 
 // Half of the eigenvector work of an item: the upward chain u (half 0) or the
 // downward chain b (half 1); at every coarse row (multiples of kCkRows) its
-// value, exponent and sums go to the checkpoints.  vs, vr: its values at the
-// source and receiver rows.
-template <class Row, int NW>
+// value, exponent and sums go to the checkpoints and, for full vectors (kV),
+// its state to `st` (stride: modes).  vs, vr: its values at the source and
+// receiver rows.
+template <class Row, int NW, bool kV>
 __device__ __forceinline__ void vector_half(const ModesArgs& A, const ProblemInfo& pi, const Panel& P, double mu,
-                                            int half, PRing& R, double* __restrict__ ck, int* __restrict__ cke,
+                                            int half, VecState* __restrict__ st, PRing& R, double* __restrict__ ck, int* __restrict__ cke,
                                             double& vs, int& Es, double& vr, int& Er) {
     constexpr int kN = kSums<Row, NW>;
     const int lane = threadIdx.x & 31;
@@ -1152,6 +1153,7 @@ __device__ __forceinline__ void vector_half(const ModesArgs& A, const ProblemInf
 #pragma unroll
         for (int n = 0; n < kN; ++n) o[32 * (1 + n)] = C.sum(n, rinv, sgn);
         cke[c * 32 + lane] = C.E;
+        if (kV && st) st[c * pi.M] = VecState{C.u, C.e, C.E, 0};
     };
     // the chain at row i of the block [a, end): from below (u) or above (b)
     auto value = [&](int i, int a, int end, double& v, int& E) {
@@ -1256,7 +1258,85 @@ struct TwistKey {
     }
 };
 
+// the chains and their sums at the row where they are joined: rows below r in
+// su (at u's exponent), rows from r on in sb
+template <int kN>
+struct TwistAt {
+    double u, b, su[kN], sb[kN];
+    int Eu, Eb, r;
+};
+
+// Full vectors on grids so coarse that a mode can live between two coarse
+// rows: beyond it a chain picks up the growing solution, by e^{g} eps of the
+// mode after a decay of g.  The coarse twist leaves at most half a chunk of
+// that; up to g = 10 it costs 2e-12 and the search below is left out.
+__device__ __forceinline__ bool fine_twist_needed(const ProblemInfo& pi) {
+    const double c0 = __longlong_as_double((long long)pi.ceffmin_bits), c1 = __longlong_as_double((long long)pi.ceffmax_bits);
+    const double kh = pi.omega * pi.dz, g = 0.5 * kCkRows * kh;
+    return g * g * (1.0 / (c0 * c0) - 1.0 / (c1 * c1)) > 100.0;
+}
+
+// the row with the largest |u b| in the two chunks around coarse row c0 (the
+// lowest of equal ones), and the sums up to it.  vfull's rows hold b meanwhile.
 template <class Row, int NW>
+__device__ __noinline__ void fine_twist(const ModesArgs& A, const ProblemInfo& pi, const Panel& P, const WorkItem& w,
+                                        double mu, double* const (&cks)[2], int c0, const VecState* st,
+                                        TwistAt<kSums<Row, NW>>& W) {
+    constexpr int kN = kSums<Row, NW>;
+    const int lane = threadIdx.x & 31, nz = P.nz, M = pi.M, nc = (nz + kCkRows - 1) / kCkRows;
+    double* tmp = A.vfull + A.vfull_off[w.problem] + w.j0 + lane;
+    const VecState* sd = st + (long long)nc * M;
+    TwistKey K{0.0, 0, 0};
+    for (int c = max(c0 - 1, 0); c <= c0; ++c) {
+        const int a = c * kCkRows, end = min(nz, a + kCkRows);
+        VecState v{0.0, -1.0, 0, 0};
+        if (c + 1 < nc) v = sd[(long long)(c + 1) * M];
+        double u = v.u, e = v.e;
+        for (int i = end - 1; i >= a; --i) {
+            u -= e;
+            e = fma(Row::sigma(P.rows, i, mu), u, e);
+            tmp[(long long)i * M] = u;
+        }
+        const VecState q = st[(long long)c * M];
+        u = q.u;
+        e = q.e;
+        for (int i = a; i < end; ++i) {
+            K.take(u, q.E, tmp[(long long)i * M], v.E, i);
+            e = fma(-Row::sigma(P.rows, i, mu), u, e);
+            u += e;
+        }
+    }
+    if (K.m == 0.0) return;
+    const int c = K.c / kCkRows, a = c * kCkRows, end = min(nz, a + kCkRows);
+    const double* wp = A.w + pi.w_off;
+    const double* gp = NW > 1 && A.g ? A.g + pi.s_off : nullptr;
+    auto add = [&](double (&s)[kN], int i, double x) {
+        const double x2 = x * x;
+        if (Row::kUnitNorm) s[0] += x2;
+        s[kN - NW] = fma(wp[i], x2, s[kN - NW]);
+        if (NW > 1) s[kN - 1] = fma(gp ? gp[i] : 1.0, x2, s[kN - 1]);
+    };
+    W.r = K.c;
+    W.Eb = 0;
+#pragma unroll
+    for (int n = 0; n < kN; ++n) {
+        W.su[n] = cks[0][((size_t)c * (1 + kN) + 1 + n) * 32 + lane];
+        W.sb[n] = c + 1 < nc ? __ldcg(cks[1] + ((size_t)(c + 1) * (1 + kN) + 1 + n) * 32 + lane) : 0.0;
+    }
+    if (c + 1 < nc) W.Eb = sd[(long long)(c + 1) * M].E;
+    for (int i = end - 1; i >= W.r; --i) add(W.sb, i, W.b = tmp[(long long)i * M]);
+    const VecState q = st[(long long)c * M];
+    double u = q.u, e = q.e;
+    for (int i = a; i < W.r; ++i) {
+        add(W.su, i, u);
+        e = fma(-Row::sigma(P.rows, i, mu), u, e);
+        u += e;
+    }
+    W.u = u;
+    W.Eu = q.E;
+}
+
+template <class Row, int NW, bool kV>
 __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemInfo& pi, const Panel& P,
                                              const WorkItem& w, double mu, PRing& R, Pair& pr, double* __restrict__ ck,
                                              int* __restrict__ cke) {
@@ -1267,7 +1347,9 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
     int* ckes[2] = {cke, cke + A.ck_stride};
     double vs, vr;
     int Es, Er;
-    vector_half<Row, NW>(A, pi, P, mu, half, R, cks[half], ckes[half], vs, Es, vr, Er);
+    VecState* st = nullptr;
+    if (kV && lane < w.m) st = A.vstate + A.vstate_off[w.problem] + w.j0 + lane;
+    vector_half<Row, NW, kV>(A, pi, P, mu, half, st ? st + (long long)half * nc * pi.M : nullptr, R, cks[half], ckes[half], vs, Es, vr, Er);
     PairBox& X = *pr.box;
     const int tb = pr.turn, t2 = tb ^ 1;
     if (half) {
@@ -1299,23 +1381,37 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
     const double us = vs, ur = vr, bs = X.v[tb][1][0][lane], br = X.v[tb][1][1][lane];
     const double eb = X.v[tb][1][2][lane];
     const int Eus = Es, Eur = Er, Ebs = __double2hiint(eb), Ebr = __double2loint(eb);
+    TwistAt<kN> W;
+    W.r = K.c * kCkRows;
     const size_t o = (size_t)K.c * (1 + kN) * 32 + lane;
-    double ut = __ldcg(cks[0] + o), bt = __ldcg(cks[1] + o);
-    const int Eu0 = __ldcg(ckes[0] + (size_t)K.c * 32 + lane), Eb0 = __ldcg(ckes[1] + (size_t)K.c * 32 + lane);
-    int Eut = Eu0, Ebt = Eb0;
+    W.u = __ldcg(cks[0] + o);
+    W.b = __ldcg(cks[1] + o);
+    W.Eu = __ldcg(ckes[0] + (size_t)K.c * 32 + lane);
+    W.Eb = __ldcg(ckes[1] + (size_t)K.c * 32 + lane);
+#pragma unroll
+    for (int n = 0; n < kN; ++n) {
+        W.su[n] = __ldcg(cks[0] + o + 32 * (1 + n));
+        W.sb[n] = __ldcg(cks[1] + o + 32 * (1 + n));
+    }
+    if (kV && fine_twist_needed(pi)) {
+        if (lane < w.m) fine_twist<Row, NW>(A, pi, P, w, mu, cks, K.c, st, W);
+        __syncwarp();
+    }
+    double ut = W.u, bt = W.b;
+    int Eut = W.Eu, Ebt = W.Eb;
     normalize(ut, Eut);
     normalize(bt, Ebt);
-    const int eut = Eut - Eu0, ebt = Ebt - Eb0;  // exponents of u and b themselves
+    const int eut = Eut - W.Eu, ebt = Ebt - W.Eb;  // exponents of u and b themselves
     const double iu2 = 1.0 / (ut * ut), ib2 = 1.0 / (bt * bt);
     auto total = [&](int n) {  // sum over all rows in units of z_r^2
-        double x = __ldcg(cks[0] + o + 32 * (1 + n)), y = __ldcg(cks[1] + o + 32 * (1 + n));
+        double x = W.su[n], y = W.sb[n];
         int ex = 0, ey = 0;
         normalize(x, ex);
         normalize(y, ey);
         // both sums were taken at the exponents of u and b at the twist
         return x * iu2 * pow2(ex - 2 * eut) + y * ib2 * pow2(ey - 2 * ebt);
     };
-    const int r = K.c * kCkRows, isrc = pi.isrc, ircv = pi.ircv;
+    const int r = W.r, isrc = pi.isrc, ircv = pi.ircv;
     const int n1 = Row::kUnitNorm ? 0 : kN - 1, nw = kN - NW;
     const double nrm = total(n1);  // sum z^2 / z_r^2
     const double f2 = Row::kUnitNorm ? 1.0 : 1.0 / (1.0 + (mu / pi.dz) * (mu / pi.dz));
@@ -1331,6 +1427,7 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
         A.ki[i] = kp.imag();
         A.vs[i] = zs * scale;
         A.vr[i] = zr * scale;
+        if (kV) A.vtwist[i] = VecTwist{mu, scale / ut, scale / bt, Eut, Ebt, r, 0};
         if (Row::kUnitNorm && NW > 1) {
             const double vph = pi.omega / kp.real();
             A.vg[i] = 1.0 / (vph * (total(nw + 1) / nrm));
@@ -1345,7 +1442,7 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
 // values of the eigenvalues in mu, 3 both.  The pairs take items from the
 // cost-ordered list as they get free (sched: a zeroed counter), or round-robin.
 // ---------------------------------------------------------------------------
-template <class Row, int NW, int kDo>
+template <class Row, int NW, int kDo, bool kV>
 __global__ void __launch_bounds__(kPWarps * 32, kPanelCtas) k_panel_modes(ModesArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int kSl = kTD + NW * kWD;
@@ -1384,16 +1481,85 @@ __global__ void __launch_bounds__(kPWarps * 32, kPanelCtas) k_panel_modes(ModesA
         } else if (lane < w.m) {
             x = A.mu[pi.off + w.j0 + lane];
         }
-        if (kDo & 2) panel_vector<Row, NW>(A, pi, P, w, x, R, pr, ck, cke);
+        if (kDo & 2) panel_vector<Row, NW, kV>(A, pi, P, w, x, R, pr, ck, cke);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// full vectors: every mode at every row, from the states that the mode-value
+// pass left at the coarse rows: a warp takes 32 modes x kCkRows rows, up from
+// the lower state below the twist and down from the upper one above it (the
+// growing direction of either chain).  A first launch finds each mode's largest
+// |value|, where modes are positive; computing the values twice (2 FMAs each)
+// is cheaper than reading and turning them.  Bound by the writes (8 B a value),
+// which run along the modes as the rows are stored; a block of 128 rows is a
+// serial chain of about 2 us, with thousands of them in flight.
+// 0.3 Hz, 20000 rows: 31 us for both launches after 130 us of states (one kernel
+// before,
+// whose warps walked 32 modes up and down all rows, 3.8 ms)
+// ---------------------------------------------------------------------------
+template <class Row, bool kPeak>
+__global__ void __launch_bounds__(256) k_panel_fill(int p0, ModesArgs A) {
+    const int p = p0 + blockIdx.z;
+    const ProblemInfo& pi = A.pinfo[p];
+    const int M = pi.M, nz = pi.nz, nc = (nz + kCkRows - 1) / kCkRows;
+    const int c = blockIdx.y * 8 + (threadIdx.x >> 5), j = blockIdx.x * 32 + (threadIdx.x & 31);
+    if (c >= nc || j >= M) return;
+    const double* rows = A.rows + (size_t)pi.s_off * Row::kW;
+    const VecTwist t = A.vtwist[pi.off + j];
+    const VecState* st = A.vstate + A.vstate_off[p] + j;
+    unsigned long long* key = A.vpeak + pi.off + j;
+    const int a = c * kCkRows, end = min(nz, a + kCkRows);
+    double* out = A.vfull + A.vfull_off[p] + j;
+    double sg = 1.0, top = 0.0;  // top: the value of largest magnitude
+    if (!kPeak) {
+        sg = (*key & 1ull) ? -1.0 : 1.0;
+        if (c == 0 && sg < 0.0) {
+            A.vs[pi.off + j] = -A.vs[pi.off + j];
+            A.vr[pi.off + j] = -A.vr[pi.off + j];
+        }
+    }
+    auto put = [&](int i, double u) {
+        if (kPeak) top = fabs(u) > fabs(top) ? u : top;
+        else out[(long long)i * M] = u;
+    };
+    const int mid = min(max(t.r, a), end);  // rows from the twist on come from above
+    if (a < mid) {
+        const VecState v = st[(long long)c * M];
+        const double f = sg * t.fu * pow2(v.E - t.Eu);
+        double u = v.u * f, e = v.e * f;
+#pragma unroll 16
+        for (int i = a; i < mid; ++i) {
+            put(i, u);
+            e = fma(-Row::sigma(rows, i, t.mu), u, e);
+            u += e;
+        }
+    }
+    if (mid < end) {
+        VecState v{0.0, -1.0, 0, 0};
+        if (c + 1 < nc) v = st[(long long)(nc + c + 1) * M];
+        const double f = sg * t.fb * pow2(v.E - t.Eb);
+        double u = v.u * f, e = v.e * f;
+#pragma unroll 16
+        for (int i = end - 1; i >= mid; --i) {
+            u -= e;
+            e = fma(Row::sigma(rows, i, t.mu), u, e);
+            put(i, u);
+        }
+    }
+    if (kPeak) {  // magnitude, with the sign in the last bit
+        const unsigned long long b = (unsigned long long)__double_as_longlong(fabs(top));
+        atomicMax(key, (b & ~1ull) | (top < 0.0 ? 1ull : 0ull));
     }
 }
 
 template <class Row, int NW>
 int modes_launch(cudaStream_t st, int grid, const ModesArgs& a, int what) {
     const size_t sm = kRingBytes<kTD + NW * kWD> + (kPWarps / 2) * sizeof(PairBox);
-    void (*f)(ModesArgs) = what == 1   ? k_panel_modes<Row, NW, 1>
-                           : what == 2 ? k_panel_modes<Row, NW, 2>
-                                       : k_panel_modes<Row, NW, 3>;
+    const bool v = a.vstate != nullptr;
+    void (*f)(ModesArgs) = what == 1   ? k_panel_modes<Row, NW, 1, false>
+                           : what == 2 ? (v ? k_panel_modes<Row, NW, 2, true> : k_panel_modes<Row, NW, 2, false>)
+                                       : (v ? k_panel_modes<Row, NW, 3, true> : k_panel_modes<Row, NW, 3, false>);
     cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     f<<<grid, kPWarps * 32, sm, st>>>(a);
     return 1;
@@ -1546,6 +1712,18 @@ int launch_panel_expand(cudaStream_t st, int n_desc, int nz_max, const ProblemIn
                         const double* s, const double* w, const double* g, double* T, double* W0, double* W1) {
     return g ? expand_launch<EssPanel, 2>(st, n_desc, nz_max, pinfo, desc, s, w, g, T, W0, W1)
              : expand_launch<EssPanel, 1>(st, n_desc, nz_max, pinfo, desc, s, w, nullptr, T, W0, nullptr);
+}
+
+int launch_panel_fill(cudaStream_t st, int P, int nz_max, int m_max, const ModesArgs& a) {
+    int n = 0;
+    const int ny = ((nz_max + kCkRows - 1) / kCkRows + 7) / 8;
+    for (int p0 = 0; p0 < P && m_max > 0; p0 += 32768) {
+        const dim3 grid((m_max + 31) / 32, ny, std::min(P - p0, 32768));
+        k_panel_fill<EssPanel, true><<<grid, 256, 0, st>>>(p0, a);
+        k_panel_fill<EssPanel, false><<<grid, 256, 0, st>>>(p0, a);
+        n += 2;
+    }
+    return n;
 }
 
 int launch_panel_modes(cudaStream_t st, int grid, const ModesArgs& a, int what) {
