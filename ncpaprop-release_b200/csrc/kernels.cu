@@ -6,18 +6,14 @@
 //  K1  matrix build on the Nz grid (ESSModeSolver::getModalTrace,
 //      ESSModeSolver.cpp:531-559; EigenEngine.cpp:57-83 assembly)
 //  K2  WKB window (ESSModeSolver.cpp:561-621)
-//  K3  Sturm isolation scan + multisection/bisection (replaces the SLEPc
-//      spectrum slice of EigenEngine::doESSCalculation, EigenEngine.cpp:10-172)
-//  K4  twisted-factorisation eigenvectors with the perturbative attenuation
-//      and group-speed integrals fused in (ModeSolver::doPerturb,
-//      ModeSolver.cpp:263-284; ESSModeSolver.cpp:738-744)
+//  K3, K4  eigenvalues and mode values: panel.cu (here only the mode values of
+//      the calls without allocations, K4s)
 //  K5  modal sums for 1-D / 2-D transmission loss (ModeSolver.cpp:292-565)
 //  K6  ModBB transfer function + pulse synthesis
 //      (ModalBroadbandPropagator.cpp:245-277, BroadbandPropagator.cpp:327-662)
 #include <algorithm>
 
 #include "device_common.cuh"
-#include "item_sched.cuh"
 #include "kernels.hpp"
 
 #include <cuda/std/complex>
@@ -558,971 +554,6 @@ int launch_window(cudaStream_t st, int P, ProblemInfo* pinfo, const double* kz2,
     return n;
 }
 
-// K3a-1: the size of each problem's isolation scan.  The number of
-// eigenvalues of S (diagonal s_i, unit off-diagonals) below x is close to the
-// sum over the rows of theta_i / pi with cos theta_i = (s_i - x) / 2 clipped
-// to [-1, 1] (each row's local band is [s_i - 2, s_i + 2]); on the 20000-point
-// grids of 0.002-0.5 Hz it gives the mode count in [lo, hi] within one mode.
-// The scan takes about two shifts per mode plus 32, in steps of 64 (one scan
-// unit), between 64 and kScanMax: problems with many close
-// eigenvalues start their bisection better isolated, those with few stop
-// paying for shifts that isolate nothing.
-constexpr int kSizeThreads = 256;
-__global__ void __launch_bounds__(kSizeThreads) k_scan_size(ProblemInfo* __restrict__ pinfo,
-                                                           const double* __restrict__ s) {
-    __shared__ float part[kSizeThreads / 32];
-    const int p = blockIdx.x;
-    const ProblemInfo pi = pinfo[p];
-    const double* row = s + pi.s_off;
-    float acc = 0.f;
-    for (int i = threadIdx.x; i < pi.nz; i += kSizeThreads) {
-        const double v = row[i];
-        const float ch = fminf(fmaxf((float)((v - pi.hi) * 0.5), -1.f), 1.f);
-        const float cl = fminf(fmaxf((float)((v - pi.lo) * 0.5), -1.f), 1.f);
-        acc += acosf(ch) - acosf(cl);
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.f;
-        for (int w = 0; w < kSizeThreads / 32; ++w) t += part[w];
-        const float m_est = fmaxf(t * (float)(1.0 / kPi), 0.f);
-        const int n = ((int)(2.f * m_est) + 32 + kScanStep - 1) / kScanStep * kScanStep;
-        pinfo[p].n_scan = min(max(n, kScanStep), kScanMax);
-        pinfo[p].n_scan_raw = pinfo[p].n_scan;
-        pinfo[p].m_est = m_est;
-    }
-}
-
-// K3: per-warp multisection + safeguarded Newton.
-//
-// Each warp owns a work item of m <= 32 consecutive eigen-indices of one
-// problem (lane l owns eigenvalue slot l: bracket [a, b] with the Sturm counts
-// at its ends, Newton iterate x, mode) and streams that problem's diagonal
-// through its own TMA ring in shared memory (kWBuf chunks of kWChunk doubles,
-// one mbarrier per slot), so warps never wait on each other.  Each lane runs
-// up to two Sturm chains (virtual lanes v = lane, lane + 32).  Every round:
-//  * eigenvalues isolated in their bracket (Sturm counts J and J + 1 at its
-//    ends) take a safeguarded Newton step on det(S - x): one virtual lane
-//    (chain 0) carries the x-derivative of the recurrence; the Sturm count at
-//    the iterate shrinks the bracket and a step leaving the bracket falls back
-//    to its midpoint.  An eigenvalue is final when the correction is below
-//    tol, or when two Newton steps in a row stayed inside the bracket, the
-//    correction shrank at least fourfold and the quadratic-convergence model
-//    predicts the next one below tol (|d_k|^3 <= tol |d_{k-1}|^2), which
-//    saves the sweep that would only confirm it;
-//  * the other virtual lanes are dealt round-robin over the eigenvalues not
-//    yet isolated (G_e lanes each), which cut their bracket into G_e + 1
-//    pieces.  Rounds with Newton slots only sweep a single chain.
-constexpr int kWChunk = 512;
-constexpr int kWBuf = 3;
-constexpr int kWarpsPerCta = 4;
-
-struct WarpRing {
-    double* buf;     // [kWBuf][kWChunk]
-    uint64_t* bars;  // [kWBuf]
-    unsigned loads;  // identical in all lanes
-};
-
-__device__ __forceinline__ void wring_issue(WarpRing& r, unsigned k, const double* src) {
-    const int slot = k % kWBuf;
-    mbar_expect_tx(&r.bars[slot], kWChunk * 8);
-    tma_load_1d(r.buf + slot * kWChunk, src, kWChunk * 8, &r.bars[slot]);
-}
-
-// position of the n-th (0-based) set bit of m
-__device__ __forceinline__ int nth_bit(unsigned m, int n) {
-    int pos = 0;
-#pragma unroll
-    for (int sh = 16; sh >= 1; sh >>= 1) {
-        const unsigned low = m & ((1u << sh) - 1u);
-        const int c = __popc(low);
-        if (n >= c) {
-            n -= c;
-            m >>= sh;
-            pos += sh;
-        } else {
-            m = low;
-        }
-    }
-    return pos;
-}
-
-// One sweep over the rows (Row format; kWChunk doubles per ring chunk, so
-// kWChunk / Row::kW rows).  mode 0: chains A and B, counts only; 1: chain A
-// with derivative(s) + chain B; 2: chain A with derivative(s) only.  p_init
-// starts both chains (Row::p_init).  For Newton rows rat0 is chain A's Newton
-// correction; for Laguerre rows (Row::kLaguerre) chain A also carries the
-// second derivative and rat0 = det'/det, h0 = rat0^2 - det''/det.
-template <class Row>
-__device__ void warp_sweep(const double* __restrict__ s, int nz, double p_init, double x0, double x1, int mode,
-                           WarpRing& r, unsigned* err, int& c0, int& c1, double& rat0, double& h0) {
-    constexpr int kW = Row::kW;
-    constexpr int kRows = kWChunk / kW;
-    const int lane = threadIdx.x & 31;
-    const int nch = (nz + kRows - 1) / kRows;
-    const unsigned base = r.loads;
-    if (lane == 0)
-        for (int c = 0; c < nch && c < kWBuf; ++c) wring_issue(r, base + c, s + (size_t)c * kWChunk);
-    __syncwarp();
-    SturmState A, B;
-    A.reset();
-    B.reset();
-    if (kW != 1) {
-        A.p0 = p_init;
-        B.p0 = p_init;
-    }
-    double da0 = 0.0, da1 = 0.0, ea0 = 0.0, ea1 = 0.0;
-    for (int c = 0; c < nch; ++c) {
-        const unsigned k = base + c;
-        const int slot = k % kWBuf;
-        mbar_wait_bounded(&r.bars[slot], (k / kWBuf) & 1u, err);
-        const double* b = r.buf + slot * kWChunk;
-        const int valid = min(kRows, nz - c * kRows);
-        const int nw = valid >> 5;
-        if (mode == 0) {
-            for (int w = 0; w < nw; ++w) Row::pair(A, B, b + 32 * kW * w, x0, x1);
-            for (int i = nw * 32; i < valid; ++i) {
-                Row::step(A, b, i, x0);
-                Row::step(B, b, i, x1);
-            }
-        } else if constexpr (Row::kLaguerre) {
-            if (mode == 1) {
-                for (int w = 0; w < nw; ++w) Row::deriv2_pair(A, da0, da1, ea0, ea1, B, b + 32 * kW * w, x0, x1);
-                for (int i = nw * 32; i < valid; ++i) {
-                    Row::step_deriv2(A, b, i, x0, da0, da1, ea0, ea1);
-                    Row::step(B, b, i, x1);
-                }
-            } else {
-                for (int w = 0; w < nw; ++w) Row::word_deriv2(A, b + 32 * kW * w, x0, da0, da1, ea0, ea1);
-                for (int i = nw * 32; i < valid; ++i) Row::step_deriv2(A, b, i, x0, da0, da1, ea0, ea1);
-            }
-        } else if (mode == 1) {
-            for (int w = 0; w < nw; ++w) Row::deriv_pair(A, da0, da1, B, b + 32 * kW * w, x0, x1);
-            for (int i = nw * 32; i < valid; ++i) {
-                Row::step_deriv(A, b, i, x0, da0, da1);
-                Row::step(B, b, i, x1);
-            }
-        } else {
-            for (int w = 0; w < nw; ++w) Row::word_deriv(A, b + 32 * kW * w, x0, da0, da1);
-            for (int i = nw * 32; i < valid; ++i) Row::step_deriv(A, b, i, x0, da0, da1);
-        }
-        __syncwarp();
-        if (lane == 0 && c + kWBuf < nch) {
-            fence_proxy_async();
-            wring_issue(r, base + c + kWBuf, s + (size_t)(c + kWBuf) * kWChunk);
-        }
-    }
-    r.loads = base + nch;
-    c0 = A.cnt;
-    c1 = B.cnt;
-    h0 = 0.0;
-    if constexpr (Row::kLaguerre) {
-        rat0 = mode >= 1 ? da1 / A.p1 : 0.0;
-        h0 = mode >= 1 ? fma(rat0, rat0, -(ea1 / A.p1)) : 0.0;
-    } else {
-        rat0 = mode >= 1 ? Row::newton(A.p1, da1) : 0.0;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Twisted Sturm sweep.  The rows [0, h) run the forward recurrence p
-// (top-down) and the rows [h, n) the backward recurrence q (bottom-up,
-// q_n = 1, q_{n+1} = 0) at the same time, so each chain is half as long and a
-// lane carries twice the independent chains.  With the twist at row h
-// (T - x = N Delta N^T, Delta = diag(D+_0..D+_{h-1}, gamma_h, D-_{h+1}..)):
-//   count = sign changes of p_{-1..h-1} + sign changes of q_{n..h+1}
-//           + [gamma_h < 0],  gamma_h = det / (p_{h-1} q_{h+1}),
-//   det = p_{h-1} q_h - p_{h-2} q_{h+1},
-// and det' follows by the product rule from the chains' derivatives.  The
-// inertia is that of the sequential count; the scan's counts, which fix the
-// mode numbers, stay sequential.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned sgnbit(double v) { return static_cast<unsigned>(__double2hiint(v)) >> 31; }
-
-// count of the twisted factorisation from the final forward chain F and
-// backward chain B (B.p1 = q_h, B.p0 = q_{h+1}); det returned
-__device__ __forceinline__ int twist_count(const SturmState& F, const SturmState& B, double& det) {
-    det = F.p1 * B.p1 - F.p0 * B.p0;
-    const int last = static_cast<int>(sgnbit(B.p1) ^ sgnbit(B.p0));
-    const int gam = static_cast<int>(sgnbit(det) ^ sgnbit(F.p1) ^ sgnbit(B.p0));
-    return F.cnt + B.cnt - last + gam;
-}
-
-// 32 front rows (ascending, fb) and 32 back rows (descending, bb) in one
-// loop.  kMode 0: four count chains (A, B forward and backward); 1: A chains
-// with derivatives + B chains; 2: A chains with derivatives only.  With kMode
-// >= 1 the A chains also carry second derivatives (fe, be: Laguerre steps).
-template <int kMode>
-__device__ __forceinline__ void tw_word(EssRows, SturmState& Af, SturmState& Bf, SturmState& Ab, SturmState& Bb,
-                                        double& fd0, double& fd1, double& bd0, double& bd1, double& fe0,
-                                        double& fe1, double& be0, double& be1, const double* __restrict__ fb,
-                                        const double* __restrict__ bb, double xa, double xb) {
-    unsigned waf = 0u, wbf = 0u, wab = 0u, wbb = 0u;
-    double af0 = Af.p0, af1 = Af.p1, ab0 = Ab.p0, ab1 = Ab.p1;
-    double bf0 = Bf.p0, bf1 = Bf.p1, bb0 = Bb.p0, bb1 = Bb.p1;
-#pragma unroll
-    for (int u = 0; u < 32; u += 2) {
-        const double2 f = *reinterpret_cast<const double2*>(fb + u);
-        const double2 g = *reinterpret_cast<const double2*>(bb + 30 - u);
-        // front row u, back row 31 - u
-        const double ta = f.x - xa, ua = g.y - xa;
-        const double qaf = fma(ta, af1, -af0), qab = fma(ua, ab1, -ab0);
-        if (kMode >= 1) {
-            const double ef = fma(ta, fd1, -(af1 + fd0)), eb = fma(ua, bd1, -(ab1 + bd0));
-            const double gf = fma(ta, fe1, -fma(2.0, fd1, fe0)), gb = fma(ua, be1, -fma(2.0, bd1, be0));
-            fd0 = fd1;
-            fd1 = ef;
-            bd0 = bd1;
-            bd1 = eb;
-            fe0 = fe1;
-            fe1 = gf;
-            be0 = be1;
-            be1 = gb;
-        }
-        waf = __funnelshift_l(__double2hiint(qaf), waf, 1);
-        wab = __funnelshift_l(__double2hiint(qab), wab, 1);
-        af0 = af1;
-        af1 = qaf;
-        ab0 = ab1;
-        ab1 = qab;
-        if (kMode <= 1) {
-            const double qbf = fma(f.x - xb, bf1, -bf0), qbb = fma(g.y - xb, bb1, -bb0);
-            wbf = __funnelshift_l(__double2hiint(qbf), wbf, 1);
-            wbb = __funnelshift_l(__double2hiint(qbb), wbb, 1);
-            bf0 = bf1;
-            bf1 = qbf;
-            bb0 = bb1;
-            bb1 = qbb;
-        }
-        // front row u + 1, back row 30 - u
-        const double ta2 = f.y - xa, ua2 = g.x - xa;
-        const double qaf2 = fma(ta2, af1, -af0), qab2 = fma(ua2, ab1, -ab0);
-        if (kMode >= 1) {
-            const double ef = fma(ta2, fd1, -(af1 + fd0)), eb = fma(ua2, bd1, -(ab1 + bd0));
-            const double gf = fma(ta2, fe1, -fma(2.0, fd1, fe0)), gb = fma(ua2, be1, -fma(2.0, bd1, be0));
-            fd0 = fd1;
-            fd1 = ef;
-            bd0 = bd1;
-            bd1 = eb;
-            fe0 = fe1;
-            fe1 = gf;
-            be0 = be1;
-            be1 = gb;
-        }
-        waf = __funnelshift_l(__double2hiint(qaf2), waf, 1);
-        wab = __funnelshift_l(__double2hiint(qab2), wab, 1);
-        af0 = af1;
-        af1 = qaf2;
-        ab0 = ab1;
-        ab1 = qab2;
-        if (kMode <= 1) {
-            const double qbf = fma(f.y - xb, bf1, -bf0), qbb = fma(g.x - xb, bb1, -bb0);
-            wbf = __funnelshift_l(__double2hiint(qbf), wbf, 1);
-            wbb = __funnelshift_l(__double2hiint(qbb), wbb, 1);
-            bf0 = bf1;
-            bf1 = qbf;
-            bb0 = bb1;
-            bb1 = qbb;
-        }
-    }
-    Af.p0 = af0;
-    Af.p1 = af1;
-    Ab.p0 = ab0;
-    Ab.p1 = ab1;
-    if (kMode >= 1) {
-        sturm_fold_deriv2(Af, waf, fd0, fd1, fe0, fe1);
-        sturm_fold_deriv2(Ab, wab, bd0, bd1, be0, be1);
-    } else {
-        sturm_fold(Af, waf);
-        sturm_fold(Ab, wab);
-    }
-    if (kMode <= 1) {
-        Bf.p0 = bf0;
-        Bf.p1 = bf1;
-        Bb.p0 = bb0;
-        Bb.p1 = bb1;
-        sturm_fold(Bf, wbf);
-        sturm_fold(Bb, wbb);
-    }
-}
-
-template <int kMode>
-__device__ __forceinline__ void tw_word(WmodRows, SturmState& Af, SturmState& Bf, SturmState& Ab, SturmState& Bb,
-                                        double& fd0, double& fd1, double& bd0, double& bd1, double&, double&, double&,
-                                        double&, const double* __restrict__ fb, const double* __restrict__ bb,
-                                        double xa, double xb) {
-    const double ca = fma(-xa, xa, -2.0), cb = fma(-xb, xb, -2.0);
-    unsigned waf = 0u, wbf = 0u, wab = 0u, wbb = 0u;
-    double af0 = Af.p0, af1 = Af.p1, ab0 = Ab.p0, ab1 = Ab.p1;
-    double bf0 = Bf.p0, bf1 = Bf.p1, bb0 = Bb.p0, bb1 = Bb.p1;
-#pragma unroll
-    for (int u = 0; u < 32; ++u) {
-        const double2 f = *reinterpret_cast<const double2*>(fb + 2 * u);
-        const double2 g = *reinterpret_cast<const double2*>(bb + 2 * (31 - u));
-        const double df = fma(-f.y, xa, f.x), dg = fma(-g.y, xa, g.x);
-        const double ta = fma(df, df, ca), ua = fma(dg, dg, ca);
-        const double qaf = fma(ta, af1, -af0), qab = fma(ua, ab1, -ab0);
-        if (kMode >= 1) {
-            const double ef = fma(ta, fd1, fma(fma(f.y, df, xa), af1, -fd0));
-            const double eb = fma(ua, bd1, fma(fma(g.y, dg, xa), ab1, -bd0));
-            fd0 = fd1;
-            fd1 = ef;
-            bd0 = bd1;
-            bd1 = eb;
-        }
-        waf = __funnelshift_l(__double2hiint(qaf), waf, 1);
-        wab = __funnelshift_l(__double2hiint(qab), wab, 1);
-        af0 = af1;
-        af1 = qaf;
-        ab0 = ab1;
-        ab1 = qab;
-        if (kMode <= 1) {
-            const double dbf = fma(-f.y, xb, f.x), dbb = fma(-g.y, xb, g.x);
-            const double qbf = fma(fma(dbf, dbf, cb), bf1, -bf0), qbb = fma(fma(dbb, dbb, cb), bb1, -bb0);
-            wbf = __funnelshift_l(__double2hiint(qbf), wbf, 1);
-            wbb = __funnelshift_l(__double2hiint(qbb), wbb, 1);
-            bf0 = bf1;
-            bf1 = qbf;
-            bb0 = bb1;
-            bb1 = qbb;
-        }
-    }
-    Af.p0 = af0;
-    Af.p1 = af1;
-    Ab.p0 = ab0;
-    Ab.p1 = ab1;
-    if (kMode >= 1) {
-        sturm_fold_deriv(Af, waf, fd0, fd1);
-        sturm_fold_deriv(Ab, wab, bd0, bd1);
-    } else {
-        sturm_fold(Af, waf);
-        sturm_fold(Ab, wab);
-    }
-    if (kMode <= 1) {
-        Bf.p0 = bf0;
-        Bf.p1 = bf1;
-        Bb.p0 = bb0;
-        Bb.p1 = bb1;
-        sturm_fold(Bf, wbf);
-        sturm_fold(Bb, wbb);
-    }
-}
-
-// one twisted sweep in mode kMode (see warp_sweep); each ring slot holds a
-// front part and a back part of kWChunk / 2 doubles
-template <class Row, int kMode>
-__device__ void warp_sweep_tw_mode(const double* __restrict__ s, int nz, double p_init, double x0, double x1,
-                                   WarpRing& r, unsigned* err, int& c0, int& c1, double& rat0, double& h0) {
-    constexpr int kW = Row::kW;
-    constexpr int kHD = kWChunk / 2;  // doubles per part
-    constexpr int kHR = kHD / kW;     // rows per part
-    constexpr int kHW = kHR / 32;     // 32-row words per part
-    const int lane = threadIdx.x & 31;
-    const int nparts = (nz + kHR - 1) / kHR;
-    const int nf = (nparts + 1) / 2, nb = nparts - nf;  // front parts 0..nf-1, back parts nparts-1 .. nf
-    const unsigned base = r.loads;
-    auto issue = [&](unsigned k, int j) {
-        const int slot = k % kWBuf;
-        mbar_expect_tx(&r.bars[slot], (j < nb ? 2 : 1) * kHD * 8);
-        tma_load_1d(r.buf + slot * kWChunk, s + (size_t)j * kHD, kHD * 8, &r.bars[slot]);
-        if (j < nb)
-            tma_load_1d(r.buf + slot * kWChunk + kHD, s + (size_t)(nparts - 1 - j) * kHD, kHD * 8, &r.bars[slot]);
-    };
-    if (lane == 0)
-        for (int j = 0; j < nf && j < kWBuf; ++j) issue(base + j, j);
-    __syncwarp();
-    SturmState Af, Bf, Ab, Bb;
-    Af.reset();
-    Bf.reset();
-    Ab.reset();
-    Bb.reset();
-    if (kW != 1) {
-        Af.p0 = p_init;
-        Bf.p0 = p_init;
-    }
-    double fd0 = 0.0, fd1 = 0.0, bd0 = 0.0, bd1 = 0.0, fe0 = 0.0, fe1 = 0.0, be0 = 0.0, be1 = 0.0;
-    for (int j = 0; j < nf; ++j) {
-        const unsigned k = base + j;
-        const int slot = k % kWBuf;
-        mbar_wait_bounded(&r.bars[slot], (k / kWBuf) & 1u, err);
-        const double* fb = r.buf + slot * kWChunk;
-        const double* bb = fb + kHD;
-        int nwb = 0;
-        if (j < nb) {
-            const int valid_b = min(kHR, nz - (nparts - 1 - j) * kHR);
-            nwb = valid_b >> 5;
-            for (int i = valid_b - 1; i >= nwb * 32; --i) {  // ragged top of the last part, descending
-                if (kMode >= 1) {
-                    if constexpr (Row::kLaguerre) Row::step_deriv2(Ab, bb, i, x0, bd0, bd1, be0, be1);
-                    else Row::step_deriv(Ab, bb, i, x0, bd0, bd1);
-                } else {
-                    Row::step(Ab, bb, i, x0);
-                }
-                if (kMode <= 1) Row::step(Bb, bb, i, x1);
-            }
-            for (int w = 0; w < nwb; ++w)
-                tw_word<kMode>(Row{}, Af, Bf, Ab, Bb, fd0, fd1, bd0, bd1, fe0, fe1, be0, be1, fb + 32 * kW * w,
-                               bb + 32 * kW * (nwb - 1 - w), x0, x1);
-        }
-        for (int w = nwb; w < kHW; ++w) {  // front words without a back partner
-            if (kMode == 0) {
-                Row::pair(Af, Bf, fb + 32 * kW * w, x0, x1);
-            } else if constexpr (Row::kLaguerre) {
-                if (kMode == 1) Row::deriv2_pair(Af, fd0, fd1, fe0, fe1, Bf, fb + 32 * kW * w, x0, x1);
-                else Row::word_deriv2(Af, fb + 32 * kW * w, x0, fd0, fd1, fe0, fe1);
-            } else {
-                if (kMode == 1) Row::deriv_pair(Af, fd0, fd1, Bf, fb + 32 * kW * w, x0, x1);
-                else Row::word_deriv(Af, fb + 32 * kW * w, x0, fd0, fd1);
-            }
-        }
-        __syncwarp();
-        if (lane == 0 && j + kWBuf < nf) {
-            fence_proxy_async();
-            issue(base + j + kWBuf, j + kWBuf);
-        }
-    }
-    r.loads = base + nf;
-    double det;
-    c0 = twist_count(Af, Ab, det);
-    c1 = 0;
-    if (kMode <= 1) {
-        double detb;
-        c1 = twist_count(Bf, Bb, detb);
-    }
-    rat0 = 0.0;
-    h0 = 0.0;
-    if (kMode >= 1) {
-        // det = F1 B1 - F0 B0 (F the forward chain p_{h-1}, p_{h-2}; B the
-        // backward chain q_h, q_{h+1}); derivatives by the product rule
-        const double dd = fd1 * Ab.p1 + Af.p1 * bd1 - fd0 * Ab.p0 - Af.p0 * bd0;
-        if constexpr (Row::kLaguerre) {
-            const double d2 = fe1 * Ab.p1 + 2.0 * fd1 * bd1 + Af.p1 * be1 -
-                              (fe0 * Ab.p0 + 2.0 * fd0 * bd0 + Af.p0 * be0);
-            rat0 = dd / det;
-            h0 = fma(rat0, rat0, -(d2 / det));
-        } else {
-            rat0 = Row::newton(det, dd);
-        }
-    }
-}
-
-// the twisted sweep; grids of one part (nz <= kWChunk / 2 / kW rows) run the
-// sequential sweep
-template <class Row>
-__device__ void warp_sweep_tw(const double* __restrict__ s, int nz, double p_init, double x0, double x1, int mode,
-                              WarpRing& r, unsigned* err, int& c0, int& c1, double& rat0, double& h0) {
-    if (!Row::kTwist || nz <= kWChunk / 2 / Row::kW) {
-        warp_sweep<Row>(s, nz, p_init, x0, x1, mode, r, err, c0, c1, rat0, h0);
-        return;
-    }
-    if (mode == 0) warp_sweep_tw_mode<Row, 0>(s, nz, p_init, x0, x1, r, err, c0, c1, rat0, h0);
-    else if (mode == 1) warp_sweep_tw_mode<Row, 1>(s, nz, p_init, x0, x1, r, err, c0, c1, rat0, h0);
-    else warp_sweep_tw_mode<Row, 2>(s, nz, p_init, x0, x1, r, err, c0, c1, rat0, h0);
-}
-
-// K3a-2: the isolation scan in units of kScanStep shifts, numbered over the
-// problems in order (problem p has n_scan_raw / kScanStep units, less the
-// trim below).  A warp sweeps a unit (warp_sweep: the sequential count, two
-// shifts per lane) through its own ring; it finds the unit's problem with a
-// warp-wide prefix sum of the units per problem, 32 problems at a time.
-// Every unit is the same work; k_scan says which warp takes which unit.  Trim: with slots > 0 (the device's warp
-// schedulers) and U units in all, the batch drops U mod slots units when that
-// is at most a quarter of U, so each scheduler sweeps the same whole number of
-// units: one unit each from the first problems (in order) that keep at least
-// 1.75 shifts per estimated mode.  Every warp computes the same trim from the
-// raw sizes; the warp that sweeps a problem's first unit records the final
-// size in n_scan for the kernels that follow.
-__device__ __forceinline__ bool scan_trimmable(const ProblemInfo& q) {
-    const int u = q.n_scan_raw / kScanStep;
-    return u >= 2 && q.m_est >= 0.f && (float)((u - 1) * kScanStep) >= 1.75f * q.m_est;
-}
-
-// unit u of the (trimmed) scan: its problem p, first shift tb and the
-// problem's scan size n; p = -1 past the last unit.  Every warp lane takes
-// part (warp-wide prefix sums over the problems, 32 at a time).
-__device__ void scan_unit(int P, const ProblemInfo* pinfo, int remove, long long u, int& p, int& tb, int& n) {
-    const int lane = threadIdx.x & 31;
-    long long before = 0;  // units of the problems before the current block of 32
-    int trimmed = 0;       // trimmable problems before the current block of 32
-    p = -1;
-    tb = n = 0;
-    for (int base = 0; base < P && p < 0; base += 32) {
-        const int q = base + lane;
-        int units = 0, tr = 0;
-        if (q < P) {
-            const ProblemInfo& pq = pinfo[q];
-            units = pq.n_scan_raw / kScanStep;
-            tr = remove > 0 && scan_trimmable(pq) ? 1 : 0;
-        }
-        int tincl = tr;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, tincl, off);
-            if (lane >= off) tincl += v;
-        }
-        if (tr && trimmed + tincl - 1 < remove) --units;
-        trimmed += __shfl_sync(0xffffffffu, tincl, 31);
-        int incl = units;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, off);
-            if (lane >= off) incl += v;
-        }
-        const bool mine = u >= before + incl - units && u < before + incl;
-        const unsigned hit = __ballot_sync(0xffffffffu, mine);
-        if (hit) {
-            const int src = __ffs(hit) - 1;
-            const int excl = __shfl_sync(0xffffffffu, incl - units, src);
-            p = base + src;
-            tb = (int)(u - before - excl) * kScanStep;
-            n = __shfl_sync(0xffffffffu, units, src) * kScanStep;
-        }
-        before += __shfl_sync(0xffffffffu, incl, 31);
-    }
-}
-
-// With sched (kSchedInts ints, zeroed), the units are claimed through the
-// bisection's item scheduler: on each warp scheduler the first
-// ceil(units / slots) warps to arrive take units until none are left, so
-// every scheduler sweeps the same number of units wherever the CTAs land
-// (launch slots CTAs: the whole grid resident).  Without it, warp w of the
-// grid sweeps unit w.
-__global__ void __launch_bounds__(kWarpsPerCta * 32) k_scan(int P, ProblemInfo* pinfo, const double* __restrict__ s,
-                                                           int* __restrict__ counts, unsigned* err, int slots,
-                                                           int* sched) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int remove = 0;  // units the trim takes off (one per trimmable problem)
-    int U = 0, E = 0;
-    for (int q = lane; q < P; q += 32) {
-        U += pinfo[q].n_scan_raw / kScanStep;
-        E += scan_trimmable(pinfo[q]) ? 1 : 0;
-    }
-    U = __reduce_add_sync(0xffffffffu, U);
-    E = __reduce_add_sync(0xffffffffu, E);
-    if (slots > 0) {
-        const int rem = U % slots;
-        if (U >= slots && 4 * rem <= U) remove = rem;
-    }
-    const int total = U - min(remove, E);  // the units after the trim
-    WarpRing r;
-    r.buf = reinterpret_cast<double*>(smem_raw) + (size_t)wid * kWBuf * kWChunk;
-    r.bars = reinterpret_cast<uint64_t*>(smem_raw + (size_t)kWarpsPerCta * kWBuf * kWChunk * 8) + wid * kWBuf;
-    r.loads = 0;
-    bool ring_ready = false;
-    ItemSched sc(slots > 0 ? sched : nullptr, slots > 0 ? max(1, (total + slots - 1) / slots) : 1);
-    long long walk = (long long)blockIdx.x * kWarpsPerCta + wid;
-    for (long long u; (u = sc.next(total, walk, (long long)gridDim.x * kWarpsPerCta)) >= 0;) {
-        int p, tb, n;
-        scan_unit(P, pinfo, remove, u, p, tb, n);
-        if (p < 0) continue;  // past the last unit (warp-uniform)
-        if (tb == 0 && lane == 0) pinfo[p].n_scan = n;
-        if (!ring_ready) {
-            if (lane == 0) {
-                for (int k = 0; k < kWBuf; ++k) mbar_init(&r.bars[k], 1);
-                fence_mbar_init();
-            }
-            __syncwarp();
-            ring_ready = true;
-        }
-        const double lo = pinfo[p].lo, hi = pinfo[p].hi;
-        const long long s_off = pinfo[p].s_off;
-        const int nz = pinfo[p].nz;
-        const int t0 = tb + 2 * lane, t1 = t0 + 1;
-        int c0, c1;
-        double rat, hq;
-        warp_sweep<EssRows>(s + s_off, nz, 0.0, scan_x(lo, hi, t0, n), scan_x(lo, hi, t1, n), 0, r, err, c0, c1,
-                            rat, hq);
-        counts[(size_t)p * kScanMax + t0] = c0;
-        counts[(size_t)p * kScanMax + t1] = c1;
-        __syncwarp();
-        if (lane == 0) fence_proxy_async();  // the ring's buffers are refilled by the next unit's copies
-        __syncwarp();
-    }
-}
-
-int launch_scan(cudaStream_t st, int P, ProblemInfo* pinfo, const double* s, int* counts, unsigned* err,
-                int slots, int* sched) {
-    k_scan_size<<<P, kSizeThreads, 0, st>>>(pinfo, s);
-    const size_t sm = (size_t)kWarpsPerCta * (kWBuf * kWChunk * 8 + kWBuf * 8);
-    const long long units = (long long)P * (kScanMax / kScanStep);
-    cudaFuncSetAttribute(k_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    // claimed units: one CTA per slot (4 per SM, the whole grid resident)
-    const long long grid = (sched && slots > 0) ? slots : (units + kWarpsPerCta - 1) / kWarpsPerCta;
-    k_scan<<<(unsigned)grid, kWarpsPerCta * 32, sm, st>>>(P, pinfo, s, counts, err, slots, sched);
-    return 2;
-}
-
-// One bisection work item (<= 32 eigenvalues of one problem) on this warp,
-// with its TMA ring r: the eigenvalues to mu in the row format's units.
-template <class Row>
-__device__ __forceinline__ void bisect_item(const ProblemInfo* __restrict__ pinfo, const double* __restrict__ s,
-                                            const int* __restrict__ counts, const WorkItem w, double tol_in,
-                                            double* __restrict__ mu, unsigned* err,
-                                            unsigned long long* step_counter, WarpRing& r) {
-    const int lane = threadIdx.x & 31;
-    const ProblemInfo pi = pinfo[w.problem];
-    const int* cnt = counts + (size_t)w.problem * kScanMax;
-    const double* sp = s + (size_t)pi.s_off * Row::kW;
-    const int nz = pi.nz;
-    const double lo = Row::scan_lo(pi), hi = Row::scan_hi(pi);
-    const double tol = tol_in * Row::tol_scale(pi);
-    const double p_init = Row::p_init(pi);
-    // state of eigen slot `lane`
-    const int J = pi.c_lo + w.j0 + lane;
-    double a = lo, b = lo, x = lo;
-    double dprev = 0.0;  // size of the previous Newton correction (0: none yet)
-    int ca = 0, cb = 0, mode = 2;
-    if (lane < w.m) {  // initial bracket from the isolation scan
-        int t0 = 0;
-        const int n_scan = pi.n_scan;
-        for (int t = 0; t < n_scan; ++t)
-            if (cnt[t] <= J) t0 = t;
-        int t1 = n_scan - 1;
-        for (int t = n_scan - 1; t > t0; --t)
-            if (cnt[t] > J) t1 = t;
-        if (cnt[t1] <= J) atomicOr(err, kErrBracket);
-        a = scan_x(lo, hi, t0, n_scan);
-        b = scan_x(lo, hi, t1, n_scan);
-        ca = cnt[t0];
-        cb = cnt[t1];
-        x = 0.5 * (a + b);
-        mode = !(b - a > tol) ? 2 : ((ca == J && cb == J + 1) ? 1 : 0);
-    }
-    for (int round = 0; round < 512; ++round) {
-        const unsigned nm = __ballot_sync(0xffffffffu, mode == 1);
-        const unsigned bm = __ballot_sync(0xffffffffu, mode == 0);
-        const int nN = __popc(nm), nB = __popc(bm);
-        if (nN + nB == 0) break;
-        const int nlB = 64 - nN;
-        // roles of this lane's two virtual lanes v = lane + 32 h
-        double xv[2];
-        int gv[2], Gv[2];
-        bool newton0 = false;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int v = lane + 32 * h;
-            int e = 0;
-            gv[h] = 0;
-            Gv[h] = 1;
-            bool nt = false;
-            if (v < nN) {
-                nt = true;
-                e = nth_bit(nm, v);
-            } else if (nB > 0) {
-                const int t = v - nN, k = t % nB;
-                e = nth_bit(bm, k);
-                gv[h] = t / nB;
-                Gv[h] = (nlB - 1 - k) / nB + 1;
-            }
-            const double ae = __shfl_sync(0xffffffffu, a, e);
-            const double be = __shfl_sync(0xffffffffu, b, e);
-            const double xe = __shfl_sync(0xffffffffu, x, e);
-            xv[h] = nt ? xe : ae + (be - ae) * ((double)(gv[h] + 1) / (double)(Gv[h] + 1));
-            if (h == 0) newton0 = nt;
-        }
-        (void)newton0;
-        int cv0, cv1;
-        double rat, hq;
-        const int smode = nN == 0 ? 0 : (nB > 0 ? 1 : 2);
-        warp_sweep_tw<Row>(sp, nz, p_init, xv[0], xv[1], smode, r, err, cv0, cv1, rat, hq);
-        if (step_counter && lane == 0) {
-            // [0]: chain steps of every kind; [1]: steps of chains carrying
-            // derivatives (Laguerre / Newton chains: 32 per sweep in modes 1, 2)
-            atomicAdd(step_counter, (unsigned long long)(smode == 2 ? 32 : 64) * (unsigned long long)nz);
-            if (smode >= 1) atomicAdd(step_counter + 1, 32ull * (unsigned long long)nz);
-        }
-        // updates.  Every __shfl_sync is executed by all 32 lanes.
-        const bool isN = mode == 1, isB = mode == 0;
-        const int vN = isN ? __popc(nm & ((1u << lane) - 1u)) : 0;  // Newton virtual lane (chain 0)
-        const int cN = __shfl_sync(0xffffffffu, cv0, vN);
-        const double rN = __shfl_sync(0xffffffffu, rat, vN);
-        const double hN = Row::kLaguerre ? __shfl_sync(0xffffffffu, hq, vN) : 0.0;
-        const int k = isB ? __popc(bm & ((1u << lane) - 1u)) : 0;
-        const int G = isB ? (nlB - 1 - k) / nB + 1 : 0;
-        const int Gmax = nB > 0 ? (nlB - 1) / nB + 1 : 0;
-        int gb = -1, cgb = ca;
-        for (int g = 0; g < Gmax; ++g) {
-            const int v = nN + k + g * nB;
-            const int c0 = __shfl_sync(0xffffffffu, cv0, v & 31), c1 = __shfl_sync(0xffffffffu, cv1, v & 31);
-            const int c = (v >> 5) ? c1 : c0;
-            if (isB && g < G && c <= J) {
-                gb = g;
-                cgb = c;
-            }
-        }
-        const int g1 = gb + 1;
-        const int v1 = nN + k + g1 * nB;
-        const int src1 = (isB && g1 < G) ? (v1 & 31) : lane;
-        const int cU0 = __shfl_sync(0xffffffffu, cv0, src1), cU1 = __shfl_sync(0xffffffffu, cv1, src1);
-        if (isN) {
-            const double xo = x;
-            if (cN <= J) {
-                a = xo;
-                ca = cN;
-            } else {
-                b = xo;
-                cb = cN;
-            }
-            // the correction: Laguerre's step toward the eigenvalue (above x
-            // when x lies below it) or Newton's
-            const double corr = Row::kLaguerre ? laguerre_step(rN, hN, (double)nz, cN <= J) : rN;
-            const double ad = fabs(corr);
-            if (ad <= tol) {
-                x = fmin(fmax(xo - corr, a), b);
-                mode = 2;
-            } else {
-                const double xn = xo - corr;
-                const bool ok = isfinite(xn) && xn > a && xn < b;
-                x = ok ? xn : 0.5 * (a + b);
-                const double ad2 = ad * ad, dp2 = dprev * dprev;
-                // cubic (Laguerre) / quadratic (Newton) convergence: the next
-                // correction would be about ad^4 / dprev^3 (ad^3 / dprev^2) <= tol,
-                // so x = xn is final
-                const bool settled =
-                    Row::kLaguerre ? ad2 * ad2 <= tol * dp2 * dprev : ad2 * ad <= tol * dp2;
-                if (!(b - a > tol)) {
-                    mode = 2;
-                } else if (ok && dprev > 0.0 && ad <= 0.25 * dprev && settled) {
-                    mode = 2;
-                }
-                dprev = ok ? ad : 0.0;
-            }
-        } else if (isB) {
-            const double A0 = a, B0 = b;
-            const double na = gb >= 0 ? A0 + (B0 - A0) * ((double)(gb + 1) / (double)(G + 1)) : A0;
-            const double nb = g1 < G ? A0 + (B0 - A0) * ((double)(gb + 2) / (double)(G + 1)) : B0;
-            if (gb >= 0) ca = cgb;
-            if (g1 < G) cb = (v1 >> 5) ? cU1 : cU0;
-            a = na;
-            b = nb;
-            x = 0.5 * (na + nb);
-            if (!(nb - na > tol) || (na == A0 && nb == B0)) {
-                mode = 2;
-            } else if (ca == J && cb == J + 1) {
-                mode = 1;  // isolated: safeguarded Newton from here
-            }
-        }
-        // a ring wait gave up: abandon the item (warp-uniform decision)
-        if (__any_sync(0xffffffffu, (*((volatile unsigned*)err) & kErrTimeout) != 0u)) break;
-    }
-    if (lane < w.m) mu[pi.off + w.j0 + lane] = x;
-}
-
-// Row: the row format (EssRows: shifts in h^2 k^2; WmodRows: kappa = h k);
-// tol is scaled per problem by Row::tol_scale.
-template <class Row>
-__global__ void __launch_bounds__(kWarpsPerCta * 32, 4)
-    k_bisect(const ProblemInfo* __restrict__ pinfo, const double* __restrict__ s, const int* __restrict__ counts,
-             const WorkItem* __restrict__ items, int n_items, int* counter, double tol_in, double* __restrict__ mu,
-             unsigned* err, unsigned long long* step_counter, const int* __restrict__ n_items_dev, int* sched,
-             int workers) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    if (n_items_dev) n_items = *n_items_dev;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    WarpRing r;
-    r.buf = reinterpret_cast<double*>(smem_raw) + (size_t)wid * kWBuf * kWChunk;
-    r.bars = reinterpret_cast<uint64_t*>(smem_raw + (size_t)kWarpsPerCta * kWBuf * kWChunk * 8) + wid * kWBuf;
-    r.loads = 0;
-    if (lane == 0) {
-        for (int k = 0; k < kWBuf; ++k) mbar_init(&r.bars[k], 1);
-        fence_mbar_init();
-    }
-    __syncwarp();
-    // items to warps: ItemSched
-    (void)counter;
-    ItemSched sc(sched, workers);
-    long long walk = (long long)blockIdx.x * kWarpsPerCta + wid;
-    for (long long it; (it = sc.next(n_items, walk, (long long)gridDim.x * kWarpsPerCta)) >= 0;)
-        bisect_item<Row>(pinfo, s, counts, items[it], tol_in, mu, err, step_counter, r);
-}
-
-static size_t bisect_smem() { return (size_t)kWarpsPerCta * (kWBuf * kWChunk * 8 + kWBuf * 8); }
-
-template <class Row>
-static int bisect_launch(cudaStream_t st, int grid, const ProblemInfo* pinfo, const double* s, const int* counts,
-                         const WorkItem* items, int n_items, int* counter, double tol, double* mu, unsigned* err,
-                         unsigned long long* step_counter, const int* n_items_dev, int* sched, int workers) {
-    const size_t sm = bisect_smem();
-    cudaFuncSetAttribute(k_bisect<Row>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_bisect<Row><<<grid, kWarpsPerCta * 32, sm, st>>>(pinfo, s, counts, items, n_items, counter, tol, mu, err,
-                                                       step_counter, n_items_dev, sched, workers);
-    return 1;
-}
-
-template <class Row>
-static int bisect_fit() {
-    int n = 1;
-    const size_t sm = bisect_smem();
-    cudaFuncSetAttribute(k_bisect<Row>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_bisect<Row>, kWarpsPerCta * 32, sm) != cudaSuccess)
-        n = 1;
-    return n < 1 ? 1 : n;
-}
-
-int launch_bisect(cudaStream_t st, int grid, const ProblemInfo* pinfo, const double* s, const int* counts,
-                  const WorkItem* items, int n_items, int* counter, double tol, double* mu, unsigned* err,
-                  unsigned long long* step_counter, const int* n_items_dev, int* sched, int workers) {
-    return bisect_launch<EssRows>(st, grid, pinfo, s, counts, items, n_items, counter, tol, mu, err, step_counter,
-                                  n_items_dev, sched, workers);
-}
-
-int bisect_ctas_per_sm() { return bisect_fit<EssRows>(); }
-
-int launch_bisect_wmod(cudaStream_t st, int grid, const ProblemInfo* pinfo, const double* rows, const int* counts,
-                       const WorkItem* items, double tol, double* mu, unsigned* err,
-                       unsigned long long* step_counter, const int* n_items_dev, int* sched, int workers) {
-    return bisect_launch<WmodRows>(st, grid, pinfo, rows, counts, items, 0, nullptr, tol, mu, err, step_counter,
-                                   n_items_dev, sched, workers);
-}
-
-int bisect_wmod_ctas_per_sm() { return bisect_fit<WmodRows>(); }
-
-// ===========================================================================
-// Work items on the device (one CTA): the host-side item building of the
-// solve without a round trip
-// ===========================================================================
-constexpr int kItemThreads = 1024;
-
-// exclusive block scan of v over the CTA; returns the prefix, *total the sum
-__device__ int block_exclusive_scan(int v, int* sh, int* total) {
-    const int t = threadIdx.x;
-    sh[t] = v;
-    __syncthreads();
-    for (int o = 1; o < kItemThreads; o <<= 1) {
-        const int a = t >= o ? sh[t - o] : 0;
-        __syncthreads();
-        sh[t] += a;
-        __syncthreads();
-    }
-    const int incl = sh[t];
-    *total = sh[kItemThreads - 1];
-    __syncthreads();
-    return incl - v;
-}
-
-// Cost-ordered bisection items.  Every item of a problem sweeps the problem's
-// nz rows once per multisection round, and the items of problems with more
-// eigenvalues per item and more modes need more rounds, so an item's cost is
-// taken as nz x m x (1 + M / 512) (m = M / items of the problem).  With order
-// set and P <= kRankMax, the problems are ranked by that cost (descending,
-// ties by index, so the list is deterministic) and their bisection items are
-// listed in rank order; the warp mapping of the bisection kernels then puts
-// the heaviest items on different warp schedulers.  Eigenvector items and the
-// mode offsets stay in problem order.
-constexpr int kRankMax = 4096;
-
-__device__ __forceinline__ float item_cost(int nz, int M, int nb) {
-    return nb > 0 ? (float)nz * ((float)M / (float)nb) * (1.0f + (float)M * (1.0f / 512.0f)) : 0.0f;
-}
-
-__global__ void __launch_bounds__(kItemThreads) k_make_items(int P, ProblemInfo* __restrict__ pinfo,
-                                                             const int* __restrict__ counts, int max_modes,
-                                                             int bis_item, WorkItem* __restrict__ bis, int bis_cap,
-                                                             WorkItem* __restrict__ ev, int ev_cap,
-                                                             int* __restrict__ tot, unsigned* __restrict__ err,
-                                                             int* __restrict__ pstat, int order) {
-    __shared__ int sh[kItemThreads];
-    __shared__ float skey[kRankMax];
-    __shared__ int sperm[kRankMax];
-    const bool ranked = order != 0 && P <= kRankMax;
-    int base_m = 0, base_b = 0, base_e = 0;
-    for (int p0 = 0; p0 < P; p0 += kItemThreads) {
-        const int p = p0 + threadIdx.x;
-        int M = 0, nb = 0, ne = 0;
-        if (p < P) {
-            const int c_lo = counts[(size_t)p * kScanMax];
-            const int c_hi = counts[(size_t)p * kScanMax + pinfo[p].n_scan - 1];
-            M = max(0, c_hi - c_lo);
-            if (M > max_modes) {
-                atomicOr(err, kErrTooMany);
-                M = max_modes;
-            }
-            pinfo[p].c_lo = c_lo;
-            pinfo[p].c_hi = c_hi;
-            pinfo[p].M = M;
-            nb = (M + bis_item - 1) / bis_item;
-            ne = (M + kEvItem - 1) / kEvItem;
-            if (ranked) skey[p] = item_cost(pinfo[p].nz, M, nb);
-        }
-        int tm, tb, te;
-        const int om = block_exclusive_scan(M, sh, &tm);
-        const int ob = block_exclusive_scan(nb, sh, &tb);
-        const int oe = block_exclusive_scan(ne, sh, &te);
-        if (p < P && pstat) {  // readiness data of the fused launch
-            const int e0 = min(base_e + oe, ev_cap);
-            pstat[p] = nb;                          // bisection items still to finish
-            pstat[P + p] = e0;                      // first eigenvector item
-            pstat[2 * P + p] = min(ne, ev_cap - e0);  // eigenvector items
-        }
-        if (p < P) {
-            pinfo[p].off = base_m + om;
-            if (!ranked)
-                for (int k = 0; k < nb; ++k) {
-                    const int j0 = (int)((long long)M * k / nb), j1 = (int)((long long)M * (k + 1) / nb);
-                    const int q = base_b + ob + k;
-                    if (q < bis_cap) bis[q] = WorkItem{p, j0, j1 - j0, 0};
-                }
-            for (int k = 0; k < ne; ++k) {
-                const int q = base_e + oe + k;
-                if (q < ev_cap) ev[q] = WorkItem{p, k * kEvItem, min(kEvItem, M - k * kEvItem), 0};
-            }
-        }
-        base_m += tm;
-        base_b += tb;
-        base_e += te;
-    }
-    if (ranked) {
-        __syncthreads();  // skey and this block's pinfo[].M writes visible
-        for (int p = threadIdx.x; p < P; p += kItemThreads) {
-            const float kp = skey[p];
-            int r = 0;
-            for (int q = 0; q < P; ++q) {
-                const float kq = skey[q];
-                r += (kq > kp || (kq == kp && q < p)) ? 1 : 0;
-            }
-            sperm[r] = p;
-        }
-        __syncthreads();
-        int base_r = 0;
-        for (int r0 = 0; r0 < P; r0 += kItemThreads) {
-            const int r = r0 + threadIdx.x;
-            int p = 0, M = 0, nb = 0;
-            if (r < P) {
-                p = sperm[r];
-                M = pinfo[p].M;
-                nb = (M + bis_item - 1) / bis_item;
-            }
-            int tb;
-            const int ob = block_exclusive_scan(nb, sh, &tb);
-            for (int k = 0; k < nb; ++k) {
-                const int j0 = (int)((long long)M * k / nb), j1 = (int)((long long)M * (k + 1) / nb);
-                const int q = base_r + ob + k;
-                if (q < bis_cap) bis[q] = WorkItem{p, j0, j1 - j0, 0};
-            }
-            base_r += tb;
-        }
-    }
-    if (threadIdx.x == 0) {
-        if (base_b > bis_cap || base_e > ev_cap) atomicOr(err, kErrTooMany);
-        tot[0] = min(base_b, bis_cap);
-        tot[1] = min(base_e, ev_cap);
-        tot[2] = base_m;
-    }
-}
-
-int launch_make_items(cudaStream_t st, int P, ProblemInfo* pinfo, const int* counts, int max_modes, int bis_item,
-                      WorkItem* bis_items, int bis_cap, WorkItem* ev_items, int ev_cap, int* tot, unsigned* err,
-                      int* pstat, int order) {
-    if (bis_item < 1 || bis_item > kWItem) return -1;
-    k_make_items<<<1, kItemThreads, 0, st>>>(P, pinfo, counts, max_modes, bis_item, bis_items, bis_cap, ev_items,
-                                             ev_cap, tot, err, pstat, order);
-    return 1;
-}
-
 // ===========================================================================
 // FP64 FMA throughput probe (denominator of the bisection roofline)
 // ===========================================================================
@@ -1547,21 +578,17 @@ int launch_fp64_probe(cudaStream_t st, int grid, int block, int n_iter, double* 
 }
 
 // ===========================================================================
-// K4: eigenvectors by twisted factorisation, one eigenvalue per lane, one work
-// item (<= 32 eigenvalues of a problem) per warp.  For S - mu with unit
-// off-diagonals the forward solution of rows 0..i-1 is z_i = (-1)^i p_{i-1}
-// and the backward solution of rows i+1..n-1 is z_i = (-1)^(n-1-i) q_{i+1}
-// (q_n = 1); with the twist r maximising |p_{r-1} q_{r+1}|,
+// K4s: mode values by twisted factorisation on the rows themselves, for the
+// calls that keep their memory in the library's image (noalloc.cu; everything
+// else runs on panel.cu).  One eigenvalue per lane, one work item (<= 32
+// eigenvalues of a problem) per warp.  For S - mu with unit off-diagonals the
+// forward solution of rows 0..i-1 is z_i = (-1)^i p_{i-1} and the backward
+// solution of rows i+1..n-1 is z_i = (-1)^(n-1-i) q_{i+1} (q_n = 1); with the
+// twist r maximising |p_{r-1} q_{r+1}|,
 //   z_i = (-1)^i p_{i-1} q_{r+1} (i <= r),  z_i = (-1)^i p_{r-1} q_{i+1} (i >= r)
-// solves (S - mu) z = gamma_r e_r: one inverse-iteration step from e_r.  Each warp streams the diagonal s (and the weights w, g)
-// through its own TMA ring, so warps never wait on each other.
-//  pass 1  backward recurrence q top-down; every kBlk rows a checkpoint
-//          (q_c, q_{c+1}, exponent) goes to global scratch;
-//  pass 2  forward recurrence p bottom-up; each block's q values are re-created
-//          from its checkpoint in registers; the twist r = argmax |p_{r-1} q_{r+1}|
-//          is tracked and sum z^2, sum z^2 w, sum z^2 g are accumulated below r
-//          (forward part) and above r (backward part, restarted at each new r);
-//  pass 3  (optional) writes the normalised eigenvector.
+// solves (S - mu) z = gamma_r e_r: one inverse-iteration step from e_r.  Each
+// warp streams the diagonal s and the weights w through its own TMA ring, so
+// warps never wait on each other.
 // ===========================================================================
 constexpr int kEvC = 256;     // doubles per chunk and array
 constexpr int kEvB = 3;       // ring slots per warp
@@ -1570,98 +597,24 @@ constexpr int kEvWarps = 4;   // warps per CTA
 struct EvRing {
     double* s;       // [kEvB][kEvC]
     double* w;
-    double* g;
     uint64_t* bars;  // [kEvB]
     unsigned loads;
 };
 
-// chunk c of the rows (kW doubles per row) and, when given, of w and g
-template <int kW>
-__device__ __forceinline__ void evr_issue(EvRing& r, unsigned k, int c, const double* sp, const double* wp,
-                                          const double* gp) {
+// chunk c of the rows and of w
+__device__ __forceinline__ void evr_issue(EvRing& r, unsigned k, int c, const double* sp, const double* wp) {
     const int slot = k % kEvB;
-    const uint32_t bytes = kEvC * 8 * (kW + (wp ? 1 : 0) + (gp ? 1 : 0));
-    mbar_expect_tx(&r.bars[slot], bytes);
-    tma_load_1d(r.s + slot * kEvC * kW, sp + (size_t)c * kEvC * kW, kEvC * 8 * kW, &r.bars[slot]);
-    if (wp) tma_load_1d(r.w + slot * kEvC, wp + (size_t)c * kEvC, kEvC * 8, &r.bars[slot]);
-    if (gp) tma_load_1d(r.g + slot * kEvC, gp + (size_t)c * kEvC, kEvC * 8, &r.bars[slot]);
+    mbar_expect_tx(&r.bars[slot], 2 * kEvC * 8);
+    tma_load_1d(r.s + slot * kEvC, sp + (size_t)c * kEvC, kEvC * 8, &r.bars[slot]);
+    tma_load_1d(r.w + slot * kEvC, wp + (size_t)c * kEvC, kEvC * 8, &r.bars[slot]);
 }
 
-// forward-pass state of one eigenvalue
-struct FwdState {
-    double pm2, pm1;     // p_{i-2}, p_{i-1}
-    int Ep;              // exponent of p
-    double An, Aw, Ag;   // running sums of p^2, p^2 w, p^2 g
-    double thr;          // best |p q| so far, in units 2^Ethr
-    int Ethr;
-    int r, Epr, Eqr;     // twist, exponents of p and q at the twist
-    double Anr, Awr, Agr, sqr, pr, qr;
-    double Tn, Tw, Tg;   // sums of (q / q_r)^2 (w, g) above the twist, units 2^(2 Eqr)
-    double fq;           // 2^(Eb - Eqr) for the current block
-    double ps, qs, prc, qrc;
-    int Eps, Eqs, Eprc, Eqrc;
-};
-
-// one forward step at row i (local row li of the staged chunk sb)
-template <class Row, bool kGroup, bool kGuard>
-__device__ __forceinline__ void fwd_step(FwdState& F, int i, int nz, const double* sb, int li, double wi, double gi,
-                                         double qn, int Eb, const typename Row::Shift& sh, int isrc, int ircv) {
-    if (kGuard && i >= nz) return;
-    const double sq = F.pm1 * F.pm1;
-    F.An = F.An + sq;
-    F.Aw = fma(sq, wi, F.Aw);
-    const double t = qn * F.fq;
-    const double t2 = t * t;
-    F.Tn = F.Tn + t2;
-    F.Tw = fma(t2, wi, F.Tw);
-    if (kGroup) {
-        F.Ag = fma(sq, gi, F.Ag);
-        F.Tg = fma(t2, gi, F.Tg);
-    }
-    const double prod = fabs(F.pm1 * qn);
-    if (prod > F.thr) {
-        F.thr = prod;
-        F.r = i;
-        F.Anr = F.An;
-        F.Awr = F.Aw;
-        F.Agr = F.Ag;
-        F.sqr = sq;
-        F.pr = F.pm1;
-        F.Epr = F.Ep;
-        F.qr = qn;
-        F.Eqr = Eb;
-        F.fq = 1.0;
-        F.Tn = 0.0;
-        F.Tw = 0.0;
-        F.Tg = 0.0;
-    }
-    if (kGuard) {
-        if (i == isrc) {
-            F.ps = F.pm1;
-            F.Eps = F.Ep;
-            F.qs = qn;
-            F.Eqs = Eb;
-        }
-        if (i == ircv) {
-            F.prc = F.pm1;
-            F.Eprc = F.Ep;
-            F.qrc = qn;
-            F.Eqrc = Eb;
-        }
-    }
-    const double pn = fma(Row::t(sb, li, sh), F.pm1, -F.pm2);
-    F.pm2 = F.pm1;
-    F.pm1 = pn;
-}
-
-// Reduction-only eigenvector item (no full vector wanted): two passes and a
-// twist chosen among the coarse rows c = 0, kCk, 2 kCk, ...
-//  pass 1  backward recurrence q with the sums T = sum_{i > c} q_{i+1}^2 (1, w,
-//          g) over the rows above; at every coarse row c the slot keeps
-//          q_{c+1}, its exponent and T (5 values per kCk rows instead of the
-//          q checkpoints every kBlk rows that a full vector needs);
-//  pass 2  forward recurrence p with the sums A = sum_{i <= c} p_{i-1}^2 (1, w,
-//          g); at each coarse row the twist key |p_{c-1} q_{c+1}| (proportional
+// One item: two passes and a twist chosen among the coarse rows c = 0, kCk, 2 kCk, ...
+//  pass 1  backward recurrence q with the sums T = sum_{i > c} q_{i+1}^2 (1, w)
+//          over the rows above; at every coarse row c the slot keeps q_{c+1}, its
+//          exponent and T;
+//  pass 2  forward recurrence p with the sums A = sum_{i <= c} p_{i-1}^2 (1, w);
+//          at each coarse row the twist key |p_{c-1} q_{c+1}| (proportional
 //          to |z_c|) picks the best twist r so far.
 // Then sum z^2 / z_r^2 = A_r / p_{r-1}^2 + T_r / q_{r+1}^2 (each in its own
 // recurrence's scale).  Restricting r to the coarse rows costs at most the
@@ -1672,22 +625,17 @@ __device__ __forceinline__ void fwd_step(FwdState& F, int i, int nz, const doubl
 constexpr int kCk = kCkRows;  // rows between coarse twist candidates
 static_assert(kEvC % kCk == 0 && kCk % kBlk == 0, "coarse rows start blocks and chunks");
 
-template <class Row, bool kGroup>
-__device__ __forceinline__ void eigvec_item_coarse(const EigvecArgs& A, const WorkItem w, EvRing& R, double* ckq,
-                                                   double* ckt, int* cke) {
-    constexpr int kW = Row::kW;
+__device__ __forceinline__ void eigvec_item(const EigvecArgs& A, const WorkItem w, EvRing& R, double* ckq, double* ckt,
+                                            int* cke) {
     const int lane = threadIdx.x & 31;
     const ProblemInfo pi = A.pinfo[w.problem];
     const int nz = pi.nz;
     const int nch = (nz + kEvC - 1) / kEvC;
     const int isrc = pi.isrc, ircv = pi.ircv;
-    const double* sp = A.s + (size_t)pi.s_off * kW;
+    const double* sp = A.s + pi.s_off;
     const double* wp = A.w + pi.w_off;
-    const double* gp = kGroup ? A.g + pi.s_off : nullptr;
     const bool active = lane < w.m;
-    // through L2: in the fused launch another warp wrote mu in this kernel
-    const double mu = active ? __ldcg(A.mu + pi.off + w.j0 + lane) : Row::idle_shift(pi);
-    const typename Row::Shift sh = Row::shift(mu);
+    const double mu = active ? A.mu[pi.off + w.j0 + lane] : pi.lo;
 
     // ---------------- pass 1: backward recurrence, coarse checkpoints ----------
     double qs = 1.0, qrc = 1.0;  // q_{isrc+1}, q_{ircv+1}
@@ -1695,26 +643,24 @@ __device__ __forceinline__ void eigvec_item_coarse(const EigvecArgs& A, const Wo
     {
         const unsigned base = R.loads;
         if (lane == 0)
-            for (int o = 0; o < nch && o < kEvB; ++o) evr_issue<kW>(R, base + o, nch - 1 - o, sp, wp, gp);
+            for (int o = 0; o < nch && o < kEvB; ++o) evr_issue(R, base + o, nch - 1 - o, sp, wp);
         __syncwarp();
         double q1 = 1.0, q2 = 0.0;  // q_{i+1}, q_{i+2} before row i; q_n = 1, q_{n+1} = 0
-        double Tn = 0.0, Tw = 0.0, Tg = 0.0;
+        double Tn = 0.0, Tw = 0.0;
         int E = 0;
         for (int o = 0; o < nch; ++o) {
             const int c = nch - 1 - o;
             const unsigned k = base + o;
             const int slot = k % kEvB;
             mbar_wait_bounded(&R.bars[slot], (k / kEvB) & 1u, A.err);
-            const double* sb = R.s + slot * kEvC * kW;
+            const double* sb = R.s + slot * kEvC;
             const double* wb = R.w + slot * kEvC;
-            const double* gb = kGroup ? R.g + slot * kEvC : nullptr;
             const int valid = min(kEvC, nz - c * kEvC);
             auto row = [&](int li) {
                 const double qq = q1 * q1;
                 Tn = Tn + qq;
                 Tw = fma(qq, wb[li], Tw);
-                if (kGroup) Tg = fma(qq, gb[li], Tg);
-                const double qi = fma(Row::t(sb, li, sh), q1, -q2);
+                const double qi = fma(sb[li] - mu, q1, -q2);
                 q2 = q1;
                 q1 = qi;
             };
@@ -1722,9 +668,8 @@ __device__ __forceinline__ void eigvec_item_coarse(const EigvecArgs& A, const Wo
                 const size_t ci = (size_t)(gbase / kCk) * 32 + lane;
                 ckq[ci] = q1;
                 cke[ci] = E;
-                ckt[ci * 3] = Tn;
-                ckt[ci * 3 + 1] = Tw;
-                ckt[ci * 3 + 2] = Tg;
+                ckt[ci * 2] = Tn;
+                ckt[ci * 2 + 1] = Tw;
             };
             for (int lb = ((valid - 1) / kBlk) * kBlk; lb >= 0; lb -= kBlk) {
                 const int gbase = c * kEvC + lb;
@@ -1759,14 +704,13 @@ __device__ __forceinline__ void eigvec_item_coarse(const EigvecArgs& A, const Wo
                     q2 *= sc;
                     Tn *= sc2;
                     Tw *= sc2;
-                    Tg *= sc2;
                     E += sft;
                 }
             }
             __syncwarp();
             if (lane == 0 && o + kEvB < nch) {
                 fence_proxy_async();
-                evr_issue<kW>(R, base + o + kEvB, nch - 1 - (o + kEvB), sp, wp, gp);
+                evr_issue(R, base + o + kEvB, nch - 1 - (o + kEvB), sp, wp);
             }
         }
         R.loads = base + nch;
@@ -1774,39 +718,37 @@ __device__ __forceinline__ void eigvec_item_coarse(const EigvecArgs& A, const Wo
     __syncwarp();  // the slot's checkpoints written by every lane before they are read
 
     // ---------------- pass 2: forward recurrence, coarse twist ----------------
-    double pm2 = Row::p_init(pi), pm1 = 1.0;  // p_{i-2}, p_{i-1}
+    double pm2 = 0.0, pm1 = 1.0;  // p_{i-2}, p_{i-1}
     int Ep = 0;
-    double An = 0.0, Aw = 0.0, Ag = 0.0;
+    double An = 0.0, Aw = 0.0;
     double best = -INFINITY;
     int r = 0, Epr = 0, Eqr = 0;
-    double Anr = 1.0, Awr = 0.0, Agr = 0.0, pr = 1.0, qr = 1.0, Tnr = 0.0, Twr = 0.0, Tgr = 0.0;
+    double Anr = 1.0, Awr = 0.0, pr = 1.0, qr = 1.0, Tnr = 0.0, Twr = 0.0;
     double ps = 1.0, prc = 1.0;  // p_{isrc-1}, p_{ircv-1}
     int Eps = 0, Eprc = 0;
     {
         const unsigned base = R.loads;
         if (lane == 0)
-            for (int c = 0; c < nch && c < kEvB; ++c) evr_issue<kW>(R, base + c, c, sp, wp, gp);
+            for (int c = 0; c < nch && c < kEvB; ++c) evr_issue(R, base + c, c, sp, wp);
         __syncwarp();
         // checkpoint of the next coarse row, loaded one candidate ahead
-        double nq = ckq[lane], nt0 = ckt[lane * 3], nt1 = ckt[lane * 3 + 1], nt2 = ckt[lane * 3 + 2];
+        double nq = ckq[lane], nt0 = ckt[lane * 2], nt1 = ckt[lane * 2 + 1];
         int nE = cke[lane];
         const int n_coarse = (nz + kCk - 1) / kCk;
         for (int c = 0; c < nch; ++c) {
             const unsigned k = base + c;
             const int slot = k % kEvB;
             mbar_wait_bounded(&R.bars[slot], (k / kEvB) & 1u, A.err);
-            const double* sb = R.s + slot * kEvC * kW;
+            const double* sb = R.s + slot * kEvC;
             const double* wb = R.w + slot * kEvC;
-            const double* gb = kGroup ? R.g + slot * kEvC : nullptr;
             const int valid = min(kEvC, nz - c * kEvC);
             auto row = [&](int li) {
                 const double sq = pm1 * pm1;
                 An = An + sq;
                 Aw = fma(sq, wb[li], Aw);
-                if (kGroup) Ag = fma(sq, gb[li], Ag);
             };
             auto step = [&](int li) {
-                const double pn = fma(Row::t(sb, li, sh), pm1, -pm2);
+                const double pn = fma(sb[li] - mu, pm1, -pm2);
                 pm2 = pm1;
                 pm1 = pn;
             };
@@ -1818,23 +760,20 @@ __device__ __forceinline__ void eigvec_item_coarse(const EigvecArgs& A, const Wo
                     r = gbase;
                     Anr = An;
                     Awr = Aw;
-                    Agr = Ag;
                     pr = pm1;
                     Epr = Ep;
                     qr = nq;
                     Eqr = nE;
                     Tnr = nt0;
                     Twr = nt1;
-                    Tgr = nt2;
                 }
                 const int kc = gbase / kCk + 1;
                 if (kc < n_coarse) {
                     const size_t ci = (size_t)kc * 32 + lane;
                     nq = ckq[ci];
                     nE = cke[ci];
-                    nt0 = ckt[ci * 3];
-                    nt1 = ckt[ci * 3 + 1];
-                    nt2 = ckt[ci * 3 + 2];
+                    nt0 = ckt[ci * 2];
+                    nt1 = ckt[ci * 2 + 1];
                 }
             };
             for (int lb = 0; lb < valid; lb += kBlk) {
@@ -1873,14 +812,13 @@ __device__ __forceinline__ void eigvec_item_coarse(const EigvecArgs& A, const Wo
                     pm2 *= sc;
                     An *= sc2;
                     Aw *= sc2;
-                    Ag *= sc2;
                     Ep += sft;
                 }
             }
             __syncwarp();
             if (lane == 0 && c + kEvB < nch) {
                 fence_proxy_async();
-                evr_issue<kW>(R, base + c + kEvB, c + kEvB, sp, wp, gp);
+                evr_issue(R, base + c + kEvB, c + kEvB, sp, wp);
             }
         }
         R.loads = base + nch;
@@ -1888,16 +826,13 @@ __device__ __forceinline__ void eigvec_item_coarse(const EigvecArgs& A, const Wo
     // ---------------- combine ----------------------------------------
     const double ip2 = 1.0 / (pr * pr), iq2 = 1.0 / (qr * qr);
     const double nrm = Anr * ip2 + Tnr * iq2;
-    // the wide-angle vectors carry SLEPc's normalisation of the linearised
-    // pencil's [v; k v] (EigenEngine.cpp:368-379): sum v^2 dz = 1 / (1 + k^2)
-    const double f2 = kW == 1 ? 1.0 : 1.0 / (1.0 + (mu / pi.dz) * (mu / pi.dz));
-    const double scale = kW == 1 ? 1.0 / sqrt(nrm * pi.dz) : sqrt(f2 / (nrm * pi.dz));
+    const double scale = 1.0 / sqrt(nrm * pi.dz);
     double zs = (isrc <= r) ? (ps / pr) * pow2(Eps - Epr) : (qs / qr) * pow2(Eqs - Eqr);
     double zr = (ircv <= r) ? (prc / pr) * pow2(Eprc - Epr) : (qrc / qr) * pow2(Eqrc - Eqr);
     if ((isrc - r) & 1) zs = -zs;
     if ((ircv - r) & 1) zr = -zr;
-    const double absorption = (Awr * ip2 + Twr * iq2) / nrm * f2;
-    const double ks = kW == 1 ? sqrt(mu / (pi.dz * pi.dz)) : mu / pi.dz;
+    const double absorption = (Awr * ip2 + Twr * iq2) / nrm;
+    const double ks = sqrt(mu / (pi.dz * pi.dz));
     const double kk = ks * ks;
     const auto kp = csqrt_principal(kk, absorption);
     if (active) {
@@ -1906,335 +841,18 @@ __device__ __forceinline__ void eigvec_item_coarse(const EigvecArgs& A, const Wo
         A.ki[o] = kp.imag();
         A.vs[o] = zs * scale;
         A.vr[o] = zr * scale;
-        if (kGroup) {
-            const double gsum = (Agr * ip2 + Tgr * iq2) / nrm;
-            const double vph = pi.omega / kp.real();
-            A.vg[o] = 1.0 / (vph * gsum);
-        } else if (A.vg) {
-            A.vg[o] = 0.0;
-        }
+        if (A.vg) A.vg[o] = 0.0;
     }
 }
 
-// One eigenvector work item (<= 32 modes of one problem) on this warp, with
-// its TMA ring R and its checkpoint slot (ck1, ck2, cke).
-template <class Row, bool kGroup, bool kVec>
-__device__ __forceinline__ void eigvec_item(const EigvecArgs& A, const WorkItem w, EvRing& R, double* ck1,
-                                            double* ck2, int* cke) {
-    constexpr int kW = Row::kW;
-    if constexpr (!kVec) {
-        // reductions only: the two-pass coarse-twist item
-        eigvec_item_coarse<Row, kGroup>(A, w, R, ck1, ck2, cke);
-        return;
-    }
-    const int lane = threadIdx.x & 31;
-    const ProblemInfo pi = A.pinfo[w.problem];
-    const int nz = pi.nz;
-    auto load_ck = [&](int kb, double& a1, double& a2, int& ae) {
-        if (min((kb + 1) * kBlk, nz) >= nz) {
-            a1 = 1.0;
-            a2 = 0.0;
-            ae = 0;
-        } else {
-            const size_t ci = (size_t)kb * 32 + lane;
-            a1 = ck1[ci];
-            a2 = ck2[ci];
-            ae = cke[ci];
-        }
-    };
-    const int nch = (nz + kEvC - 1) / kEvC;
-    const int nblk = (nz + kBlk - 1) / kBlk;
-    const int isrc = pi.isrc, ircv = pi.ircv;
-    const double* sp = A.s + (size_t)pi.s_off * kW;
-    const double* wp = A.w + pi.w_off;
-    const double* gp = kGroup ? A.g + pi.s_off : nullptr;
-    const bool active = lane < w.m;
-    // through L2: in the fused launch another warp wrote mu in this kernel
-    const double mu = active ? __ldcg(A.mu + pi.off + w.j0 + lane) : Row::idle_shift(pi);
-    const typename Row::Shift sh = Row::shift(mu);
-
-    // ---------------- pass 1: backward recurrence, checkpoints ----------
-    {
-        const unsigned base = R.loads;
-        if (lane == 0)
-            for (int o = 0; o < nch && o < kEvB; ++o)
-                evr_issue<kW>(R, base + o, nch - 1 - o, sp, nullptr, nullptr);
-        __syncwarp();
-        double q1 = 1.0, q2 = 0.0;  // q_i, q_{i+1}; q_n = 1, q_{n+1} = 0
-        int E = 0;
-        for (int o = 0; o < nch; ++o) {
-            const int c = nch - 1 - o;
-            const unsigned k = base + o;
-            const int slot = k % kEvB;
-            mbar_wait_bounded(&R.bars[slot], (k / kEvB) & 1u, A.err);
-            const double* sb = R.s + slot * kEvC * kW;
-            const int valid = min(kEvC, nz - c * kEvC);
-            for (int lb = ((valid - 1) / kBlk) * kBlk; lb >= 0; lb -= kBlk) {
-                if (lb + kBlk <= valid) {
-#pragma unroll
-                    for (int u = kBlk - 1; u >= 0; --u) {
-                        const double qi = fma(Row::t(sb, lb + u, sh), q1, -q2);
-                        q2 = q1;
-                        q1 = qi;
-                    }
-                } else {
-                    for (int u = valid - 1 - lb; u >= 0; --u) {
-                        const double qi = fma(Row::t(sb, lb + u, sh), q1, -q2);
-                        q2 = q1;
-                        q1 = qi;
-                    }
-                }
-                const int gbase = c * kEvC + lb;
-                if (gbase > 0) {
-                    const size_t ci = (size_t)(gbase / kBlk - 1) * 32 + lane;
-                    ck1[ci] = q1;
-                    ck2[ci] = q2;
-                    cke[ci] = E;
-                }
-                const int sh = grow_shift(q1, q2);
-                if (sh) {
-                    const double sc = pow2(-sh);
-                    q1 *= sc;
-                    q2 *= sc;
-                    E += sh;
-                }
-            }
-            __syncwarp();
-            if (lane == 0 && o + kEvB < nch) {
-                fence_proxy_async();
-                evr_issue<kW>(R, base + o + kEvB, nch - 1 - (o + kEvB), sp, nullptr, nullptr);
-            }
-        }
-        R.loads = base + nch;
-    }
-
-    // ---------------- pass 2: forward recurrence, twist, sums ----------
-    FwdState F;
-    F.pm2 = Row::p_init(pi);
-    F.pm1 = 1.0;
-    F.Ep = 0;
-    F.An = F.Aw = F.Ag = 0.0;
-    F.thr = -1.0;
-    F.Ethr = 0;
-    F.r = 0;
-    F.Epr = F.Eqr = 0;
-    F.Anr = 1.0;
-    F.Awr = F.Agr = 0.0;
-    F.sqr = F.pr = F.qr = 1.0;
-    F.Tn = F.Tw = F.Tg = 0.0;
-    F.fq = 1.0;
-    F.ps = F.qs = F.prc = F.qrc = 1.0;
-    F.Eps = F.Eqs = F.Eprc = F.Eqrc = 0;
-    {
-        const unsigned base = R.loads;
-        if (lane == 0)
-            for (int c = 0; c < nch && c < kEvB; ++c) evr_issue<kW>(R, base + c, c, sp, wp, gp);
-        __syncwarp();
-        double nq1, nq2;
-        int nE;
-        load_ck(0, nq1, nq2, nE);
-        for (int c = 0; c < nch; ++c) {
-            const unsigned k = base + c;
-            const int slot = k % kEvB;
-            mbar_wait_bounded(&R.bars[slot], (k / kEvB) & 1u, A.err);
-            const double* sb = R.s + slot * kEvC * kW;
-            const double* wb = R.w + slot * kEvC;
-            const double* gb = kGroup ? R.g + slot * kEvC : nullptr;
-            const int valid = min(kEvC, nz - c * kEvC);
-            for (int lb = 0; lb < valid; lb += kBlk) {
-                const int gbase = c * kEvC + lb;
-                const int kb = gbase / kBlk;
-                double q1 = nq1, q2 = nq2;
-                const int Eb = nE;
-                if (kb + 1 < nblk) load_ck(kb + 1, nq1, nq2, nE);
-                const int Enew = F.Ep + Eb;
-                if (Enew != F.Ethr) {
-                    F.thr *= pow2(F.Ethr - Enew);
-                    F.Ethr = Enew;
-                }
-                F.fq = pow2(Eb - F.Eqr);
-                // q_{gbase+1 .. gbase+kBlk}, units 2^Eb
-                double qb[kBlk];
-                const int ctop = min(gbase + kBlk, nz);
-                const bool full = gbase + kBlk <= nz;
-                if (ctop == gbase + kBlk) {
-                    qb[kBlk - 1] = q1;
-#pragma unroll
-                    for (int jj = kBlk - 2; jj >= 0; --jj) {
-                        const double qi = fma(Row::t(sb, lb + jj + 1, sh), q1, -q2);
-                        qb[jj] = qi;
-                        q2 = q1;
-                        q1 = qi;
-                    }
-                } else {
-#pragma unroll
-                    for (int jj = kBlk - 1; jj >= 0; --jj) {
-                        const int idx = gbase + 1 + jj;
-                        if (idx == ctop) {
-                            qb[jj] = q1;
-                        } else if (idx < ctop) {
-                            const double qi = fma(Row::t(sb, lb + jj + 1, sh), q1, -q2);
-                            qb[jj] = qi;
-                            q2 = q1;
-                            q1 = qi;
-                        } else {
-                            qb[jj] = 0.0;
-                        }
-                    }
-                }
-                const bool special = !full || (isrc >= gbase && isrc < gbase + kBlk) ||
-                                     (ircv >= gbase && ircv < gbase + kBlk);
-                if (!special) {
-#pragma unroll
-                    for (int jj = 0; jj < kBlk; ++jj)
-                        fwd_step<Row, kGroup, false>(F, gbase + jj, nz, sb, lb + jj, wb[lb + jj],
-                                                     kGroup ? gb[lb + jj] : 0.0, qb[jj], Eb, sh, isrc, ircv);
-                } else {
-#pragma unroll
-                    for (int jj = 0; jj < kBlk; ++jj) {
-                        const int li = min(lb + jj, valid - 1);
-                        fwd_step<Row, kGroup, true>(F, gbase + jj, nz, sb, li, wb[li], kGroup ? gb[li] : 0.0,
-                                                    qb[jj], Eb, sh, isrc, ircv);
-                    }
-                }
-                const int sh = grow_shift(F.pm1, F.pm2);
-                if (sh) {
-                    const double sc = pow2(-sh), sc2 = pow2(-2 * sh);
-                    F.pm1 *= sc;
-                    F.pm2 *= sc;
-                    F.An *= sc2;
-                    F.Aw *= sc2;
-                    F.Ag *= sc2;
-                    F.Ep += sh;
-                }
-            }
-            __syncwarp();
-            if (lane == 0 && c + kEvB < nch) {
-                fence_proxy_async();
-                evr_issue<kW>(R, base + c + kEvB, c + kEvB, sp, wp, gp);
-            }
-        }
-        R.loads = base + nch;
-    }
-    // ---------------- combine ----------------------------------------
-    const double iq2 = 1.0 / (F.qr * F.qr);
-    const double isq = 1.0 / F.sqr;
-    const double nrm = F.Anr * isq + F.Tn * iq2;
-    // the wide-angle vectors carry SLEPc's normalisation of the linearised
-    // pencil's [v; k v] (EigenEngine.cpp:368-379): sum v^2 dz = 1 / (1 + k^2)
-    const double f2 = kW == 1 ? 1.0 : 1.0 / (1.0 + (mu / pi.dz) * (mu / pi.dz));
-    const double scale = kW == 1 ? 1.0 / sqrt(nrm * pi.dz) : sqrt(f2 / (nrm * pi.dz));
-    const int r = F.r;
-    double zs = (isrc <= r) ? (F.ps / F.pr) * pow2(F.Eps - F.Epr) : (F.qs / F.qr) * pow2(F.Eqs - F.Eqr);
-    double zr = (ircv <= r) ? (F.prc / F.pr) * pow2(F.Eprc - F.Epr) : (F.qrc / F.qr) * pow2(F.Eqrc - F.Eqr);
-    if ((isrc - r) & 1) zs = -zs;
-    if ((ircv - r) & 1) zr = -zr;
-    const double absorption = kW == 1 ? (F.Awr * isq + F.Tw * iq2) / nrm : (F.Awr * isq + F.Tw * iq2) / nrm * f2;
-    const double ks = kW == 1 ? sqrt(mu / (pi.dz * pi.dz)) : mu / pi.dz;
-    const double kk = ks * ks;
-    const auto kp = csqrt_principal(kk, absorption);
-    if (active) {
-        const int o = pi.off + w.j0 + lane;
-        A.kr[o] = kp.real();
-        A.ki[o] = kp.imag();
-        A.vs[o] = zs * scale;
-        A.vr[o] = zr * scale;
-        if (kGroup) {
-            const double gsum = (F.Agr * isq + F.Tg * iq2) / nrm;
-            const double vph = pi.omega / kp.real();
-            A.vg[o] = 1.0 / (vph * gsum);
-        } else if (A.vg) {
-            A.vg[o] = 0.0;
-        }
-    }
-    // ---------------- pass 3 (optional): full eigenvector --------------
-    if (kVec) {
-        double* vout = A.vfull + A.vfull_off[w.problem];
-        const int M = pi.M;
-        const unsigned base = R.loads;
-        if (lane == 0)
-            for (int c = 0; c < nch && c < kEvB; ++c) evr_issue<kW>(R, base + c, c, sp, nullptr, nullptr);
-        __syncwarp();
-        double pa = Row::p_init(pi), pb = 1.0;
-        int Ea = 0;
-        double nq1, nq2;
-        int nE;
-        load_ck(0, nq1, nq2, nE);
-        const double ipr = 1.0 / F.pr, iqr = 1.0 / F.qr;
-        for (int c = 0; c < nch; ++c) {
-            const unsigned k = base + c;
-            const int slot = k % kEvB;
-            mbar_wait_bounded(&R.bars[slot], (k / kEvB) & 1u, A.err);
-            const double* sb = R.s + slot * kEvC * kW;
-            const int valid = min(kEvC, nz - c * kEvC);
-            for (int lb = 0; lb < valid; lb += kBlk) {
-                const int gbase = c * kEvC + lb;
-                const int kb = gbase / kBlk;
-                double q1 = nq1, q2 = nq2;
-                const int Eb = nE;
-                if (kb + 1 < nblk) load_ck(kb + 1, nq1, nq2, nE);
-                double qb[kBlk];
-                const int ctop = min(gbase + kBlk, nz);
-#pragma unroll
-                for (int jj = kBlk - 1; jj >= 0; --jj) {
-                    const int idx = gbase + 1 + jj;
-                    if (idx == ctop) {
-                        qb[jj] = q1;
-                    } else if (idx < ctop) {
-                        const double qi = fma(Row::t(sb, lb + jj + 1, sh), q1, -q2);
-                        qb[jj] = qi;
-                        q2 = q1;
-                        q1 = qi;
-                    } else {
-                        qb[jj] = 0.0;
-                    }
-                }
-                const double fp = pow2(Ea - F.Epr) * ipr * scale;
-                const double fqq = pow2(Eb - F.Eqr) * iqr * scale;
-#pragma unroll
-                for (int jj = 0; jj < kBlk; ++jj) {
-                    const int i = gbase + jj;
-                    if (i < nz) {
-                        double zi = (i <= r) ? pb * fp : qb[jj] * fqq;
-                        if ((i - r) & 1) zi = -zi;
-                        if (active) vout[(size_t)i * M + w.j0 + lane] = zi;
-                        const double pn = fma(Row::t(sb, lb + jj, sh), pb, -pa);
-                        pa = pb;
-                        pb = pn;
-                    }
-                }
-                const int sh = grow_shift(pb, pa);
-                if (sh) {
-                    const double sc = pow2(-sh);
-                    pa *= sc;
-                    pb *= sc;
-                    Ea += sh;
-                }
-            }
-            __syncwarp();
-            if (lane == 0 && c + kEvB < nch) {
-                fence_proxy_async();
-                evr_issue<kW>(R, base + c + kEvB, c + kEvB, sp, nullptr, nullptr);
-            }
-        }
-        R.loads = base + nch;
-    }
-}
-
-// Row: the row format (EssRows, WmodRows in device_common.cuh); mu holds the
-// shift of each mode in the row format's units (h^2 k^2, or kappa = h k)
-template <class Row, bool kGroup, bool kVec>
 __global__ void __launch_bounds__(kEvWarps * 32, 4) k_eigvec(EigvecArgs A) {
-    constexpr int kW = Row::kW;
-    constexpr int NA = kW + (kGroup ? 2 : 1);
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    double* wb0 = reinterpret_cast<double*>(smem_raw) + (size_t)wid * kEvB * NA * kEvC;
+    double* wb0 = reinterpret_cast<double*>(smem_raw) + (size_t)wid * kEvB * 2 * kEvC;
     EvRing R;
     R.s = wb0;
-    R.w = wb0 + kEvB * kEvC * kW;
-    R.g = kGroup ? wb0 + (kW + 1) * kEvB * kEvC : nullptr;
-    R.bars = reinterpret_cast<uint64_t*>(smem_raw + (size_t)kEvWarps * kEvB * NA * kEvC * 8) + wid * kEvB;
+    R.w = wb0 + kEvB * kEvC;
+    R.bars = reinterpret_cast<uint64_t*>(smem_raw + (size_t)kEvWarps * kEvB * 2 * kEvC * 8) + wid * kEvB;
     R.loads = 0;
     if (lane == 0) {
         for (int k = 0; k < kEvB; ++k) mbar_init(&R.bars[k], 1);
@@ -2245,196 +863,16 @@ __global__ void __launch_bounds__(kEvWarps * 32, 4) k_eigvec(EigvecArgs A) {
     double* ck1 = A.ck_q1 + gw * A.ck_slot_stride;
     double* ck2 = A.ck_q2 + gw * A.ck_slot_stride;
     int* cke = A.ck_e + gw * A.ck_slot_stride;
-    const int n_items_all = A.n_items_dev ? *A.n_items_dev : A.n_items;
-    // static round-robin over the grid's warps (see k_bisect)
-    const int warps_total = gridDim.x * kEvWarps;
-    for (int it = blockIdx.x * kEvWarps + wid; it < n_items_all; it += warps_total) {
-        if (A.ev_done && A.ev_done[it]) continue;  // done in the fused launch
-        eigvec_item<Row, kGroup, kVec>(A, A.items[it], R, ck1, ck2, cke);
-    }
+    // static round-robin over the grid's warps
+    for (int it = blockIdx.x * kEvWarps + wid; it < A.n_items; it += gridDim.x * kEvWarps)
+        eigvec_item(A, A.items[it], R, ck1, ck2, cke);
 }
 
-template <class Row, bool G, bool V>
-static void* eigvec_fn() {
-    return (void*)k_eigvec<Row, G, V>;
-}
-
-template <class Row>
-static size_t eigvec_smem(const EigvecArgs& a) {
-    const int na = Row::kW + (a.g ? 2 : 1);
-    return (size_t)kEvWarps * (kEvB * na * kEvC * 8 + kEvB * 8);
-}
-
-template <class Row>
-static void* eigvec_select(const EigvecArgs& a) {
-    const bool grp = a.g != nullptr, vec = a.vfull != nullptr;
-    if (grp && vec) return eigvec_fn<Row, true, true>();
-    if (grp) return eigvec_fn<Row, true, false>();
-    if (vec) return eigvec_fn<Row, false, true>();
-    return eigvec_fn<Row, false, false>();
-}
-
-template <class Row>
-static int eigvec_fit(const EigvecArgs& a) {
-    int n = 1;
-    void* f = eigvec_select<Row>(a);
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eigvec_smem<Row>(a));
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, kEvWarps * 32, eigvec_smem<Row>(a)) != cudaSuccess)
-        n = 1;
-    return n < 1 ? 1 : n;
-}
-
-template <class Row>
-static int eigvec_launch(cudaStream_t st, int grid, const EigvecArgs& a) {
-    const size_t sm = eigvec_smem<Row>(a);
-    const bool grp = a.g != nullptr, vec = a.vfull != nullptr;
-    cudaFuncSetAttribute(eigvec_select<Row>(a), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (grp && vec) k_eigvec<Row, true, true><<<grid, kEvWarps * 32, sm, st>>>(a);
-    else if (grp) k_eigvec<Row, true, false><<<grid, kEvWarps * 32, sm, st>>>(a);
-    else if (vec) k_eigvec<Row, false, true><<<grid, kEvWarps * 32, sm, st>>>(a);
-    else k_eigvec<Row, false, false><<<grid, kEvWarps * 32, sm, st>>>(a);
+int launch_eigvec(cudaStream_t st, int grid, const EigvecArgs& a) {
+    const size_t sm = (size_t)kEvWarps * (kEvB * 2 * kEvC * 8 + kEvB * 8);
+    cudaFuncSetAttribute(k_eigvec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_eigvec<<<grid, kEvWarps * 32, sm, st>>>(a);
     return 1;
-}
-
-int eigvec_ctas_per_sm(const EigvecArgs& a) { return eigvec_fit<EssRows>(a); }
-
-int launch_eigvec(cudaStream_t st, int grid, const EigvecArgs& a) { return eigvec_launch<EssRows>(st, grid, a); }
-
-int eigvec_wmod_ctas_per_sm(const EigvecArgs& a) { return eigvec_fit<WmodRows>(a); }
-
-// the wide-angle instantiation carries no group speeds
-int launch_eigvec_wmod(cudaStream_t st, int grid, const EigvecArgs& a) {
-    if (a.g) return -1;
-    return eigvec_launch<WmodRows>(st, grid, a);
-}
-
-// ===========================================================================
-// K3+K4 fused: bisection and eigenvectors in one launch.  Every warp first
-// runs its bisection items (the static mapping of k_bisect); the warp that
-// finishes a problem's last bisection item appends the problem's eigenvector
-// items to a ready queue.  Then every warp takes queue slots in order and
-// runs the eigenvector item it finds there, so eigenvectors of finished
-// problems overlap the bisection of the others.  Producers never wait on
-// consumers; a consumer waits for its slot to be filled (bounded: it gives
-// up after F.wait_ns or on a device error), and every item it did not
-// finish is left to the k_eigvec launch that follows (items marked done are
-// skipped there), so no result depends on all CTAs being resident.
-// ===========================================================================
-template <class Row>
-__global__ void __launch_bounds__(kWarpsPerCta * 32, 4) k_bisect_eigvec(FusedArgs F) {
-    static_assert(kWarpsPerCta == kEvWarps, "one warp layout for both phases");
-    constexpr int kW = Row::kW;
-    constexpr int kBisD = kWBuf * kWChunk, kEvD = kEvB * (kW + 1) * kEvC;
-    constexpr int kWarpD = kBisD > kEvD ? kBisD : kEvD;  // doubles of one warp's ring buffer
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    double* wbuf = reinterpret_cast<double*>(smem_raw) + (size_t)wid * kWarpD;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + (size_t)kWarpsPerCta * kWarpD * 8) + wid * (kWBuf + kEvB);
-    WarpRing r;
-    r.buf = wbuf;
-    r.bars = bars;
-    r.loads = 0;
-    EvRing R;
-    R.s = wbuf;
-    R.w = wbuf + kEvB * kEvC * kW;
-    R.g = nullptr;
-    R.bars = bars + kWBuf;
-    R.loads = 0;
-    if (lane == 0) {
-        for (int k = 0; k < kWBuf + kEvB; ++k) mbar_init(&bars[k], 1);
-        fence_mbar_init();
-    }
-    __syncwarp();
-    const int P = F.P;
-    // ---- bisection items; the last item of a problem publishes its eigenvector items ----
-    const int n_bis = *F.n_bis_dev;
-    ItemSched sc(F.sched, F.workers);
-    long long walk = (long long)blockIdx.x * kWarpsPerCta + wid;
-    for (long long it; (it = sc.next(n_bis, walk, (long long)gridDim.x * kWarpsPerCta)) >= 0;) {
-        const WorkItem w = F.bis[it];
-        bisect_item<Row>(F.pinfo, F.s, F.counts, w, F.tol, F.mu, F.err, nullptr, r);
-        __threadfence();  // this lane's eigenvalues visible before the count below
-        __syncwarp();
-        if (lane == 0 && atomicSub(&F.pstat[w.problem], 1) == 1) {
-            const int e0 = F.pstat[P + w.problem], ne = F.pstat[2 * P + w.problem];
-            if (ne > 0) {
-                const int t = atomicAdd(F.q_tail, ne);
-                for (int i = 0; i < ne; ++i) atomicExch(&F.queue[t + i], e0 + i + 1);
-            }
-        }
-        __syncwarp();
-    }
-    // ---- eigenvector items from the ready queue ----
-    // with ev_workers_only, warps that ran no bisection leave the eigenvector
-    // items to the bisection warps (as those finish) and to the k_eigvec
-    // launch that follows, instead of competing with the bisection
-    if (F.ev_workers_only && !sc.worker) return;
-    const int n_ev = *F.ea.n_items_dev;
-    const size_t gw = (size_t)blockIdx.x * kEvWarps + wid;
-    double* ck1 = F.ea.ck_q1 + gw * F.ea.ck_slot_stride;
-    double* ck2 = F.ea.ck_q2 + gw * F.ea.ck_slot_stride;
-    int* cke = F.ea.ck_e + gw * F.ea.ck_slot_stride;
-    if (lane == 0) fence_proxy_async();  // the shared buffer now feeds the other ring
-    __syncwarp();
-    for (;;) {
-        int h = 0;
-        if (lane == 0) h = atomicAdd(F.q_head, 1);
-        h = __shfl_sync(0xffffffffu, h, 0);
-        if (h >= n_ev) break;
-        int v = 0;
-        if (lane == 0) {
-            const uint64_t t0 = global_ns();
-            for (;;) {
-                v = *((volatile int*)(F.queue + h));
-                if (v != 0) break;
-                if ((*((volatile unsigned*)F.err) & (kErrTimeout | kErrTooMany)) != 0u ||
-                    global_ns() - t0 > F.wait_ns)
-                    break;
-                __nanosleep(2000);
-            }
-        }
-        v = __shfl_sync(0xffffffffu, v, 0);
-        if (v == 0) break;  // gave up: the following k_eigvec launch runs this item
-        __threadfence();   // the item's eigenvalues, written by another warp, before reading them
-        const int it = v - 1;
-        eigvec_item<Row, false, false>(F.ea, F.ea.items[it], R, ck1, ck2, cke);
-        __syncwarp();
-        if (lane == 0) F.ev_done[it] = 1;
-    }
-}
-
-template <class Row>
-static size_t fused_smem() {
-    constexpr int kBisD = kWBuf * kWChunk, kEvD = kEvB * (Row::kW + 1) * kEvC;
-    constexpr int kWarpD = kBisD > kEvD ? kBisD : kEvD;
-    return (size_t)kWarpsPerCta * (kWarpD * 8 + (kWBuf + kEvB) * 8);
-}
-
-template <class Row>
-static int fused_fit() {
-    int n = 1;
-    const size_t sm = fused_smem<Row>();
-    cudaFuncSetAttribute(k_bisect_eigvec<Row>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_bisect_eigvec<Row>, kWarpsPerCta * 32, sm) !=
-        cudaSuccess)
-        n = 1;
-    return n < 1 ? 1 : n;
-}
-
-template <class Row>
-static int fused_launch(cudaStream_t st, int grid, const FusedArgs& a) {
-    if (a.ea.g || a.ea.vfull || !a.ev_done || !a.pstat || !a.queue) return -1;
-    const size_t sm = fused_smem<Row>();
-    cudaFuncSetAttribute(k_bisect_eigvec<Row>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_bisect_eigvec<Row><<<grid, kWarpsPerCta * 32, sm, st>>>(a);
-    return 1;
-}
-
-int fused_ctas_per_sm() { return fused_fit<EssRows>(); }
-int launch_bisect_eigvec(cudaStream_t st, int grid, const FusedArgs& a) { return fused_launch<EssRows>(st, grid, a); }
-int fused_wmod_ctas_per_sm() { return fused_fit<WmodRows>(); }
-int launch_bisect_eigvec_wmod(cudaStream_t st, int grid, const FusedArgs& a) {
-    return fused_launch<WmodRows>(st, grid, a);
 }
 
 // ===========================================================================

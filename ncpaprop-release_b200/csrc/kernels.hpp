@@ -73,26 +73,19 @@ constexpr int kScanMax = 512;      // count slots per problem of the isolation s
 constexpr int kScanStep = 64;      // shifts per scan unit (one warp, two per lane)
 constexpr int kScanDefault = 256;  // shifts per problem unless the scan sizes them (wide-angle rows)
 constexpr int kChunk = 1024;      // doubles per TMA chunk of the diagonal
-constexpr int kBlk = 16;          // eigenvector checkpoint interval
-constexpr int kCkRows = 128;      // twist candidates of the reduction-only eigenvector items
-// elements of each eigenvector checkpoint array per warp slot for grids of up
-// to nz points: q every kBlk rows (items that write full vectors) or three
-// sums every kCkRows rows (items that only reduce)
+constexpr int kBlk = 16;          // rows between rescalings in k_eigvec
+constexpr int kCkRows = 128;      // rows between twist candidates
+// elements of each checkpoint array per warp slot of k_eigvec for grids of up
+// to nz points (room for the sums of every coarse row)
 inline long long ck_slot_elems(long long nz) {
     const long long a = (nz + kBlk - 1) / kBlk, b = 3 * ((nz + kCkRows - 1) / kCkRows);
     return (a > b ? a : b) * 32;
 }
 // elements per warp slot of the coarse rows of grids of up to nz points
 inline long long coarse_slot_elems(long long nz) { return (nz + kCkRows - 1) / kCkRows * 32; }
-constexpr int kThreads = 256;     // threads of the scan CTAs
 constexpr int kWItem = 32;        // eigenvalues per warp work item of the bisection
 constexpr int kEvItem = 32;       // eigenvalues per warp work item of the eigenvector kernel
 constexpr int kEvWarpsPerCta = 4; // warps per eigenvector CTA
-// bisection item scheduler state (ints): ticket, heavy-end and light-end
-// counters, then one arrival counter per (SM < kSchedSms, sub-partition)
-constexpr int kSchedSms = 256;
-constexpr int kSchedInts = 3 + 4 * kSchedSms;
-constexpr int kSchedWorkers = 2;  // default bisection warps per warp scheduler
 
 // knot-level derived quantities
 int launch_steffen(cudaStream_t st, int n, const double* x, const double* y, int batch, int ystride,
@@ -122,97 +115,29 @@ int launch_build_matrix(cudaStream_t st, int nk, const double* zk, const double*
 // WKB window and scaled bounds (K2); the records carry wkb_trial = kWkbNone
 int launch_window(cudaStream_t st, int P, ProblemInfo* pinfo, const double* kz2, int wkb, int wvnum,
                   double c_min, double c_max, unsigned* err);
-// isolation scan (K3a): sizes each problem's scan (ProblemInfo::n_scan) from
-// an estimate of its mode count, then pinfo[p].n_scan Sturm counts per
-// problem at counts[p * kScanMax + t]
-// slots > 0 (warp schedulers of the device: 4 x SMs) trims the batch's scan
-// to a whole number of units per scheduler; sched (kSchedInts ints, zeroed)
-// then has the units claimed per scheduler (see k_scan)
-int launch_scan(cudaStream_t st, int P, ProblemInfo* pinfo, const double* s, int* counts, unsigned* err,
-                int slots = 0, int* sched = nullptr);
-// multisection/bisection over work items (K3); step_counter (optional)
-// accumulates the Sturm recurrence steps swept; sched (kSchedInts ints,
-// zeroed) runs a cost-ordered item list (order = 1 in launch_make_items) with
-// `workers` warps per warp scheduler (the first from the heavy end of the
-// list, the others from the light end); null maps items round-robin
-int launch_bisect(cudaStream_t st, int grid, const ProblemInfo* pinfo, const double* s, const int* counts,
-                  const WorkItem* items, int n_items, int* counter, double tol, double* mu, unsigned* err,
-                  unsigned long long* step_counter, const int* n_items_dev = nullptr, int* sched = nullptr,
-                  int workers = kSchedWorkers);
-int bisect_ctas_per_sm();
 // FP64 throughput probe: each thread runs n_iter iterations of 8 independent
 // FMA chains; out receives a value that keeps the chains live
 int launch_fp64_probe(cudaStream_t st, int grid, int block, int n_iter, double* out);
-// twisted-factorisation eigenvectors + fused reductions (K4)
+// mode values by twisted factorisation of the rows (K4s, noalloc.cu)
 struct EigvecArgs {
     const ProblemInfo* pinfo;
-    const double* s;   // rows at pinfo[p].s_off
-    const double* w;   // rows at pinfo[p].w_off
-    const double* g;   // rows at pinfo[p].s_off, or null
+    const double* s;  // rows at pinfo[p].s_off
+    const double* w;  // rows at pinfo[p].w_off
     const WorkItem* items;
     int n_items;
-    const int* n_items_dev;  // when set, the item count is read here (built on the device)
-    const int* ev_done;      // when set, items with ev_done[it] != 0 are skipped (done in the fused launch)
-    int* counter;
     const double* mu;
     double* kr;
     double* ki;
     double* vs;
     double* vr;
     double* vg;
-    double* vfull;            // optional: per problem [nz x M] at vfull_off[p]
-    const long long* vfull_off;
-    double* ck_q1;            // checkpoint scratch, one slot per warp of the grid
+    double* ck_q1;  // checkpoint scratch, one slot per warp of the grid
     double* ck_q2;
     int* ck_e;
-    long long ck_slot_stride; // elements per warp slot (blocks of the largest grid x 32)
+    long long ck_slot_stride;  // elements per warp slot (blocks of the largest grid x 32)
     unsigned* err;
 };
 int launch_eigvec(cudaStream_t st, int grid, const EigvecArgs& a);
-// Bisection and eigenvectors in one launch (ESS rows, no group speeds, no
-// full vectors): bisection items as launch_bisect, then eigenvector items of
-// finished problems from a ready queue.  pstat[3 P] from k_make_items;
-// queue[ev_cap], q_head, q_tail and ev_done[ev_cap] zeroed before the launch.
-// A k_eigvec launch with ea.ev_done = ev_done must follow: it runs the items
-// this launch did not finish.
-struct FusedArgs {
-    int P;
-    const ProblemInfo* pinfo;
-    const double* s;
-    const int* counts;
-    const WorkItem* bis;
-    const int* n_bis_dev;
-    double tol;
-    double* mu;
-    unsigned* err;
-    int* pstat;
-    int* queue;
-    int* q_head;
-    int* q_tail;
-    int* ev_done;
-    unsigned long long wait_ns;  // a consumer gives up on an empty slot after this long
-    int* sched;                  // bisection item scheduler (kSchedInts, zeroed) or null (round-robin)
-    int workers;                 // bisection warps per warp scheduler with sched
-    int ev_workers_only;         // only warps that ran bisection take eigenvector items
-    EigvecArgs ea;
-};
-int launch_bisect_eigvec(cudaStream_t st, int grid, const FusedArgs& a);
-int fused_ctas_per_sm();
-// the same on the wide-angle rows (mu = kappa; follow with launch_eigvec_wmod)
-int launch_bisect_eigvec_wmod(cudaStream_t st, int grid, const FusedArgs& a);
-int fused_wmod_ctas_per_sm();
-// Work items built on the device from the Sturm scan: per problem c_lo, c_hi,
-// M and CSR offset in pinfo; bisection items (<= bis_item eigenvalues, sizes
-// balanced inside a problem) and eigenvector items (kEvItem) appended;
-// tot = {n_bisect_items, n_eigvec_items, total modes}.  Sets kErrTooMany if a
-// problem exceeds max_modes (its M is then clamped) or a capacity is exceeded.
-// pstat (optional, 3 P ints): per problem the number of bisection items, the
-// first eigenvector item and the number of eigenvector items.  order = 1
-// lists the bisection items by estimated cost, heaviest problems first (for
-// P <= 4096; problem order otherwise)
-int launch_make_items(cudaStream_t st, int P, ProblemInfo* pinfo, const int* counts, int max_modes, int bis_item,
-                      WorkItem* bis_items, int bis_cap, WorkItem* ev_items, int ev_cap, int* tot, unsigned* err,
-                      int* pstat = nullptr, int order = 0);
 // The eigen-solve on panel expansions (panel.cu) of the ESS rows or, wide, of
 // the wide-angle rows (mu = kappa = h k; W1 for a weight of ones).  T: block
 // transfer matrices (kRecT doubles a record), W0, W1: their derivatives for the
@@ -278,8 +203,6 @@ int launch_panel_modes(cudaStream_t st, bool wide, int grid, const ModesArgs& a,
 int launch_panel_fill(cudaStream_t st, bool wide, int P, int nz_max, int m_max, const ModesArgs& a);
 int panel_ctas_per_sm();
 
-// resident eigenvector CTAs per SM for the variant selected by a
-int eigvec_ctas_per_sm(const EigvecArgs& a);
 // modal sums
 int launch_tl1d(cudaStream_t st, int P, const ProblemInfo* pinfo, const double* kr, const double* ki,
                 const double* vs, const double* vr, int nr, double dr, int lossless, double* re, double* im,
@@ -311,8 +234,7 @@ int launch_bb_pulse(cudaStream_t st, int nfreq, const double* f, const double* s
 int launch_src_dft(cudaStream_t st, int n, const double* x, double dt, int nfft, int nfreq, const double* tw,
                    double* s);
 
-// Wide-angle (WMod) modes (wmod.cu).  Rows of T(k) h^2 in the WmodRows
-// format (device_common.cuh): two doubles per row, (B_i, U_i) interleaved, at
+// Wide-angle (WMod) modes (wmod.cu).  Rows of T(k) h^2: two doubles per row, (B_i, U_i) interleaved, at
 // 2 * pinfo[p].s_off (the s layout, rows padded to kChunk); row 0's ground
 // term goes to pinfo[p].g0.  The eigen-solve runs in kappa = h k: pinfo
 // k_min / k_max bound the window in k, kappa_min = k_min dz.
@@ -322,19 +244,6 @@ int launch_wmod_build(cudaStream_t st, int nk, const double* zk, const double* c
                       const double* wck, const double* wcc, const double* ceffk, const double* ceffc, int n_az,
                       int P, ProblemInfo* pinfo, int nz, int nz_pad, double z_min, double dz_grid, double dz,
                       double admittance, double* rows, double* kz2);
-int launch_wscan(cudaStream_t st, int P, const ProblemInfo* pinfo, const double* rows, int* counts, unsigned* err);
-// k_bisect on the wide-angle rows: mu receives kappa = h k; tol is relative
-// to kappa_max; step_counter (optional) counts chain steps (3 FMA each) as
-// launch_bisect does
-int launch_bisect_wmod(cudaStream_t st, int grid, const ProblemInfo* pinfo, const double* rows, const int* counts,
-                       const WorkItem* items, double tol, double* mu, unsigned* err,
-                       unsigned long long* step_counter, const int* n_items_dev, int* sched = nullptr,
-                       int workers = kSchedWorkers);
-int bisect_wmod_ctas_per_sm();
-// eigenvectors of the wide-angle rows: EigvecArgs with s = rows, mu = kappa,
-// g = null; vectors normalised to sum v^2 dz = 1 / (1 + k^2)
-int launch_eigvec_wmod(cudaStream_t st, int grid, const EigvecArgs& a);
-int eigvec_wmod_ctas_per_sm(const EigvecArgs& a);
 
 // K5 modal sum on the tensor cores (modal_sum.cu)
 struct MsPlan {

@@ -111,7 +111,7 @@ struct ncpa_ctx {
     long long launches = 0;
     int num_sms = 148;
     DevBuf d_err;                  // device status word
-    DevBuf ck1, ck2, cke;          // eigenvector checkpoint scratch
+    DevBuf ck1, cke;               // eigenvector checkpoint scratch
     DevBuf ex;                     // panel expansions
     std::map<int, DevBuf> twiddle; // per nfft
     DevBuf bb_out;                 // waveforms kept in HBM (NULL host buffer)
@@ -127,15 +127,10 @@ struct ncpa_ctx {
     int ms_last_variant = 0, ms_last_fmt = 0;
     std::vector<double> ms_last_times;  // per variant, ms, of the last tuning run
     int item_override = 0;         // eigenvalues per bisection item (0: chosen per solve); NCPA_BISECT_ITEM
-    // bisection items listed by estimated cost and spread over the warp
-    // schedulers (heaviest first); NCPA_BISECT_ORDER=0 keeps problem order and
+    // work items listed by estimated cost, heaviest first, and taken by the
+    // warps as they get free; NCPA_BISECT_ORDER=0 keeps problem order and
     // round-robin warps.  Results do not depend on it.
     bool bis_order = true;
-    int bis_workers = ncpa::kSchedWorkers;  // bisection warps per warp scheduler; NCPA_BISECT_WORKERS
-    // fused launch: only the bisection warps take eigenvector items (as their
-    // bisection ends), the others leave them to the k_eigvec launch that
-    // follows; NCPA_FUSE_EV_WORKERS=0 lets every warp of the launch take them
-    bool fuse_ev_workers = true;
     // modal sum of ncpa_tl_2d (the front ends' tloss_2d.nm): NCPA_SUM_FP64,
     // or NCPA_SUM_TC_GUARDED with NCPA_TL2D_SUM=3
     int tl2d_method = NCPA_SUM_FP64;
@@ -143,9 +138,6 @@ struct ncpa_ctx {
     // NCPA_SCAN_TRIM=0 keeps every problem's own estimate
     bool scan_trim = true;
     bool fuse_solve = true;        // fused bisection + eigenvector launch; NCPA_FUSE_SOLVE=0 turns it off
-    // how long a consumer of the fused launch waits for an empty queue slot
-    // before leaving the item to the following launch; NCPA_FUSE_WAIT_NS
-    unsigned long long fuse_wait_ns = 1000000000ull;
     double* h_pin = nullptr;       // small pinned host buffer for scalars read back per solve
     int* h_tot = nullptr;          // pinned: item and mode totals of a device-built solve
     size_t h_pin_n = 0;
@@ -1258,17 +1250,11 @@ ncpa_status ncpa_ctx_create(ncpa_ctx** out, const ncpa_ctx_opts* opts) {
         const char* tv = std::getenv("NCPA_TIMING");
         ctx->timing = tv && tv[0] == '1';
         if (const char* fv = std::getenv("NCPA_FUSE_SOLVE")) ctx->fuse_solve = fv[0] != '0';
-        if (const char* wv = std::getenv("NCPA_FUSE_WAIT_NS")) ctx->fuse_wait_ns = std::strtoull(wv, nullptr, 10);
         if (const char* mv = std::getenv("NCPA_MS_TUNE")) ctx->ms_tune = mv[0] != '0';
         if (const char* ov = std::getenv("NCPA_BISECT_ORDER")) ctx->bis_order = ov[0] != '0';
-        if (const char* ev = std::getenv("NCPA_FUSE_EV_WORKERS")) ctx->fuse_ev_workers = ev[0] != '0';
         if (const char* sv = std::getenv("NCPA_SCAN_TRIM")) ctx->scan_trim = sv[0] != '0';
         if (const char* tv2 = std::getenv("NCPA_TL2D_SUM"))
             ctx->tl2d_method = std::atoi(tv2) == NCPA_SUM_TC_GUARDED ? NCPA_SUM_TC_GUARDED : NCPA_SUM_FP64;
-        if (const char* wv = std::getenv("NCPA_BISECT_WORKERS")) {
-            const int v = std::atoi(wv);
-            if (v >= 1 && v <= 16) ctx->bis_workers = v;
-        }
         // tuning override of the eigenvalues per bisection item (1..32)
         if (const char* iv = std::getenv("NCPA_BISECT_ITEM")) {
             const int v = std::atoi(iv);
@@ -1290,7 +1276,6 @@ ncpa_status ncpa_ctx_destroy(ncpa_ctx* ctx) {
     ctx->d_stats.release();
     ctx->ex.release();
     ctx->ck1.release();
-    ctx->ck2.release();
     ctx->cke.release();
     ctx->d_err.release();
     for (DevBuf* b : {&ctx->ms_img, &ctx->ms_q, &ctx->ms_tab, &ctx->ms_raw, &ctx->ms_vz, &ctx->ms_idx, &ctx->ms_re,

@@ -136,18 +136,14 @@ extern "C" ncpa_status ncpa_eigvec_static(const double* s, const double* w, int 
     a.pinfo = reinterpret_cast<const ProblemInfo*>(base + kOffInfo);
     a.s = reinterpret_cast<const double*>(base + kOffS);
     a.w = reinterpret_cast<const double*>(base + kOffW);
-    a.g = nullptr;
     a.items = reinterpret_cast<const WorkItem*>(base + kOffItems);
     a.n_items = (n_modes + ncpa::kEvItem - 1) / ncpa::kEvItem;
-    a.counter = reinterpret_cast<int*>(base + kOffCounter);
     a.mu = mu;
     a.kr = re_k;
     a.ki = im_k;
     a.vs = v_src;
     a.vr = v_rcv;
     a.vg = nullptr;
-    a.vfull = nullptr;
-    a.vfull_off = nullptr;
     a.ck_q1 = reinterpret_cast<double*>(base + kOffQ1);
     a.ck_q2 = reinterpret_cast<double*>(base + kOffQ2);
     a.ck_e = reinterpret_cast<int*>(base + kOffE);

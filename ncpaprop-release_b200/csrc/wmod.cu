@@ -21,20 +21,6 @@
 
 namespace ncpa {
 
-namespace {
-
-constexpr int kWScanThreads = kScanDefault / 2;  // two shifts per thread
-constexpr int kWsRows = 512;                    // rows per scan ring chunk (8 KB)
-constexpr int kWsBuf = 4;                       // scan ring slots
-
-__device__ __forceinline__ double wscan_x(double lo, double hi, int t) {
-    if (t == 0) return lo;
-    if (t == kScanDefault - 1) return hi;
-    return lo + (hi - lo) * ((double)t / (double)(kScanDefault - 1));
-}
-
-}  // namespace
-
 // wind component along each azimuth at the knots (the wc term of
 // k_ceff_knots, same expression)
 __global__ void k_wc_knots(int n, int n_az, const double* __restrict__ az, const double* __restrict__ ws,
@@ -137,70 +123,6 @@ int launch_wmod_build(cudaStream_t st, int nk, const double* zk, const double* c
     dim3 grid((nz_pad + 255) / 256, n_az, (n_f + kWbFreqs - 1) / kWbFreqs);
     k_wmod_build<<<grid, 256, 0, st>>>(nk, zk, c0k, c0c, wck, wcc, ceffk, ceffc, n_az, n_f, pinfo, nz, nz_pad, z_min,
                                        dz_grid, dz, admittance, reinterpret_cast<double2*>(rows), kz2);
-    return 1;
-}
-
-// ---------------------------------------------------------------------------
-// Isolation scan: kScanDefault counts per problem on an even grid of
-// [kappa_min, kappa_max] (the layout k_make_items reads); the CTA streams the
-// rows through a kWsBuf-deep TMA ring, each thread runs two shifts
-// (WmodRows::pair: p_{-2} = -g0, p_{-1} = 1, p_i = t_i p_{i-1} - p_{i-2}).
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kWScanThreads) k_wscan(const ProblemInfo* __restrict__ pinfo,
-                                                         const double* __restrict__ rows, int* __restrict__ counts,
-                                                         unsigned* err) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    double* buf = reinterpret_cast<double*>(smem_raw);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + (size_t)kWsBuf * kWsRows * 16);
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < kWsBuf; ++k) mbar_init(&bars[k], 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
-    const int p = blockIdx.x;
-    const ProblemInfo pi = pinfo[p];
-    const double* src = rows + 2 * pi.s_off;
-    const double lo = WmodRows::scan_lo(pi), hi = WmodRows::scan_hi(pi);
-    const int t0 = threadIdx.x, t1 = threadIdx.x + kWScanThreads;
-    const double xa = wscan_x(lo, hi, t0), xb = wscan_x(lo, hi, t1);
-    const int nz = pi.nz;
-    const int nch = (nz + kWsRows - 1) / kWsRows;
-    if (threadIdx.x == 0)
-        for (int c = 0; c < nch && c < kWsBuf; ++c) {
-            mbar_expect_tx(&bars[c], kWsRows * 16);
-            tma_load_1d(buf + (size_t)c * 2 * kWsRows, src + (size_t)c * 2 * kWsRows, kWsRows * 16, &bars[c]);
-        }
-    SturmState A, B;
-    A.reset();
-    B.reset();
-    A.p0 = B.p0 = WmodRows::p_init(pi);
-    for (int c = 0; c < nch; ++c) {
-        const int slot = c % kWsBuf;
-        mbar_wait_bounded(&bars[slot], (c / kWsBuf) & 1u, err);
-        const double* b = buf + (size_t)slot * 2 * kWsRows;
-        const int valid = min(kWsRows, nz - c * kWsRows);
-        const int nw = valid >> 5;
-        for (int w = 0; w < nw; ++w) WmodRows::pair(A, B, b + 64 * w, xa, xb);
-        for (int i = nw * 32; i < valid; ++i) {
-            WmodRows::step(A, b, i, xa);
-            WmodRows::step(B, b, i, xb);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0 && c + kWsBuf < nch) {
-            fence_proxy_async();
-            mbar_expect_tx(&bars[slot], kWsRows * 16);
-            tma_load_1d(buf + (size_t)slot * 2 * kWsRows, src + (size_t)(c + kWsBuf) * 2 * kWsRows, kWsRows * 16,
-                        &bars[slot]);
-        }
-    }
-    counts[(size_t)p * kScanMax + t0] = A.cnt;
-    counts[(size_t)p * kScanMax + t1] = B.cnt;
-}
-
-int launch_wscan(cudaStream_t st, int P, const ProblemInfo* pinfo, const double* rows, int* counts, unsigned* err) {
-    if (P <= 0) return 0;
-    const size_t sm = (size_t)kWsBuf * kWsRows * 16 + kWsBuf * 8;
-    k_wscan<<<P, kWScanThreads, sm, st>>>(pinfo, rows, counts, err);
     return 1;
 }
 
