@@ -38,20 +38,24 @@ __device__ double steffen_slope(int n, const double* __restrict__ x, const doubl
     return (sgn1(sl) + sgn1(sr)) * m;
 }
 
+// coefficients of the interval i
+__device__ __forceinline__ void steffen_coef(int n, const double* __restrict__ x, const double* __restrict__ y, int i,
+                                             double* __restrict__ c) {
+    const double y0 = steffen_slope(n, x, y, i), y1 = steffen_slope(n, x, y, i + 1);
+    const double h = x[i + 1] - x[i];
+    const double s = (y[i + 1] - y[i]) / h;
+    c[0] = (y0 + y1 - 2.0 * s) / h / h;
+    c[1] = (3.0 * s - 2.0 * y0 - y1) / h;
+    c[2] = y0;
+    c[3] = y[i];
+}
+
 __global__ void k_steffen(int n, const double* __restrict__ x, const double* __restrict__ yall, int batch,
                           int ystride, double* __restrict__ call, int cstride) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     int b = blockIdx.y;
     if (i >= n - 1 || b >= batch) return;
-    const double* y = yall + (size_t)b * ystride;
-    double y0 = steffen_slope(n, x, y, i), y1 = steffen_slope(n, x, y, i + 1);
-    double h = x[i + 1] - x[i];
-    double s = (y[i + 1] - y[i]) / h;
-    double* c = call + (size_t)b * cstride + 4 * i;
-    c[0] = (y0 + y1 - 2.0 * s) / h / h;
-    c[1] = (3.0 * s - 2.0 * y0 - y1) / h;
-    c[2] = y0;
-    c[3] = y[i];
+    steffen_coef(n, x, yall + (size_t)b * ystride, i, call + (size_t)b * cstride + 4 * i);
 }
 
 int launch_steffen(cudaStream_t st, int n, const double* x, const double* y, int batch, int ystride,
@@ -211,93 +215,105 @@ __device__ double sb_alpha(const SbKnot& K, double freq) {
     return a_cl + a_rot + a_diff + a_vib;
 }
 
-constexpr int kSbFreqs = 8;  // frequencies per thread of k_alpha_knots
+// Knot-level fields of every group and their Steffen coefficients in one
+// launch: c_eff per azimuth (and, for wide-angle rows, the wind component and
+// c0), absorption per frequency.  A block takes kKnotStep intervals of one
+// field, or of kSbFreqs frequencies' absorptions (the knot's part is evaluated
+// once), with the knots around them in shared memory.  Bound by launch latency:
+// 32 groups of one problem took 128 launches for this (with their uploads and
+// allocations 1.9 ms a solve, now 0.1).
+constexpr int kSbFreqs = 8;  // frequencies of an absorption block
+constexpr int kKnotThreads = 128, kKnotStep = kKnotThreads - 3;
 
-__global__ void k_alpha_knots(int n, int n_f, const double* __restrict__ freqs, const double* __restrict__ z,
-                              const double* __restrict__ t, const double* __restrict__ p,
-                              const double* __restrict__ rho, double* __restrict__ alpha) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int f0 = blockIdx.y * kSbFreqs;
-    if (k >= n) return;
-    const SbKnot K = sb_knot(z[k] * 0.001, t[k], p[k], rho[k]);
-    const int f1 = min(n_f, f0 + kSbFreqs);
-    for (int f = f0; f < f1; ++f) alpha[(size_t)f * n + k] = sb_alpha(K, freqs[f]);
+__global__ void __launch_bounds__(kKnotThreads) k_knots(const GroupDesc* __restrict__ desc, int tiles) {
+    __shared__ double ys[kKnotThreads];
+    const GroupDesc& G = desc[blockIdx.z];
+    const int n = G.nk, t = threadIdx.x, k0 = (blockIdx.x % tiles) * kKnotStep - 1;
+    if (k0 + 1 >= n - 1) return;
+    int row = blockIdx.x / tiles;
+    const int k = min(max(k0 + t, 0), n - 1);
+    const bool own = k0 + t == k && ((t >= 1 && t <= kKnotStep) || k == n - 1);
+    // one field: its value v at this thread's knot, y and coefficients to global
+    auto field = [&](double v, double* __restrict__ y, double* __restrict__ coef) {
+        ys[t] = v;
+        if (own) y[k] = v;
+        __syncthreads();
+        const int i = k0 + t;
+        if (t >= 1 && t <= kKnotStep && i < n - 1) steffen_coef(n, G.zk, ys - k0, i, coef + 4 * i);
+        __syncthreads();
+    };
+    if (row < G.n_az * (G.wide ? 2 : 1)) {
+        const int a = row % G.n_az;
+        const double az_rad = G.az[a] * kPi / 180.0;
+        const double dir = G.wd[k] * kPi / 180.0;
+        const double wc = G.ws[k] * cos(dir - az_rad);
+        if (row < G.n_az) field(wc + G.c0[k], G.ceffk + (size_t)a * n, G.ceffc + (size_t)a * 4 * (n - 1));
+        else field(wc, G.wck + (size_t)a * n, G.wcc + (size_t)a * 4 * (n - 1));
+        return;
+    }
+    row -= G.n_az * (G.wide ? 2 : 1);
+    if (G.wide) {
+        if (row == 0) {
+            field(G.c0[k], G.c0k, G.c0c);
+            return;
+        }
+        --row;
+    }
+    const int f0 = row * kSbFreqs, f1 = min(G.n_f, f0 + kSbFreqs);
+    if (f0 >= f1) return;
+    SbKnot K;
+    if (!G.attn) K = sb_knot(G.zk[k] * 0.001, G.t[k], G.p[k], G.rho[k]);
+    for (int f = f0; f < f1; ++f)
+        field(G.attn ? G.attn[k] : sb_alpha(K, G.freqs[f]), G.alpha + (size_t)f * n, G.alphac + (size_t)f * 4 * (n - 1));
 }
 
-int launch_alpha_knots(cudaStream_t st, int n, int n_f, const double* freqs, const double* z, const double* t,
-                       const double* p, const double* rho, double* alpha) {
-    dim3 grid((n + 127) / 128, (n_f + kSbFreqs - 1) / kSbFreqs);
-    k_alpha_knots<<<grid, 128, 0, st>>>(n, n_f, freqs, z, t, p, rho, alpha);
-    return 1;
-}
+// rho at the source and receiver rows and the weights w_i = ((omega / c_T)
+// alpha_i) 2 of doPerturb, c_T = sqrt(1.4 P / rho), of every group.  A thread
+// takes one grid point and kAwFreqs frequencies: one knot search, every value
+// by spline_get's expression; padding rows are zero.
+constexpr int kAwFreqs = 16;
 
-__global__ void k_grid_common(int nk, const double* __restrict__ zk, const double* __restrict__ rho,
-                              const double* __restrict__ rcoef, const double* __restrict__ p,
-                              const double* __restrict__ pcoef, int nz, double z_min, double dz_grid,
-                              double* __restrict__ rho_g, double* __restrict__ ct_g) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nz) return;
-    double h = z_min + i * dz_grid;
-    double r = spline_get(nk, zk, rho, rcoef, h);
-    double pv = spline_get(nk, zk, p, pcoef, h);
-    rho_g[i] = r;
-    ct_g[i] = sqrt(1.4 * pv / r);
-}
-
-int launch_grid_common(cudaStream_t st, int nk, const double* zk, const double* rho, const double* rcoef,
-                       const double* p, const double* pcoef, int nz, double z_min, double dz_grid,
-                       double* rho_g, double* ct_g) {
-    k_grid_common<<<(nz + 255) / 256, 256, 0, st>>>(nk, zk, rho, rcoef, p, pcoef, nz, z_min, dz_grid, rho_g,
-                                                    ct_g);
-    return 1;
-}
-
-// w_i = ((omega / c_T) alpha_i) 2, the integrand weight of doPerturb.  A
-// thread takes one grid point and kAwFreqs frequencies: the knot search is
-// shared, each alpha_f(z_i) is spline_get's expression.
-constexpr int kAwFreqs = 8;
-
-__global__ void k_attn_weight(int nk, const double* __restrict__ zk, const double* __restrict__ alpha,
-                              const double* __restrict__ acoef, int n_f, const double* __restrict__ freqs,
-                              int nz, double z_min, double dz_grid, const double* __restrict__ ct_g,
-                              double* __restrict__ w, int wstride) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int f0 = blockIdx.y * kAwFreqs;
-    if (i >= nz) return;
-    const double h = z_min + i * dz_grid;
+__global__ void __launch_bounds__(256) k_grid_fields(const GroupDesc* __restrict__ desc) {
+    const GroupDesc& G = desc[blockIdx.z];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, nk = G.nk;
+    const int f0 = blockIdx.y * kAwFreqs, f1 = min(G.n_f, f0 + kAwFreqs);
+    if (i >= G.nz_pad || f0 >= f1) return;
+    if (i >= G.nz) {
+        for (int f = f0; f < f1; ++f) G.w[(size_t)f * G.nz_pad + i] = 0.0;
+        return;
+    }
+    const double h = G.z_min + i * G.dz_grid;
     int where = 0, kn = 0;  // 0 inside the knots, 1 above, 2 below
     double t = 0.0;
-    if (h > zk[nk - 1]) {
+    if (h > G.zk[nk - 1]) {
         where = 1;
-    } else if (h < zk[0]) {
+    } else if (h < G.zk[0]) {
         where = 2;
     } else {
-        kn = knot_search(nk, zk, h);
-        t = h - zk[kn];
+        kn = knot_search(nk, G.zk, h);
+        t = h - G.zk[kn];
     }
-    const double ct = ct_g[i];
-    const int f1 = min(n_f, f0 + kAwFreqs);
+    auto at = [&](const double* __restrict__ y, const double* __restrict__ coef) {
+        if (where == 1) return y[nk - 1];
+        if (where == 2) return y[0];
+        const double* c = coef + 4 * kn;
+        return c[3] + t * (c[2] + t * (c[1] + t * c[0]));
+    };
+    const double r = at(G.rho, G.rcoef), pv = at(G.p, G.pcoef);
+    if (blockIdx.y == 0) {
+        if (i == G.isrc) G.rho_pair[0] = r;
+        if (i == G.ircv) G.rho_pair[1] = r;
+    }
+    const double ct = sqrt(1.4 * pv / r);
+    const double *__restrict__ al = G.alpha, *__restrict__ ac = G.alphac, *__restrict__ fr = G.freqs;
+    double* __restrict__ w = G.w + i;
+    const int wstride = G.nz_pad;
+#pragma unroll 4
     for (int f = f0; f < f1; ++f) {
-        double a;
-        if (where == 1) {
-            a = alpha[(size_t)f * nk + nk - 1];
-        } else if (where == 2) {
-            a = alpha[(size_t)f * nk];
-        } else {
-            const double* c = acoef + (size_t)f * 4 * (nk - 1) + 4 * kn;
-            a = c[3] + t * (c[2] + t * (c[1] + t * c[0]));
-        }
-        const double omega = 2 * kPi * freqs[f];
-        w[(size_t)f * wstride + i] = ((omega / ct) * a) * 2;
+        const double a = at(al + (size_t)f * nk, ac + (size_t)f * 4 * (nk - 1));
+        const double omega = 2 * kPi * fr[f];
+        w[(size_t)f * wstride] = ((omega / ct) * a) * 2;
     }
-}
-
-int launch_attn_weight(cudaStream_t st, int nk, const double* zk, const double* alpha, const double* acoef,
-                       int n_f, const double* freqs, int nz, double z_min, double dz_grid, const double* ct_g,
-                       double* w, int wstride) {
-    dim3 grid((nz + 255) / 256, (n_f + kAwFreqs - 1) / kAwFreqs);
-    k_attn_weight<<<grid, 256, 0, st>>>(nk, zk, alpha, acoef, n_f, freqs, nz, z_min, dz_grid, ct_g, w, wstride);
-    return 1;
 }
 
 // ===========================================================================
@@ -318,18 +334,19 @@ __device__ __forceinline__ double warp_max(double v) {
 // c_eff is sampled once and every problem's entries use the same expressions.
 constexpr int kBmFreqs = 16;
 
-__global__ void __launch_bounds__(256) k_build_matrix(int nk, const double* __restrict__ zk,
-                                                      const double* __restrict__ ceffk,
-                                                      const double* __restrict__ ceffcoef, int n_az, int n_f,
-                                                      ProblemInfo* __restrict__ pinfo, int nz, int nz_pad,
-                                                      double z_min, double dz_grid, double dz, double admittance,
-                                                      double* __restrict__ s, double* __restrict__ kz2,
-                                                      double* __restrict__ g) {
+__global__ void __launch_bounds__(256) k_build_matrix(const GroupDesc* __restrict__ desc, int tiles) {
+    const GroupDesc& G = desc[blockIdx.z];
     const int a = blockIdx.y;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int f0 = blockIdx.z * kBmFreqs, f1 = min(n_f, f0 + kBmFreqs);
-    const double* ck = ceffk + (size_t)a * nk;
-    const double* cc = ceffcoef + (size_t)a * 4 * (nk - 1);
+    const int i = (blockIdx.x % tiles) * blockDim.x + threadIdx.x;
+    const int n_f = G.n_f, n_az = G.n_az, nk = G.nk, nz = G.nz, nz_pad = G.nz_pad;
+    const int f0 = (blockIdx.x / tiles) * kBmFreqs, f1 = min(n_f, f0 + kBmFreqs);
+    if (a >= n_az || f0 >= f1 || (blockIdx.x % tiles) * blockDim.x >= nz_pad) return;
+    const double* __restrict__ zk = G.zk;
+    const double* __restrict__ ck = G.ceffk + (size_t)a * nk;
+    const double* __restrict__ cc = G.ceffc + (size_t)a * 4 * (nk - 1);
+    const double z_min = G.z_min, dz_grid = G.dz_grid, dz = G.dz, admittance = G.admittance;
+    ProblemInfo* __restrict__ pinfo = G.pinfo;
+    double *__restrict__ s = G.s, *__restrict__ kz2 = G.kz2, *__restrict__ g = G.gs;
     const double h2 = dz * dz;
     const double bnd = (1. / (dz * admittance + 1)) / (dz * dz);
     double cmin = 1e300, cmax = -1e300;
@@ -392,15 +409,24 @@ __global__ void __launch_bounds__(256) k_build_matrix(int nk, const double* __re
     }
 }
 
-int launch_build_matrix(cudaStream_t st, int nk, const double* zk, const double* ceffk, const double* ceffcoef,
-                        int n_az, int P, ProblemInfo* pinfo, int nz, int nz_pad, double z_min, double dz_grid,
-                        double dz, double admittance, double* s, double* kz2, double* g) {
-    if (n_az < 1 || P % n_az != 0) return -1;
-    const int n_f = P / n_az;
-    dim3 grid((nz_pad + 255) / 256, n_az, (n_f + kBmFreqs - 1) / kBmFreqs);
-    k_build_matrix<<<grid, 256, 0, st>>>(nk, zk, ceffk, ceffcoef, n_az, n_f, pinfo, nz, nz_pad, z_min, dz_grid, dz,
-                                         admittance, s, kz2, g);
-    return 1;
+int launch_groups(cudaStream_t st, const GroupDesc* desc, const GroupDims& d) {
+    int n = 0;
+    for (int g0 = 0; g0 < d.n; g0 += 65535, n += 2) {  // grid.z limit
+        const int m = std::min(65535, d.n - g0);
+        const int tiles = (d.nk - 1 + kKnotStep - 1) / kKnotStep, rows = d.n_fields + (d.n_f + kSbFreqs - 1) / kSbFreqs;
+        k_knots<<<dim3(tiles * rows, 1, m), kKnotThreads, 0, st>>>(desc + g0, tiles);
+        k_grid_fields<<<dim3((d.nz_pad + 255) / 256, (d.n_f + kAwFreqs - 1) / kAwFreqs, m), 256, 0, st>>>(desc + g0);
+    }
+    return n;
+}
+
+int launch_build_matrix(cudaStream_t st, const GroupDesc* desc, const GroupDims& d) {
+    const int tiles = (d.nz_pad + 255) / 256;
+    int n = 0;
+    for (int g0 = 0; g0 < d.n; g0 += 65535, ++n)
+        k_build_matrix<<<dim3(tiles * ((d.n_f + kBmFreqs - 1) / kBmFreqs), d.n_az, std::min(65535, d.n - g0)), 256, 0,
+                         st>>>(desc + g0, tiles);
+    return n;
 }
 
 // ===========================================================================

@@ -95,23 +95,31 @@ int launch_profile_derived(cudaStream_t st, int n, const double* z, const double
                            int have_c0, double* c0, double* ws, double* wd);
 int launch_ceff_knots(cudaStream_t st, int n, int n_az, const double* az, const double* c0, const double* ws,
                       const double* wd, double* ceff);
-int launch_alpha_knots(cudaStream_t st, int n, int n_f, const double* freqs, const double* z, const double* t,
-                       const double* p, const double* rho, double* alpha);
-// grid sampling of the frequency-independent fields: rho, P on the grid and
-// c_T = sqrt(1.4 P / rho)
-int launch_grid_common(cudaStream_t st, int nk, const double* zk, const double* rho, const double* rcoef,
-                       const double* p, const double* pcoef, int nz, double z_min, double dz_grid,
-                       double* rho_g, double* ct_g);
-// attenuation weight w = 2 alpha omega / c_T for every frequency [n_f x nz]
-int launch_attn_weight(cudaStream_t st, int nk, const double* zk, const double* alpha, const double* acoef,
-                       int n_f, const double* freqs, int nz, double z_min, double dz_grid, const double* ct_g,
-                       double* w, int wstride);
-// matrix build (K1): s, optional kz2 = (omega/c)^2 and g = 1/c^2, each
-// [P x nz_pad]; fills ceff extrema / ground / top in ProblemInfo (the P
-// problems of one launch share one grid; their rows are nz_pad apart)
-int launch_build_matrix(cudaStream_t st, int nk, const double* zk, const double* ceffk, const double* ceffcoef,
-                        int n_az, int P, ProblemInfo* pinfo, int nz, int nz_pad, double z_min, double dz_grid,
-                        double dz, double admittance, double* s, double* kz2, double* g);
+// One group (a profile's frequencies x azimuths on one grid): what the knot-
+// and grid-level kernels read and write.  Problem p = frequency n_az + azimuth;
+// its rows are nz_pad apart in s (doubles, or (B, U) pairs when wide), gs and
+// kz2 (or null), its weights per frequency in w.
+struct GroupDesc {
+    int nk, nz, nz_pad, n_f, n_az, wide, isrc, ircv;
+    double z_min, dz_grid, dz, admittance;
+    const double *zk, *c0, *ws, *wd, *t, *p, *rho, *rcoef, *pcoef;
+    const double* attn;  // user attenuation at the knots, or null: Sutherland-Bass
+    const double *freqs, *az;
+    double *ceffk, *ceffc, *alpha, *alphac;  // [n_az | n_f][nk], coefficients [..][4 (nk - 1)]
+    double *wck, *wcc, *c0k, *c0c;           // wide: wind component, c0
+    double* rho_pair;                        // rho at the source and receiver rows
+    ProblemInfo* pinfo;
+    double *s, *w, *gs, *kz2;
+};
+// the largest of the groups' sizes (n groups; n_fields: c_eff and wide fields)
+struct GroupDims {
+    int n, nk, nz_pad, n_f, n_az, n_fields;
+};
+// knot- and grid-level fields of every group
+int launch_groups(cudaStream_t st, const GroupDesc* desc, const GroupDims& d);
+// matrix build (K1): s, optional kz2 = (omega/c)^2 and gs = 1/c^2; fills ceff
+// extrema / ground / top in ProblemInfo
+int launch_build_matrix(cudaStream_t st, const GroupDesc* desc, const GroupDims& d);
 // WKB window and scaled bounds (K2); the records carry wkb_trial = kWkbNone
 int launch_window(cudaStream_t st, int P, ProblemInfo* pinfo, const double* kz2, int wkb, int wvnum,
                   double c_min, double c_max, unsigned* err);
@@ -238,12 +246,7 @@ int launch_src_dft(cudaStream_t st, int n, const double* x, double dt, int nfft,
 // 2 * pinfo[p].s_off (the s layout, rows padded to kChunk); row 0's ground
 // term goes to pinfo[p].g0.  The eigen-solve runs in kappa = h k: pinfo
 // k_min / k_max bound the window in k, kappa_min = k_min dz.
-int launch_wc_knots(cudaStream_t st, int n, int n_az, const double* az, const double* ws, const double* wd,
-                    double* wc);
-int launch_wmod_build(cudaStream_t st, int nk, const double* zk, const double* c0k, const double* c0c,
-                      const double* wck, const double* wcc, const double* ceffk, const double* ceffc, int n_az,
-                      int P, ProblemInfo* pinfo, int nz, int nz_pad, double z_min, double dz_grid, double dz,
-                      double admittance, double* rows, double* kz2);
+int launch_wmod_build(cudaStream_t st, const GroupDesc* desc, const GroupDims& d);
 
 // K5 modal sum on the tensor cores (modal_sum.cu)
 struct MsPlan {

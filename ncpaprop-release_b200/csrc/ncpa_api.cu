@@ -394,71 +394,106 @@ double lamb_admittance(ncpa_ctx* ctx, const ncpa_profile* prof, double z_min) {
     return -der / val / 2.0;
 }
 
-// Device buffers of one group's knot-level and grid-level stages.
-struct GroupBufs {
-    DevBuf freqs, az, ceffk, ceffc, alpha, alphac, rho_g, ct_g;
-    double admittance = 0.0;
+// Device buffers of the groups' knot- and grid-level stages: one table of
+// records, one pool of values.
+struct GroupTable {
+    DevBuf desc, axes, vals, rho;
+    ncpa::GroupDims dims{};
+    bool wide = false;
 };
 
-// Allocates a group's buffers, uploads its frequencies and azimuths and, with
-// the Lamb-wave condition, computes the ground admittance (host work that
-// stays outside any captured graph).
-void prepare_group(ncpa_ctx* ctx, const ncpa_ess_params* prm, const Group& g, GroupBufs& b) {
+// Allocates the buffers, uploads frequencies, azimuths and records and, with
+// the Lamb-wave condition, computes the ground admittances (host work that
+// stays outside any captured graph).  d_pinfo, s, w, gs, kz2 (the last two may
+// be null) are the arrays the groups' offsets refer to.
+void prepare_groups(ncpa_ctx* ctx, const ncpa_ess_params* prm, const std::vector<Group>& groups, ProblemInfo* d_pinfo,
+                    double* s, double* w, double* gs, double* kz2, GroupTable& t) {
     cudaStream_t st = ctx->stream;
-    const int nk = g.prof->n;
-    upload(b.freqs, g.freqs, g.n_freq, st);
-    upload(b.az, g.az, g.n_az, st);
-    b.ceffk.alloc((size_t)g.n_az * nk * 8, st);
-    b.ceffc.alloc((size_t)g.n_az * 4 * (nk - 1) * 8, st);
-    b.alpha.alloc((size_t)g.n_freq * nk * 8, st);
-    b.alphac.alloc((size_t)g.n_freq * 4 * (nk - 1) * 8, st);
-    b.rho_g.alloc((size_t)g.nz * 8, st);
-    b.ct_g.alloc((size_t)g.nz * 8, st);
-    b.admittance = prm->lamb_wave_bc ? lamb_admittance(ctx, g.prof, g.geo.z_min) : 0.0;
+    t.wide = prm->method == NCPA_METHOD_WMOD;
+    const size_t n = groups.size();
+    std::vector<ncpa::GroupDesc> desc(n);
+    std::vector<double> axes;
+    size_t n_val = 0;
+    for (const Group& g : groups) {
+        const size_t nk = g.prof->n, rows = (t.wide ? 2 * g.n_az + 1 : g.n_az) + (size_t)g.n_freq;
+        n_val += rows * (nk + 4 * (nk - 1));
+        axes.insert(axes.end(), g.freqs, g.freqs + g.n_freq);
+        axes.insert(axes.end(), g.az, g.az + g.n_az);
+    }
+    t.vals.alloc(n_val * 8, st);
+    t.rho.alloc(2 * n * 8, st);
+    upload(t.axes, axes, st);
+    double* v = t.vals.as<double>();
+    const double* ax = t.axes.as<double>();
+    ncpa::GroupDims& d = t.dims;
+    d = ncpa::GroupDims{};
+    d.n = (int)n;
+    for (size_t i = 0; i < n; ++i) {
+        const Group& g = groups[i];
+        const ncpa_profile* f = g.prof;
+        ncpa::GroupDesc& D = desc[i];
+        D.nk = f->n;
+        D.nz = g.nz;
+        D.nz_pad = g.nz_pad;
+        D.n_f = g.n_freq;
+        D.n_az = g.n_az;
+        D.wide = t.wide ? 1 : 0;
+        D.isrc = g.geo.isrc;
+        D.ircv = g.geo.ircv;
+        D.z_min = g.geo.z_min;
+        D.dz_grid = g.geo.dz_grid;
+        D.dz = g.geo.dz;
+        D.admittance = prm->lamb_wave_bc ? lamb_admittance(ctx, f, g.geo.z_min) : 0.0;
+        D.zk = f->z.as<double>();
+        D.c0 = f->c0.as<double>();
+        D.ws = f->ws.as<double>();
+        D.wd = f->wd.as<double>();
+        D.t = f->t.as<double>();
+        D.p = f->p.as<double>();
+        D.rho = f->rho.as<double>();
+        D.rcoef = f->rcoef.as<double>();
+        D.pcoef = f->pcoef.as<double>();
+        D.attn = f->has_attn ? f->attn.as<double>() : nullptr;
+        D.freqs = ax;
+        D.az = ax + g.n_freq;
+        ax += g.n_freq + g.n_az;
+        auto take = [&](int rows, double*& y, double*& coef) {
+            y = v;
+            v += (size_t)rows * D.nk;
+            coef = v;
+            v += (size_t)rows * 4 * (D.nk - 1);
+        };
+        take(g.n_az, D.ceffk, D.ceffc);
+        take(g.n_freq, D.alpha, D.alphac);
+        if (t.wide) {
+            take(g.n_az, D.wck, D.wcc);
+            take(1, D.c0k, D.c0c);
+        }
+        D.rho_pair = t.rho.as<double>() + 2 * i;
+        D.pinfo = d_pinfo + g.p0;
+        D.s = s + (t.wide ? 2 : 1) * g.s_base;
+        D.w = w + g.w_base;
+        D.gs = gs ? gs + g.s_base : nullptr;
+        D.kz2 = kz2 ? kz2 + g.s_base : nullptr;
+        d.nk = std::max(d.nk, D.nk);
+        d.nz_pad = std::max(d.nz_pad, D.nz_pad);
+        d.n_f = std::max(d.n_f, D.n_f);
+        d.n_az = std::max(d.n_az, D.n_az);
+    }
+    d.n_fields = t.wide ? 2 * d.n_az + 1 : d.n_az;
+    upload(t.desc, desc, st);
 }
 
-// Knot-level fields, grid fields and matrices of one group's problems: only
-// kernel launches, device copies and memsets, plus one copy of rho at the
-// source and receiver grid points to rho_pair[0..1] (pinned host memory when
-// captured).  d_pinfo, s, w, gs, kz2 point at the group's first problem / row.
-void enqueue_group(ncpa_ctx* ctx, PhaseTimer& tm, const Group& g, GroupBufs& b, bool wkb, ProblemInfo* d_pinfo,
-                   double* s, double* w, double* gs, double* kz2, double* rho_pair) {
+// Knot-level fields, grid fields and matrices of all groups: kernel launches
+// and one copy of rho at the source and receiver grid points to rho_pairs
+// (pinned host memory).
+void enqueue_groups(ncpa_ctx* ctx, PhaseTimer& tm, const GroupTable& t, double* rho_pairs) {
     cudaStream_t st = ctx->stream;
-    const ncpa_profile* prof = g.prof;
-    const int nk = prof->n;
-    const int P = g.n_freq * g.n_az;
-    check_launch(ctx, ncpa::launch_ceff_knots(st, nk, g.n_az, b.az.as<double>(), prof->c0.as<double>(),
-                                              prof->ws.as<double>(), prof->wd.as<double>(), b.ceffk.as<double>()));
-    check_launch(ctx, ncpa::launch_steffen(st, nk, prof->z.as<double>(), b.ceffk.as<double>(), g.n_az, nk,
-                                           b.ceffc.as<double>(), 4 * (nk - 1)));
-    if (prof->has_attn) {
-        for (int f = 0; f < g.n_freq; ++f)
-            CK(cudaMemcpyAsync(b.alpha.as<double>() + (size_t)f * nk, prof->attn.p, nk * 8, cudaMemcpyDeviceToDevice,
-                               st));
-    } else {
-        check_launch(ctx, ncpa::launch_alpha_knots(st, nk, g.n_freq, b.freqs.as<double>(), prof->z.as<double>(),
-                                                   prof->t.as<double>(), prof->p.as<double>(),
-                                                   prof->rho.as<double>(), b.alpha.as<double>()));
-    }
-    check_launch(ctx, ncpa::launch_steffen(st, nk, prof->z.as<double>(), b.alpha.as<double>(), g.n_freq, nk,
-                                           b.alphac.as<double>(), 4 * (nk - 1)));
-    // ---- grid fields ----
-    CK(cudaMemsetAsync(w, 0, (size_t)g.n_freq * g.nz_pad * 8, st));
-    check_launch(ctx, ncpa::launch_grid_common(st, nk, prof->z.as<double>(), prof->rho.as<double>(),
-                                               prof->rcoef.as<double>(), prof->p.as<double>(),
-                                               prof->pcoef.as<double>(), g.nz, g.geo.z_min, g.geo.dz_grid,
-                                               b.rho_g.as<double>(), b.ct_g.as<double>()));
-    check_launch(ctx, ncpa::launch_attn_weight(st, nk, prof->z.as<double>(), b.alpha.as<double>(),
-                                               b.alphac.as<double>(), g.n_freq, b.freqs.as<double>(), g.nz,
-                                               g.geo.z_min, g.geo.dz_grid, b.ct_g.as<double>(), w, g.nz_pad));
-    CK(cudaMemcpyAsync(rho_pair, b.rho_g.as<double>() + g.geo.isrc, 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(rho_pair + 1, b.rho_g.as<double>() + g.geo.ircv, 8, cudaMemcpyDeviceToHost, st));
+    const ncpa::GroupDesc* desc = t.desc.as<ncpa::GroupDesc>();
+    check_launch(ctx, ncpa::launch_groups(st, desc, t.dims));
+    CK(cudaMemcpyAsync(rho_pairs, t.rho.p, (size_t)t.dims.n * 16, cudaMemcpyDeviceToHost, st));
     tm.mark("knots+grid");
-    // ---- K1 matrix ----
-    check_launch(ctx, ncpa::launch_build_matrix(st, nk, prof->z.as<double>(), b.ceffk.as<double>(),
-                                                b.ceffc.as<double>(), g.n_az, P, d_pinfo, g.nz, g.nz_pad,
-                                                g.geo.z_min, g.geo.dz_grid, g.geo.dz, b.admittance, s,
-                                                wkb ? kz2 : nullptr, gs));
+    check_launch(ctx, t.wide ? ncpa::launch_wmod_build(st, desc, t.dims) : ncpa::launch_build_matrix(st, desc, t.dims));
     tm.mark("matrix");
 }
 
@@ -818,45 +853,7 @@ void layout_panels(ncpa_modes* M, const std::vector<Group>& groups, const ncpa_e
         }
 }
 
-void solve_groups(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, std::vector<Group>& groups) {
-    cudaStream_t st = ctx->stream;
-    PhaseTimer tm(ctx);
-    tm.mark("start");
-    long long s_tot = 0, w_tot = 0;
-    layout_groups(M, groups, s_tot, w_tot);
-    layout_panels(M, groups, prm, 1.0);
-    upload(M->d_pinfo, M->info, st);
-    const bool wkb = wants_wkb(prm);
-    DevBuf s, w, gs, kz2;
-    s.alloc((size_t)s_tot * 8, st);
-    w.alloc((size_t)w_tot * 8, st);
-    if (wkb) kz2.alloc((size_t)s_tot * 8, st);
-    if (prm->want_group_speed) gs.alloc((size_t)s_tot * 8, st);
-    double* rho_pairs = pinned(ctx, 2 * groups.size());
-    ProblemInfo* d_pinfo = M->d_pinfo.as<ProblemInfo>();
-    std::vector<GroupBufs> gb(groups.size());
-    for (size_t gi = 0; gi < groups.size(); ++gi) prepare_group(ctx, prm, groups[gi], gb[gi]);
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
-        const Group& g = groups[gi];
-        enqueue_group(ctx, tm, g, gb[gi], wkb, d_pinfo + g.p0, s.as<double>() + g.s_base, w.as<double>() + g.w_base,
-                      prm->want_group_speed ? gs.as<double>() + g.s_base : nullptr,
-                      wkb ? kz2.as<double>() + g.s_base : nullptr, rho_pairs + 2 * gi);
-    }
-    solve_core(ctx, tm, M, prm, wkb, s, w, gs, kz2);
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
-        const Group& g = groups[gi];
-        const int np = g.n_freq * g.n_az;
-        for (int k = 0; k < np; ++k) {
-            M->rho_src_p[g.p0 + k] = rho_pairs[2 * gi];
-            M->rho_rcv_p[g.p0 + k] = rho_pairs[2 * gi + 1];
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// WMod (wide-angle) solve: WModeSolver::solve (WModeSolver.cpp:257-486)
-// ---------------------------------------------------------------------------
-// the matrix spacing of WModeSolver::solve, (maxheight - z_min) / Nz_grid
+// WMod (wide-angle): the matrix spacing of WModeSolver::solve, (maxheight - z_min) / Nz_grid
 // (WModeSolver.cpp:281; the sampling grid keeps setParams' spacing), and the
 // source / receiver rows on it
 void wmod_geometry(Group& g, const ncpa_ess_params* prm) {
@@ -870,93 +867,33 @@ void wmod_geometry(Group& g, const ncpa_ess_params* prm) {
         throw ApiError(NCPA_EINVAL, "source/receiver height outside the grid");
 }
 
-struct WmodBufs {
-    GroupBufs gb;           // frequencies, azimuths, c_eff and alpha knots, grid fields
-    DevBuf wck, wcc, c0c;   // wind component knots and splines, c0 spline
-};
-
-// knot-level fields, attenuation weights and coefficient rows of one group
-void enqueue_wmod_group(ncpa_ctx* ctx, PhaseTimer& tm, const Group& g, WmodBufs& wb, bool wkb, ProblemInfo* d_pinfo,
-                        double* rows, double* w, double* kz2, double* rho_pair) {
-    cudaStream_t st = ctx->stream;
-    const ncpa_profile* prof = g.prof;
-    const int nk = prof->n;
-    GroupBufs& b = wb.gb;
-    check_launch(ctx, ncpa::launch_ceff_knots(st, nk, g.n_az, b.az.as<double>(), prof->c0.as<double>(),
-                                              prof->ws.as<double>(), prof->wd.as<double>(), b.ceffk.as<double>()));
-    check_launch(ctx, ncpa::launch_steffen(st, nk, prof->z.as<double>(), b.ceffk.as<double>(), g.n_az, nk,
-                                           b.ceffc.as<double>(), 4 * (nk - 1)));
-    check_launch(ctx, ncpa::launch_wc_knots(st, nk, g.n_az, b.az.as<double>(), prof->ws.as<double>(),
-                                            prof->wd.as<double>(), wb.wck.as<double>()));
-    check_launch(ctx, ncpa::launch_steffen(st, nk, prof->z.as<double>(), wb.wck.as<double>(), g.n_az, nk,
-                                           wb.wcc.as<double>(), 4 * (nk - 1)));
-    check_launch(ctx, ncpa::launch_steffen(st, nk, prof->z.as<double>(), prof->c0.as<double>(), 1, nk,
-                                           wb.c0c.as<double>(), 4 * (nk - 1)));
-    if (prof->has_attn) {
-        for (int f = 0; f < g.n_freq; ++f)
-            CK(cudaMemcpyAsync(b.alpha.as<double>() + (size_t)f * nk, prof->attn.p, nk * 8, cudaMemcpyDeviceToDevice,
-                               st));
-    } else {
-        check_launch(ctx, ncpa::launch_alpha_knots(st, nk, g.n_freq, b.freqs.as<double>(), prof->z.as<double>(),
-                                                   prof->t.as<double>(), prof->p.as<double>(),
-                                                   prof->rho.as<double>(), b.alpha.as<double>()));
-    }
-    check_launch(ctx, ncpa::launch_steffen(st, nk, prof->z.as<double>(), b.alpha.as<double>(), g.n_freq, nk,
-                                           b.alphac.as<double>(), 4 * (nk - 1)));
-    CK(cudaMemsetAsync(w, 0, (size_t)g.n_freq * g.nz_pad * 8, st));
-    check_launch(ctx, ncpa::launch_grid_common(st, nk, prof->z.as<double>(), prof->rho.as<double>(),
-                                               prof->rcoef.as<double>(), prof->p.as<double>(),
-                                               prof->pcoef.as<double>(), g.nz, g.geo.z_min, g.geo.dz_grid,
-                                               b.rho_g.as<double>(), b.ct_g.as<double>()));
-    check_launch(ctx, ncpa::launch_attn_weight(st, nk, prof->z.as<double>(), b.alpha.as<double>(),
-                                               b.alphac.as<double>(), g.n_freq, b.freqs.as<double>(), g.nz,
-                                               g.geo.z_min, g.geo.dz_grid, b.ct_g.as<double>(), w, g.nz_pad));
-    CK(cudaMemcpyAsync(rho_pair, b.rho_g.as<double>() + g.geo.isrc, 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(rho_pair + 1, b.rho_g.as<double>() + g.geo.ircv, 8, cudaMemcpyDeviceToHost, st));
-    tm.mark("knots+grid");
-    check_launch(ctx, ncpa::launch_wmod_build(st, nk, prof->z.as<double>(), prof->c0.as<double>(),
-                                              wb.c0c.as<double>(), wb.wck.as<double>(), wb.wcc.as<double>(),
-                                              b.ceffk.as<double>(), b.ceffc.as<double>(), g.n_az,
-                                              g.n_freq * g.n_az, d_pinfo, g.nz, g.nz_pad, g.geo.z_min,
-                                              g.geo.dz_grid, g.geo.dz, b.admittance, rows, wkb ? kz2 : nullptr));
-    tm.mark("matrix");
-}
-
-void solve_wmod(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, std::vector<Group>& groups) {
+void solve_groups(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, std::vector<Group>& groups) {
     cudaStream_t st = ctx->stream;
     PhaseTimer tm(ctx);
     tm.mark("start");
-    for (Group& g : groups) wmod_geometry(g, prm);
+    const bool wide = prm->method == NCPA_METHOD_WMOD;
+    if (wide)
+        for (Group& g : groups) wmod_geometry(g, prm);
     long long s_tot = 0, w_tot = 0;
     layout_groups(M, groups, s_tot, w_tot);
     layout_panels(M, groups, prm, 1.0);
     upload(M->d_pinfo, M->info, st);
     const bool wkb = wants_wkb(prm);
-    DevBuf rows, w, kz2;
-    rows.alloc((size_t)s_tot * 16, st);
+    DevBuf s, w, gs, kz2;
+    s.alloc((size_t)s_tot * (wide ? 16 : 8), st);
     w.alloc((size_t)w_tot * 8, st);
     if (wkb) kz2.alloc((size_t)s_tot * 8, st);
+    if (prm->want_group_speed && !wide) gs.alloc((size_t)s_tot * 8, st);
     double* rho_pairs = pinned(ctx, 2 * groups.size());
     ProblemInfo* d_pinfo = M->d_pinfo.as<ProblemInfo>();
-    std::vector<WmodBufs> wbs(groups.size());
+    GroupTable gt;
+    prepare_groups(ctx, prm, groups, d_pinfo, s.as<double>(), w.as<double>(), gs.as<double>(), kz2.as<double>(), gt);
+    enqueue_groups(ctx, tm, gt, rho_pairs);
+    solve_core(ctx, tm, M, prm, wkb, s, w, gs, kz2);
     for (size_t gi = 0; gi < groups.size(); ++gi) {
         const Group& g = groups[gi];
-        prepare_group(ctx, prm, g, wbs[gi].gb);
-        const int nk = g.prof->n;
-        wbs[gi].wck.alloc((size_t)g.n_az * nk * 8, st);
-        wbs[gi].wcc.alloc((size_t)g.n_az * 4 * (nk - 1) * 8, st);
-        wbs[gi].c0c.alloc((size_t)4 * (nk - 1) * 8, st);
-    }
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
-        const Group& g = groups[gi];
-        enqueue_wmod_group(ctx, tm, g, wbs[gi], wkb, d_pinfo + g.p0, rows.as<double>() + 2 * g.s_base,
-                           w.as<double>() + g.w_base, wkb ? kz2.as<double>() + g.s_base : nullptr, rho_pairs + 2 * gi);
-    }
-    DevBuf none;
-    solve_core(ctx, tm, M, prm, wkb, rows, w, none, kz2);
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
-        const Group& g = groups[gi];
-        for (int k = 0; k < g.n_freq * g.n_az; ++k) {
+        const int np = g.n_freq * g.n_az;
+        for (int k = 0; k < np; ++k) {
             M->rho_src_p[g.p0 + k] = rho_pairs[2 * gi];
             M->rho_rcv_p[g.p0 + k] = rho_pairs[2 * gi + 1];
         }
@@ -977,7 +914,7 @@ struct PlanData {
     ncpa_ess_params prm{};
     std::vector<std::vector<double>> freqs, azs;  // host copies the groups point at
     std::vector<Group> groups;
-    std::vector<GroupBufs> gb;
+    GroupTable gt;
     DevBuf s, w, gs, kz2, pinfo_init;
     SolveBufs sb;
     Tuning tuning;
@@ -1002,12 +939,7 @@ void enqueue_plan(PlanData& pl, const Tuning& t) {
     CK(cudaMemcpyAsync(d_pinfo, pl.pinfo_init.p, (size_t)M->P * sizeof(ProblemInfo), cudaMemcpyDeviceToDevice, st));
     CK(cudaMemsetAsync(ctx->d_err.p, 0, sizeof(unsigned), st));
     const bool grp = pl.prm.want_group_speed != 0;
-    for (size_t gi = 0; gi < pl.groups.size(); ++gi) {
-        const Group& g = pl.groups[gi];
-        enqueue_group(ctx, tm, g, pl.gb[gi], pl.wkb, d_pinfo + g.p0, pl.s.as<double>() + g.s_base,
-                      pl.w.as<double>() + g.w_base, grp ? pl.gs.as<double>() + g.s_base : nullptr,
-                      pl.wkb ? pl.kz2.as<double>() + g.s_base : nullptr, pl.h_rho + 2 * gi);
-    }
+    enqueue_groups(ctx, tm, pl.gt, pl.h_rho);
     enqueue_solve(ctx, tm, M, &pl.prm, pl.wkb, pl.s.as<double>(), pl.w.as<double>(), grp ? pl.gs.as<double>() : nullptr,
                   pl.kz2.as<double>(), pl.sb, t, false, pl.h_tot, pl.h_info, pl.h_err);
     if (pl.with_tl)
@@ -1563,8 +1495,7 @@ ncpa_status ncpa_ess_solve(ncpa_ctx* ctx, const ncpa_profile* prof, const ncpa_e
         M->na = n_az;
         M->freqs.assign(freqs, freqs + n_freq);
         M->az.assign(az_deg, az_deg + n_az);
-        if (prm->method == NCPA_METHOD_WMOD) solve_wmod(ctx, M.get(), prm, groups);
-        else solve_groups(ctx, M.get(), prm, groups);
+        solve_groups(ctx, M.get(), prm, groups);
         *out = M.release();
         return NCPA_OK;
     });
@@ -1602,8 +1533,7 @@ ncpa_status ncpa_ess_solve_jobs(ncpa_ctx* ctx, const ncpa_ess_job* jobs, int n_j
             for (int f = 0; f < g.n_freq; ++f)
                 for (int a = 0; a < g.n_az; ++a) M->freqs.push_back(g.freqs[f]);
         M->az.assign(1, groups[0].az[0]);
-        if (prm->method == NCPA_METHOD_WMOD) solve_wmod(ctx, M.get(), prm, groups);
-        else solve_groups(ctx, M.get(), prm, groups);
+        solve_groups(ctx, M.get(), prm, groups);
         *out = M.release();
         return NCPA_OK;
     });
@@ -2343,8 +2273,8 @@ ncpa_status ncpa_ess_plan_create(ncpa_ctx* ctx, const ncpa_ess_job* jobs, int n_
         CK(cudaHostAlloc((void**)&pl.h_tot, 4 * sizeof(int), cudaHostAllocDefault));
         CK(cudaHostAlloc((void**)&pl.h_err, sizeof(unsigned), cudaHostAllocDefault));
         CK(cudaHostAlloc((void**)&pl.h_rho, 2 * pl.groups.size() * sizeof(double), cudaHostAllocDefault));
-        pl.gb.resize(pl.groups.size());
-        for (size_t gi = 0; gi < pl.groups.size(); ++gi) prepare_group(ctx, prm, pl.groups[gi], pl.gb[gi]);
+        prepare_groups(ctx, prm, pl.groups, M->d_pinfo.as<ProblemInfo>(), pl.s.as<double>(), pl.w.as<double>(),
+                       pl.gs.as<double>(), pl.kz2.as<double>(), pl.gt);
         const int kMinItem = 16;  // smallest bisection item the tuner tries
         pl.sb.own_ck = true;
         prepare_solve(ctx, M, &pl.prm, tune ? kMinItem : ncpa::kWItem, pl.sb);

@@ -16,29 +16,12 @@
 // and each eigenvector is the null vector of T: panel.cu with the WmodPanel
 // rows (64 frequencies x 20000 points: 6.5 -> 2.3 ms a call against sweeps of
 // the rows themselves).  This file builds the rows.
+#include <algorithm>
+
 #include "device_common.cuh"
 #include "kernels.hpp"
 
 namespace ncpa {
-
-// wind component along each azimuth at the knots (the wc term of
-// k_ceff_knots, same expression)
-__global__ void k_wc_knots(int n, int n_az, const double* __restrict__ az, const double* __restrict__ ws,
-                           const double* __restrict__ wd, double* __restrict__ wc) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int a = blockIdx.y;
-    if (k >= n || a >= n_az) return;
-    const double az_rad = az[a] * kPi / 180.0;
-    const double dir = wd[k] * kPi / 180.0;
-    wc[(size_t)a * n + k] = ws[k] * cos(dir - az_rad);
-}
-
-int launch_wc_knots(cudaStream_t st, int n, int n_az, const double* az, const double* ws, const double* wd,
-                    double* wc) {
-    dim3 grid((n + 255) / 256, n_az);
-    k_wc_knots<<<grid, 256, 0, st>>>(n, n_az, az, ws, wd, wc);
-    return 1;
-}
 
 // Rows (B_i, U_i) of one group's problems (nz_pad rows apart, problem p =
 // frequency-major over n_az azimuths) on the sampling grid z_min + i dz_grid
@@ -49,17 +32,20 @@ int launch_wc_knots(cudaStream_t st, int n, int n_az, const double* az, const do
 // (azimuth, grid point) and kWbFreqs frequencies: the profile is sampled once.
 constexpr int kWbFreqs = 16;
 
-__global__ void __launch_bounds__(256) k_wmod_build(int nk, const double* __restrict__ zk,
-                                                    const double* __restrict__ c0k, const double* __restrict__ c0c,
-                                                    const double* __restrict__ wck, const double* __restrict__ wcc,
-                                                    const double* __restrict__ ceffk,
-                                                    const double* __restrict__ ceffc, int n_az, int n_f,
-                                                    ProblemInfo* __restrict__ pinfo, int nz, int nz_pad,
-                                                    double z_min, double dz_grid, double dz, double admittance,
-                                                    double2* __restrict__ rows, double* __restrict__ kz2) {
+__global__ void __launch_bounds__(256) k_wmod_build(const GroupDesc* __restrict__ desc, int tiles) {
+    const GroupDesc& G = desc[blockIdx.z];
     const int az = blockIdx.y;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int f0 = blockIdx.z * kWbFreqs, f1 = min(n_f, f0 + kWbFreqs);
+    const int i = (blockIdx.x % tiles) * blockDim.x + threadIdx.x;
+    const int n_f = G.n_f, n_az = G.n_az, nk = G.nk, nz = G.nz, nz_pad = G.nz_pad;
+    const int f0 = (blockIdx.x / tiles) * kWbFreqs, f1 = min(n_f, f0 + kWbFreqs);
+    if (az >= n_az || f0 >= f1 || (blockIdx.x % tiles) * blockDim.x >= nz_pad) return;
+    const double *__restrict__ zk = G.zk, *__restrict__ c0k = G.c0k, *__restrict__ c0c = G.c0c;
+    const double *__restrict__ wck = G.wck, *__restrict__ wcc = G.wcc;
+    const double *__restrict__ ceffk = G.ceffk, *__restrict__ ceffc = G.ceffc;
+    const double z_min = G.z_min, dz_grid = G.dz_grid, dz = G.dz, admittance = G.admittance;
+    ProblemInfo* __restrict__ pinfo = G.pinfo;
+    double2* __restrict__ rows = reinterpret_cast<double2*>(G.s);
+    double* __restrict__ kz2 = G.kz2;
     double cmin = 1e300, cmax = -1e300;
     const int top = nz - (nz / 10);
     const int itop = top + 1 < nz ? top + 1 : nz - 1;
@@ -114,16 +100,13 @@ __global__ void __launch_bounds__(256) k_wmod_build(int nk, const double* __rest
     }
 }
 
-int launch_wmod_build(cudaStream_t st, int nk, const double* zk, const double* c0k, const double* c0c,
-                      const double* wck, const double* wcc, const double* ceffk, const double* ceffc, int n_az,
-                      int P, ProblemInfo* pinfo, int nz, int nz_pad, double z_min, double dz_grid, double dz,
-                      double admittance, double* rows, double* kz2) {
-    if (n_az < 1 || P % n_az != 0) return -1;
-    const int n_f = P / n_az;
-    dim3 grid((nz_pad + 255) / 256, n_az, (n_f + kWbFreqs - 1) / kWbFreqs);
-    k_wmod_build<<<grid, 256, 0, st>>>(nk, zk, c0k, c0c, wck, wcc, ceffk, ceffc, n_az, n_f, pinfo, nz, nz_pad, z_min,
-                                       dz_grid, dz, admittance, reinterpret_cast<double2*>(rows), kz2);
-    return 1;
+int launch_wmod_build(cudaStream_t st, const GroupDesc* desc, const GroupDims& d) {
+    const int tiles = (d.nz_pad + 255) / 256;
+    int n = 0;
+    for (int g0 = 0; g0 < d.n; g0 += 65535, ++n)
+        k_wmod_build<<<dim3(tiles * ((d.n_f + kWbFreqs - 1) / kWbFreqs), d.n_az, std::min(65535, d.n - g0)), 256, 0,
+                       st>>>(desc + g0, tiles);
+    return n;
 }
 
 }  // namespace ncpa
