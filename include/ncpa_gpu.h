@@ -239,6 +239,9 @@ enum { NCPA_SUM_FP64 = 0, NCPA_SUM_TC_BF16X3 = 1, NCPA_SUM_TC_TF32 = 2, NCPA_SUM
 ncpa_status ncpa_tl_multi(ncpa_ctx *ctx, const ncpa_modes *modes, int problem, int n_rcv,
                           const double *rcv_height_m, const ncpa_tl_params *tp, int method, double *re,
                           double *im);
+/* The same to one array of (re, im) pairs [n_rcv x n_ranges x 2]. */
+ncpa_status ncpa_tl_multi_pairs(ncpa_ctx *ctx, const ncpa_modes *modes, int problem, int n_rcv,
+                                const double *rcv_height_m, const ncpa_tl_params *tp, int method, double *p);
 
 /* Modal starter of one problem (ESSModeSolver::getModalStarter,
  * ESSModeSolver.cpp:670-723; needs want_vectors).  Call with NULL outputs to

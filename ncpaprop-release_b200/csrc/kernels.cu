@@ -1466,6 +1466,18 @@ __global__ void __launch_bounds__(256) k_src_dft(int n, const double* __restrict
 
 // out[c][r] = in[r][c] for a rows x cols matrix of doubles, 32 x 32 tiles
 // staged in shared memory (both sides coalesced)
+// out[i] = (re[i], im[i])
+__global__ void __launch_bounds__(256) k_pairs(size_t n, const double* __restrict__ re, const double* __restrict__ im,
+                                               double2* __restrict__ out) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = make_double2(re[i], im[i]);
+}
+
+int launch_pairs(cudaStream_t st, size_t n, const double* re, const double* im, double* out) {
+    k_pairs<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, re, im, reinterpret_cast<double2*>(out));
+    return 1;
+}
+
 __global__ void __launch_bounds__(256) k_transpose(int rows, int cols, const double* __restrict__ in,
                                                    double* __restrict__ out) {
     __shared__ double t[32][33];

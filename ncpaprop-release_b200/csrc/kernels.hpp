@@ -222,6 +222,8 @@ size_t modal_sum_scratch(int M, int nr);
 int launch_modal_sum(cudaStream_t st, int M, const double* kr, const double* ki, const double* vs_src,
                      const double* vec, const int* rows, int nj, int nr, double dr, int lossless, bool range_major,
                      int num_sms, void* scratch, double* re, double* im);
+// out[2 i], out[2 i + 1] = re[i], im[i]
+int launch_pairs(cudaStream_t st, size_t n, const double* re, const double* im, double* out);
 // out[c][r] = in[r][c] (rows x cols doubles)
 int launch_transpose(cudaStream_t st, int rows, int cols, const double* in, double* out);
 // broadband synthesis

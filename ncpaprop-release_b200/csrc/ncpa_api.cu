@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "atmosphere.hpp"
+#include "host_copy.hpp"
 #include "kernels.hpp"
 
 using ncpa::ProblemInfo;
@@ -139,7 +140,8 @@ struct ncpa_ctx {
     bool scan_trim = true;
     bool fuse_solve = true;        // fused bisection + eigenvector launch; NCPA_FUSE_SOLVE=0 turns it off
     double* h_pin = nullptr;       // small pinned host buffer for scalars read back per solve
-    int* h_tot = nullptr;          // pinned: item and mode totals of a device-built solve
+    int* h_tot = nullptr;          // pinned: item and mode totals of a device-built solve, status word at [8]
+    ncpa::HostCopier copier;       // results to pageable host memory
     size_t h_pin_n = 0;
     DevBuf d_stats;                // device counters (Sturm sequences)
     bool timing = false;           // NCPA_TIMING=1: per-phase times on stderr
@@ -245,16 +247,26 @@ void check_launch(ncpa_ctx* ctx, int n) {
     if (e != cudaSuccess) throw CudaError(std::string("kernel launch: ") + cudaGetErrorString(e));
 }
 
-void check_device_status(ncpa_ctx* ctx) {
-    unsigned h = 0;
-    CK(cudaMemcpyAsync(&h, ctx->d_err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+// throws for the device status h
+void check_status(ncpa_ctx* ctx, unsigned h) {
     if (h) {
         CK(cudaMemsetAsync(ctx->d_err.p, 0, sizeof(unsigned), ctx->stream));
         if (h & ncpa::kErrTimeout) throw ApiError(NCPA_ETIMEDOUT, "a bounded device wait gave up");
         if (h & ncpa::kErrBracket) throw ApiError(NCPA_ECUDA, "bisection bracket inconsistent with Sturm counts");
         if (h & ncpa::kErrWkb) throw ApiError(NCPA_ECUDA, "WKB window search exceeded its trial count");
     }
+}
+
+void check_device_status(ncpa_ctx* ctx) {
+    unsigned* h = reinterpret_cast<unsigned*>(ctx->h_tot + 8);
+    CK(cudaMemcpyAsync(h, ctx->d_err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    check_status(ctx, *h);
+}
+
+// device results to host memory; the stream is idle on return
+void copy_to_host(ncpa_ctx* ctx, std::initializer_list<ncpa::HostCopier::Part> parts) {
+    CK(ctx->copier.run(ctx->device, ctx->stream, parts.begin(), parts.size()));
 }
 
 const double* twiddle(ncpa_ctx* ctx, int nfft) {
@@ -268,21 +280,15 @@ const double* twiddle(ncpa_ctx* ctx, int nfft) {
     return p;
 }
 
-// copy the mode arrays of a solve to its host mirror (stream-ordered)
+// copy the mode arrays of a solve to its host mirror
 void fetch_modes(const ncpa_modes* M) {
-    cudaStream_t st = M->ctx->stream;
-    M->kr.resize(M->Mtot);
-    M->ki.resize(M->Mtot);
-    M->vs.resize(M->Mtot);
-    M->vr.resize(M->Mtot);
-    M->vg.resize(M->Mtot);
-    if (M->Mtot > 0) {
-        CK(cudaMemcpyAsync(M->kr.data(), M->d_kr.p, M->Mtot * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(M->ki.data(), M->d_ki.p, M->Mtot * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(M->vs.data(), M->d_vs.p, M->Mtot * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(M->vr.data(), M->d_vr.p, M->Mtot * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(M->vg.data(), M->d_vg.p, M->Mtot * 8, cudaMemcpyDeviceToHost, st));
-    }
+    const size_t n = (size_t)M->Mtot * 8;
+    for (std::vector<double>* v : {&M->kr, &M->ki, &M->vs, &M->vr, &M->vg}) v->resize(M->Mtot);
+    copy_to_host(M->ctx, {{M->kr.data(), M->d_kr.p, n},
+                          {M->ki.data(), M->d_ki.p, n},
+                          {M->vs.data(), M->d_vs.p, n},
+                          {M->vr.data(), M->d_vr.p, n},
+                          {M->vg.data(), M->d_vg.p, n}});
     M->host_valid = true;
 }
 
@@ -714,23 +720,25 @@ void finish_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const int* tot, 
     M->Mtot = tot[2];
     M->host_valid = false;
     if (!M->prm.keep_on_device) fetch_modes(M);
-    check_device_status(ctx);
+    check_status(ctx, *err);
     tm.mark("fetch");
 }
 
 // Window, Sturm scan, work items, bisection and eigenvectors over all
 // problems of M (their matrices built; each problem's rows of s, w, g and kz2
-// at the offsets in its ProblemInfo).
+// at the offsets in its ProblemInfo).  h_info: P records, pinned or M->info.
 void solve_core(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_params* prm, bool wkb, DevBuf& s,
-                DevBuf& w, DevBuf& g, DevBuf& kz2) {
+                DevBuf& w, DevBuf& g, DevBuf& kz2, ProblemInfo* h_info) {
     Tuning t;
     if (ctx->item_override > 0) t.bis_item = std::min(ctx->item_override, ncpa::kWItem);
     SolveBufs b;
     prepare_solve(ctx, M, prm, t.bis_item, b);
-    unsigned h_err = 0;
+    unsigned* h_err = reinterpret_cast<unsigned*>(ctx->h_tot + 8);
     enqueue_solve(ctx, tm, M, prm, wkb, s.as<double>(), w.as<double>(), g.as<double>(), kz2.as<double>(), b, t,
-                  ctx->stats && !ctx->stats_fused, ctx->h_tot, M->info.data(), &h_err);
-    finish_solve(ctx, tm, M, ctx->h_tot, &h_err);
+                  ctx->stats && !ctx->stats_fused, ctx->h_tot, h_info, h_err);
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (h_info != M->info.data()) std::copy(h_info, h_info + M->P, M->info.begin());
+    finish_solve(ctx, tm, M, ctx->h_tot, h_err);
 }
 
 void init_modes(ncpa_modes* M, ncpa_ctx* ctx, const ncpa_ess_params* prm, int P) {
@@ -884,12 +892,17 @@ void solve_groups(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, std:
     w.alloc((size_t)w_tot * 8, st);
     if (wkb) kz2.alloc((size_t)s_tot * 8, st);
     if (prm->want_group_speed && !wide) gs.alloc((size_t)s_tot * 8, st);
-    double* rho_pairs = pinned(ctx, 2 * groups.size());
+    static_assert(sizeof(ProblemInfo) % 8 == 0, "records behind the densities");
+    // the records come back behind the densities; very many of them (4 MB and
+    // up) straight to their place, at the driver's pace
+    const bool stage = (size_t)M->P * sizeof(ProblemInfo) <= (4u << 20);
+    double* rho_pairs = pinned(ctx, 2 * groups.size() + (stage ? (size_t)M->P * (sizeof(ProblemInfo) / 8) : 0));
+    ProblemInfo* h_info = stage ? reinterpret_cast<ProblemInfo*>(rho_pairs + 2 * groups.size()) : M->info.data();
     ProblemInfo* d_pinfo = M->d_pinfo.as<ProblemInfo>();
     GroupTable gt;
     prepare_groups(ctx, prm, groups, d_pinfo, s.as<double>(), w.as<double>(), gs.as<double>(), kz2.as<double>(), gt);
     enqueue_groups(ctx, tm, gt, rho_pairs);
-    solve_core(ctx, tm, M, prm, wkb, s, w, gs, kz2);
+    solve_core(ctx, tm, M, prm, wkb, s, w, gs, kz2, h_info);
     for (size_t gi = 0; gi < groups.size(); ++gi) {
         const Group& g = groups[gi];
         const int np = g.n_freq * g.n_az;
@@ -1580,7 +1593,6 @@ ncpa_status ncpa_modes_get(const ncpa_modes* m, int problem, double* re_k, doubl
     if (!m->host_valid) {
         ncpa_status s = guarded(m->ctx, [&]() -> ncpa_status {
             fetch_modes(m);
-            CK(cudaStreamSynchronize(m->ctx->stream));
             return NCPA_OK;
         });
         if (s != NCPA_OK) return s;
@@ -1602,15 +1614,21 @@ ncpa_status ncpa_modes_get_all(const ncpa_modes* m, int* mode_off, double* re_k,
     mode_off[m->P] = m->Mtot;
     if (!re_k && !im_k && !v_src && !v_rcv && !v_group) return NCPA_OK;
     return guarded(m->ctx, [&]() -> ncpa_status {
-        cudaStream_t st = m->ctx->stream;
         const size_t n = (size_t)m->Mtot * 8;
-        if (n) {
-            const std::pair<double*, const DevBuf*> cols[] = {
-                {re_k, &m->d_kr}, {im_k, &m->d_ki}, {v_src, &m->d_vs}, {v_rcv, &m->d_vr}, {v_group, &m->d_vg}};
-            for (const auto& c : cols)
-                if (c.first) CK(cudaMemcpyAsync(c.first, c.second->p, n, cudaMemcpyDeviceToHost, st));
+        if (m->host_valid) {
+            const ncpa::HostCopier::Part parts[] = {{re_k, m->kr.data(), re_k ? n : 0},
+                                                    {im_k, m->ki.data(), im_k ? n : 0},
+                                                    {v_src, m->vs.data(), v_src ? n : 0},
+                                                    {v_rcv, m->vr.data(), v_rcv ? n : 0},
+                                                    {v_group, m->vg.data(), v_group ? n : 0}};
+            m->ctx->copier.host(m->ctx->device, parts, 5);
+        } else {
+            copy_to_host(m->ctx, {{re_k, m->d_kr.p, re_k ? n : 0},
+                                  {im_k, m->d_ki.p, im_k ? n : 0},
+                                  {v_src, m->d_vs.p, v_src ? n : 0},
+                                  {v_rcv, m->d_vr.p, v_rcv ? n : 0},
+                                  {v_group, m->d_vg.p, v_group ? n : 0}});
         }
-        CK(cudaStreamSynchronize(st));
         return NCPA_OK;
     });
 }
@@ -1620,11 +1638,7 @@ ncpa_status ncpa_modes_get_vectors(const ncpa_modes* m, int problem, double* v) 
     if (!m->prm.want_vectors) return fail(m->ctx, NCPA_EINVAL, "solve was run without want_vectors");
     return guarded(m->ctx, [&]() -> ncpa_status {
         const size_t n = (size_t)m->info[problem].M * m->info[problem].nz;
-        if (n) {
-            CK(cudaMemcpyAsync(v, m->d_vfull.as<double>() + m->vfull_off[problem], n * 8, cudaMemcpyDeviceToHost,
-                               m->ctx->stream));
-            CK(cudaStreamSynchronize(m->ctx->stream));
-        }
+        copy_to_host(m->ctx, {{v, m->d_vfull.as<double>() + m->vfull_off[problem], n * 8}});
         return NCPA_OK;
     });
 }
@@ -1654,12 +1668,8 @@ ncpa_status ncpa_tl_1d(ncpa_ctx* ctx, const ncpa_modes* m, const ncpa_tl_params*
                                             m->d_ki.as<double>(), m->d_vs.as<double>(), m->d_vr.as<double>(),
                                             tp->n_ranges, tp->dr_m, tp->lossless, dre.as<double>(), dim.as<double>(),
                                             dinc.as<double>()));
-        if (!keep) {
-            CK(cudaMemcpyAsync(re, dre.p, n * 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(im, dim.p, n * 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(incoh, dinc.p, n * 8, cudaMemcpyDeviceToHost, st));
-        }
-        CK(cudaStreamSynchronize(st));
+        if (!keep) copy_to_host(ctx, {{re, dre.p, n * 8}, {im, dim.p, n * 8}, {incoh, dinc.p, n * 8}});
+        else CK(cudaStreamSynchronize(st));
         return NCPA_OK;
     });
 }
@@ -1682,10 +1692,7 @@ ncpa_status ncpa_tl_1d_range(ncpa_ctx* ctx, const ncpa_modes* m, int first, int 
                                             m->d_ki.as<double>(), m->d_vs.as<double>(), m->d_vr.as<double>(),
                                             tp->n_ranges, tp->dr_m, tp->lossless, dre.as<double>(), dim.as<double>(),
                                             dinc.as<double>()));
-        CK(cudaMemcpyAsync(re, dre.p, n * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(im, dim.p, n * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(incoh, dinc.p, n * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
+        copy_to_host(ctx, {{re, dre.p, n * 8}, {im, dim.p, n * 8}, {incoh, dinc.p, n * 8}});
         return NCPA_OK;
     });
 }
@@ -1896,9 +1903,7 @@ ncpa_status ncpa_tl_2d(ncpa_ctx* ctx, const ncpa_modes* m, int problem, const nc
             tim.alloc(n * 8, st);
             check_launch(ctx, ncpa::launch_transpose(st, nzo, nr, ctx->ms_re.as<double>(), tre.as<double>()));
             check_launch(ctx, ncpa::launch_transpose(st, nzo, nr, ctx->ms_im.as<double>(), tim.as<double>()));
-            CK(cudaMemcpyAsync(re, tre.p, n * 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(im, tim.p, n * 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
+            copy_to_host(ctx, {{re, tre.p, n * 8}, {im, tim.p, n * 8}});
             check_device_status(ctx);
             return NCPA_OK;
         }
@@ -1918,16 +1923,16 @@ ncpa_status ncpa_tl_2d(ncpa_ctx* ctx, const ncpa_modes* m, int problem, const nc
                                                  vec + (size_t)pi.isrc * Mm, vec, drows.as<int>(), nzo, tp->n_ranges,
                                                  tp->dr_m, tp->lossless, true, ctx->num_sms, ctx->ms_vz.p,
                                                  dre.as<double>(), dim.as<double>()));
-        CK(cudaMemcpyAsync(re, dre.p, n * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(im, dim.p, n * 8, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
+        copy_to_host(ctx, {{re, dre.p, n * 8}, {im, dim.p, n * 8}});
         return NCPA_OK;
     });
 }
 
 
-ncpa_status ncpa_tl_multi(ncpa_ctx* ctx, const ncpa_modes* m, int problem, int n_rcv, const double* rcv_height_m,
-                          const ncpa_tl_params* tp, int method, double* re, double* im) {
+namespace {
+// the sum at receivers, to re and im, to pairs (re, im), or kept on the device
+ncpa_status tl_multi(ncpa_ctx* ctx, const ncpa_modes* m, int problem, int n_rcv, const double* rcv_height_m,
+                     const ncpa_tl_params* tp, int method, double* re, double* im, double* pairs) {
     if (!ctx || !m || !tp || !rcv_height_m || n_rcv < 1 || problem < 0 || problem >= m->P) return NCPA_EINVAL;
     if ((re == nullptr) != (im == nullptr)) return NCPA_EINVAL;
     if (method != NCPA_SUM_FP64 && method != NCPA_SUM_TC_BF16X3 && method != NCPA_SUM_TC_TF32 &&
@@ -1951,12 +1956,29 @@ ncpa_status ncpa_tl_multi(ncpa_ctx* ctx, const ncpa_modes* m, int problem, int n
         const size_t nout = (size_t)n_rcv * nr;
         modal_sum_rows(ctx, m, problem, idx, tp, method);
         if (re) {
-            CK(cudaMemcpyAsync(re, ctx->ms_re.p, nout * 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(im, ctx->ms_im.p, nout * 8, cudaMemcpyDeviceToHost, st));
+            copy_to_host(ctx, {{re, ctx->ms_re.p, nout * 8}, {im, ctx->ms_im.p, nout * 8}});
+        } else if (pairs) {
+            DevBuf z;
+            z.alloc(nout * 16, st);
+            check_launch(ctx, ncpa::launch_pairs(st, nout, ctx->ms_re.as<double>(), ctx->ms_im.as<double>(),
+                                                 z.as<double>()));
+            copy_to_host(ctx, {{pairs, z.p, nout * 16}});
         }
         check_device_status(ctx);
         return NCPA_OK;
     });
+}
+}  // namespace
+
+ncpa_status ncpa_tl_multi(ncpa_ctx* ctx, const ncpa_modes* m, int problem, int n_rcv, const double* rcv_height_m,
+                          const ncpa_tl_params* tp, int method, double* re, double* im) {
+    return tl_multi(ctx, m, problem, n_rcv, rcv_height_m, tp, method, re, im, nullptr);
+}
+
+ncpa_status ncpa_tl_multi_pairs(ncpa_ctx* ctx, const ncpa_modes* m, int problem, int n_rcv,
+                                const double* rcv_height_m, const ncpa_tl_params* tp, int method, double* p) {
+    if (!p) return NCPA_EINVAL;
+    return tl_multi(ctx, m, problem, n_rcv, rcv_height_m, tp, method, nullptr, nullptr, p);
 }
 
 // ---------------------------------------------------------------------------
@@ -1991,8 +2013,8 @@ ncpa_status bb_common(ncpa_ctx* ctx, int nfreq, const double* d_f, const int* d_
                                                dh.as<double>()));
     check_launch(ctx, ncpa::launch_bb_pulse(st, nfreq, d_f, dsrc.as<double>(), dh.as<double>(), nr, dt0.as<double>(),
                                             nfft, tw, dout.as<double>()));
-    if (waveforms) CK(cudaMemcpyAsync(waveforms, dout.p, (size_t)nr * nfft * 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    if (waveforms) copy_to_host(ctx, {{waveforms, dout.p, (size_t)nr * nfft * 8}});
+    else CK(cudaStreamSynchronize(st));
     return NCPA_OK;
 }
 }  // namespace
@@ -2363,12 +2385,8 @@ ncpa_status ncpa_ess_plan_tl(ncpa_plan* plan, double* re, double* im, double* in
     if (!pl.with_tl) return fail(pl.ctx, NCPA_EINVAL, "the plan has no TL range grid");
     if (!pl.ran) return fail(pl.ctx, NCPA_EINVAL, "the plan has not run");
     return guarded(pl.ctx, [&]() -> ncpa_status {
-        cudaStream_t st = pl.ctx->stream;
         const size_t n = (size_t)pl.M->P * pl.tp.n_ranges * 8;
-        CK(cudaMemcpyAsync(re, pl.M->tl_re.p, n, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(im, pl.M->tl_im.p, n, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(incoh, pl.M->tl_inc.p, n, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
+        copy_to_host(pl.ctx, {{re, pl.M->tl_re.p, n}, {im, pl.M->tl_im.p, n}, {incoh, pl.M->tl_inc.p, n}});
         return NCPA_OK;
     });
 }

@@ -29,7 +29,7 @@ EXPORTED = [
     "ncpa_kernel_launches", "ncpa_ctx_stream", "ncpa_ctx_set_timing", "ncpa_ctx_phase_stats",
     "ncpa_ctx_reset_stats", "ncpa_ctx_sturm_steps", "ncpa_probe_fp64_peak", "ncpa_source_spectrum_builtin",
     "ncpa_eigvec_static", "ncpa_profile_set_attn", "ncpa_profile_load_attn", "ncpa_profile_knots", "ncpa_profile_z0",
-    "ncpa_modal_starter", "ncpa_source_waveform", "ncpa_tl_multi", "ncpa_ess_solve_jobs", "ncpa_server_opts_default", "ncpa_server_create",
+    "ncpa_modal_starter", "ncpa_source_waveform", "ncpa_tl_multi", "ncpa_tl_multi_pairs", "ncpa_ess_solve_jobs", "ncpa_server_opts_default", "ncpa_server_create",
     "ncpa_server_submit", "ncpa_server_wait", "ncpa_server_release", "ncpa_server_stats_get", "ncpa_server_destroy", "ncpa_modes_get_all",
     "ncpa_ess_plan_create", "ncpa_ess_plan_run", "ncpa_ess_plan_modes", "ncpa_ess_plan_tl", "ncpa_ess_plan_tuning",
     "ncpa_ess_plan_destroy", "ncpa_profile_update", "ncpa_g2s_convert", "ncpa_profile_load_g2s",
@@ -166,6 +166,7 @@ def lib():
         L.ncpa_tl_1d.argtypes = [_vp, _vp, ctypes.POINTER(_TlParams), _dp, _dp, _dp]
         L.ncpa_tl_2d_heights.argtypes = [_vp, _c_int, _ip]
         L.ncpa_tl_2d.argtypes = [_vp, _vp, _c_int, ctypes.POINTER(_TlParams), _dp, _dp, _dp]
+        L.ncpa_tl_multi_pairs.argtypes = [_vp, _vp, _c_int, _c_int, _dp, ctypes.POINTER(_TlParams), _c_int, _dp]
         L.ncpa_tl_multi.argtypes = [_vp, _vp, _c_int, _c_int, _dp, ctypes.POINTER(_TlParams), _c_int, _dp, _dp]
         L.ncpa_bb_synthesize.argtypes = [_vp, ctypes.POINTER(_DispDesc), ctypes.POINTER(_BbParams), _dp]
         L.ncpa_bb_synthesize_modes.argtypes = [_vp, _vp, _c_int, ctypes.POINTER(_BbParams), _dp]
@@ -551,11 +552,14 @@ class Modes:
         """Modal sum at many receivers: complex P [n_rcv x n_ranges]."""
         h = _f64(heights_m)
         tp = _TlParams(int(n_ranges), float(dr_m), int(lossless))
-        re = np.empty((len(h), n_ranges)) if to_host else None
-        im = np.empty((len(h), n_ranges)) if to_host else None
-        self.ctx.check(lib().ncpa_tl_multi(self.ctx.h, self.h, p, len(h), _p(h), ctypes.byref(tp), int(method),
-                                           _p(re), _p(im)), "ncpa_tl_multi")
-        return (re + 1j * im) if to_host else None
+        if not to_host:
+            self.ctx.check(lib().ncpa_tl_multi(self.ctx.h, self.h, p, len(h), _p(h), ctypes.byref(tp), int(method),
+                                               None, None), "ncpa_tl_multi")
+            return None
+        out = np.empty((len(h), n_ranges), dtype=np.complex128)
+        self.ctx.check(lib().ncpa_tl_multi_pairs(self.ctx.h, self.h, p, len(h), _p(h), ctypes.byref(tp), int(method),
+                                                 out.ctypes.data_as(_dp)), "ncpa_tl_multi_pairs")
+        return out
 
     def bb_synthesize(self, ranges_m, max_celerity, nfft, src_re, src_im, zero_attn=False, to_host=True, out=None):
         rng, sre, sim = _f64(ranges_m), _f64(src_re), _f64(src_im)
