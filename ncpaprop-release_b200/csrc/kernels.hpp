@@ -201,6 +201,7 @@ struct ModesArgs {
     double* vfull;              // [row][mode] per problem at vfull_off
     const long long* vfull_off;
     int* sched;  // item counter (zeroed) or null: round-robin
+    int num_sms;
     unsigned* err;
     unsigned long long* steps;  // optional counter of row steps
 };

@@ -680,6 +680,7 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
     a.ck_e = (b.own_ck ? b.cke : ctx->cke).as<int>();
     a.ck_stride = ncpa::coarse_slot_elems(M->nz_max);
     a.sched = ctx->bis_order ? b.sched.as<int>() : nullptr;
+    a.num_sms = ctx->num_sms;
     a.err = err;
     if (prm->want_vectors) {
         a.vstate = v.state.as<ncpa::VecState>();

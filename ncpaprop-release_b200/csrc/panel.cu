@@ -1528,14 +1528,22 @@ __global__ void __launch_bounds__(kPWarps * 32, kPanelCtas) k_panel_modes(ModesA
     const long long gp = (long long)blockIdx.x * (kPWarps / 2) + pr.id;
     double* ck = A.ck_u + gp * 2 * A.ck_stride * (1 + kSums<Row, NW>);
     int* cke = A.ck_e + gp * 2 * A.ck_stride;
-    long long walk = gp;
+    // first items: one to the first pair of as many CTAs as there are SMs (which
+    // start on different ones), then to their second pairs, then to the next
+    // CTAs, so that few items have a scheduler for each warp; later ones as the
+    // pairs get free (sched), or round-robin
+    const int n_pairs = gridDim.x * (kPWarps / 2), row = blockIdx.x / A.num_sms;
+    const int width = min(A.num_sms, (int)gridDim.x - row * A.num_sms);  // CTAs of this row
+    long long walk = (long long)row * A.num_sms * (kPWarps / 2) + pr.id * width + blockIdx.x % A.num_sms;
+    bool first = true;
     for (int turn = 0;; turn ^= 1) {
         if (pr.half == 0 && lane == 0) {
             long long it = walk;
-            if (A.sched) it = atomicAdd(A.sched, 1);
+            if (A.sched && !first) it = n_pairs + atomicAdd(A.sched, 1);
             pr.box->item[turn] = it < n_items ? (int)it : -1;
         }
-        walk += (long long)gridDim.x * (kPWarps / 2);
+        walk += n_pairs;
+        first = false;
         pr.sync();
         const int it = pr.box->item[turn];
         if (it < 0) break;
