@@ -212,10 +212,12 @@ int launch_panel_modes(cudaStream_t st, bool wide, int grid, const ModesArgs& a,
 int launch_panel_fill(cudaStream_t st, bool wide, int P, int nz_max, int m_max, const ModesArgs& a);
 int panel_ctas_per_sm();
 
-// modal sums
+// 1-D TL; m_max: at least the most modes of a problem; scratch of tl1d_scratch
+// bytes (0: none)
+size_t tl1d_scratch(int P, int nr, int m_max, int num_sms);
 int launch_tl1d(cudaStream_t st, int P, const ProblemInfo* pinfo, const double* kr, const double* ki,
                 const double* vs, const double* vr, int nr, double dr, int lossless, double* re, double* im,
-                double* incoh);
+                double* incoh, int m_max, int num_sms, double* scratch);
 // FP64 modal sum at heights rows[j] (rows of vec, M values each):
 // re/im [nr x nj] with range_major, else [nj x nr]; scratch of
 // modal_sum_scratch bytes

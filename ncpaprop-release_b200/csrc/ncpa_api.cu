@@ -114,6 +114,7 @@ struct ncpa_ctx {
     DevBuf d_err;                  // device status word
     DevBuf ck1, cke;               // eigenvector checkpoint scratch
     DevBuf ex;                     // panel expansions
+    DevBuf tl_part;                // 1-D TL sums of single mode tiles
     std::map<int, DevBuf> twiddle; // per nfft
     DevBuf bb_out;                 // waveforms kept in HBM (NULL host buffer)
     DevBuf ms_img, ms_q, ms_tab, ms_raw, ms_vz, ms_idx, ms_re, ms_im;  // modal-sum scratch (grow-only)
@@ -929,7 +930,7 @@ struct PlanData {
     std::vector<std::vector<double>> freqs, azs;  // host copies the groups point at
     std::vector<Group> groups;
     GroupTable gt;
-    DevBuf s, w, gs, kz2, pinfo_init;
+    DevBuf s, w, gs, kz2, pinfo_init, tl_part;
     SolveBufs sb;
     Tuning tuning;
     bool wkb = false, with_tl = false, ran = false;
@@ -960,7 +961,8 @@ void enqueue_plan(PlanData& pl, const Tuning& t) {
         check_launch(ctx, ncpa::launch_tl1d(st, M->P, d_pinfo, M->d_kr.as<double>(), M->d_ki.as<double>(),
                                             M->d_vs.as<double>(), M->d_vr.as<double>(), pl.tp.n_ranges, pl.tp.dr_m,
                                             pl.tp.lossless, M->tl_re.as<double>(), M->tl_im.as<double>(),
-                                            M->tl_inc.as<double>()));
+                                            M->tl_inc.as<double>(), M->prm.max_modes, ctx->num_sms,
+                                            pl.tl_part.as<double>()));
 }
 
 // Captures the plan's sequence with launch shapes t and instantiates it.
@@ -1221,6 +1223,7 @@ ncpa_status ncpa_ctx_destroy(ncpa_ctx* ctx) {
     ctx->bb_out.release();
     ctx->d_stats.release();
     ctx->ex.release();
+    ctx->tl_part.release();
     ctx->ck1.release();
     ctx->cke.release();
     ctx->d_err.release();
@@ -1647,6 +1650,14 @@ ncpa_status ncpa_modes_get_vectors(const ncpa_modes* m, int problem, double* v) 
 // ---------------------------------------------------------------------------
 // transmission loss
 // ---------------------------------------------------------------------------
+namespace {
+int most_modes(const ncpa_modes* m, int first, int count) {
+    int n = 0;
+    for (int p = first; p < first + count; ++p) n = std::max(n, m->info[p].M);
+    return n;
+}
+}  // namespace
+
 ncpa_status ncpa_tl_1d(ncpa_ctx* ctx, const ncpa_modes* m, const ncpa_tl_params* tp, double* re, double* im,
                        double* incoh) {
     if (!ctx || !m || !tp) return NCPA_EINVAL;
@@ -1665,10 +1676,12 @@ ncpa_status ncpa_tl_1d(ncpa_ctx* ctx, const ncpa_modes* m, const ncpa_tl_params*
         dre.alloc(n * 8, st);
         dim.alloc(n * 8, st);
         dinc.alloc(n * 8, st);
+        const int m_max = most_modes(m, 0, m->P);
+        ctx->tl_part.alloc(ncpa::tl1d_scratch(m->P, tp->n_ranges, m_max, ctx->num_sms), st);
         check_launch(ctx, ncpa::launch_tl1d(st, m->P, m->d_pinfo.as<ProblemInfo>(), m->d_kr.as<double>(),
                                             m->d_ki.as<double>(), m->d_vs.as<double>(), m->d_vr.as<double>(),
                                             tp->n_ranges, tp->dr_m, tp->lossless, dre.as<double>(), dim.as<double>(),
-                                            dinc.as<double>()));
+                                            dinc.as<double>(), m_max, ctx->num_sms, ctx->tl_part.as<double>()));
         if (!keep) copy_to_host(ctx, {{re, dre.p, n * 8}, {im, dim.p, n * 8}, {incoh, dinc.p, n * 8}});
         else CK(cudaStreamSynchronize(st));
         return NCPA_OK;
@@ -1688,11 +1701,13 @@ ncpa_status ncpa_tl_1d_range(ncpa_ctx* ctx, const ncpa_modes* m, int first, int 
         dre.alloc(n * 8, st);
         dim.alloc(n * 8, st);
         dinc.alloc(n * 8, st);
+        const int m_max = most_modes(m, first, count);
+        ctx->tl_part.alloc(ncpa::tl1d_scratch(count, tp->n_ranges, m_max, ctx->num_sms), st);
         // the problem records carry absolute mode offsets: start at `first`
         check_launch(ctx, ncpa::launch_tl1d(st, count, m->d_pinfo.as<ProblemInfo>() + first, m->d_kr.as<double>(),
                                             m->d_ki.as<double>(), m->d_vs.as<double>(), m->d_vr.as<double>(),
                                             tp->n_ranges, tp->dr_m, tp->lossless, dre.as<double>(), dim.as<double>(),
-                                            dinc.as<double>()));
+                                            dinc.as<double>(), m_max, ctx->num_sms, ctx->tl_part.as<double>()));
         copy_to_host(ctx, {{re, dre.p, n * 8}, {im, dim.p, n * 8}, {incoh, dinc.p, n * 8}});
         return NCPA_OK;
     });
@@ -2308,6 +2323,7 @@ ncpa_status ncpa_ess_plan_create(ncpa_ctx* ctx, const ncpa_ess_job* jobs, int n_
             M->tl_re.alloc(n, st);
             M->tl_im.alloc(n, st);
             M->tl_inc.alloc(n, st);
+            pl.tl_part.alloc(ncpa::tl1d_scratch(P, tl->n_ranges, M->prm.max_modes, ctx->num_sms), st);
         }
         CK(cudaStreamSynchronize(st));
         char key[160];
