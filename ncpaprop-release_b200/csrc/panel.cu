@@ -650,8 +650,75 @@ __device__ __forceinline__ void laguerre_half(const Panel& P, const double* __re
     }
 }
 
+// The transfer matrix of the chunks [c0, c1) at NC shifts per lane (its two
+// columns u, e and v, f up to a common scale) and the sign changes of the
+// column that starts with u = 0 (v), by which those of any state that enters
+// follow from the parity.
+template <class Row, int NC>
+__device__ __forceinline__ void count_segment(const Panel& P, const double* __restrict__ Trec, const double (&x)[NC],
+                                              int c0, int c1, PRing& R, unsigned* err, double (&u)[NC],
+                                              double (&e)[NC], double (&v)[NC], double (&f)[NC], int (&zeros)[NC]) {
+    typename Row::Shift sh[NC];
+#pragma unroll
+    for (int n = 0; n < NC; ++n) {
+        u[n] = f[n] = 1.0;
+        e[n] = v[n] = 0.0;
+        zeros[n] = 0;
+        sh[n] = typename Row::Shift(P, x[n]);
+    }
+    const double* src = Trec + (size_t)P.rec * kRecT;
+    ring_stream(
+        R, max(c1 - c0, 0), err,
+        [&](double* dst, uint64_t* bar, int o) {
+            mbar_expect_tx(bar, kTD * 8);
+            tma_load_1d(dst, src + (size_t)(c0 + o) * kTD, kTD * 8, bar);
+        },
+        [&](const double* rec, int o) {
+            const int nb = min(kPanelChunk, P.nblk - (c0 + o) * kPanelChunk);
+            for (int q = 0; q < nb; q += 2, rec += 2 * kRecT) {
+                double p[2][NC][4], t[2][NC];
+#pragma unroll
+                for (int n = 0; n < NC; ++n) {
+                    t[0][n] = sh[n].at(rec);
+                    t[1][n] = sh[n].at(rec + kRecT);
+                }
+                horner_blocks<NC>(rec, rec + kRecT, t, p);
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    if (q + b >= nb) break;
+                    const int n2 = __double2loint(rec[b * kRecT + kRecZeros]);
+#pragma unroll
+                    for (int n = 0; n < NC; ++n) {
+                        const double(&m)[4] = p[b][n];
+                        const double un = fma(m[0], u[n], m[1] * e[n]), vn = fma(m[0], v[n], m[1] * f[n]);
+                        e[n] = fma(m[2], u[n], m[3] * e[n]);
+                        f[n] = fma(m[2], v[n], m[3] * f[n]);
+                        zeros[n] += block_zeros(v[n], vn, m[1], t[b][n], n2);
+                        u[n] = un;
+                        v[n] = vn;
+                    }
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < NC; ++n) {
+                const int s = rescale_shift(fmax(fabs(u[n]), fabs(v[n])), fmax(fabs(e[n]), fabs(f[n])));
+                if (s) {
+                    const double sc = pow2(-s);
+                    u[n] *= sc;
+                    e[n] *= sc;
+                    v[n] *= sc;
+                    f[n] *= sc;
+                }
+            }
+        });
+}
+
 // ---------------------------------------------------------------------------
-// isolation scan: units of kScanStep shifts, one warp each
+// Isolation scan: units of kScanStep shifts, a CTA each, whose four warps take
+// a quarter of the blocks: with one warp to a unit a single problem's scan was
+// a chain of 157 blocks on 2 to 8 warps (0.1 Hz 49 us, 2 Hz 183 us; now 22 and 73),
+// and that of 256 problems ended with half of the chip idle (143 us, now 89).  The
+// second column costs 8 more instructions a block next to 120 of Horner's rule.
 // ---------------------------------------------------------------------------
 template <class Row>
 __global__ void __launch_bounds__(kPWarps * 32) k_panel_scan(const ProblemInfo* __restrict__ pinfo,
@@ -660,7 +727,7 @@ __global__ void __launch_bounds__(kPWarps * 32) k_panel_scan(const ProblemInfo* 
                                                              unsigned* err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int slot = blockIdx.x * kPWarps + wid, p = slot / kScanSlots, unit = slot % kScanSlots;
+    const int p = blockIdx.x / kScanSlots, unit = blockIdx.x % kScanSlots;
     const ProblemInfo& pi = pinfo[p];
     const int n = pi.n_scan;
     if (unit * kScanStep >= n) return;
@@ -670,7 +737,44 @@ __global__ void __launch_bounds__(kPWarps * 32) k_panel_scan(const ProblemInfo* 
     const double lo = Row::lo(pi), hi = Row::hi(pi);
     const double x[2] = {scan_x(lo, hi, t0, n), scan_x(lo, hi, t0 + 1, n)};
     int c[2];
-    count_sweep<Row, 2>(P, T, x, R, err, c);
+    if (!P.blk) {  // raw rows: one chain, on the first warp
+        if (wid) return;
+        count_sweep<Row, 2>(P, T, x, R, err, c);
+    } else {
+        struct Seg {
+            double m[4][2][32];
+            int z[2][32];
+        };
+        Seg* box = reinterpret_cast<Seg*>(smem_raw + kRingBytes<kTD>);
+        const int nch = (P.nblk + kPanelChunk - 1) / kPanelChunk;
+        double u[2], e[2], v[2], f[2];
+        int z[2];
+        count_segment<Row, 2>(P, T, x, nch * wid / kPWarps, nch * (wid + 1) / kPWarps, R, err, u, e, v, f, z);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            box[wid].m[0][k][lane] = u[k];
+            box[wid].m[1][k][lane] = e[k];
+            box[wid].m[2][k][lane] = v[k];
+            box[wid].m[3][k][lane] = f[k];
+            box[wid].z[k][lane] = z[k];
+        }
+        __syncthreads();
+        if (wid) return;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {  // the state (1, e0) through the segments
+            double a = 1.0, b = P.e0;
+            int zeros = 0;
+            for (int s = 0; s < kPWarps; ++s) {
+                const double an = fma(box[s].m[0][k][lane], a, box[s].m[2][k][lane] * b);
+                b = fma(box[s].m[1][k][lane], a, box[s].m[3][k][lane] * b);
+                const int n2 = box[s].z[k][lane];
+                zeros += n2 + static_cast<int>((neg(a) ^ neg(an)) ^ static_cast<unsigned>(n2 & 1));
+                a = an;
+                scale2(a, b);
+            }
+            c[k] = P.nz - zeros;
+        }
+    }
     *reinterpret_cast<int2*>(counts + (size_t)p * kScanMax + t0) = make_int2(c[0], c[1]);
 }
 
@@ -1771,8 +1875,10 @@ int scan_launch(cudaStream_t st, int P, int nz_max, const ProblemInfo* pinfo, co
         dim3 grid(expand_ctas(nz_max), kScanSlots * std::min(step, P - p0));
         k_expand_scan<Row><<<grid, kExpThreads, 0, st>>>(pinfo, p0, rows, T);
     }
-    static_assert(kScanSlots % kPWarps == 0, "a CTA's units belong to one problem");
-    k_panel_scan<Row><<<P * (kScanSlots / kPWarps), kPWarps * 32, kRingBytes<kTD>, st>>>(pinfo, rows, T, counts, err);
+    // the warps' rings, then their segments
+    const size_t sm = kRingBytes<kTD> + kPWarps * (4 * 2 * 32 * 8 + 2 * 32 * 4);
+    cudaFuncSetAttribute(k_panel_scan<Row>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_panel_scan<Row><<<P * kScanSlots, kPWarps * 32, sm, st>>>(pinfo, rows, T, counts, err);
     return n;
 }
 
