@@ -186,6 +186,7 @@ struct ModesArgs {
     const int* counts;
     const WorkItem* items;
     const int* n_items_dev;
+    int item_cap;  // at most this many
     double tol;
     double* mu;
     double *kr, *ki, *vs, *vr, *vg;
@@ -200,8 +201,9 @@ struct ModesArgs {
     unsigned long long* vpeak;  // zeroed
     double* vfull;              // [row][mode] per problem at vfull_off
     const long long* vfull_off;
-    int* sched;  // item counter (zeroed) or null: round-robin
+    int* sched;  // two item counters (zeroed) or null: round-robin
     int num_sms;
+    int min_items, max_items;  // (set by the launcher) a launch returns for other item counts
     unsigned* err;
     unsigned long long* steps;  // optional counter of row steps
 };

@@ -670,6 +670,7 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
     a.counts = b.counts.as<int>();
     a.items = b.items.as<WorkItem>();
     a.n_items_dev = b.tot.as<int>();
+    a.item_cap = b.item_cap;
     a.tol = wide ? kWmodTol : kBisectTol;
     a.mu = b.mu.as<double>();
     a.kr = M->d_kr.as<double>();

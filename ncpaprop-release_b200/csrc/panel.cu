@@ -47,6 +47,7 @@
 // eigenvalue's: 1e-6 of Im k for ducted modes, whose weights aloft are 1e9
 // times those in the duct.)
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 #include "device_common.cuh"
@@ -536,12 +537,12 @@ __device__ __forceinline__ void count_sweep(const Panel& P, const double* __rest
 }
 
 // ---------------------------------------------------------------------------
-// Laguerre sweeps.  The lower half of the blocks runs upwards (u), the upper
-// half downwards (b), one warp each, both with their first and half second
-// derivatives in t; at the block between, W = u e^b - e u^b is -u_{nz-1}, the
-// determinant up to sign, and its derivatives follow by the product rule.  An
-// isolated eigenvalue needs no counts: the sign of the determinant is the
-// parity of the count.
+// Laguerre sweeps, in four segments of the blocks: the first runs a state
+// upwards (u), the last one downwards (b), those between the two columns of
+// their transfer matrices, all with first and half second derivatives in t.
+// Put together, W = u e^b - e u^b is -u_{nz-1}, the determinant up to sign, and
+// its derivatives follow by the product rule.  An isolated eigenvalue needs no
+// counts: the sign of the determinant is the parity of the count.
 // ---------------------------------------------------------------------------
 struct LagChain {
     double u, e, u1, e1, u2, e2;
@@ -558,6 +559,24 @@ struct LagChain {
         }
     }
 };
+
+// two chains by a common factor
+__device__ __forceinline__ void rescale_pair(LagChain& A, LagChain& B) {
+    const double mu = fmax(fmax(fmax(fabs(A.u), fabs(A.u1)), fabs(A.u2)), fmax(fmax(fabs(B.u), fabs(B.u1)), fabs(B.u2)));
+    const double me = fmax(fmax(fmax(fabs(A.e), fabs(A.e1)), fabs(A.e2)), fmax(fmax(fabs(B.e), fabs(B.e1)), fabs(B.e2)));
+    const int sh = rescale_shift(mu, me);
+    if (sh) {
+        const double sc = pow2(-sh);
+        for (LagChain* C : {&A, &B}) {
+            C->u *= sc;
+            C->e *= sc;
+            C->u1 *= sc;
+            C->e1 *= sc;
+            C->u2 *= sc;
+            C->e2 *= sc;
+        }
+    }
+}
 
 // entries at t with first (d) and, for k2, half second (s) derivatives
 template <bool k2>
@@ -578,75 +597,82 @@ __device__ __forceinline__ void horner_der(const double* __restrict__ c, double 
     if (!k2) s[0] = s[1] = s[2] = s[3] = 0.0;
 }
 
+// one block's matrix on a chain: values, first and half second derivatives
 template <class Row>
-__device__ __forceinline__ void laguerre_half(const Panel& P, const double* __restrict__ Trec, double x, int half,
-                                              PRing& R, unsigned* err, LagChain& C) {
-    C = half ? LagChain{0.0, -1.0, 0.0, 0.0, 0.0, 0.0} : LagChain{1.0, P.e0, 0.0, 0.0, 0.0, 0.0};
-    if (P.blk) {
-        const typename Row::Shift sh(P, x);
-        const double* src = Trec + (size_t)P.rec * kRecT;
-        const int nch = (P.nblk + kPanelChunk - 1) / kPanelChunk, nu = (nch + 1) / 2;  // chunks; those of u
-        ring_stream(
-            R, half ? nch - nu : nu, err,
-            [&](double* dst, uint64_t* bar, int o) {
-                const size_t c = half ? nch - 1 - o : o;
-                mbar_expect_tx(bar, kTD * 8);
-                tma_load_1d(dst, src + c * kTD, kTD * 8, bar);
-            },
-            [&](const double* buf, int o) {
-                const int c = half ? nch - 1 - o : o, nb = min(kPanelChunk, P.nblk - c * kPanelChunk);
-                for (int i = 0; i < nb; ++i) {
-                    const double* rec = buf + (half ? nb - 1 - i : i) * kRecT;
-                    double p[4], d[4], s[4];
-                    horner_der<Row::kLaguerre>(rec, sh.at(rec), p, d, s);
-                    if (half) {  // the inverses: (u, e) -> (p3 u - p1 e, p0 e - p2 u)
-                        const double m[4] = {p[3], -p[1], -p[2], p[0]}, f[4] = {d[3], -d[1], -d[2], d[0]},
-                                     g[4] = {s[3], -s[1], -s[2], s[0]};
+__device__ __forceinline__ void lag_step(const double (&p)[4], const double (&d)[4], const double (&s)[4],
+                                         LagChain& C) {
+    double u2 = 0.0, e2 = 0.0;
+    if (Row::kLaguerre) {
+        u2 = fma(p[0], C.u2, p[1] * C.e2) + fma(d[0], C.u1, d[1] * C.e1) + fma(s[0], C.u, s[1] * C.e);
+        e2 = fma(p[2], C.u2, p[3] * C.e2) + fma(d[2], C.u1, d[3] * C.e1) + fma(s[2], C.u, s[3] * C.e);
+    }
+    const double u1 = fma(p[0], C.u1, p[1] * C.e1) + fma(d[0], C.u, d[1] * C.e);
+    const double e1 = fma(p[2], C.u1, p[3] * C.e1) + fma(d[2], C.u, d[3] * C.e);
+    const double u = fma(p[0], C.u, p[1] * C.e), e = fma(p[2], C.u, p[3] * C.e);
+    C = LagChain{u, e, u1, e1, u2, e2};
+}
+
+// NC chains through the chunks [c0, c1), upwards or down
+template <class Row, int NC>
+__device__ __forceinline__ void lag_segment(const Panel& P, const double* __restrict__ Trec, double x, int c0, int c1,
+                                            bool down, PRing& R, unsigned* err, LagChain (&C)[NC]) {
+    const typename Row::Shift sh(P, x);
+    const double* src = Trec + (size_t)P.rec * kRecT;
+    ring_stream(
+        R, max(c1 - c0, 0), err,
+        [&](double* dst, uint64_t* bar, int o) {
+            const size_t c = down ? c1 - 1 - o : c0 + o;
+            mbar_expect_tx(bar, kTD * 8);
+            tma_load_1d(dst, src + c * kTD, kTD * 8, bar);
+        },
+        [&](const double* buf, int o) {
+            const int c = down ? c1 - 1 - o : c0 + o, nb = min(kPanelChunk, P.nblk - c * kPanelChunk);
+            for (int i = 0; i < nb; ++i) {
+                const double* rec = buf + (down ? nb - 1 - i : i) * kRecT;
+                double p[4], d[4], s[4];
+                horner_der<Row::kLaguerre>(rec, sh.at(rec), p, d, s);
+                if (down) {  // the inverses: (u, e) -> (p3 u - p1 e, p0 e - p2 u)
+                    const double m[4] = {p[3], -p[1], -p[2], p[0]}, f[4] = {d[3], -d[1], -d[2], d[0]},
+                                 g[4] = {s[3], -s[1], -s[2], s[0]};
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            p[j] = m[j];
-                            d[j] = f[j];
-                            s[j] = g[j];
-                        }
-                    }
-                    double u2 = 0.0, e2 = 0.0;
-                    if (Row::kLaguerre) {
-                        u2 = fma(p[0], C.u2, p[1] * C.e2) + fma(d[0], C.u1, d[1] * C.e1) + fma(s[0], C.u, s[1] * C.e);
-                        e2 = fma(p[2], C.u2, p[3] * C.e2) + fma(d[2], C.u1, d[3] * C.e1) + fma(s[2], C.u, s[3] * C.e);
-                    }
-                    const double u1 = fma(p[0], C.u1, p[1] * C.e1) + fma(d[0], C.u, d[1] * C.e);
-                    const double e1 = fma(p[2], C.u1, p[3] * C.e1) + fma(d[2], C.u, d[3] * C.e);
-                    const double u = fma(p[0], C.u, p[1] * C.e), e = fma(p[2], C.u, p[3] * C.e);
-                    C = LagChain{u, e, u1, e1, u2, e2};
+                    for (int n = 0; n < NC; ++n) lag_step<Row>(m, f, g, C[n]);
+                } else {
+#pragma unroll
+                    for (int n = 0; n < NC; ++n) lag_step<Row>(p, d, s, C[n]);
                 }
-                C.rescale();
-            });
-    } else {
-        const int h = P.nz / 2, n = half ? P.nz - h : h;
-        for (int j = 0; j < n; ++j) {
-            const int i = half ? P.nz - 1 - j : j;
-            const double sg = Row::sigma(P.rows, i, x), sl = Row::slope(P.rows, i, x);
-            if (half) {
-                C.u -= C.e;
-                C.u1 -= C.e1;
-                if (Row::kLaguerre) {
-                    C.u2 -= C.e2;
-                    C.e2 = fma(sg, C.u2, fma(-sl, C.u1, C.e2));
-                }
-                C.e1 = fma(sg, C.u1, fma(-sl, C.u, C.e1));
-                C.e = fma(sg, C.u, C.e);
-            } else {
-                if (Row::kLaguerre) {
-                    C.e2 = fma(-sg, C.u2, fma(sl, C.u1, C.e2));
-                    C.u2 += C.e2;
-                }
-                C.e1 = fma(-sg, C.u1, fma(sl, C.u, C.e1));
-                C.e = fma(-sg, C.u, C.e);
-                C.u += C.e;
-                C.u1 += C.e1;
             }
-            if ((j & 15) == 15) C.rescale();
+            if (NC == 1) C[0].rescale();
+            else rescale_pair(C[0], C[NC - 1]);
+        });
+}
+
+// the raw rows' two halves
+template <class Row>
+__device__ __forceinline__ void lag_raw(const Panel& P, double x, int half, LagChain& C) {
+    const int h = P.nz / 2, n = half ? P.nz - h : h;
+    for (int j = 0; j < n; ++j) {
+        const int i = half ? P.nz - 1 - j : j;
+        const double sg = Row::sigma(P.rows, i, x), sl = Row::slope(P.rows, i, x);
+        if (half) {
+            C.u -= C.e;
+            C.u1 -= C.e1;
+            if (Row::kLaguerre) {
+                C.u2 -= C.e2;
+                C.e2 = fma(sg, C.u2, fma(-sl, C.u1, C.e2));
+            }
+            C.e1 = fma(sg, C.u1, fma(-sl, C.u, C.e1));
+            C.e = fma(sg, C.u, C.e);
+        } else {
+            if (Row::kLaguerre) {
+                C.e2 = fma(-sg, C.u2, fma(sl, C.u1, C.e2));
+                C.u2 += C.e2;
+            }
+            C.e1 = fma(-sg, C.u1, fma(sl, C.u, C.e1));
+            C.e = fma(-sg, C.u, C.e);
+            C.u += C.e;
+            C.u1 += C.e1;
         }
+        if ((j & 15) == 15) C.rescale();
     }
 }
 
@@ -967,23 +993,41 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_panel_groups(int P, const P
 }
 
 // ---------------------------------------------------------------------------
-// A work item runs on a pair of warps: of a Laguerre sweep they take the front
-// and the back rows, of a counting sweep 32 shifts each, of the eigenvectors the
-// upward and the downward pass.  Both keep the state of every slot and take the
-// same decisions from what they exchange, one barrier a round.
+// A work item runs on a pair of warps or on a team of four: of every sweep of its
+// eigenvalues they take two or one of four segments of the blocks (so the sums
+// are the same), of the eigenvectors the first two take the upward and the
+// downward pass.  All keep the state of every slot and take the same decisions
+// from what they exchange.
 // ---------------------------------------------------------------------------
 struct PairBox {
-    double v[2][2][6][32];  // [round parity][half][value][lane]
+    double v[2][2][3][32];  // [parity][half][value][lane]: of the eigenvector passes
     int c[2][2][32];        // counts
-    int err[2][2];
+    int err[2][4];
     int item[2];
 };
 
-struct Pair {
+// The W warps (2 or 4) of an item: warp `half` of W.  The segments' results are
+// exchanged through the rings, which are idle between sweeps.
+template <int W>
+struct Team {
     PairBox* box;
+    double* area;  // ring of the team's first warp
+    int stride;    // doubles of a warp's ring
     int id, half;
     int turn;  // buffer of the next exchange
-    __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, 64;" ::"r"(1 + id) : "memory"); }
+    __device__ __forceinline__ void sync() const {
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + id), "n"(32 * W) : "memory");
+    }
+    // the first two warps
+    __device__ __forceinline__ void sync2() const {
+        if (W == 2) sync();
+        else asm volatile("bar.sync 8, 64;" ::: "memory");
+    }
+    // where segment s puts its results (n doubles a segment of the first kind a warp takes)
+    __device__ __forceinline__ double* slot(int s, int n) const {
+        if (W == 4) return area + s * stride;
+        return area + (s >> 1) * stride + ((s == 1 || s == 2) ? n : 0);
+    }
 };
 
 // position of the n-th (0-based) set bit of m
@@ -1010,11 +1054,11 @@ __device__ __forceinline__ int nth_set(unsigned m, int n) {
 // dealt over the slots not yet isolated and cut their brackets.  A slot is final
 // when the correction is below tol, or when the last two steps stayed inside
 // the bracket and the cubic model predicts the next one below tol.
-template <class Row>
+template <class Row, int W>
 __device__ __forceinline__ double panel_bisect(const ProblemInfo& pi, const Panel& P, const WorkItem& w,
                                                const double* __restrict__ Trec, const int* __restrict__ counts,
                                                double tol_in, unsigned* err, unsigned long long* steps, PRing& R,
-                                               Pair& pr) {
+                                               Team<W>& pr) {
     const int lane = threadIdx.x & 31;
     const double lo = Row::lo(pi), hi = Row::hi(pi);
     const int nz = pi.nz, n = pi.n_scan;
@@ -1043,29 +1087,99 @@ __device__ __forceinline__ double panel_bisect(const ProblemInfo& pi, const Pane
         PairBox& X = *pr.box;
         const int tb = pr.turn;
         pr.turn ^= 1;
-        if (nB > 0) {  // counts: this half's virtual lanes
-            const int v = lane + 32 * pr.half;
-            const bool on = v >= nN;
-            const int t = on ? v - nN : 0, k = t % nB, g = t / nB, G = (nlB - 1 - k) / nB + 1;
-            const int e = nth_set(bm, k);
-            const double ae = __shfl_sync(0xffffffffu, a, e);
-            const double be = __shfl_sync(0xffffffffu, b, e);
-            const double xs[1] = {ae + (be - ae) * ((double)(g + 1) / (double)(G + 1))};
-            int c[1];
-            count_sweep<Row, 1>(P, Trec, xs, R, err, c);
-            X.c[tb][pr.half][lane] = c[0];
+        // segments of this warp: one of four, or an end and its neighbour
+        constexpr int kSegs = 4 / W;
+        auto seg_of = [&](int i) { return W == 4 ? pr.half : (pr.half ? 3 - i : i); };
+        const int nch = (P.nblk + kPanelChunk - 1) / kPanelChunk;
+        if (nB > 0) {  // counts: virtual lanes v = lane, lane + 32 of every warp
+            double xs[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int v = lane + 32 * h;
+                const int t = v >= nN ? v - nN : 0, k = t % nB, g = t / nB, G = (nlB - 1 - k) / nB + 1;
+                const int e = nth_set(bm, k);
+                const double ae = __shfl_sync(0xffffffffu, a, e);
+                const double be = __shfl_sync(0xffffffffu, b, e);
+                xs[h] = ae + (be - ae) * ((double)(g + 1) / (double)(G + 1));
+            }
+            constexpr int kN = 5 * 64;  // doubles of a segment
+            if (P.blk) {
+                double su[kSegs][2], se[kSegs][2], sv[kSegs][2], sf[kSegs][2];
+                int z[kSegs][2];
+#pragma unroll
+                for (int i = 0; i < kSegs; ++i) {
+                    const int s = seg_of(i);
+                    count_segment<Row, 2>(P, Trec, xs, nch * s / 4, nch * (s + 1) / 4, R, err, su[i], se[i], sv[i],
+                                          sf[i], z[i]);
+                }
+#pragma unroll
+                for (int i = 0; i < kSegs; ++i) {
+                    double* o = pr.slot(seg_of(i), kN);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int v = lane + 32 * h;
+                        o[v] = su[i][h];
+                        o[64 + v] = se[i][h];
+                        o[128 + v] = sv[i][h];
+                        o[192 + v] = sf[i][h];
+                        o[256 + v] = __hiloint2double(0, z[i][h]);
+                    }
+                }
+                pr.sync();
+                if (pr.half < 2) {  // shifts lane + 32 half: the state (1, e0) through the segments
+                    const int v = lane + 32 * pr.half;
+                    double ua = 1.0, eb = P.e0;
+                    int zeros = 0;
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        const double* o = pr.slot(s, kN);
+                        const double un = fma(o[v], ua, o[128 + v] * eb);
+                        eb = fma(o[64 + v], ua, o[192 + v] * eb);
+                        const int n2 = __double2loint(o[256 + v]);
+                        zeros += n2 + static_cast<int>((neg(ua) ^ neg(un)) ^ static_cast<unsigned>(n2 & 1));
+                        ua = un;
+                        scale2(ua, eb);
+                    }
+                    X.c[tb][pr.half][lane] = nz - zeros;
+                }
+                pr.sync();  // the rings are free again
+            } else if (pr.half == 0) {
+                int c[2];
+                count_sweep<Row, 2>(P, Trec, xs, R, err, c);
+                X.c[tb][0][lane] = c[0];
+                X.c[tb][1][lane] = c[1];
+            }
         }
+        constexpr int kL = 6 * 32;  // doubles of a chain
         if (nN > 0) {  // Laguerre chains of slots nth_set(nm, lane)
             const double xe = __shfl_sync(0xffffffffu, x, lane < nN ? nth_set(nm, lane) : 0);
-            LagChain C;
-            laguerre_half<Row>(P, Trec, xe, pr.half, R, err, C);
-            double(&o)[6][32] = X.v[tb][pr.half];
-            o[0][lane] = C.u;
-            o[1][lane] = C.e;
-            o[2][lane] = C.u1;
-            o[3][lane] = C.e1;
-            o[4][lane] = C.u2;
-            o[5][lane] = C.e2;
+            auto put = [&](double* o, const LagChain& C) {
+                o[lane] = C.u;
+                o[32 + lane] = C.e;
+                o[64 + lane] = C.u1;
+                o[96 + lane] = C.e1;
+                o[128 + lane] = C.u2;
+                o[160 + lane] = C.e2;
+            };
+            LagChain S[1], M[2];
+            S[0] = pr.half ? LagChain{0.0, -1.0, 0.0, 0.0, 0.0, 0.0} : LagChain{1.0, P.e0, 0.0, 0.0, 0.0, 0.0};
+            M[0] = LagChain{1.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            M[1] = LagChain{0.0, 1.0, 0.0, 0.0, 0.0, 0.0};
+            if (W == 2 || pr.half == 0 || pr.half == 3) {
+                const int s = pr.half ? 3 : 0;
+                if (P.blk) lag_segment<Row, 1>(P, Trec, xe, nch * s / 4, nch * (s + 1) / 4, s == 3, R, err, S);
+                else lag_raw<Row>(P, xe, s == 3, S[0]);
+            }
+            if (P.blk && (W == 2 || pr.half == 1 || pr.half == 2)) {
+                const int s = W == 4 ? pr.half : 1 + pr.half;
+                lag_segment<Row, 2>(P, Trec, xe, nch * s / 4, nch * (s + 1) / 4, false, R, err, M);
+            }
+            if (W == 2 || pr.half == 0 || pr.half == 3) put(pr.slot(pr.half ? 3 : 0, kL), S[0]);
+            if (W == 2 || pr.half == 1 || pr.half == 2) {
+                double* o = pr.slot(W == 4 ? pr.half : 1 + pr.half, kL);
+                put(o, M[0]);
+                put(o + kL, M[1]);
+            }
         }
         if (steps && lane == 0 && pr.half == 0) {
             atomicAdd(steps, (unsigned long long)((nB > 0 ? 64 : 0) + (nN > 0 ? 32 : 0)) * (unsigned long long)nz);
@@ -1075,25 +1189,38 @@ __device__ __forceinline__ double panel_bisect(const ProblemInfo& pi, const Pane
         pr.sync();
         if (mode == 1) {
             const int v = __popc(nm & ((1u << lane) - 1u));
-            const double(&F)[6][32] = X.v[tb][0];
-            const double(&B)[6][32] = X.v[tb][1];
-            const double u = F[0][v], e = F[1][v], u1 = F[2][v], e1 = F[3][v], u2 = F[4][v], e2 = F[5][v];
-            const double y = B[0][v], z = B[1][v], y1 = B[2][v], z1 = B[3][v], y2 = B[4][v], z2 = B[5][v];
-            const double W = u * z - e * y;
-            const double W1 = u1 * z + u * z1 - (e1 * y + e * y1);
+            auto get = [&](const double* o) {
+                return LagChain{o[v], o[32 + v], o[64 + v], o[96 + v], o[128 + v], o[160 + v]};
+            };
+            LagChain U = get(pr.slot(0, kL));
+            const LagChain D = get(pr.slot(3, kL));
+            if (P.blk) {
+#pragma unroll
+                for (int s = 1; s <= 2; ++s) {  // through the segments between
+                    const LagChain A = get(pr.slot(s, kL)), B = get(pr.slot(s, kL) + kL);
+                    const double m[4] = {A.u, B.u, A.e, B.e}, d[4] = {A.u1, B.u1, A.e1, B.e1},
+                                 q[4] = {A.u2, B.u2, A.e2, B.e2};
+                    lag_step<Row>(m, d, q, U);
+                    U.rescale();
+                }
+            }
+            const double u = U.u, e = U.e, u1 = U.u1, e1 = U.e1, u2 = U.u2, e2 = U.e2;
+            const double y = D.u, z = D.e, y1 = D.u1, z1 = D.e1, y2 = D.u2, z2 = D.e2;
+            const double w0 = u * z - e * y;
+            const double w1 = u1 * z + u * z1 - (e1 * y + e * y1);
             // below the eigenvalue the count nz - (sign changes of u) is J, above
-            // it J + 1; W = -u_{nz-1}
-            const bool below = ((neg(W) ^ 1u) ^ static_cast<unsigned>(nz & 1)) == static_cast<unsigned>(J & 1);
+            // it J + 1; w0 = -u_{nz-1}
+            const bool below = ((neg(w0) ^ 1u) ^ static_cast<unsigned>(nz & 1)) == static_cast<unsigned>(J & 1);
             const double xo = x;
             if (below) a = xo;
             else b = xo;
             double corr;
             if (Row::kLaguerre) {
-                const double W2 = u2 * z + u1 * z1 + u * z2 - (e2 * y + e1 * y1 + e * y2);  // half W''
-                const double rinv = 1.0 / P.r, g = W1 / W * rinv, h = fma(g, g, -(2.0 * (W2 / W) * rinv * rinv));
+                const double w2 = u2 * z + u1 * z1 + u * z2 - (e2 * y + e1 * y1 + e * y2);  // half W''
+                const double rinv = 1.0 / P.r, g = w1 / w0 * rinv, h = fma(g, g, -(2.0 * (w2 / w0) * rinv * rinv));
                 corr = laguerre_step(g, h, (double)nz, below);
             } else {
-                corr = W / W1 * P.r;
+                corr = w0 / w1 * P.r;
             }
             const double ad = fabs(corr);
             if (ad <= tol) {
@@ -1137,7 +1264,9 @@ __device__ __forceinline__ double panel_bisect(const ProblemInfo& pi, const Pane
             if (!(b - a > tol) || (a == A0 && b == B0)) mode = 2;
             else if (ca == J && cb == J + 1) mode = 1;
         }
-        if (X.err[tb][0] | X.err[tb][1]) break;  // a ring wait gave up: abandon the item
+        const bool gave_up = (X.err[tb][0] | X.err[tb][1] | (W == 4 ? X.err[tb][2] | X.err[tb][3] : 0)) != 0;
+        pr.sync();  // the rings are free again
+        if (gave_up) break;  // a ring wait ran out: abandon the item
     }
     return x;
 }
@@ -1511,9 +1640,9 @@ __device__ __noinline__ void fine_twist(const ModesArgs& A, const ProblemInfo& p
     W.Eu = q.E;
 }
 
-template <class Row, int NW, bool kV>
+template <class Row, int NW, bool kV, int W>
 __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemInfo& pi, const Panel& P,
-                                             const WorkItem& w, double mu, PRing& R, Pair& pr, double* __restrict__ ck,
+                                             const WorkItem& w, double mu, PRing& R, Team<W>& pr, double* __restrict__ ck,
                                              int* __restrict__ cke) {
     constexpr int kN = kSums<Row, NW>;
     const int lane = threadIdx.x & 31, half = pr.half;
@@ -1532,7 +1661,7 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
         X.v[tb][1][1][lane] = vr;
         X.v[tb][1][2][lane] = __hiloint2double(Es, Er);
     }
-    pr.sync();  // checkpoints of both halves (and the box) visible to both
+    pr.sync2();  // checkpoints of both halves (and the box) visible to both
     // the twist: the coarse row with the largest |u b|, the lowest of equal ones;
     // each half looks through half of the rows
     TwistKey K{0.0, 0, 0};
@@ -1546,7 +1675,7 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
         X.v[t2][1][0][lane] = K.m;
         X.v[t2][1][1][lane] = __hiloint2double(K.E, K.c);
     }
-    pr.sync();
+    pr.sync2();
     if (half) return;
     {
         const double m = X.v[t2][1][0][lane], ec = X.v[t2][1][1][lane];
@@ -1556,37 +1685,37 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
     const double us = vs, ur = vr, bs = X.v[tb][1][0][lane], br = X.v[tb][1][1][lane];
     const double eb = X.v[tb][1][2][lane];
     const int Eus = Es, Eur = Er, Ebs = __double2hiint(eb), Ebr = __double2loint(eb);
-    TwistAt<kN> W;
-    W.r = K.c * kCkRows;
+    TwistAt<kN> tw;
+    tw.r = K.c * kCkRows;
     const size_t o = (size_t)K.c * (1 + kN) * 32 + lane;
-    W.u = __ldcg(cks[0] + o);
-    W.b = __ldcg(cks[1] + o);
-    W.Eu = __ldcg(ckes[0] + (size_t)K.c * 32 + lane);
-    W.Eb = __ldcg(ckes[1] + (size_t)K.c * 32 + lane);
+    tw.u = __ldcg(cks[0] + o);
+    tw.b = __ldcg(cks[1] + o);
+    tw.Eu = __ldcg(ckes[0] + (size_t)K.c * 32 + lane);
+    tw.Eb = __ldcg(ckes[1] + (size_t)K.c * 32 + lane);
 #pragma unroll
     for (int n = 0; n < kN; ++n) {
-        W.su[n] = __ldcg(cks[0] + o + 32 * (1 + n));
-        W.sb[n] = __ldcg(cks[1] + o + 32 * (1 + n));
+        tw.su[n] = __ldcg(cks[0] + o + 32 * (1 + n));
+        tw.sb[n] = __ldcg(cks[1] + o + 32 * (1 + n));
     }
     if (kV && fine_twist_needed(pi)) {
-        if (lane < w.m) fine_twist<Row, NW>(A, pi, P, w, mu, cks, K.c, st, W);
+        if (lane < w.m) fine_twist<Row, NW>(A, pi, P, w, mu, cks, K.c, st, tw);
         __syncwarp();
     }
-    double ut = W.u, bt = W.b;
-    int Eut = W.Eu, Ebt = W.Eb;
+    double ut = tw.u, bt = tw.b;
+    int Eut = tw.Eu, Ebt = tw.Eb;
     normalize(ut, Eut);
     normalize(bt, Ebt);
-    const int eut = Eut - W.Eu, ebt = Ebt - W.Eb;  // exponents of u and b themselves
+    const int eut = Eut - tw.Eu, ebt = Ebt - tw.Eb;  // exponents of u and b themselves
     const double iu2 = 1.0 / (ut * ut), ib2 = 1.0 / (bt * bt);
     auto total = [&](int n) {  // sum over all rows in units of z_r^2
-        double x = W.su[n], y = W.sb[n];
+        double x = tw.su[n], y = tw.sb[n];
         int ex = 0, ey = 0;
         normalize(x, ex);
         normalize(y, ey);
         // both sums were taken at the exponents of u and b at the twist
         return x * iu2 * pow2(ex - 2 * eut) + y * ib2 * pow2(ey - 2 * ebt);
     };
-    const int r = W.r, isrc = pi.isrc, ircv = pi.ircv;
+    const int r = tw.r, isrc = pi.isrc, ircv = pi.ircv;
     const int n1 = Row::kUnitNorm ? 0 : kN - 1, nw = kN - NW;
     const double nrm = total(n1);  // sum z^2 / z_r^2
     const double f2 = Row::kUnitNorm ? 1.0 : 1.0 / (1.0 + (mu / pi.dz) * (mu / pi.dz));
@@ -1615,30 +1744,38 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
 // ---------------------------------------------------------------------------
 // eigenvalues and mode values of every item.  kDo: 1 eigenvalues to mu, 2 mode
 // values of the eigenvalues in mu, 3 both.  The pairs take items from the
-// cost-ordered list as they get free (sched: a zeroed counter), or round-robin.
+// cost-ordered list as they get free (sched: two zeroed counters), or round-robin.
 // ---------------------------------------------------------------------------
-template <class Row, int NW, int kDo, bool kV>
+// doubles of a ring slot: eigenvalues alone need no weights
+template <int NW, int kDo>
+constexpr int kModesSl = kTD + (kDo == 1 ? 0 : NW) * kWD;
+
+template <class Row, int NW, int kDo, bool kV, int W>
 __global__ void __launch_bounds__(kPWarps * 32, kPanelCtas) k_panel_modes(ModesArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    constexpr int kSl = kTD + NW * kWD;
+    constexpr int kSl = kModesSl<NW, kDo>;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int n_items = *A.n_items_dev;
+    if (n_items < A.min_items || n_items > A.max_items) return;  // another launch's
     PRing R = make_ring(smem_raw, wid, kSl);
-    Pair pr;
-    pr.box = reinterpret_cast<PairBox*>(smem_raw + kRingBytes<kSl>) + (wid >> 1);
-    pr.id = wid >> 1;
-    pr.half = wid & 1;
+    constexpr int kTeams = kPWarps / W;
+    Team<W> pr;
+    pr.id = wid / W;
+    pr.half = wid % W;
+    pr.box = reinterpret_cast<PairBox*>(smem_raw + kRingBytes<kSl>) + pr.id;
+    pr.stride = kPBuf * kSl;
+    pr.area = reinterpret_cast<double*>(smem_raw) + (size_t)pr.id * W * pr.stride;
     pr.turn = 0;
-    const long long gp = (long long)blockIdx.x * (kPWarps / 2) + pr.id;
+    const long long gp = (long long)blockIdx.x * kTeams + pr.id;
     double* ck = A.ck_u + gp * 2 * A.ck_stride * (1 + kSums<Row, NW>);
     int* cke = A.ck_e + gp * 2 * A.ck_stride;
-    // first items: one to the first pair of as many CTAs as there are SMs (which
-    // start on different ones), then to their second pairs, then to the next
+    // first items: one to the first team of as many CTAs as there are SMs (which
+    // start on different ones), then to their second teams, then to the next
     // CTAs, so that few items have a scheduler for each warp; later ones as the
-    // pairs get free (sched), or round-robin
-    const int n_pairs = gridDim.x * (kPWarps / 2), row = blockIdx.x / A.num_sms;
+    // teams get free (sched), or round-robin
+    const int n_pairs = gridDim.x * kTeams, row = blockIdx.x / A.num_sms;
     const int width = min(A.num_sms, (int)gridDim.x - row * A.num_sms);  // CTAs of this row
-    long long walk = (long long)row * A.num_sms * (kPWarps / 2) + pr.id * width + blockIdx.x % A.num_sms;
+    long long walk = (long long)row * A.num_sms * kTeams + pr.id * width + blockIdx.x % A.num_sms;
     bool first = true;
     for (int turn = 0;; turn ^= 1) {
         if (pr.half == 0 && lane == 0) {
@@ -1659,12 +1796,12 @@ __global__ void __launch_bounds__(kPWarps * 32, kPanelCtas) k_panel_modes(ModesA
         const Panel P = panel_of<Row>(pi, d, A.rows);
         double x = P.xc;
         if (kDo & 1) {
-            x = panel_bisect<Row>(pi, P, w, A.T, A.counts, A.tol, A.err, A.steps, R, pr);
+            x = panel_bisect<Row, W>(pi, P, w, A.T, A.counts, A.tol, A.err, A.steps, R, pr);
             if (pr.half == 0 && lane < w.m) A.mu[pi.off + w.j0 + lane] = x;
         } else if (lane < w.m) {
             x = A.mu[pi.off + w.j0 + lane];
         }
-        if (kDo & 2) panel_vector<Row, NW, kV>(A, pi, P, w, x, R, pr, ck, cke);
+        if ((kDo & 2) && pr.half < 2) panel_vector<Row, NW, kV, W>(A, pi, P, w, x, R, pr, ck, cke);
     }
 }
 
@@ -1736,16 +1873,60 @@ __global__ void __launch_bounds__(256) k_panel_fill(int p0, ModesArgs A) {
     }
 }
 
-template <class Row, int NW>
-int modes_launch(cudaStream_t st, int grid, const ModesArgs& a, int what) {
-    const size_t sm = kRingBytes<kTD + NW * kWD> + (kPWarps / 2) * sizeof(PairBox);
-    const bool v = a.vstate != nullptr;
-    void (*f)(ModesArgs) = what == 1   ? k_panel_modes<Row, NW, 1, false>
-                           : what == 2 ? (v ? k_panel_modes<Row, NW, 2, true> : k_panel_modes<Row, NW, 2, false>)
-                                       : (v ? k_panel_modes<Row, NW, 3, true> : k_panel_modes<Row, NW, 3, false>);
+template <class Row, int NW, int kDo, bool kV, int W>
+void modes_run(cudaStream_t st, int grid, const ModesArgs& a) {
+    constexpr int kSl = kModesSl<NW, kDo>;
+    static_assert(kSl * kPBuf >= 18 * 32 && kSl * kPBuf >= 2 * 5 * 64, "a warp's segments fit its ring");
+    const size_t sm = kRingBytes<kSl> + (kPWarps / 2) * sizeof(PairBox);
+    auto* f = k_panel_modes<Row, NW, kDo, kV, W>;
     cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     f<<<grid, kPWarps * 32, sm, st>>>(a);
-    return 1;
+}
+
+template <class Row, int NW, int kDo, int W>
+void modes_run(cudaStream_t st, int grid, const ModesArgs& a) {
+    if (kDo != 1 && a.vstate) modes_run<Row, NW, kDo, kDo != 1, W>(st, grid, a);
+    else modes_run<Row, NW, kDo, false, W>(st, grid, a);
+}
+
+// How many warps an item gets, by the number of items (known on the device: a
+// launch that it does not ask for returns at once; those beyond item_cap are
+// left out).  The arithmetic is the same.
+//  up to two an SM     teams of four, both stages in one launch: an item alone on
+//                      its SM has a scheduler for each warp (0.1 Hz: 77 + 102
+//                      us as pairs 129 + 107; 32 requests 289 + 205 as pairs 543
+//                      + 207)
+//  up to 4 x the pairs teams of four for the eigenvalues, pairs for the mode
+//  that fit            values: items are finished sooner, so fewer idle at the
+//                      end (256 frequencies, 1.3 x: 553 us, as pairs 603; 64
+//                      wide-angle ones 408, as pairs 659)
+//  more                pairs: 6 % less work than in the transfer matrices of the
+//                      inner segments twice over (45-azimuth sweep 1906 us, as
+//                      teams 1962)
+// The stages apart where SMs are full: in one kernel their code shares the
+// instruction cache (256 frequencies: 1118 us in one launch of pairs, 950 in two).
+template <class Row, int NW>
+int modes_launch(cudaStream_t st, int grid, const ModesArgs& a, int what) {
+    ModesArgs few = a, some = a, many = a, rest = a;
+    few.min_items = 0;
+    few.max_items = std::min(grid, 2 * a.num_sms);
+    rest.min_items = some.min_items = few.max_items + 1;
+    some.max_items = std::max(4 * (kPWarps / 2) * grid, few.max_items);
+    many.min_items = some.max_items + 1;
+    rest.max_items = many.max_items = INT_MAX;
+    if (what == 1) modes_run<Row, 1, 1, 4>(st, few.max_items, few);
+    if (what == 2) modes_run<Row, NW, 2, 4>(st, few.max_items, few);
+    if (what == 3) modes_run<Row, NW, 3, 4>(st, few.max_items, few);
+    int n = 1;
+    if (what & 1) {
+        if (a.item_cap >= some.min_items) modes_run<Row, 1, 1, 4>(st, grid, some), ++n;
+        if (a.item_cap >= many.min_items) modes_run<Row, 1, 1, 2>(st, grid, many), ++n;
+    }
+    if (what & 2 && a.item_cap >= rest.min_items) {
+        if (what == 3 && rest.sched) ++rest.sched;  // a counter of its own
+        modes_run<Row, NW, 2, 2>(st, grid, rest), ++n;
+    }
+    return n;
 }
 
 // CTAs per panel: enough for one thread per column of 128-row blocks, more
