@@ -1316,9 +1316,23 @@ __device__ __forceinline__ void adj_add(const double (&d)[4], double u, double e
 template <class Row, int NW>
 constexpr int kSums = (Row::kUnitNorm ? 1 : 0) + NW;
 
-// a chain (u, e) with its derivatives d/dt and d/deps
-template <class Row, int NW>
+// What a warp of the mode-value pass carries beside its chain (part 0: all).  A
+// team of four splits it: the norm to one warp and the weights to the other, or
+// a weight each.
+template <class Row, int NW, int kPart>
+struct Part {
+    static constexpr bool norm = Row::kUnitNorm && kPart != 2;
+    static constexpr int lo = kPart == 2 && !Row::kUnitNorm ? 1 : 0;
+    static constexpr int hi = kPart == 1 ? (Row::kUnitNorm ? 0 : 1) : NW;  // weights [lo, hi)
+};
+
+// a chain (u, e) with its derivatives d/dt and d/deps.  The common exponent
+// follows u and e alone (so that it does not depend on the part): the
+// derivatives are at most some 2^130 above, where the chain has decayed to its
+// rounding while they have grown, and their products stay finite.
+template <class Row, int NW, int kPart>
 struct VecChain {
+    using Q = Part<Row, NW, kPart>;
     double u, e, u1, e1, uw[NW], ew[NW];
     int E;  // common exponent
     __device__ __forceinline__ void start(double u0, double e0) {
@@ -1330,27 +1344,17 @@ struct VecChain {
         E = 0;
     }
     __device__ __forceinline__ void rescale() {
-        double m = fabs(u), k = fabs(e);
-        if (Row::kUnitNorm) {
-            m = fmax(m, fabs(u1));
-            k = fmax(k, fabs(e1));
-        }
-#pragma unroll
-        for (int n = 0; n < NW; ++n) {
-            m = fmax(m, fabs(uw[n]));
-            k = fmax(k, fabs(ew[n]));
-        }
-        const int x = max(biased_exp(m), biased_exp(k)), sh = x - 1023;
+        const int x = max(biased_exp(u), biased_exp(e)), sh = x - 1023;
         if (x != 0 && (sh > 240 || sh < -240)) {  // products of two stay finite
             const double sc = pow2(-sh);
             u *= sc;
             e *= sc;
-            if (Row::kUnitNorm) {
+            if (Q::norm) {
                 u1 *= sc;
                 e1 *= sc;
             }
 #pragma unroll
-            for (int n = 0; n < NW; ++n) {
+            for (int n = Q::lo; n < Q::hi; ++n) {
                 uw[n] *= sc;
                 ew[n] *= sc;
             }
@@ -1366,8 +1370,9 @@ struct VecChain {
 };
 
 // matrices of two blocks at t: values, d/dt (Row::kUnitNorm) and the weights'
-template <class Row, int NW>
+template <class Row, int NW, int kPart>
 struct VecMats {
+    using Q = Part<Row, NW, kPart>;
     double p[2][4], d[2][4], w[2][NW][4];
     __device__ __forceinline__ void eval(const double* const (&T)[2], const double* const (&W)[2],
                                          const double (&t)[2]) {
@@ -1380,12 +1385,12 @@ struct VecMats {
                 const double cf[4] = {v0.x, v0.y, v1.x, v1.y};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    if (Row::kUnitNorm && k < kPD) d[b][j] = k == kPD - 1 ? p[b][j] : fma(d[b][j], t[b], p[b][j]);
+                    if (Q::norm && k < kPD) d[b][j] = k == kPD - 1 ? p[b][j] : fma(d[b][j], t[b], p[b][j]);
                     p[b][j] = k == kPD ? cf[j] : fma(p[b][j], t[b], cf[j]);
                 }
                 if (k <= kPW) {
 #pragma unroll
-                    for (int n = 0; n < NW; ++n) {
+                    for (int n = Q::lo; n < Q::hi; ++n) {
                         const double2* r = reinterpret_cast<const double2*>(W[b] + n * kWD);
                         const double2 w0 = r[2 * k], w1 = r[2 * k + 1];
                         const double wf[4] = {w0.x, w0.y, w1.x, w1.y};
@@ -1395,15 +1400,15 @@ struct VecMats {
                 }
             }
     }
-    __device__ __forceinline__ void up(int b, VecChain<Row, NW>& C) const {
+    __device__ __forceinline__ void up(int b, VecChain<Row, NW, kPart>& C) const {
         const double(&m)[4] = p[b];
-        if (Row::kUnitNorm) {
+        if (Q::norm) {
             const double v = fma(m[0], C.u1, m[1] * C.e1) + fma(d[b][0], C.u, d[b][1] * C.e);
             C.e1 = fma(m[2], C.u1, m[3] * C.e1) + fma(d[b][2], C.u, d[b][3] * C.e);
             C.u1 = v;
         }
 #pragma unroll
-        for (int n = 0; n < NW; ++n) {
+        for (int n = Q::lo; n < Q::hi; ++n) {
             const double(&g)[4] = w[b][n];
             const double v = fma(m[0], C.uw[n], m[1] * C.ew[n]) + fma(g[0], C.u, g[1] * C.e);
             C.ew[n] = fma(m[2], C.uw[n], m[3] * C.ew[n]) + fma(g[2], C.u, g[3] * C.e);
@@ -1413,13 +1418,13 @@ struct VecMats {
         C.e = fma(m[2], C.u, m[3] * C.e);
         C.u = un;
     }
-    __device__ __forceinline__ void down(int b, VecChain<Row, NW>& C) const {
-        if (Row::kUnitNorm) {
+    __device__ __forceinline__ void down(int b, VecChain<Row, NW, kPart>& C) const {
+        if (Q::norm) {
             adj_apply(p[b], C.u1, C.e1);
             adj_add(d[b], C.u, C.e, C.u1, C.e1);
         }
 #pragma unroll
-        for (int n = 0; n < NW; ++n) {
+        for (int n = Q::lo; n < Q::hi; ++n) {
             adj_apply(p[b], C.uw[n], C.ew[n]);
             adj_add(w[b][n], C.u, C.e, C.uw[n], C.ew[n]);
         }
@@ -1432,10 +1437,11 @@ struct VecMats {
 // value, exponent and sums go to the checkpoints and, for full vectors (kV),
 // its state to `st` (stride: modes).  vs, vr: its values at the source and
 // receiver rows.
-template <class Row, int NW, bool kV>
+template <class Row, int NW, bool kV, int kPart>
 __device__ __forceinline__ void vector_half(const ModesArgs& A, const ProblemInfo& pi, const Panel& P, double mu,
                                             int half, VecState* __restrict__ st, PRing& R, double* __restrict__ ck, int* __restrict__ cke,
                                             double& vs, int& Es, double& vr, int& Er) {
+    using Q = Part<Row, NW, kPart>;
     constexpr int kN = kSums<Row, NW>;
     const int lane = threadIdx.x & 31;
     const int nz = P.nz, isrc = pi.isrc, ircv = pi.ircv;
@@ -1444,7 +1450,7 @@ __device__ __forceinline__ void vector_half(const ModesArgs& A, const ProblemInf
     const double* wp = A.w + pi.w_off;
     const double* gp = NW > 1 && A.g ? A.g + pi.s_off : nullptr;
     auto weight = [&](int n, int i) { return n == 0 ? __ldg(wp + i) : (gp ? __ldg(gp + i) : 1.0); };
-    VecChain<Row, NW> C;
+    VecChain<Row, NW, kPart> C;
     if (half == 0) C.start(1.0, P.e0);
     else C.start(0.0, -1.0);
     vs = vr = 0.0;
@@ -1453,15 +1459,18 @@ __device__ __forceinline__ void vector_half(const ModesArgs& A, const ProblemInf
         if (a % kCkRows) return;
         const size_t c = (size_t)(a / kCkRows);
         double* o = ck + c * (1 + kN) * 32 + lane;
-        o[0] = C.u;
+        if (kPart != 2) {
+            o[0] = C.u;
+            cke[c * 32 + lane] = C.E;
+        }
+        if (Q::norm) o[32] = C.sum(0, rinv, sgn);
 #pragma unroll
-        for (int n = 0; n < kN; ++n) o[32 * (1 + n)] = C.sum(n, rinv, sgn);
-        cke[c * 32 + lane] = C.E;
-        if (kV && st) st[c * pi.M] = VecState{C.u, C.e, C.E, 0};
+        for (int n = Q::lo; n < Q::hi; ++n) o[32 * (1 + kN - NW + n)] = C.sum(kN - NW + n, rinv, sgn);
+        if (kV && kPart != 2 && st) st[c * pi.M] = VecState{C.u, C.e, C.E, 0};
     };
     // the chain at row i of the block [a, end): from below (u) or above (b)
     auto value = [&](int i, int a, int end, double& v, int& E) {
-        if (i < a || i >= end) return;
+        if (kPart == 2 || i < a || i >= end) return;
         double f = C.e;
         v = C.u;
         E = C.E;
@@ -1476,17 +1485,17 @@ __device__ __forceinline__ void vector_half(const ModesArgs& A, const ProblemInf
             R, nch, A.err,
             [&](double* dst, uint64_t* bar, int o) {
                 const size_t c = half ? nch - 1 - o : o;
-                mbar_expect_tx(bar, (kTD + NW * kWD) * 8);
+                mbar_expect_tx(bar, (kTD + (Q::hi - Q::lo) * kWD) * 8);
                 tma_load_1d(dst, src + c * kTD, kTD * 8, bar);
 #pragma unroll
-                for (int n = 0; n < NW; ++n) tma_load_1d(dst + kTD + n * kWD, sw[n] + c * kWD, kWD * 8, bar);
+                for (int n = Q::lo; n < Q::hi; ++n) tma_load_1d(dst + kTD + n * kWD, sw[n] + c * kWD, kWD * 8, bar);
             },
             [&](const double* buf, int o) {
                 const int c = half ? nch - 1 - o : o, nb = min(kPanelChunk, P.nblk - c * kPanelChunk);
                 for (int q0 = 0; q0 < kPanelChunk; q0 += 2) {
                     const int qa = half ? kPanelChunk - 1 - q0 : q0, qb = half ? qa - 1 : qa + 1;
                     if (min(qa, qb) >= nb) continue;
-                    VecMats<Row, NW> M;
+                    VecMats<Row, NW, kPart> M;
                     const double* const Ts[2] = {buf + qa * kRecT, buf + qb * kRecT};
                     const double* const Ws[2] = {buf + kTD + qa * kRecW, buf + kTD + qb * kRecW};
                     const double t[2] = {sh.at(Ts[0]), sh.at(Ts[1])};
@@ -1520,20 +1529,22 @@ __device__ __forceinline__ void vector_half(const ModesArgs& A, const ProblemInf
                 const int i = half ? a + end - 1 - j : j;
                 const double sg = Row::sigma(P.rows, i, mu), sl = Row::slope(P.rows, i, mu);
                 if (half == 0) {
-                    C.e1 = fma(-sg, C.u1, fma(sl, C.u, C.e1));
+                    if (Q::norm) C.e1 = fma(-sg, C.u1, fma(sl, C.u, C.e1));
 #pragma unroll
-                    for (int n = 0; n < NW; ++n) C.ew[n] = fma(-sg, C.uw[n], fma(-weight(n, i), C.u, C.ew[n]));
+                    for (int n = Q::lo; n < Q::hi; ++n) C.ew[n] = fma(-sg, C.uw[n], fma(-weight(n, i), C.u, C.ew[n]));
                     C.e = fma(-sg, C.u, C.e);
                     C.u += C.e;
-                    C.u1 += C.e1;
+                    if (Q::norm) C.u1 += C.e1;
 #pragma unroll
-                    for (int n = 0; n < NW; ++n) C.uw[n] += C.ew[n];
+                    for (int n = Q::lo; n < Q::hi; ++n) C.uw[n] += C.ew[n];
                 } else {
                     C.u -= C.e;
-                    C.u1 -= C.e1;
-                    C.e1 = fma(sg, C.u1, fma(-sl, C.u, C.e1));
+                    if (Q::norm) {
+                        C.u1 -= C.e1;
+                        C.e1 = fma(sg, C.u1, fma(-sl, C.u, C.e1));
+                    }
 #pragma unroll
-                    for (int n = 0; n < NW; ++n) {
+                    for (int n = Q::lo; n < Q::hi; ++n) {
                         C.uw[n] -= C.ew[n];
                         C.ew[n] = fma(sg, C.uw[n], fma(weight(n, i), C.u, C.ew[n]));
                     }
@@ -1642,10 +1653,10 @@ __device__ __noinline__ void fine_twist(const ModesArgs& A, const ProblemInfo& p
 
 template <class Row, int NW, bool kV, int W>
 __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemInfo& pi, const Panel& P,
-                                             const WorkItem& w, double mu, PRing& R, Team<W>& pr, double* __restrict__ ck,
-                                             int* __restrict__ cke) {
+                                             const WorkItem& w, double mu, PRing& R, Team<W>& pr, bool split,
+                                             double* __restrict__ ck, int* __restrict__ cke) {
     constexpr int kN = kSums<Row, NW>;
-    const int lane = threadIdx.x & 31, half = pr.half;
+    const int lane = threadIdx.x & 31, half = pr.half & 1;
     const int nc = (P.nz + kCkRows - 1) / kCkRows;
     double* cks[2] = {ck, ck + A.ck_stride * (1 + kN)};
     int* ckes[2] = {cke, cke + A.ck_stride};
@@ -1653,15 +1664,27 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
     int Es, Er;
     VecState* st = nullptr;
     if (kV && lane < w.m) st = A.vstate + A.vstate_off[w.problem] + w.j0 + lane;
-    vector_half<Row, NW, kV>(A, pi, P, mu, half, st ? st + (long long)half * nc * pi.M : nullptr, R, cks[half], ckes[half], vs, Es, vr, Er);
+    if (kV && st) st += (long long)half * nc * pi.M;
+    // a team alone on its SM splits the sums (1185 modes: 403 -> 294 us);
+    // two of them fill it, and the transfer matrices evaluated twice cost more
+    // than the idle warps (36 azimuths of 0.5 Hz: both stages 286 us, split 300)
+    double* c = cks[half];
+    int* ce = ckes[half];
+    if (W == 4 && split) {
+        if (pr.half < 2) vector_half<Row, NW, kV, 1>(A, pi, P, mu, half, st, R, c, ce, vs, Es, vr, Er);
+        else vector_half<Row, NW, kV, 2>(A, pi, P, mu, half, st, R, c, ce, vs, Es, vr, Er);
+    } else if (pr.half < 2) {
+        vector_half<Row, NW, kV, 0>(A, pi, P, mu, half, st, R, c, ce, vs, Es, vr, Er);
+    }
     PairBox& X = *pr.box;
     const int tb = pr.turn, t2 = tb ^ 1;
-    if (half) {
+    if (pr.half == 1) {
         X.v[tb][1][0][lane] = vs;
         X.v[tb][1][1][lane] = vr;
         X.v[tb][1][2][lane] = __hiloint2double(Es, Er);
     }
-    pr.sync2();  // checkpoints of both halves (and the box) visible to both
+    pr.sync();  // checkpoints of both halves (and the box) visible to both
+    if (pr.half >= 2) return;
     // the twist: the coarse row with the largest |u b|, the lowest of equal ones;
     // each half looks through half of the rows
     TwistKey K{0.0, 0, 0};
@@ -1801,7 +1824,7 @@ __global__ void __launch_bounds__(kPWarps * 32, kPanelCtas) k_panel_modes(ModesA
         } else if (lane < w.m) {
             x = A.mu[pi.off + w.j0 + lane];
         }
-        if ((kDo & 2) && pr.half < 2) panel_vector<Row, NW, kV, W>(A, pi, P, w, x, R, pr, ck, cke);
+        if (kDo & 2) panel_vector<Row, NW, kV, W>(A, pi, P, w, x, R, pr, n_items <= A.num_sms, ck, cke);
     }
 }
 
