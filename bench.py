@@ -304,7 +304,7 @@ def run_ours(args):
     sturm_steps, deriv_steps = ctx.bisect_steps()
     phases = {ph: ctx.phase_stats(ph)[0] / n_ph for ph in
               ("knots+grid", "matrix", "window", "scan", "host-items", "bisect", "eigvec", "fetch")}
-    # the fused bisection + eigenvector launch the timed steps run, timed alone
+    # eigenvalues and mode values as the timed steps launch them, timed alone
     ctx.reset_stats()
     ctx.set_timing(2)
     for _ in range(n_ph):
@@ -314,7 +314,6 @@ def run_ours(args):
     ctx.set_timing(False)
     fused_ms, fused_n = ctx.phase_stats("bisect+eigvec")
     phases["bisect+eigvec (fused)"] = fused_ms / max(fused_n, 1)
-    phases["eigvec-rest"] = ctx.phase_stats("eigvec-rest")[0] / n_ph
     m_cnt = ctx.solve(prof, params_dev, freqs, az)
     modes_total = m_cnt.total_modes()
     m_cnt.close()
@@ -354,16 +353,15 @@ def run_ours(args):
         solves = NFREQ * args.steps * world
         value = solves / (ms_dev / 1e3)
         e2e_value = solves / (ms_e2e / 1e3)
-        # bisection kernel roofline, steps counted by the kernel: 3 FP64 flops
-        # per step of a count-only chain (subtract + fused multiply-add), 10
-        # per step of a Laguerre chain (p, p', p'': subtract, four FMAs, one add)
-        flops = 3.0 * (sturm_steps - deriv_steps) + 10.0 * deriv_steps  # over the bis_n timed launches
+        # eigenvalue sweeps, row steps (one shift over one grid point) counted by
+        # the kernel.  At 128 rows a block: a count's four polynomials of degree
+        # 14 and two columns are 126 FP64 flops a block, 1.0 a row; a Laguerre
+        # chain's, with first and second derivatives, 375, 2.9 a row
+        flops = 1.0 * (sturm_steps - deriv_steps) + 2.9 * deriv_steps  # over the bis_n timed launches
         achieved = flops / (bis_ms / 1e3) / 1e12 if bis_ms > 0 else None
-        # the fused launch: the same bisection work plus the reduction-only
-        # eigenvector items, 7 flops per row and pass (square, add, multiply-
-        # add with the weight, subtract, multiply-add of the recurrence), two
-        # passes per mode
-        ev_flops = 14.0 * NZ * modes_total
+        # with the mode values: two directions per mode, 338 flops a block each
+        # (entries, their derivative and the weight's), 5.3 a row in all
+        ev_flops = 5.3 * NZ * modes_total
         fused_flops = (flops / bis_n if bis_n else 0.0) + ev_flops
         fused_launch_ms = fused_ms / max(fused_n, 1)
         fused_achieved = fused_flops / (fused_launch_ms / 1e3) / 1e12 if fused_ms > 0 else None
@@ -377,31 +375,32 @@ def run_ours(args):
                        "profile": "analytic 0-150 km (T piecewise linear, 60+20 m/s jets)", "nz_grid": NZ,
                        "n_freq": NFREQ, "df_hz": 0.5 / NFREQ, "azimuth_deg": az[0], "tl_ranges": N_TL,
                        "synthesis_ranges_km": "200-300/10", "nfft": nfft, "l2": "flushed (256 MiB write) between steps",
-                       "eigen_solve": "fused bisection + eigenvector launch in the timed steps; phases_ms and the "
-                                      "roofline time k_bisect and k_eigvec alone (per-phase timing runs them "
-                                      "separately) and the fused launch alone (roofline.fused)",
+                       "eigen_solve": "panel expansions; phases_ms and the roofline time the eigenvalue and the "
+                                      "mode-value launches alone and both as the timed steps run them "
+                                      "(roofline.fused)",
                        "parallelism": "replicas (one 256-frequency job per GPU)"},
             "e2e": {"value": round(e2e_value, 2), "unit": METRIC, "h2d_bytes_per_step": int(h2d[0]),
                     "d2h_bytes_per_step": int(d2h[0])},
             "gpu_launches": int(launches),
             "clocks": clocks,
-            "roofline": {"kernel": "k_bisect (Sturm multisection)", "bound": "fp64",
+            "roofline": {"kernel": "k_panel_modes (eigenvalues)", "bound": "fp64",
                          "achieved": round(achieved, 3) if achieved else None, "peak": round(fp64_peak, 3),
                          "unit": "TFLOP/s", "frac": round(achieved / fp64_peak, 4) if achieved else None,
                          "peak_source": "measured in this run (dependent-FMA probe on all SMs)",
                          "traffic": None, "traffic_source": "not measured by this run (DRAM counters need ncu)",
                          "avg_launch_ms": round(bis_ms / max(bis_n, 1), 4),
                          "flops_per_launch": flops / bis_n if bis_n else None,
-                         "flops": "3 per count-chain step, 10 per Laguerre-chain step (p, p', p'')",
+                         "flops": "1.0 per count-chain row step, 2.9 per Laguerre-chain row step (blocks of 128 "
+                                  "rows)",
                          "chain_steps_per_launch": sturm_steps / bis_n if bis_n else None,
                          "laguerre_chain_steps_per_launch": deriv_steps / bis_n if bis_n else None,
-                         "fused": {"kernel": "k_bisect_eigvec (the launch the timed steps run)",
+                         "fused": {"kernel": "k_panel_modes (eigenvalues and mode values as in the timed steps)",
                                    "avg_launch_ms": round(fused_launch_ms, 4),
                                    "flops_per_launch": fused_flops,
                                    "achieved": round(fused_achieved, 3) if fused_achieved else None,
                                    "frac": round(fused_achieved / fp64_peak, 4) if fused_achieved else None,
-                                   "flops": "the bisection's counted flops + 14 per grid row per mode for the "
-                                            "two eigenvector passes (%d modes)" % modes_total}},
+                                   "flops": "the eigenvalue sweeps' counted flops + 5.3 per grid row per mode for "
+                                            "the two directions of the mode values (%d modes)" % modes_total}},
             "phases_ms": {k: round(v, 4) for k, v in phases.items()},
             "plain_gpu": {"value": round(plain_rate, 2), "unit": METRIC,
                           "what": "one ncpa_ess_solve + TL per frequency, same workload"},
@@ -694,7 +693,7 @@ def wmod_leg(ctx, stream, prof, freqs, az, fp64_peak, flush, cpu_seconds, k=5):
     steps, dsteps = ctx.bisect_steps()
     phases = {ph: round(ctx.phase_stats(ph)[0] / n_ph, 4) for ph in
               ("knots+grid", "matrix", "window", "scan", "host-items", "bisect", "eigvec", "fetch")}
-    flops = 6.0 * (steps - dsteps) + 12.0 * dsteps
+    flops = 1.0 * (steps - dsteps) + 1.9 * dsteps  # as in the ESS roofline; Newton: first derivatives only
     achieved = flops / (bis_ms / 1e3) / 1e12 if bis_ms > 0 else None
     # CPU: the oracle's WMod restatement on a stratified sample
     O, pp, prm = _oracle_setup()
@@ -712,11 +711,11 @@ def wmod_leg(ctx, stream, prof, freqs, az, fp64_peak, flush, cpu_seconds, k=5):
                     "1-D TL at %d ranges x %g km, analytic 0-150 km profile" % (NZ, N_TL, DR_TL / 1e3),
         "modes_total": modes, "ms_per_step": round(ms, 4), "value": round(NFREQ / (ms / 1e3), 2), "unit": METRIC,
         "phases_ms": phases,
-        "roofline": {"kernel": "k_bisect<WmodRows> (Sturm multisection in kappa)", "bound": "fp64",
+        "roofline": {"kernel": "k_panel_modes (eigenvalues in kappa, wide-angle rows)", "bound": "fp64",
                      "achieved": round(achieved, 3) if achieved else None,
                      "peak": round(fp64_peak, 3) if fp64_peak else None, "unit": "TFLOP/s",
                      "frac": round(achieved / fp64_peak, 4) if achieved and fp64_peak else None,
-                     "flops": "6 per count-chain step (3 FMA), 12 per Newton-chain step (with the derivative)",
+                     "flops": "1.0 per count-chain row step, 1.9 per Newton-chain row step (blocks of 128 rows)",
                      "avg_launch_ms": round(bis_ms / max(bis_n, 1), 4)},
         "cpu_baseline": {"value": round(done / el, 3), "unit": METRIC, "cores": O.lib().orc_num_threads(),
                          "kind": "port",
