@@ -59,7 +59,17 @@ struct WorkItem {
 constexpr int kPD = 14, kPW = 11;
 constexpr int kRecT = 4 * (kPD + 1) + 2, kRecW = 4 * (kPW + 1);
 constexpr int kPanelChunk = 4;
-constexpr int kPanelMaxBlk = 128, kPanelMinBlk = 8;
+constexpr int kPanelMaxBlk = 128;
+// The shortest blocks; a panel that asks for shorter ones sweeps the rows as they
+// are.  Blocks of 16 rows cost twice the instructions of the rows, in a quarter
+// of the chain: worth it on long grids, whose solves wait for chains more than
+// for the FP64 pipe (4 Hz, 20000 rows alone 2.15 -> 1.85 ms; 36 azimuths of 2 Hz,
+// 8000 rows, wide 8.8 -> 5.8), not on short ones (90 azimuths of 1 Hz, 2500 rows
+// 1.5 -> 2.0).  Blocks of 8 cost four times the rows and were used before (2.4).
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr int panel_min_blk(int nz) { return nz >= 4096 ? 16 : 32; }
 constexpr double kRhoMax = 10.0;
 
 struct PanelDesc {
@@ -157,13 +167,13 @@ int launch_panel_scan(cudaStream_t st, bool wide, int P, int nz_max, ProblemInfo
                       int slots, unsigned* done, unsigned* err);
 // c_lo, c_hi, M and off of every problem, the work items (at most bis_item
 // eigenvalues, their panel in WorkItem::pad or -1) and the panels; tot =
-// {items, items, modes}; kErrTooMany above max_modes or cap
+// {items, items, modes, items without a panel}; kErrTooMany above
+// max_modes or cap
 int launch_panel_items(cudaStream_t st, bool wide, int P, ProblemInfo* pinfo, const int* counts, int max_modes, int bis_item,
                        WorkItem* items, int cap, PanelDesc* desc, int* tot, unsigned* err, int order);
 // expansions of the work items' panels
 int launch_panel_expand(cudaStream_t st, bool wide, int n_desc, int nz_max, const ProblemInfo* pinfo, const PanelDesc* desc,
                         const double* s, const double* w, const double* g, double* T, double* W0, double* W1);
-constexpr int kPanelSlots = 4;  // two pairs of warps, two directions each
 constexpr int kCkVals = 4;  // doubles of a coarse row's checkpoint, at most
 // full vectors: the state of a chain before a coarse row, times 2^E
 struct VecState {
@@ -190,7 +200,7 @@ struct ModesArgs {
     double tol;
     double* mu;
     double *kr, *ki, *vs, *vr, *vg;
-    double* ck_u;  // per CTA: kPanelSlots x kCkVals ck_stride doubles, kPanelSlots x ck_stride ints
+    double* ck_u;  // panel_ck_slots x kCkVals ck_stride doubles and x ck_stride ints
     int* ck_e;
     long long ck_stride;
     // full vectors (null: none): per problem at vstate_off the upward states
@@ -201,7 +211,7 @@ struct ModesArgs {
     unsigned long long* vpeak;  // zeroed
     double* vfull;              // [row][mode] per problem at vfull_off
     const long long* vfull_off;
-    int* sched;  // two item counters (zeroed) or null: round-robin
+    int* sched;  // six item counters (zeroed) or null: round-robin
     int num_sms;
     int min_items, max_items;  // (set by the launcher) a launch returns for other item counts
     unsigned* err;
@@ -213,6 +223,11 @@ int launch_panel_modes(cudaStream_t st, bool wide, int grid, const ModesArgs& a,
 // left; m_max: the most modes of a problem
 int launch_panel_fill(cudaStream_t st, bool wide, int P, int nz_max, int m_max, const ModesArgs& a);
 int panel_ctas_per_sm();
+// the items without panels, which launch_panel_modes leaves out: the same grid and
+// arguments, on any stream
+int launch_rows_modes(cudaStream_t st, bool wide, int grid, const ModesArgs& a, int what);
+// checkpoint slots of both on that many CTAs
+int panel_ck_slots(int grid, bool rows);
 
 // 1-D TL; m_max: at least the most modes of a problem; scratch of tl1d_scratch
 // bytes (0: none)

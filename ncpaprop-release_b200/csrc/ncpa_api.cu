@@ -108,6 +108,8 @@ void upload(DevBuf& d, const T* h, size_t n, cudaStream_t st) {
 struct ncpa_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
+    cudaStream_t side = nullptr;   // work items by rows, beside the others: forked from stream and joined again
+    cudaEvent_t forked = nullptr, joined = nullptr;
     std::string err;
     long long launches = 0;
     int num_sms = 148;
@@ -209,6 +211,7 @@ struct ncpa_modes {
     std::vector<ProblemInfo> info;
     long long n_blocks = 0;  // block records of the panel expansions
     int n_desc = 0;          // panels of the work items
+    bool rows = false;       // some may have none
     int Mtot = 0;
     DevBuf d_pinfo, d_kr, d_ki, d_vs, d_vr, d_vg, d_vfull, d_vfull_off;
     mutable DevBuf tl_re, tl_im, tl_inc;  // 1-D TL kept in HBM
@@ -543,7 +546,7 @@ void prepare_solve(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, int
     b.items.alloc((size_t)b.item_cap * sizeof(WorkItem), st);
     b.tot.alloc(4 * sizeof(int), st);
     b.mu.alloc(mcap * 8, st);
-    b.sched.alloc(4 * sizeof(int), st);
+    b.sched.alloc(8 * sizeof(int), st);
     const size_t nT = (size_t)M->n_blocks * ncpa::kRecT, nW = (size_t)M->n_blocks * ncpa::kRecW;
     DevBuf& ex = b.own_ck ? b.ex : ctx->ex;
     const bool two = prm->want_group_speed || prm->method == NCPA_METHOD_WMOD;  // weights of the expansions
@@ -558,7 +561,7 @@ void prepare_solve(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, int
     M->d_vs.alloc(mcap * 8, st);
     M->d_vr.alloc(mcap * 8, st);
     M->d_vg.alloc(mcap * 8, st);
-    const size_t need = (size_t)modes_grid(ctx, 0) * ncpa::kPanelSlots * ncpa::coarse_slot_elems(M->nz_max);
+    const size_t need = (size_t)ncpa::panel_ck_slots(modes_grid(ctx, 0), M->rows) * ncpa::coarse_slot_elems(M->nz_max);
     DevBuf& c1 = b.own_ck ? b.ck1 : ctx->ck1;
     DevBuf& ce = b.own_ck ? b.cke : ctx->cke;
     c1.alloc(need * ncpa::kCkVals * 8, st);
@@ -641,9 +644,9 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
     tm.mark("window");
     // ---- isolation scan ----
     // item counters of the launches below and the scan's block counter
-    CK(cudaMemsetAsync(b.sched.p, 0, 4 * sizeof(int), st));
+    CK(cudaMemsetAsync(b.sched.p, 0, 8 * sizeof(int), st));
     check_launch(ctx, ncpa::launch_panel_scan(st, wide, P, M->nz_max, d_pinfo, s, b.T, b.counts.as<int>(),
-                                              scan_slots(ctx), b.sched.as<unsigned>() + 2, err));
+                                              scan_slots(ctx), b.sched.as<unsigned>() + 7, err));
     tm.mark("scan");
     // one launch for eigenvalues and mode values, unless per-phase timing or
     // step counts ask for the two apart
@@ -692,16 +695,29 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
         a.vfull = M->d_vfull.as<double>();
         a.vfull_off = M->d_vfull_off.as<long long>();
     }
+    auto modes = [&](int what) {
+        const int grid = modes_grid(ctx, t.bis_ctas);
+        int n = 0;
+        if (M->rows) {
+            CK(cudaEventRecord(ctx->forked, st));
+            CK(cudaStreamWaitEvent(ctx->side, ctx->forked, 0));
+            n = ncpa::launch_rows_modes(ctx->side, wide, grid, a, what);
+            CK(cudaEventRecord(ctx->joined, ctx->side));
+        }
+        n += ncpa::launch_panel_modes(st, wide, grid, a, what);
+        if (M->rows) CK(cudaStreamWaitEvent(st, ctx->joined, 0));
+        check_launch(ctx, n);
+    };
     if (fuse) {
-        check_launch(ctx, ncpa::launch_panel_modes(st, wide, modes_grid(ctx, t.bis_ctas), a, 3));
+        modes(3);
         tm.mark("bisect+eigvec");
     } else {
         a.steps = count_steps ? ctx->d_stats.as<unsigned long long>() : nullptr;
-        check_launch(ctx, ncpa::launch_panel_modes(st, wide, modes_grid(ctx, t.bis_ctas), a, 1));
+        modes(1);
         tm.mark("bisect");
         a.steps = nullptr;
         if (a.sched) ++a.sched;
-        check_launch(ctx, ncpa::launch_panel_modes(st, wide, modes_grid(ctx, t.bis_ctas), a, 2));
+        modes(2);
         tm.mark("eigvec");
     }
     if (prm->want_vectors) {
@@ -822,9 +838,10 @@ std::pair<double, double> ceff_bounds(const ncpa_profile* prof, double az_deg) {
 void layout_panels(ncpa_modes* M, const std::vector<Group>& groups, const ncpa_ess_params* prm, double slack) {
     M->n_blocks = 0;
     M->n_desc = 0;
+    M->rows = false;
     const double rho = ncpa::kRhoMax, B = ncpa::kPanelMaxBlk;
     const double n_s = ncpa::kScanMax / ncpa::kScanStep;  // scan panels
-    std::map<std::pair<const ncpa_profile*, double>, std::pair<double, double>> seen;
+    std::map<std::pair<const ncpa_profile*, int>, std::pair<double, double>> seen;
     for (const Group& g : groups)
         for (int a = 0; a < g.n_az; ++a) {
             double c_lo, c_hi;
@@ -847,6 +864,8 @@ void layout_panels(ncpa_modes* M, const std::vector<Group>& groups, const ncpa_e
                 // half the window times the steepness of sigma (1, or 3 kappa_max)
                 const double win = prm->method == NCPA_METHOD_WMOD ? 3.0 / c_lo * (1.0 / c_lo - 1.0 / c_hi) : dk;
                 const double R = std::min(1.05 * slack * 0.5 * kh * kh * win, 8.0);
+                const double b = ncpa::panel_min_blk(pi.nz);
+                if (R * b * b > rho) M->rows = true;
                 // items of 16 modes, the smallest a plan tries
                 const double n_it = std::min((2.0 * pi.freq * pi.dz * nz * std::sqrt(dk * slack) + 32.0) / 16.0, 4096.0);
                 const double n = std::max(n_it, n_s);
@@ -1185,6 +1204,9 @@ ncpa_status ncpa_ctx_create(ncpa_ctx** out, const ncpa_ctx_opts* opts) {
         if (prop.major < 10) throw ApiError(NCPA_ENODEV, "this library is built for sm_100a (B200)");
         ctx->num_sms = prop.multiProcessorCount;
         CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
+        CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&ctx->forked, cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&ctx->joined, cudaEventDisableTiming));
         // keep freed blocks of the stream-ordered allocator cached in the pool
         cudaMemPool_t pool;
         CK(cudaDeviceGetDefaultMemPool(&pool, ctx->device));
@@ -1236,6 +1258,9 @@ ncpa_status ncpa_ctx_destroy(ncpa_ctx* ctx) {
     if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
     if (ctx->h_tot) cudaFreeHost(ctx->h_tot);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
+    if (ctx->side) cudaStreamDestroy(ctx->side);
+    if (ctx->forked) cudaEventDestroy(ctx->forked);
+    if (ctx->joined) cudaEventDestroy(ctx->joined);
     delete ctx;
     return NCPA_OK;
 }

@@ -64,6 +64,8 @@ constexpr int kWD = kPanelChunk * kRecW;  // doubles of a chunk of one weight's 
 constexpr int kPBuf = 3;                  // ring slots per warp
 constexpr int kPWarps = 4;                // warps per CTA (two pairs)
 constexpr int kPanelCtas = 3;             // CTAs per SM
+constexpr int kSoloMin = 6;               // items by rows per SM from which on each has a warp
+constexpr int kRowsCtas = 4;              // CTAs per SM then
 constexpr int kRecZeros = 4 * (kPD + 1), kRecMid = kRecZeros + 1;
 static_assert(kRecT == kRecMid + 1 && kRecT % 2 == 0, "T record: coefficients, zero count, split, 16-byte size");
 static_assert(kRecW == 4 * (kPW + 1), "W record: coefficients");
@@ -73,7 +75,7 @@ struct Panel {
     const double* rows;  // raw rows of the problem
     long long rec;       // first block record
     int nblk, blk, nz;   // blk = 0: no records, the sweeps run on the raw rows
-    double e0;
+    double e0, um0;  // e_{-1} and u_{-2}
 };
 
 // the coefficients of -sigma in t: s0 + s1 t + s2 t^2
@@ -98,9 +100,19 @@ struct EssPanel {
     __device__ static __forceinline__ double sigma(const double* __restrict__ row, int i, double x) {
         return (__ldg(row + i) - x) + 2.0;
     }
-    // -d sigma / dx
-    __device__ static __forceinline__ double slope(const double* __restrict__, int, double) { return 1.0; }
-    __device__ static __forceinline__ double e_init(const ProblemInfo&) { return 1.0; }  // p_{-2} = 0
+    __device__ static __forceinline__ double um_init(const ProblemInfo&) { return 0.0; }  // p_{-2} = 0
+    // a row (staged in shared memory) at a shift: 2 - sigma, and d / dx of it over kSlope
+    struct At {
+        double x;
+        __device__ __forceinline__ At() {}
+        __device__ __forceinline__ explicit At(double x_) : x(x_) {}
+        __device__ __forceinline__ double turn(const double* __restrict__ r) const { return x - r[0]; }
+        __device__ __forceinline__ double turn(const double* __restrict__ r, double& slope) const {
+            slope = 1.0;
+            return x - r[0];
+        }
+    };
+    static constexpr double kSlope = 1.0;
     __device__ static __forceinline__ double lo(const ProblemInfo& pi) { return pi.lo; }
     __device__ static __forceinline__ double hi(const ProblemInfo& pi) { return pi.hi; }
     __device__ static __forceinline__ double tol_scale(const ProblemInfo&) { return 1.0; }
@@ -152,11 +164,29 @@ struct WmodPanel {
         const double d = fma(-q.y, x, q.x);
         return fma(d, d, fma(-x, x, -2.0)) + 2.0;
     }
+    // -d sigma / dx
     __device__ static __forceinline__ double slope(const double* __restrict__ row, int i, double x) {
         const double2 q = row_at(row, i);
         return 2.0 * fma(q.y, fma(-q.y, x, q.x), x);
     }
-    __device__ static __forceinline__ double e_init(const ProblemInfo& pi) { return 1.0 - pi.g0; }
+    __device__ static __forceinline__ double um_init(const ProblemInfo& pi) { return pi.g0; }
+    struct At {
+        double x, c;
+        __device__ __forceinline__ At() {}
+        __device__ __forceinline__ explicit At(double x_) : x(x_), c(fma(-x_, x_, -2.0)) {}
+        __device__ __forceinline__ double turn(const double* __restrict__ r) const {
+            const double2 q = *reinterpret_cast<const double2*>(r);
+            const double d = fma(-q.y, x, q.x);
+            return -fma(d, d, c);
+        }
+        __device__ __forceinline__ double turn(const double* __restrict__ r, double& slope) const {
+            const double2 q = *reinterpret_cast<const double2*>(r);
+            const double d = fma(-q.y, x, q.x);
+            slope = fma(q.y, d, x);
+            return -fma(d, d, c);
+        }
+    };
+    static constexpr double kSlope = 2.0;
     __device__ static __forceinline__ double lo(const ProblemInfo& pi) { return pi.k_min * pi.dz; }
     __device__ static __forceinline__ double hi(const ProblemInfo& pi) { return pi.k_max * pi.dz; }
     __device__ static __forceinline__ double tol_scale(const ProblemInfo& pi) { return pi.k_max * pi.dz; }
@@ -195,16 +225,17 @@ __device__ __forceinline__ Panel panel_of(const ProblemInfo& pi, const PanelDesc
     P.nz = pi.nz;
     P.nblk = d.blk ? (pi.nz + d.blk - 1) / d.blk : 0;
     P.rec = d.rec;
-    P.e0 = Row::e_init(pi);
+    P.um0 = Row::um_init(pi);
+    P.e0 = 1.0 - P.um0;
     return P;
 }
 
 __device__ __forceinline__ int padded(int nblk) { return (nblk + kPanelChunk - 1) / kPanelChunk * kPanelChunk; }
 
 // rows per block for shifts within r of the centre: the most that keep r B^2
-// within kRhoMax (0: not even kPanelMinBlk)
-__device__ __forceinline__ int block_rows(double r) {
-    for (int B = kPanelMaxBlk; B >= kPanelMinBlk; B >>= 1)
+// within kRhoMax (0: not even panel_min_blk, the rows as they are)
+__device__ __forceinline__ int block_rows(double r, int nz) {
+    for (int B = kPanelMaxBlk; B >= panel_min_blk(nz); B >>= 1)
         if (r * (double)B * (double)B <= kRhoMax) return B;
     return 0;
 }
@@ -240,7 +271,7 @@ __device__ void plan_scan_panels(ProblemInfo& pi, int n) {
     }
     if (!B) {
         upp = 1;
-        B = block_rows(st * (0.5 * d * (double)(kScanStep - 1)));
+        B = block_rows(st * (0.5 * d * (double)(kScanStep - 1)), pi.nz);
     }
     const long long need = B ? (long long)((units + upp - 1) / upp) * padded((pi.nz + B - 1) / B) : 0;
     const bool fits = B != 0 && need <= pi.blk_cap;
@@ -471,71 +502,138 @@ __device__ __forceinline__ void horner_blocks(const double* __restrict__ c0, con
         }
 }
 
-// Sturm counts at NC shifts per lane
-template <class Row, int NC>
-__device__ __forceinline__ void count_sweep(const Panel& P, const double* __restrict__ Trec, const double (&x)[NC],
-                                            PRing& R, unsigned* err, int (&cnt)[NC]) {
-    double u[NC], e[NC];
-    typename Row::Shift sh[NC];
-    int zeros[NC];
+// ---------------------------------------------------------------------------
+// Rows as they are, where a panel has no records: the recurrence u_i = (2 -
+// sigma_i) u_{i-1} - u_{i-2}, upwards from the ground and, the same with the
+// indices reversed, downwards from the upper boundary (b), over half of the
+// rows each.  Two instructions a row and shift for a count, six with two
+// derivatives, five for a vector with one weight: what blocks of 32 rows cost
+// (see panel_min_blk).  The rows run through the warp's ring.
+// ---------------------------------------------------------------------------
+template <class Row>
+constexpr int kStage = 128 / Row::kW;  // rows of a chunk
+static_assert(128 <= kTD, "a slot holds a chunk of rows");
+constexpr int kRun = 16;  // rows between rescalings
+// (the sweeps are functions of their own, so that the code of the block sweeps
+// stays what it is; the ring's count comes back with their results)
+
+// Rows [i0, i1), downwards or up, in runs of at most kRun rows that start at
+// multiples of it: run(rows, x, lo, n) for the rows lo .. lo + n - 1, with x[k]
+// their values of the NX further arrays xs.
+template <class Row, int NX, bool kDown, class Run>
+__device__ __forceinline__ void rows_sweep(const Panel& P, int i0, int i1, PRing& R, unsigned* err,
+                                           const double* const* xs, Run run) {
+    constexpr int kS = kStage<Row>;
+    const int c0 = i0 / kS, nc = i1 > i0 ? (i1 + kS - 1) / kS - c0 : 0;
+    ring_stream(
+        R, nc, err,
+        [&](double* dst, uint64_t* bar, int o) {
+            const size_t c = kDown ? c0 + nc - 1 - o : c0 + o;
+            mbar_expect_tx(bar, (128 + NX * kS) * 8);
+            tma_load_1d(dst, P.rows + c * 128, 128 * 8, bar);
 #pragma unroll
-    for (int n = 0; n < NC; ++n) {
-        u[n] = 1.0;
-        e[n] = P.e0;
-        zeros[n] = 0;
-        sh[n] = typename Row::Shift(P, x[n]);
-    }
-    if (P.blk) {
-        const double* src = Trec + (size_t)P.rec * kRecT;
-        ring_stream(
-            R, (P.nblk + kPanelChunk - 1) / kPanelChunk, err,
-            [&](double* dst, uint64_t* bar, int c) {
-                mbar_expect_tx(bar, kTD * 8);
-                tma_load_1d(dst, src + (size_t)c * kTD, kTD * 8, bar);
-            },
-            [&](const double* rec, int c) {
-                const int nb = min(kPanelChunk, P.nblk - c * kPanelChunk);
-                for (int q = 0; q < nb; q += 2, rec += 2 * kRecT) {
-                    double p[2][NC][4], t[2][NC];
-#pragma unroll
-                    for (int n = 0; n < NC; ++n) {
-                        t[0][n] = sh[n].at(rec);
-                        t[1][n] = sh[n].at(rec + kRecT);
-                    }
-                    horner_blocks<NC>(rec, rec + kRecT, t, p);
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-                        if (q + b >= nb) break;
-                        const int n2 = __double2loint(rec[b * kRecT + kRecZeros]);
-#pragma unroll
-                        for (int n = 0; n < NC; ++n) {
-                            const double(&m)[4] = p[b][n];
-                            const double un = fma(m[0], u[n], m[1] * e[n]);
-                            e[n] = fma(m[2], u[n], m[3] * e[n]);
-                            zeros[n] += block_zeros(u[n], un, m[1], t[b][n], n2);
-                            u[n] = un;
-                        }
-                    }
-                }
-#pragma unroll
-                for (int n = 0; n < NC; ++n) scale2(u[n], e[n]);
-            });
-    } else {
-        // no records (a window so wide against the grid that blocks of 8 rows
-        // have no short expansion, or beyond the reserved records): row by row
-        for (int i = 0; i < P.nz; ++i) {
-#pragma unroll
-            for (int n = 0; n < NC; ++n) {
-                e[n] = fma(-Row::sigma(P.rows, i, x[n]), u[n], e[n]);
-                const double un = u[n] + e[n];
-                zeros[n] += static_cast<int>(neg(un) ^ neg(u[n]));
-                u[n] = un;
-                if ((i & 15) == 15) scale2(u[n], e[n]);
+            for (int k = 0; k < NX; ++k) tma_load_1d(dst + kTD + k * kWD, xs[k] + c * kS, kS * 8, bar);
+        },
+        [&](const double* buf, int o) {
+            const int first = (kDown ? c0 + nc - 1 - o : c0 + o) * kS;
+            for (int q = 0; q < kS / kRun; ++q) {
+                const int a = first + kRun * (kDown ? kS / kRun - 1 - q : q);
+                const int lo = max(a, i0), n = min(a + kRun, i1) - lo;
+                if (n > 0) run(buf + (lo - first) * Row::kW, buf + kTD + (lo - first), lo, n);
             }
+        });
+}
+// f(j) for the n rows of a run in order
+template <bool kDown, class F>
+__device__ __forceinline__ void run_rows(int n, F f) {
+    if (n == kRun) {
+#pragma unroll
+        for (int j = 0; j < kRun; ++j) f(kDown ? kRun - 1 - j : j);
+    } else {
+        for (int j = 0; j < n; ++j) f(kDown ? n - 1 - j : j);
+    }
+}
+
+// sign changes over the last m rows: their signs in the low bits, the one before
+// them above
+__device__ __forceinline__ int run_zeros(unsigned bits, int m) {
+    return __popc((bits ^ (bits >> 1)) & ((1u << m) - 1u));
+}
+
+// Counts of NC shifts per lane by rows: the sign changes z of a chain over rows
+// [0, h) upwards, with v = u_h and w = u_{h-1}, or over rows (h, nz) downwards,
+// with v = b_h and w = b_{h-1}.
+template <int NC>
+struct RowCounts {
+    static constexpr int kSize = NC > 0 ? NC : 1;
+    double v[kSize], w[kSize];
+    int z[kSize];
+    unsigned loads;
+};
+template <class Row, int NC, bool kDown>
+struct CountRows {
+    static constexpr int kSize = NC > 0 ? NC : 1;
+    double u[kSize], um[kSize];
+    unsigned bits[kSize];
+    int z[kSize];
+    typename Row::At at[kSize];
+    __device__ __forceinline__ CountRows(const Panel& P, double x0, double x1) {
+#pragma unroll
+        for (int n = 0; n < NC; ++n) {
+            u[n] = 1.0;
+            um[n] = kDown ? 0.0 : P.um0;
+            z[n] = 0;
+            bits[n] = 0u;
+            at[n] = typename Row::At(n ? x1 : x0);
         }
     }
+    __device__ __forceinline__ void row(const double* r) {
 #pragma unroll
-    for (int n = 0; n < NC; ++n) cnt[n] = P.nz - zeros[n];
+        for (int n = 0; n < NC; ++n) {
+            const double un = fma(at[n].turn(r), u[n], -um[n]);
+            um[n] = u[n];
+            u[n] = un;
+            bits[n] = __funnelshift_l(__double2hiint(un), bits[n], 1);
+        }
+    }
+    __device__ __forceinline__ void fold(int m) {
+#pragma unroll
+        for (int n = 0; n < NC; ++n) {
+            z[n] += run_zeros(bits[n], m);
+            scale2(u[n], um[n]);
+        }
+    }
+    __device__ __forceinline__ void end(RowCounts<NC>& out) const {
+#pragma unroll
+        for (int n = 0; n < NC; ++n) {
+            out.v[n] = kDown ? um[n] : u[n];
+            out.w[n] = kDown ? u[n] : um[n];
+            // row h is the joint's
+            out.z[n] = z[n] - (kDown ? 0 : static_cast<int>(neg(u[n]) ^ neg(um[n])));
+        }
+    }
+};
+template <class Row, int NC, bool kDown>
+__device__ __noinline__ RowCounts<NC> rows_count(const Panel P, double x0, double x1, int h, PRing R, unsigned* err) {
+    CountRows<Row, NC, kDown> C(P, x0, x1);
+    rows_sweep<Row, 0, kDown>(P, kDown ? h + 1 : 0, kDown ? P.nz : h + 1, R, err, nullptr,
+                              [&](const double* r, const double*, int, int m) {
+                                  run_rows<kDown>(m, [&](int j) { C.row(r + j * Row::kW); });
+                                  C.fold(m);
+                              });
+    RowCounts<NC> out;
+    C.end(out);
+    out.loads = R.loads;
+    return out;
+}
+
+// the count from both ends' chains at row h (values v at h and w at h - 1,
+// sign changes z): those of u over all rows are z + z' and one more or none at
+// the joint (the inertia of the twisted factorisation), by the sign of u_{nz-1}
+// = w b_h - ... , the chains' Wronskian
+__device__ __forceinline__ int rows_join(int nz, double u, double um, int zu, double b, double bm, int zb) {
+    const int z = zu + zb;
+    return nz - z - static_cast<int>(neg(u * bm - um * b) ^ static_cast<unsigned>(z & 1));
 }
 
 // ---------------------------------------------------------------------------
@@ -648,34 +746,137 @@ __device__ __forceinline__ void lag_segment(const Panel& P, const double* __rest
         });
 }
 
-// the raw rows' two halves
-template <class Row>
-__device__ __forceinline__ void lag_raw(const Panel& P, double x, int half, LagChain& C) {
-    const int h = P.nz / 2, n = half ? P.nz - h : h;
-    for (int j = 0; j < n; ++j) {
-        const int i = half ? P.nz - 1 - j : j;
-        const double sg = Row::sigma(P.rows, i, x), sl = Row::slope(P.rows, i, x);
-        if (half) {
-            C.u -= C.e;
-            C.u1 -= C.e1;
-            if (Row::kLaguerre) {
-                C.u2 -= C.e2;
-                C.e2 = fma(sg, C.u2, fma(-sl, C.u1, C.e2));
-            }
-            C.e1 = fma(sg, C.u1, fma(-sl, C.u, C.e1));
-            C.e = fma(sg, C.u, C.e);
-        } else {
-            if (Row::kLaguerre) {
-                C.e2 = fma(-sg, C.u2, fma(sl, C.u1, C.e2));
-                C.u2 += C.e2;
-            }
-            C.e1 = fma(-sg, C.u1, fma(sl, C.u, C.e1));
-            C.e = fma(-sg, C.u, C.e);
-            C.u += C.e;
-            C.u1 += C.e1;
-        }
-        if ((j & 15) == 15) C.rescale();
+// The same by rows, up over [0, nz / 2) or down over the others, with the sign
+// changes z as of rows_count (their joint is row nz / 2 - 1).
+struct RowLag {
+    LagChain C;
+    int z;
+    unsigned loads;
+};
+template <class Row, bool kDown>
+struct LagRows {
+    LagChain U;  // e: the value before
+    unsigned bits = 0u;
+    int z = 0;
+    typename Row::At at;
+    __device__ __forceinline__ LagRows(const Panel& P, double x)
+        : U{1.0, kDown ? 0.0 : P.um0, 0.0, 0.0, 0.0, 0.0}, at(x) {}
+    __device__ __forceinline__ void row(const double* r) {
+        double sl;
+        const double q = at.turn(r, sl);
+        double u2 = 0.0;
+        if (Row::kLaguerre) u2 = fma(q, U.u2, U.u1 - U.e2);
+        const double u1 = Row::kLaguerre ? fma(q, U.u1, U.u - U.e1) : fma(q, U.u1, fma(sl, U.u, -U.e1));
+        const double u = fma(q, U.u, -U.e);
+        bits = __funnelshift_l(__double2hiint(u), bits, 1);
+        U = LagChain{u, U.u, u1, U.u1, u2, U.u2};
     }
+    __device__ __forceinline__ void fold(int m) {
+        z += run_zeros(bits, m);
+        U.rescale();
+    }
+    // the state before row nz / 2; the derivative was taken over kSlope
+    __device__ __forceinline__ void end(RowLag& out) const {
+        constexpr double k = Row::kSlope;
+        out.z = z - (kDown ? 0 : static_cast<int>(neg(U.u) ^ neg(U.e)));
+        if (kDown) out.C = {U.e, U.e - U.u, k * U.e1, k * (U.e1 - U.u1), U.e2, U.e2 - U.u2};
+        else out.C = {U.u, U.u - U.e, k * U.u1, k * (U.u1 - U.e1), U.u2, U.u2 - U.e2};
+    }
+};
+template <class Row, bool kDown>
+__device__ __noinline__ RowLag rows_lag(const Panel P, double x, PRing R, unsigned* err) {
+    LagRows<Row, kDown> C(P, x);
+    const int h = P.nz / 2;
+    rows_sweep<Row, 0, kDown>(P, kDown ? h : 0, kDown ? P.nz : h, R, err, nullptr,
+                              [&](const double* r, const double*, int, int m) {
+                                  run_rows<kDown>(m, [&](int j) { C.row(r + j * Row::kW); });
+                                  C.fold(m);
+                              });
+    RowLag out;
+    C.end(out);
+    out.loads = R.loads;
+    return out;
+}
+
+// Both directions in one warp, row by row in turn, so that it has twice the
+// chains in flight: the Laguerre chains of xa (kLag) and the counts of NC shifts.
+template <int NC>
+struct RowBoth {
+    RowLag L[2];
+    RowCounts<NC> K[2];
+    unsigned loads;
+};
+template <class Row, bool kLag, int NC>
+__device__ __noinline__ RowBoth<NC> rows_both(const Panel P, double xa, double x0, double x1, PRing R, unsigned* err) {
+    constexpr int kS = kStage<Row>, kW = Row::kW;
+    static_assert(kTD + 128 <= kTD + kWD, "a slot with one weight holds two chunks of rows");
+    LagRows<Row, false> lu(P, xa);
+    LagRows<Row, true> ld(P, xa);
+    CountRows<Row, NC, false> cu(P, x0, x1);
+    CountRows<Row, NC, true> cd(P, x0, x1);
+    // the counts' joint is row h, the Laguerre chains meet before it: row h is taken
+    // by the upward counts and by the downward Laguerre chain apart
+    const int h = P.nz / 2, top = (P.nz - 1) / kS;
+    const int nf = h / kS + 1, nb = top - h / kS + 1;  // chunks with rows [0, h], [h, nz)
+    auto up = [&](const double* r, bool last) {
+        if (kLag && !last) lu.row(r);
+        cu.row(r);
+    };
+    auto dn = [&](const double* r, bool last) {
+        if (kLag) ld.row(r);
+        if (!last) cd.row(r);
+    };
+    auto fold_up = [&](int m, int ml) {
+        if (kLag && ml) lu.fold(ml);
+        cu.fold(m);
+    };
+    auto fold_dn = [&](int m, int mc) {
+        if (kLag) ld.fold(m);
+        if (mc) cd.fold(mc);
+    };
+    ring_stream(
+        R, max(nf, nb), err,
+        [&](double* dst, uint64_t* bar, int o) {
+            mbar_expect_tx(bar, ((o < nf) + (o < nb)) * 128 * 8);
+            if (o < nf) tma_load_1d(dst, P.rows + (size_t)o * 128, 128 * 8, bar);
+            if (o < nb) tma_load_1d(dst + kTD, P.rows + (size_t)(top - o) * 128, 128 * 8, bar);
+        },
+        [&](const double* buf, int o) {
+            int f = o * kS, b = o < nb ? min(P.nz, (top - o + 1) * kS) : 0;  // next row up; behind the next one down
+            const int f1 = o < nf ? min(h + 1, f + kS) : f, b0 = o < nb ? max(h, (top - o) * kS) : b;
+            const double *rf = buf - f * kW, *rb = buf + kTD - (top - o) * kS * kW;
+            while (f < f1 || b > b0) {
+                const int m = min(kRun, f1 - f), n = b - max(b0, (b - 1) / kRun * kRun);
+                if (m == kRun && n == kRun && f + kRun <= h && b - kRun > h) {
+                    const double *p = rf + f * kW, *q = rb + (b - kRun) * kW;
+#pragma unroll
+                    for (int j = 0; j < kRun; ++j) {
+                        up(p + j * kW, false);
+                        dn(q + (kRun - 1 - j) * kW, false);
+                    }
+                    fold_up(kRun, kRun);
+                    fold_dn(kRun, kRun);
+                } else {
+                    if (m > 0) {
+                        for (int j = 0; j < m; ++j) up(rf + (f + j) * kW, f + j == h);
+                        fold_up(m, m - (f + m > h));
+                    }
+                    if (n > 0) {
+                        for (int j = 0; j < n; ++j) dn(rb + (b - 1 - j) * kW, b - 1 - j == h);
+                        fold_dn(n, n - (b - n == h));
+                    }
+                }
+                f += max(m, 0);
+                b -= max(n, 0);
+            }
+        });
+    RowBoth<NC> out;
+    lu.end(out.L[0]);
+    ld.end(out.L[1]);
+    cu.end(out.K[0]);
+    cd.end(out.K[1]);
+    out.loads = R.loads;
+    return out;
 }
 
 // The transfer matrix of the chunks [c0, c1) at NC shifts per lane (its two
@@ -765,15 +966,28 @@ __global__ void __launch_bounds__(kPWarps * 32) k_panel_scan(const ProblemInfo* 
     const double lo = Row::lo(pi), hi = Row::hi(pi);
     const double x[2] = {scan_x(lo, hi, t0, n), scan_x(lo, hi, t0 + 1, n)};
     int c[2];
-    if (!P.blk) {  // raw rows: one chain, on the first warp
+    struct Seg {
+        double m[4][2][32];
+        int z[2][32];
+    };
+    Seg* box = reinterpret_cast<Seg*>(smem_raw + kRingBytes<kTD>);
+    if (!P.blk) {  // by rows: a warp takes one of the two shifts over half of them
+        const int h = P.nz / 2, k = wid >> 1;
+        const double xk = k ? x[1] : x[0];
+        const auto o = wid & 1 ? rows_count<Row, 1, true>(P, xk, 0.0, h, R, err)
+                               : rows_count<Row, 1, false>(P, xk, 0.0, h, R, err);
+        box[wid].m[0][0][lane] = o.v[0];
+        box[wid].m[1][0][lane] = o.w[0];
+        box[wid].z[0][lane] = o.z[0];
+        __syncthreads();
         if (wid) return;
-        count_sweep<Row, 2>(P, T, x, R, err, c);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const Seg &U = box[2 * k], &B = box[2 * k + 1];
+            c[k] = rows_join(P.nz, U.m[0][0][lane], U.m[1][0][lane], U.z[0][lane], B.m[0][0][lane], B.m[1][0][lane],
+                             B.z[0][lane]);
+        }
     } else {
-        struct Seg {
-            double m[4][2][32];
-            int z[2][32];
-        };
-        Seg* box = reinterpret_cast<Seg*>(smem_raw + kRingBytes<kTD>);
         const int nch = (P.nblk + kPanelChunk - 1) / kPanelChunk;
         double u[2], e[2], v[2], f[2];
         int z[2];
@@ -903,6 +1117,7 @@ __global__ void __launch_bounds__(kItemThreads) k_panel_items(int P, ProblemInfo
         tot[0] = min(base, cap);
         tot[1] = min(base, cap);
         tot[2] = base_m;
+        tot[3] = 0;
     }
 }
 
@@ -929,7 +1144,8 @@ template <class Row>
 __global__ void __launch_bounds__(kPlanWarps * 32) k_panel_groups(int P, const ProblemInfo* __restrict__ pinfo,
                                                                   const int* __restrict__ counts, int bis_item,
                                                                   WorkItem* __restrict__ items, int cap,
-                                                                  PanelDesc* __restrict__ desc) {
+                                                                  PanelDesc* __restrict__ desc,
+                                                                  int* __restrict__ tot) {
     __shared__ double xa[kPlanWarps][kPlanItems], xb[kPlanWarps][kPlanItems];
     __shared__ int grp[kPlanWarps][kPlanItems];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -964,7 +1180,7 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_panel_groups(int P, const P
                 PanelDesc d;
                 d.xc = 0.5 * (a + b);
                 d.r = fmax(0.5 * (b - a), 1e-300);
-                d.blk = block_rows(st * d.r);
+                d.blk = block_rows(st * d.r, pi.nz);
                 d.problem = p;
                 d.rec = pi.blk_off + used;
                 const int need = d.blk ? padded((pi.nz + d.blk - 1) / d.blk) : 0;
@@ -982,6 +1198,7 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_panel_groups(int P, const P
             const int k = k0 + i, q = pi.item0 + k;
             const int j0 = (int)((long long)M * k / nb), j1 = (int)((long long)M * (k + 1) / nb);
             if (q < cap) items[q] = WorkItem{p, j0, j1 - j0, grp[wid][i]};
+            if (grp[wid][i] < 0) atomicAdd(&tot[3], 1);  // sweeps its rows
         }
         __syncwarp();
         ng = __shfl_sync(0xffffffffu, ng, 0);
@@ -1018,17 +1235,25 @@ struct Team {
     int id, half;
     int turn;  // buffer of the next exchange
     __device__ __forceinline__ void sync() const {
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + id), "n"(32 * W) : "memory");
+        if (W == 1) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(1 + id), "n"(32 * W) : "memory");
     }
     // the first two warps
     __device__ __forceinline__ void sync2() const {
-        if (W == 2) sync();
+        if (W <= 2) sync();
         else asm volatile("bar.sync 8, 64;" ::: "memory");
     }
     // where segment s puts its results (n doubles a segment of the first kind a warp takes)
     __device__ __forceinline__ double* slot(int s, int n) const {
         if (W == 4) return area + s * stride;
         return area + (s >> 1) * stride + ((s == 1 || s == 2) ? n : 0);
+    }
+    // and set s of 32 shifts by rows, upwards or down
+    __device__ __forceinline__ double* rows(int s, bool down) const {
+        constexpr int kR = 7 * 32;
+        if (W == 4) return area + (2 * s + down) * stride;
+        if (W == 2) return area + down * stride + s * kR;
+        return area + (2 * s + down) * kR;
     }
 };
 
@@ -1050,13 +1275,112 @@ __device__ __forceinline__ int nth_set(unsigned m, int n) {
     return pos;
 }
 
+// A round by rows: the Laguerre chains of the first nN of 32 shifts (xe) and the
+// counts of the others and of 32 more (xs), or the counts of 64.  The chains stay
+// in pr.rows(0, .), the counts of lane v go to c[v >> 5][v & 31].
+template <class Row, int W>
+__device__ __forceinline__ void rows_round(const Panel& P, const double (&xs)[2], double xe, int nN, int nB, PRing& R,
+                                           unsigned* err, Team<W>& pr, int (&c)[2][32]) {
+    const int lane = threadIdx.x & 31, h = P.nz / 2;
+    const double xa = lane < nN || nB == 0 ? xe : xs[0];
+    constexpr int kNC = W == 4 ? 1 : 2, kDirs = W == 1 ? 2 : 1;
+    const bool down = W != 1 && (pr.half & 1);
+    const int s0 = W == 4 ? pr.half >> 1 : 0;                        // first set of this warp
+    const bool lag = nN > 0 && s0 == 0;                              // has Laguerre chains
+    const bool count = nN == 0 || (nB > 0 && s0 + kNC == 2);        // has counts,
+    const int n0 = nN > 0 ? kNC - 1 : 0;                             // of its sets from this one on
+    // the ring is in use until this warp's last sweep: results go there afterwards
+    RowLag L[kDirs];
+    RowCounts<kNC> K[kDirs];
+    auto last = [&](const RowCounts<1>& r, int d) {
+        K[d].v[kNC - 1] = r.v[0];
+        K[d].w[kNC - 1] = r.w[0];
+        K[d].z[kNC - 1] = r.z[0];
+    };
+    if constexpr (W == 1) {
+        if (nN == 0) {
+            const auto r = rows_both<Row, false, 2>(P, xa, xs[0], xs[1], R, err);
+            K[0] = r.K[0];
+            K[1] = r.K[1];
+            R.loads = r.loads;
+        } else {
+            auto keep = [&](const auto& r) {
+                L[0] = r.L[0];
+                L[1] = r.L[1];
+                R.loads = r.loads;
+            };
+            if (nB > 0) {
+                const auto r = rows_both<Row, true, 1>(P, xa, xs[1], 0.0, R, err);
+                keep(r);
+                last(r.K[0], 0);
+                last(r.K[1], 1);
+            } else {
+                keep(rows_both<Row, true, 0>(P, xa, 0.0, 0.0, R, err));
+            }
+        }
+    } else {
+        if (lag) {
+            L[0] = down ? rows_lag<Row, true>(P, xa, R, err) : rows_lag<Row, false>(P, xa, R, err);
+            R.loads = L[0].loads;
+        }
+        if (count && nN > 0) {
+            const RowCounts<1> r = down ? rows_count<Row, 1, true>(P, xs[1], 0.0, h, R, err)
+                                        : rows_count<Row, 1, false>(P, xs[1], 0.0, h, R, err);
+            last(r, 0);
+            R.loads = r.loads;
+        } else if (count) {
+            const double x0 = s0 ? xs[1] : xs[0];
+            K[0] = down ? rows_count<Row, kNC, true>(P, x0, xs[1], h, R, err)
+                        : rows_count<Row, kNC, false>(P, x0, xs[1], h, R, err);
+            R.loads = K[0].loads;
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int d = 0; d < kDirs; ++d) {
+        const bool dn = W == 1 ? d == 1 : down;
+        if (lag) {
+            double* o = pr.rows(0, dn) + lane;
+            o[0] = L[d].C.u;
+            o[32] = L[d].C.e;
+            o[64] = L[d].C.u1;
+            o[96] = L[d].C.e1;
+            o[128] = L[d].C.u2;
+            o[160] = L[d].C.e2;
+            o[192] = __hiloint2double(0, L[d].z);
+        }
+#pragma unroll
+        for (int n = 0; n < kNC; ++n) {
+            if (!count || n < n0) continue;
+            double* o = pr.rows(s0 + n, dn) + lane;
+            o[0] = K[d].v[n];
+            o[32] = K[d].w[n];
+            o[64] = __hiloint2double(0, K[d].z[n]);
+        }
+    }
+    if (nB == 0) return;
+    pr.sync();
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        if (W != 1 && pr.half != s) continue;
+        const double *a = pr.rows(s, false) + lane, *b = pr.rows(s, true) + lane;
+        if (s == 0 && nN > 0) {
+            const int z = __double2loint(a[192]) + __double2loint(b[192]);
+            const double w0 = a[0] * b[32] - a[32] * b[0];  // -u_{nz-1}
+            c[0][lane] = P.nz - z - static_cast<int>((neg(w0) ^ 1u) ^ static_cast<unsigned>(z & 1));
+        } else {
+            c[s][lane] = rows_join(P.nz, a[0], a[32], __double2loint(a[64]), b[0], b[32], __double2loint(b[64]));
+        }
+    }
+}
+
 // Eigenvalues of a work item (<= 32), lane l owning slot l, to x.  Every round:
 // slots isolated in their bracket (Sturm counts J and J + 1 at its ends) take a
 // safeguarded Laguerre step; the other virtual lanes (v = lane + 32 half) are
 // dealt over the slots not yet isolated and cut their brackets.  A slot is final
 // when the correction is below tol, or when the last two steps stayed inside
 // the bracket and the cubic model predicts the next one below tol.
-template <class Row, int W>
+template <class Row, int W, bool kRows>
 __device__ __forceinline__ double panel_bisect(const ProblemInfo& pi, const Panel& P, const WorkItem& w,
                                                const double* __restrict__ Trec, const int* __restrict__ counts,
                                                double tol_in, unsigned* err, unsigned long long* steps, PRing& R,
@@ -1093,8 +1417,8 @@ __device__ __forceinline__ double panel_bisect(const ProblemInfo& pi, const Pane
         constexpr int kSegs = 4 / W;
         auto seg_of = [&](int i) { return W == 4 ? pr.half : (pr.half ? 3 - i : i); };
         const int nch = (P.nblk + kPanelChunk - 1) / kPanelChunk;
+        double xs[2] = {x, x}, xe = x;
         if (nB > 0) {  // counts: virtual lanes v = lane, lane + 32 of every warp
-            double xs[2];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int v = lane + 32 * h;
@@ -1104,8 +1428,23 @@ __device__ __forceinline__ double panel_bisect(const ProblemInfo& pi, const Pane
                 const double be = __shfl_sync(0xffffffffu, b, e);
                 xs[h] = ae + (be - ae) * ((double)(g + 1) / (double)(G + 1));
             }
-            constexpr int kN = 5 * 64;  // doubles of a segment
-            if (P.blk) {
+        }
+        // Laguerre chains of slots nth_set(nm, lane)
+        if (nN > 0) xe = __shfl_sync(0xffffffffu, x, lane < nN ? nth_set(nm, lane) : 0);
+        constexpr int kL = 6 * 32;  // doubles of a chain
+        auto put = [&](double* o, const LagChain& C) {
+            o[lane] = C.u;
+            o[32 + lane] = C.e;
+            o[64 + lane] = C.u1;
+            o[96 + lane] = C.e1;
+            o[128 + lane] = C.u2;
+            o[160 + lane] = C.e2;
+        };
+        if constexpr (kRows) {
+            rows_round<Row, W>(P, xs, xe, nN, nB, R, err, pr, X.c[tb]);
+        } else {
+            if (nB > 0) {
+                constexpr int kN = 5 * 64;  // doubles of a segment
                 double su[kSegs][2], se[kSegs][2], sv[kSegs][2], sf[kSegs][2];
                 int z[kSegs][2];
 #pragma unroll
@@ -1145,42 +1484,26 @@ __device__ __forceinline__ double panel_bisect(const ProblemInfo& pi, const Pane
                     X.c[tb][pr.half][lane] = nz - zeros;
                 }
                 pr.sync();  // the rings are free again
-            } else if (pr.half == 0) {
-                int c[2];
-                count_sweep<Row, 2>(P, Trec, xs, R, err, c);
-                X.c[tb][0][lane] = c[0];
-                X.c[tb][1][lane] = c[1];
             }
-        }
-        constexpr int kL = 6 * 32;  // doubles of a chain
-        if (nN > 0) {  // Laguerre chains of slots nth_set(nm, lane)
-            const double xe = __shfl_sync(0xffffffffu, x, lane < nN ? nth_set(nm, lane) : 0);
-            auto put = [&](double* o, const LagChain& C) {
-                o[lane] = C.u;
-                o[32 + lane] = C.e;
-                o[64 + lane] = C.u1;
-                o[96 + lane] = C.e1;
-                o[128 + lane] = C.u2;
-                o[160 + lane] = C.e2;
-            };
-            LagChain S[1], M[2];
-            S[0] = pr.half ? LagChain{0.0, -1.0, 0.0, 0.0, 0.0, 0.0} : LagChain{1.0, P.e0, 0.0, 0.0, 0.0, 0.0};
-            M[0] = LagChain{1.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-            M[1] = LagChain{0.0, 1.0, 0.0, 0.0, 0.0, 0.0};
-            if (W == 2 || pr.half == 0 || pr.half == 3) {
-                const int s = pr.half ? 3 : 0;
-                if (P.blk) lag_segment<Row, 1>(P, Trec, xe, nch * s / 4, nch * (s + 1) / 4, s == 3, R, err, S);
-                else lag_raw<Row>(P, xe, s == 3, S[0]);
-            }
-            if (P.blk && (W == 2 || pr.half == 1 || pr.half == 2)) {
-                const int s = W == 4 ? pr.half : 1 + pr.half;
-                lag_segment<Row, 2>(P, Trec, xe, nch * s / 4, nch * (s + 1) / 4, false, R, err, M);
-            }
-            if (W == 2 || pr.half == 0 || pr.half == 3) put(pr.slot(pr.half ? 3 : 0, kL), S[0]);
-            if (W == 2 || pr.half == 1 || pr.half == 2) {
-                double* o = pr.slot(W == 4 ? pr.half : 1 + pr.half, kL);
-                put(o, M[0]);
-                put(o + kL, M[1]);
+            if (nN > 0) {
+                LagChain S[1], M[2];
+                S[0] = pr.half ? LagChain{0.0, -1.0, 0.0, 0.0, 0.0, 0.0} : LagChain{1.0, P.e0, 0.0, 0.0, 0.0, 0.0};
+                M[0] = LagChain{1.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+                M[1] = LagChain{0.0, 1.0, 0.0, 0.0, 0.0, 0.0};
+                if (W == 2 || pr.half == 0 || pr.half == 3) {
+                    const int s = pr.half ? 3 : 0;
+                    lag_segment<Row, 1>(P, Trec, xe, nch * s / 4, nch * (s + 1) / 4, s == 3, R, err, S);
+                }
+                if (W == 2 || pr.half == 1 || pr.half == 2) {
+                    const int s = W == 4 ? pr.half : 1 + pr.half;
+                    lag_segment<Row, 2>(P, Trec, xe, nch * s / 4, nch * (s + 1) / 4, false, R, err, M);
+                }
+                if (W == 2 || pr.half == 0 || pr.half == 3) put(pr.slot(pr.half ? 3 : 0, kL), S[0]);
+                if (W == 2 || pr.half == 1 || pr.half == 2) {
+                    double* o = pr.slot(W == 4 ? pr.half : 1 + pr.half, kL);
+                    put(o, M[0]);
+                    put(o + kL, M[1]);
+                }
             }
         }
         if (steps && lane == 0 && pr.half == 0) {
@@ -1194,9 +1517,9 @@ __device__ __forceinline__ double panel_bisect(const ProblemInfo& pi, const Pane
             auto get = [&](const double* o) {
                 return LagChain{o[v], o[32 + v], o[64 + v], o[96 + v], o[128 + v], o[160 + v]};
             };
-            LagChain U = get(pr.slot(0, kL));
-            const LagChain D = get(pr.slot(3, kL));
-            if (P.blk) {
+            LagChain U = get(kRows ? pr.rows(0, false) : pr.slot(0, kL));
+            const LagChain D = get(kRows ? pr.rows(0, true) : pr.slot(3, kL));
+            if (!kRows) {
 #pragma unroll
                 for (int s = 1; s <= 2; ++s) {  // through the segments between
                     const LagChain A = get(pr.slot(s, kL)), B = get(pr.slot(s, kL) + kL);
@@ -1266,7 +1589,7 @@ __device__ __forceinline__ double panel_bisect(const ProblemInfo& pi, const Pane
             if (!(b - a > tol) || (a == A0 && b == B0)) mode = 2;
             else if (ca == J && cb == J + 1) mode = 1;
         }
-        const bool gave_up = (X.err[tb][0] | X.err[tb][1] | (W == 4 ? X.err[tb][2] | X.err[tb][3] : 0)) != 0;
+        const bool gave_up = (X.err[tb][0] | (W == 1 ? 0 : X.err[tb][1]) | (W == 4 ? X.err[tb][2] | X.err[tb][3] : 0)) != 0;
         pr.sync();  // the rings are free again
         if (gave_up) break;  // a ring wait ran out: abandon the item
     }
@@ -1434,6 +1757,89 @@ struct VecMats {
     }
 };
 
+// Half of the eigenvector work of an item by rows: the sums of squares as they
+// are, five instructions a row (see vector_half for what is kept).
+struct RowVals {
+    double vs, vr;
+    int Es, Er;
+    unsigned loads;
+};
+template <class Row, int NW, bool kV, int kPart, bool kDown>
+__device__ __noinline__ RowVals rows_vector(const ModesArgs& A, const ProblemInfo& pi, const Panel P, double mu,
+                                            VecState* __restrict__ st, PRing R, double* __restrict__ ck,
+                                            int* __restrict__ cke) {
+    using Q = Part<Row, NW, kPart>;
+    constexpr int kN = kSums<Row, NW>, NX = Q::hi - Q::lo;
+    const int lane = threadIdx.x & 31, isrc = pi.isrc, ircv = pi.ircv, M = pi.M;
+    // the weights of this part (one without an array: ones, not read)
+    const double* const w[2] = {A.w + pi.w_off, NW > 1 && A.g ? A.g + pi.s_off : A.w + pi.w_off};
+    const typename Row::At at(mu);
+    double u = 1.0, um = kDown ? 0.0 : P.um0, sum[kN];
+    int E = 0;
+    RowVals out{0.0, 0.0, 0, 0, 0u};
+#pragma unroll
+    for (int n = 0; n < kN; ++n) sum[n] = 0.0;
+    auto row = [&](const double* r, const double* x) {
+        const double x2 = u * u;  // of z_i
+        if (Q::norm) sum[0] += x2;
+#pragma unroll
+        for (int n = Q::lo; n < Q::hi; ++n) {
+            double& s = sum[kN - NW + n];
+            s = n == 1 && !Row::kUnitNorm ? s + x2 : fma(x[(n - Q::lo) * kWD], x2, s);
+        }
+        const double un = fma(at.turn(r), u, -um);
+        um = u;
+        u = un;
+    };
+    // of the state before row i
+    auto keep = [&](int i) {
+        if (i % kCkRows) return;
+        const double v = kDown ? um : u, e = kDown ? um - u : u - um;
+        const size_t c = (size_t)(i / kCkRows);
+        double* o = ck + c * (1 + kN) * 32 + lane;
+        if (kPart != 2) {
+            o[0] = v;
+            cke[c * 32 + lane] = E;
+        }
+        if (Q::norm) o[32] = sum[0];
+#pragma unroll
+        for (int n = Q::lo; n < Q::hi; ++n) o[32 * (1 + kN - NW + n)] = sum[kN - NW + n];
+        if (kV && kPart != 2 && st) st[c * M] = VecState{v, e, E, 0};
+    };
+    auto value = [&](int i) {
+        const double v = kDown ? um : u;
+        if (i == isrc) out.vs = v, out.Es = E;
+        if (i == ircv) out.vr = v, out.Er = E;
+    };
+    rows_sweep<Row, NX, kDown>(
+        P, 0, P.nz, R, A.err, w + (NX > 0 ? Q::lo : 0), [&](const double* r, const double* x, int lo, int m) {
+            if (!kDown) keep(lo);
+            if (kPart != 2 && ((isrc >= lo && isrc < lo + m) || (ircv >= lo && ircv < lo + m))) {
+                for (int k = 0; k < m; ++k) {
+                    const int j = kDown ? m - 1 - k : k;
+                    if (!kDown) value(lo + j);
+                    row(r + j * Row::kW, x + j);
+                    if (kDown) value(lo + j);
+                }
+            } else {
+                run_rows<kDown>(m, [&](int j) { row(r + j * Row::kW, x + j); });
+            }
+            if (kDown) keep(lo);
+            // a run grows by 2^368 at most; a chain that decays keeps its sums
+            const int big = max(biased_exp(u), biased_exp(um)) - 1023;
+            if (big > 100) {
+                const double sc = pow2(-big);
+                u *= sc;
+                um *= sc;
+#pragma unroll
+                for (int n = 0; n < kN; ++n) sum[n] *= sc * sc;
+                E += big;
+            }
+        });
+    out.loads = R.loads;
+    return out;
+}
+
 // Half of the eigenvector work of an item: the upward chain u (half 0) or the
 // downward chain b (half 1); at every coarse row (multiples of kCkRows) its
 // value, exponent and sums go to the checkpoints and, for full vectors (kV),
@@ -1449,9 +1855,6 @@ __device__ __forceinline__ void vector_half(const ModesArgs& A, const ProblemInf
     const int nz = P.nz, isrc = pi.isrc, ircv = pi.ircv;
     const double rinv = 1.0 / P.r;
     const typename Row::Shift sh(P, mu);
-    const double* wp = A.w + pi.w_off;
-    const double* gp = NW > 1 && A.g ? A.g + pi.s_off : nullptr;
-    auto weight = [&](int n, int i) { return n == 0 ? __ldg(wp + i) : (gp ? __ldg(gp + i) : 1.0); };
     VecChain<Row, NW, kPart> C;
     if (half == 0) C.start(1.0, P.e0);
     else C.start(0.0, -1.0);
@@ -1479,84 +1882,46 @@ __device__ __forceinline__ void vector_half(const ModesArgs& A, const ProblemInf
         if (half == 0) rows_up<Row>(P.rows, a, i, mu, v, f);
         else rows_down<Row>(P.rows, end, i, mu, v, f);
     };
-    if (P.blk) {
-        const int nch = (P.nblk + kPanelChunk - 1) / kPanelChunk;
-        const double* src = A.T + (size_t)P.rec * kRecT;
-        const double* sw[2] = {A.W0 + (size_t)P.rec * kRecW, NW > 1 ? A.W1 + (size_t)P.rec * kRecW : nullptr};
-        ring_stream(
-            R, nch, A.err,
-            [&](double* dst, uint64_t* bar, int o) {
-                const size_t c = half ? nch - 1 - o : o;
-                mbar_expect_tx(bar, (kTD + (Q::hi - Q::lo) * kWD) * 8);
-                tma_load_1d(dst, src + c * kTD, kTD * 8, bar);
+    const int nch = (P.nblk + kPanelChunk - 1) / kPanelChunk;
+    const double* src = A.T + (size_t)P.rec * kRecT;
+    const double* sw[2] = {A.W0 + (size_t)P.rec * kRecW, NW > 1 ? A.W1 + (size_t)P.rec * kRecW : nullptr};
+    ring_stream(
+        R, nch, A.err,
+        [&](double* dst, uint64_t* bar, int o) {
+            const size_t c = half ? nch - 1 - o : o;
+            mbar_expect_tx(bar, (kTD + (Q::hi - Q::lo) * kWD) * 8);
+            tma_load_1d(dst, src + c * kTD, kTD * 8, bar);
 #pragma unroll
-                for (int n = Q::lo; n < Q::hi; ++n) tma_load_1d(dst + kTD + n * kWD, sw[n] + c * kWD, kWD * 8, bar);
-            },
-            [&](const double* buf, int o) {
-                const int c = half ? nch - 1 - o : o, nb = min(kPanelChunk, P.nblk - c * kPanelChunk);
-                for (int q0 = 0; q0 < kPanelChunk; q0 += 2) {
-                    const int qa = half ? kPanelChunk - 1 - q0 : q0, qb = half ? qa - 1 : qa + 1;
-                    if (min(qa, qb) >= nb) continue;
-                    VecMats<Row, NW, kPart> M;
-                    const double* const Ts[2] = {buf + qa * kRecT, buf + qb * kRecT};
-                    const double* const Ws[2] = {buf + kTD + qa * kRecW, buf + kTD + qb * kRecW};
-                    const double t[2] = {sh.at(Ts[0]), sh.at(Ts[1])};
-                    M.eval(Ts, Ws, t);
+            for (int n = Q::lo; n < Q::hi; ++n) tma_load_1d(dst + kTD + n * kWD, sw[n] + c * kWD, kWD * 8, bar);
+        },
+        [&](const double* buf, int o) {
+            const int c = half ? nch - 1 - o : o, nb = min(kPanelChunk, P.nblk - c * kPanelChunk);
+            for (int q0 = 0; q0 < kPanelChunk; q0 += 2) {
+                const int qa = half ? kPanelChunk - 1 - q0 : q0, qb = half ? qa - 1 : qa + 1;
+                if (min(qa, qb) >= nb) continue;
+                VecMats<Row, NW, kPart> M;
+                const double* const Ts[2] = {buf + qa * kRecT, buf + qb * kRecT};
+                const double* const Ws[2] = {buf + kTD + qa * kRecW, buf + kTD + qb * kRecW};
+                const double t[2] = {sh.at(Ts[0]), sh.at(Ts[1])};
+                M.eval(Ts, Ws, t);
 #pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-                        const int q = b ? qb : qa;
-                        if (q >= nb) continue;
-                        const int a = (c * kPanelChunk + q) * P.blk, end = min(nz, a + P.blk);
-                        if (half == 0) keep(a, 1.0);
-                        value(isrc, a, end, vs, Es);
-                        value(ircv, a, end, vr, Er);
-                        if (half == 0) {
-                            M.up(b, C);
-                        } else {
-                            M.down(b, C);
-                            keep(a, -1.0);
-                        }
+                for (int b = 0; b < 2; ++b) {
+                    const int q = b ? qb : qa;
+                    if (q >= nb) continue;
+                    const int a = (c * kPanelChunk + q) * P.blk, end = min(nz, a + P.blk);
+                    if (half == 0) keep(a, 1.0);
+                    value(isrc, a, end, vs, Es);
+                    value(ircv, a, end, vr, Er);
+                    if (half == 0) {
+                        M.up(b, C);
+                    } else {
+                        M.down(b, C);
+                        keep(a, -1.0);
                     }
-                }
-                C.rescale();
-            });
-    } else {
-        const int nb = (nz + 15) / 16;
-        for (int o = 0; o < nb; ++o) {
-            const int a = 16 * (half ? nb - 1 - o : o), end = min(nz, a + 16);
-            if (half == 0) keep(a, 1.0);
-            value(isrc, a, end, vs, Es);
-            value(ircv, a, end, vr, Er);
-            for (int j = a; j < end; ++j) {
-                const int i = half ? a + end - 1 - j : j;
-                const double sg = Row::sigma(P.rows, i, mu), sl = Row::slope(P.rows, i, mu);
-                if (half == 0) {
-                    if (Q::norm) C.e1 = fma(-sg, C.u1, fma(sl, C.u, C.e1));
-#pragma unroll
-                    for (int n = Q::lo; n < Q::hi; ++n) C.ew[n] = fma(-sg, C.uw[n], fma(-weight(n, i), C.u, C.ew[n]));
-                    C.e = fma(-sg, C.u, C.e);
-                    C.u += C.e;
-                    if (Q::norm) C.u1 += C.e1;
-#pragma unroll
-                    for (int n = Q::lo; n < Q::hi; ++n) C.uw[n] += C.ew[n];
-                } else {
-                    C.u -= C.e;
-                    if (Q::norm) {
-                        C.u1 -= C.e1;
-                        C.e1 = fma(sg, C.u1, fma(-sl, C.u, C.e1));
-                    }
-#pragma unroll
-                    for (int n = Q::lo; n < Q::hi; ++n) {
-                        C.uw[n] -= C.ew[n];
-                        C.ew[n] = fma(sg, C.uw[n], fma(weight(n, i), C.u, C.ew[n]));
-                    }
-                    C.e = fma(sg, C.u, C.e);
                 }
             }
-            if (half) keep(a, -1.0);
             C.rescale();
-        }
-    }
+        });
 }
 
 // |u b| at a coarse row as m 2^E, m in [1, 2) (m = 0: none yet)
@@ -1653,7 +2018,7 @@ __device__ __noinline__ void fine_twist(const ModesArgs& A, const ProblemInfo& p
     W.Eu = q.E;
 }
 
-template <class Row, int NW, bool kV, int W>
+template <class Row, int NW, bool kV, int W, bool kRows>
 __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemInfo& pi, const Panel& P,
                                              const WorkItem& w, double mu, PRing& R, Team<W>& pr, bool split,
                                              double* __restrict__ ck, int* __restrict__ cke) {
@@ -1664,6 +2029,7 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
     int* ckes[2] = {cke, cke + A.ck_stride};
     double vs, vr;
     int Es, Er;
+    RowVals above{};  // W == 1
     VecState* st = nullptr;
     if (kV && lane < w.m) st = A.vstate + A.vstate_off[w.problem] + w.j0 + lane;
     if (kV && st) st += (long long)half * nc * pi.M;
@@ -1672,7 +2038,32 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
     // than the idle warps (36 azimuths of 0.5 Hz: both stages 286 us, split 300)
     double* c = cks[half];
     int* ce = ckes[half];
-    if (W == 4 && split) {
+    if constexpr (kRows) {
+        RowVals o{};
+        if (W == 1) {
+            o = rows_vector<Row, NW, kV, 0, false>(A, pi, P, mu, st, R, cks[0], ckes[0]);
+            R.loads = o.loads;
+            VecState* sd = st ? st + (long long)nc * pi.M : st;
+            above = rows_vector<Row, NW, kV, 0, true>(A, pi, P, mu, sd, R, cks[1], ckes[1]);
+            R.loads = above.loads;
+        } else if (W == 4 && split && pr.half >= 2) {
+            o = half ? rows_vector<Row, NW, kV, 2, true>(A, pi, P, mu, st, R, c, ce)
+                     : rows_vector<Row, NW, kV, 2, false>(A, pi, P, mu, st, R, c, ce);
+            R.loads = o.loads;
+        } else if (W == 4 && split) {
+            o = half ? rows_vector<Row, NW, kV, 1, true>(A, pi, P, mu, st, R, c, ce)
+                     : rows_vector<Row, NW, kV, 1, false>(A, pi, P, mu, st, R, c, ce);
+            R.loads = o.loads;
+        } else if (pr.half < 2) {
+            o = half ? rows_vector<Row, NW, kV, 0, true>(A, pi, P, mu, st, R, c, ce)
+                     : rows_vector<Row, NW, kV, 0, false>(A, pi, P, mu, st, R, c, ce);
+            R.loads = o.loads;
+        }
+        vs = o.vs;
+        vr = o.vr;
+        Es = o.Es;
+        Er = o.Er;
+    } else if (W == 4 && split) {
         if (pr.half < 2) vector_half<Row, NW, kV, 1>(A, pi, P, mu, half, st, R, c, ce, vs, Es, vr, Er);
         else vector_half<Row, NW, kV, 2>(A, pi, P, mu, half, st, R, c, ce, vs, Es, vr, Er);
     } else if (pr.half < 2) {
@@ -1690,7 +2081,7 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
     // the twist: the coarse row with the largest |u b|, the lowest of equal ones;
     // each half looks through half of the rows
     TwistKey K{0.0, 0, 0};
-    const int c0 = half ? nc / 2 : 0, c1 = half ? nc : nc / 2;
+    const int c0 = half ? nc / 2 : 0, c1 = half || W == 1 ? nc : nc / 2;
 #pragma unroll 4
     for (int c = c0; c < c1; ++c) {
         const size_t o = (size_t)c * (1 + kN) * 32 + lane, i = (size_t)c * 32 + lane;
@@ -1702,13 +2093,14 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
     }
     pr.sync2();
     if (half) return;
-    {
+    if (W != 1) {
         const double m = X.v[t2][1][0][lane], ec = X.v[t2][1][1][lane];
         const int E = __double2hiint(ec);
         if (m > 0.0 && (K.m == 0.0 || E > K.E || (E == K.E && m > K.m))) K.c = __double2loint(ec);
     }
-    const double us = vs, ur = vr, bs = X.v[tb][1][0][lane], br = X.v[tb][1][1][lane];
-    const double eb = X.v[tb][1][2][lane];
+    const double us = vs, ur = vr, bs = W == 1 ? above.vs : X.v[tb][1][0][lane];
+    const double br = W == 1 ? above.vr : X.v[tb][1][1][lane];
+    const double eb = W == 1 ? __hiloint2double(above.Es, above.Er) : X.v[tb][1][2][lane];
     const int Eus = Es, Eur = Er, Ebs = __double2hiint(eb), Ebr = __double2loint(eb);
     TwistAt<kN> tw;
     tw.r = K.c * kCkRows;
@@ -1776,7 +2168,7 @@ template <int NW, int kDo>
 constexpr int kModesSl = kTD + (kDo == 1 ? 0 : NW) * kWD;
 
 template <class Row, int NW, int kDo, bool kV, int W>
-__global__ void __launch_bounds__(kPWarps * 32, kPanelCtas) k_panel_modes(ModesArgs A) {
+__global__ void __launch_bounds__(kPWarps * 32, kPanelCtas) k_panel_modes(const __grid_constant__ ModesArgs A) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int kSl = kModesSl<NW, kDo>;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1814,19 +2206,72 @@ __global__ void __launch_bounds__(kPWarps * 32, kPanelCtas) k_panel_modes(ModesA
         const int it = pr.box->item[turn];
         if (it < 0) break;
         const WorkItem w = A.items[it];
+        if (w.pad < 0) continue;  // k_rows_modes'
         const ProblemInfo& pi = A.pinfo[w.problem];
-        PanelDesc d{};
-        if (w.pad >= 0) d = A.desc[w.pad];
-        else d.xc = Row::lo(pi);
-        const Panel P = panel_of<Row>(pi, d, A.rows);
+        const Panel P = panel_of<Row>(pi, A.desc[w.pad], A.rows);
         double x = P.xc;
         if (kDo & 1) {
-            x = panel_bisect<Row, W>(pi, P, w, A.T, A.counts, A.tol, A.err, A.steps, R, pr);
+            x = panel_bisect<Row, W, false>(pi, P, w, A.T, A.counts, A.tol, A.err, A.steps, R, pr);
             if (pr.half == 0 && lane < w.m) A.mu[pi.off + w.j0 + lane] = x;
         } else if (lane < w.m) {
             x = A.mu[pi.off + w.j0 + lane];
         }
-        if (kDo & 2) panel_vector<Row, NW, kV, W>(A, pi, P, w, x, R, pr, n_items <= A.num_sms, ck, cke);
+        if (kDo & 2) panel_vector<Row, NW, kV, W, false>(A, pi, P, w, x, R, pr, n_items <= A.num_sms, ck, cke);
+    }
+}
+
+// The items by rows (what: 1 eigenvalues, 2 mode values, 3 both), on a stream
+// beside k_panel_modes, whose code stays smaller without them (2 Hz, 20000 rows:
+// 541 us, with the rows' sweeps in the same kernel 578).  Teams of four while the
+// items are few: a sweep is a chain over half of the rows.  A warp to an item
+// from kSoloMin an SM on, both directions in turn and no exchange: bound by FP64
+// issue and, on grids of some hundred rows, by the latency of a sweep's first
+// rows, which more items in flight hide (12 on an SM, 3 teams of four; 90
+// azimuths of 1 Hz, 2500 rows 1040 -> 730 us).  The values are the same.
+template <class Row, int NW, bool kV, int W, int kDo>
+__global__ void __launch_bounds__(kPWarps * 32, W == 1 ? kRowsCtas : kPanelCtas)
+    k_rows_modes(const __grid_constant__ ModesArgs A) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    constexpr int kSl = kTD + NW * kWD, kTeams = kPWarps / W;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int n_items = A.n_items_dev[0], n_rows = A.n_items_dev[3];
+    if (n_rows == 0 || (n_rows > kSoloMin * A.num_sms) != (W == 1)) return;  // none, or the other launch's
+    PRing R = make_ring(smem_raw, wid, kSl);
+    Team<W> pr;
+    pr.id = wid / W;
+    pr.half = wid % W;
+    pr.box = reinterpret_cast<PairBox*>(smem_raw + kRingBytes<kSl>) + pr.id;
+    pr.stride = kPBuf * kSl;
+    pr.area = reinterpret_cast<double*>(smem_raw) + (size_t)pr.id * W * pr.stride;
+    pr.turn = 0;
+    const long long slot = (long long)blockIdx.x * kTeams + pr.id;
+    double* ck = A.ck_u + slot * 2 * A.ck_stride * (1 + kSums<Row, NW>);
+    int* cke = A.ck_e + slot * 2 * A.ck_stride;
+    const int n_teams = gridDim.x * kTeams;
+    int next = pr.id * gridDim.x + blockIdx.x;  // first items on different SMs
+    for (int turn = 0;; turn ^= 1) {
+        if (pr.half == 0 && lane == 0) {
+            while (next < n_items && A.items[next].pad >= 0)  // k_panel_modes'
+                next = A.sched ? n_teams + atomicAdd(A.sched, 1) : next + n_teams;
+            pr.box->item[turn] = next < n_items ? next : -1;
+            next = A.sched ? n_teams + atomicAdd(A.sched, 1) : next + n_teams;
+        }
+        pr.sync();
+        const int it = pr.box->item[turn];
+        if (it < 0) break;
+        const WorkItem w = A.items[it];
+        const ProblemInfo& pi = A.pinfo[w.problem];
+        PanelDesc d{};
+        d.xc = Row::lo(pi);
+        const Panel P = panel_of<Row>(pi, d, A.rows);
+        double x = P.xc;
+        if (kDo & 1) {
+            x = panel_bisect<Row, W, true>(pi, P, w, A.T, A.counts, A.tol, A.err, A.steps, R, pr);
+            if (pr.half == 0 && lane < w.m) A.mu[pi.off + w.j0 + lane] = x;
+        } else if (lane < w.m) {
+            x = A.mu[pi.off + w.j0 + lane];
+        }
+        if (kDo & 2) panel_vector<Row, NW, kV, W, true>(A, pi, P, w, x, R, pr, false, ck, cke);
     }
 }
 
@@ -1898,6 +2343,9 @@ __global__ void __launch_bounds__(256) k_panel_fill(int p0, ModesArgs A) {
     }
 }
 
+// checkpoint slots of k_panel_modes: two directions of two pairs a CTA
+int panel_slots(int grid) { return 2 * (kPWarps / 2) * grid; }
+
 template <class Row, int NW, int kDo, bool kV, int W>
 void modes_run(cudaStream_t st, int grid, const ModesArgs& a) {
     constexpr int kSl = kModesSl<NW, kDo>;
@@ -1906,6 +2354,36 @@ void modes_run(cudaStream_t st, int grid, const ModesArgs& a) {
     auto* f = k_panel_modes<Row, NW, kDo, kV, W>;
     cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     f<<<grid, kPWarps * 32, sm, st>>>(a);
+}
+
+template <class Row, int NW, bool kV, int W, int kDo>
+void rows_run(cudaStream_t st, int ctas, const ModesArgs& a) {
+    constexpr int kSl = kTD + NW * kWD;
+    static_assert(kSl * kPBuf >= 4 * 7 * 32, "a warp's chains fit its ring");
+    const size_t sm = kRingBytes<kSl> + (kPWarps / W) * sizeof(PairBox);
+    auto* f = k_rows_modes<Row, NW, kV, W, kDo>;
+    cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    f<<<ctas, kPWarps * 32, sm, st>>>(a);
+}
+template <class Row, int NW, bool kV>
+int rows_run(cudaStream_t st, int grid, const ModesArgs& a, int what) {
+    ModesArgs r = a;
+    const long long used = panel_slots(grid);  // behind k_panel_modes' checkpoints
+    r.ck_u += used * kCkVals * a.ck_stride;
+    r.ck_e += used * a.ck_stride;
+    if (r.sched) r.sched += 2;
+    const int teams = std::min(grid, a.item_cap);
+    if (what == 3) rows_run<Row, NW, kV, 4, 3>(st, teams, r);
+    if (what == 1) rows_run<Row, 1, false, 4, 1>(st, teams, r);
+    if (what == 2) rows_run<Row, NW, kV, 4, 2>(st, teams, r);
+    int n = 1;
+    if (a.item_cap > kSoloMin * a.num_sms) {
+        const int ctas = std::min(grid / kPanelCtas * kRowsCtas, (a.item_cap + kPWarps - 1) / kPWarps);
+        if (what & 1) rows_run<Row, 1, false, 1, 1>(st, ctas, r), ++n;
+        if (what == 3 && r.sched) ++r.sched;
+        if (what & 2) rows_run<Row, NW, kV, 1, 2>(st, ctas, r), ++n;
+    }
+    return n;
 }
 
 template <class Row, int NW, int kDo, int W>
@@ -2121,7 +2599,7 @@ int launch_panel_items(cudaStream_t st, bool wide, int P, ProblemInfo* pinfo, co
     if (bis_item < 1 || bis_item > kWItem) return -1;
     k_panel_items<<<1, kItemThreads, 0, st>>>(P, pinfo, counts, max_modes, bis_item, cap, tot, err, order);
     auto* f = wide ? k_panel_groups<WmodPanel> : k_panel_groups<EssPanel>;
-    f<<<(P + kPlanWarps - 1) / kPlanWarps, kPlanWarps * 32, 0, st>>>(P, pinfo, counts, bis_item, items, cap, desc);
+    f<<<(P + kPlanWarps - 1) / kPlanWarps, kPlanWarps * 32, 0, st>>>(P, pinfo, counts, bis_item, items, cap, desc, tot);
     return 2;
 }
 
@@ -2147,11 +2625,21 @@ int launch_panel_fill(cudaStream_t st, bool wide, int P, int nz_max, int m_max, 
     return n;
 }
 
+int launch_rows_modes(cudaStream_t st, bool wide, int grid, const ModesArgs& a, int what) {
+    if (wide) return a.vstate ? rows_run<WmodPanel, 2, true>(st, grid, a, what) : rows_run<WmodPanel, 2, false>(st, grid, a, what);
+    if (a.g) return a.vstate ? rows_run<EssPanel, 2, true>(st, grid, a, what) : rows_run<EssPanel, 2, false>(st, grid, a, what);
+    return a.vstate ? rows_run<EssPanel, 1, true>(st, grid, a, what) : rows_run<EssPanel, 1, false>(st, grid, a, what);
+}
+
 int launch_panel_modes(cudaStream_t st, bool wide, int grid, const ModesArgs& a, int what) {
     if (wide) return modes_launch<WmodPanel, 2>(st, grid, a, what);
     return a.g ? modes_launch<EssPanel, 2>(st, grid, a, what) : modes_launch<EssPanel, 1>(st, grid, a, what);
 }
 
 int panel_ctas_per_sm() { return kPanelCtas; }
+
+int panel_ck_slots(int grid, bool rows) {
+    return panel_slots(grid) + (rows ? 2 * kPWarps * (grid / kPanelCtas * kRowsCtas) : 0);
+}
 
 }  // namespace ncpa
