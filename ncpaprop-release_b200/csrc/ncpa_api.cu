@@ -196,6 +196,7 @@ struct ncpa_profile {
     int has_z0 = 0;
     double z_lo = 0.0, z_hi = 0.0;
     std::vector<double> h_c0, h_u, h_v;  // host copies: bounds of c_eff size the panel expansions
+    double h_wind = 0.0;                 // the largest wind speed
     int plan_refs = 0;  // plans whose graphs read this profile's arrays
 };
 
@@ -808,9 +809,12 @@ void layout_groups(ncpa_modes* M, std::vector<Group>& groups, long long& s_tot, 
     }
 }
 
-// extremes of c_eff = c0 + u sin(az) + v cos(az) at the knots
-std::pair<double, double> ceff_bounds(const ncpa_profile* prof, double az_deg) {
-    const double s = std::sin(az_deg * kPi / 180.0), c = std::cos(az_deg * kPi / 180.0);
+// Bounds of c_eff = c0 + u sin(az) + v cos(az) at the knots for the azimuths of
+// sector k of kSectors: at the sector's middle, and half a sector times the
+// largest wind to either side.
+constexpr int kSectors = 32;
+std::pair<double, double> ceff_bounds(const ncpa_profile* prof, int k) {
+    const double az = (k + 0.5) * (2.0 * kPi / kSectors), s = std::sin(az), c = std::cos(az);
     const double *c0 = prof->h_c0.data(), *u = prof->h_u.data(), *v = prof->h_v.data();
     double lo[4] = {INFINITY, INFINITY, INFINITY, INFINITY}, hi[4] = {0.0, 0.0, 0.0, 0.0};
     const int n = prof->n;
@@ -821,8 +825,9 @@ std::pair<double, double> ceff_bounds(const ncpa_profile* prof, double az_deg) {
             lo[k] = x < lo[k] ? x : lo[k];
             hi[k] = x > hi[k] ? x : hi[k];
         }
-    return {std::min(std::min(lo[0], lo[1]), std::min(lo[2], lo[3])),
-            std::max(std::max(hi[0], hi[1]), std::max(hi[2], hi[3]))};
+    const double edge = prof->h_wind * (kPi / kSectors);
+    return {std::min(std::min(lo[0], lo[1]), std::min(lo[2], lo[3])) - edge,
+            std::max(std::max(hi[0], hi[1]), std::max(hi[2], hi[3])) + edge};
 }
 
 // Reserves the panels and block records of every problem (panel.cu).  With
@@ -849,9 +854,12 @@ void layout_panels(ncpa_modes* M, const std::vector<Group>& groups, const ncpa_e
                 c_lo = std::min(prm->c_min, prm->c_max);
                 c_hi = std::max(prm->c_min, prm->c_max);
             } else {
-                // jobs of a sweep share their profile and azimuths
-                auto [it, fresh] = seen.try_emplace({g.prof, g.az[a]});
-                if (fresh) it->second = ceff_bounds(g.prof, g.az[a]);
+                // a pass over the knots a sector: with one an azimuth 720 of them
+                // took 0.8 ms of host time
+                const double turn = g.az[a] / 360.0;
+                const int k = std::max(0, std::min((int)((turn - std::floor(turn)) * kSectors), kSectors - 1));
+                auto [it, fresh] = seen.try_emplace({g.prof, k});
+                if (fresh) it->second = ceff_bounds(g.prof, k);
                 c_lo = it->second.first;
                 c_hi = it->second.second;
             }
@@ -1288,6 +1296,8 @@ void fill_profile(ncpa_ctx* ctx, ncpa_profile* P, const ncpa_profile_desc* d) {
     for (int i = 0; i < n; ++i) P->h_c0[i] = d->c0 ? d->c0[i] : std::sqrt(1.4 * d->p[i] / d->rho[i]);
     P->h_u.assign(d->u, d->u + n);
     P->h_v.assign(d->v, d->v + n);
+    P->h_wind = 0.0;
+    for (int i = 0; i < n; ++i) P->h_wind = std::max(P->h_wind, std::sqrt(d->u[i] * d->u[i] + d->v[i] * d->v[i]));
     const std::pair<DevBuf*, const double*> cols[] = {{&P->z, d->z}, {&P->u, d->u}, {&P->v, d->v},
                                                       {&P->t, d->t}, {&P->p, d->p}, {&P->rho, d->rho}};
     for (const auto& c : cols) CK(cudaMemcpyAsync(c.first->p, c.second, n * sizeof(double), cudaMemcpyHostToDevice, st));
