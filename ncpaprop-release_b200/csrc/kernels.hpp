@@ -42,6 +42,7 @@ struct ProblemInfo {
     int blk_cap;           // block records reserved (the scan's panels, then the work items')
     long long blk_off;     // the first of them
     double g0;             // wide-angle rows: ground term of row 0, 1 / (dz admittance + 1)
+    unsigned long long c0min_bits;  // wide-angle rows: least c_0
 };
 
 constexpr int kWkbNone = 1 << 30;

@@ -795,6 +795,7 @@ void layout_groups(ncpa_modes* M, std::vector<Group>& groups, long long& s_tot, 
                 pi.az = g.az[a];
                 pi.ceffmin_bits = 0x7ff0000000000000ull;
                 pi.ceffmax_bits = 0ull;
+                pi.c0min_bits = 0x7ff0000000000000ull;
                 pi.wkb_trial = ncpa::kWkbNone;
                 pi.dz = g.geo.dz;
                 pi.nz = g.nz;
@@ -878,8 +879,11 @@ void layout_panels(ncpa_modes* M, const std::vector<Group>& groups, const ncpa_e
                 const double n_it = std::min((2.0 * pi.freq * pi.dz * nz * std::sqrt(dk * slack) + 32.0) / 16.0, 4096.0);
                 const double n = std::max(n_it, n_s);
                 const double n_g = std::ceil(std::min(2.0 * R * B * B / rho + 2.0, n_it));
+                // a narrow window far above the band of most rows has short blocks for their
+                // growth (most_rows; |sigma| about (h k_max)^2 at most): two such panels
+                const double k = kh / c_lo, b_min = std::max(std::min(B, 60.0 / std::acosh(1.0 + 0.5 * k * k)), 8.0);
                 const double blocks = std::min(2.0 * nz * R * B / rho, 2.0 * nz * std::sqrt(n * R / rho)) +
-                                      2.0 * std::ceil(nz / B);
+                                      2.0 * std::ceil(nz / b_min);
                 pi.grp_off = M->n_desc;
                 pi.grp_cap = (int)n_g;
                 M->n_desc += pi.grp_cap;

@@ -63,6 +63,11 @@ constexpr int kTD = kPanelChunk * kRecT;  // doubles of a chunk of T records
 constexpr int kWD = kPanelChunk * kRecW;  // doubles of a chunk of one weight's records
 constexpr int kPBuf = 3;                  // ring slots per warp
 constexpr int kPWarps = 4;                // warps per CTA (two pairs)
+// a chunk's growth in bits, at most, and where the mode values' chains are
+// rescaled: sums are products of u at kVecBits + kGrowBits and a derivative
+// at 130 more
+constexpr int kGrowBits = 400, kVecBits = 20;
+static_assert(480 + kGrowBits + 130 < 1023 && 2 * (kVecBits + kGrowBits) + 130 < 1023, "the sweeps stay finite");
 constexpr int kPanelCtas = 3;             // CTAs per SM
 constexpr int kSoloMin = 6;               // items by rows per SM from which on each has a warp
 constexpr int kRowsCtas = 4;              // CTAs per SM then
@@ -117,6 +122,13 @@ struct EssPanel {
     __device__ static __forceinline__ double hi(const ProblemInfo& pi) { return pi.hi; }
     __device__ static __forceinline__ double tol_scale(const ProblemInfo&) { return 1.0; }
     __device__ static __forceinline__ double steepness(const ProblemInfo&) { return 1.0; }  // of sigma in x
+    // a bound of |sigma| = |h^2 omega^2 / c_eff^2 - x| in the window
+    __device__ static __forceinline__ float span(const ProblemInfo& pi) {
+        const float wh = (float)(pi.omega * pi.dz), lo = (float)pi.lo, hi = (float)pi.hi;
+        const float k0 = wh / (float)__longlong_as_double((long long)pi.ceffmax_bits);
+        const float k1 = wh / (float)__longlong_as_double((long long)pi.ceffmin_bits);
+        return fmaxf(k1 * k1 - fminf(lo, hi), fmaxf(lo, hi) - k0 * k0);
+    }
     // The shift that a row sees.  The stored rows are multiples of 2^-52 in (-2,
     // -1] (but for the ground row and very coarse grids).  So in doubles s_i - x
     // is s_i less x rounded to that grid where it lies above -2, and below,
@@ -193,6 +205,16 @@ struct WmodPanel {
     // |d sigma / d kappa| = 2 (kappa + U d), U d < kappa / 2 at winds below half
     // the speed of sound
     __device__ static __forceinline__ double steepness(const ProblemInfo& pi) { return 3.0 * (pi.k_max * pi.dz); }
+    // A bound of |sigma| = |d^2 - kappa^2|: at phase speed c, d = h omega (1 - w /
+    // c) / c_0 is at most h omega / c_0 downwind, and upwind, with c_0 = c_eff -
+    // w, at most h omega / min c_eff (for c from there on)
+    __device__ static __forceinline__ float span(const ProblemInfo& pi) {
+        const float c = fminf((float)__longlong_as_double((long long)pi.ceffmin_bits),
+                              (float)__longlong_as_double((long long)pi.c0min_bits));
+        const float dz = (float)pi.dz, d = (float)pi.omega * dz / c;
+        const float a = (float)pi.k_min * dz, b = (float)pi.k_max * dz, k0 = fminf(a, b), k1 = fmaxf(a, b);
+        return fmaxf(fmaxf(d, k1) * fmaxf(d, k1) - k0 * k0, k1 * k1);
+    }
     // An evaluation of the rows rounds -kappa^2 - 2 once for all of them, a
     // common shift of sigma by up to 2e-16; the blocks take the kappa that
     // shifts theirs alike (by the middle row's slope).
@@ -232,10 +254,23 @@ __device__ __forceinline__ Panel panel_of(const ProblemInfo& pi, const PanelDesc
 
 __device__ __forceinline__ int padded(int nblk) { return (nblk + kPanelChunk - 1) / kPanelChunk * kPanelChunk; }
 
-// rows per block for shifts within r of the centre: the most that keep r B^2
-// within kRhoMax (0: not even panel_min_blk, the rows as they are)
-__device__ __forceinline__ int block_rows(double r, int nz) {
-    for (int B = kPanelMaxBlk; B >= panel_min_blk(nz); B >>= 1)
+// The most rows of a block, for the growth of a chain over a chunk of them: with
+// |sigma| <= S a row multiplies the state by at most e^lambda, cosh lambda = 1 +
+// S / 2 (the comparison recurrence |e'| = |e| + S |u|, |u'| = |u| + |e'|).  The
+// sweeps rescale once a chunk, so that a state below 2^480 stays finite, and the
+// mode values' chains, whose sums are products of two, one below 2^kVecBits.  (In
+// single precision, whose errors the bits to spare cover: in double 3 us a solve.)
+__device__ __forceinline__ int most_rows(float S) {
+    const float h = 0.5f * S, bits = log1pf(h + sqrtf(h * (h + 2.f))) * 1.4426950f;
+    int B = kPanelMaxBlk;
+    while (B > 0 && !(bits * (float)(kPanelChunk * B) <= (float)kGrowBits)) B >>= 1;
+    return B;
+}
+
+// rows per block for shifts within r of the centre: the most (of `most`) that
+// keep r B^2 within kRhoMax (0: not even panel_min_blk, the rows as they are)
+__device__ __forceinline__ int block_rows(double r, int nz, int most) {
+    for (int B = most; B >= panel_min_blk(nz); B >>= 1)
         if (r * (double)B * (double)B <= kRhoMax) return B;
     return 0;
 }
@@ -261,17 +296,18 @@ __device__ void plan_scan_panels(ProblemInfo& pi, int n) {
     const int units = n / kScanStep;
     const double st = Row::steepness(pi);
     const double d = fabs(Row::hi(pi) - Row::lo(pi)) / (double)(n - 1);
-    int upp = units, B = 0;
+    const int most = most_rows(Row::span(pi));
+    int upp = most >= panel_min_blk(pi.nz) ? units : 0, B = 0;
     for (; upp >= 1; --upp) {
         const double r = 0.5 * d * (double)(upp * kScanStep - 1);
-        if (st * r * (double)kPanelMaxBlk * (double)kPanelMaxBlk <= kRhoMax) {
-            B = kPanelMaxBlk;
+        if (st * r * (double)most * (double)most <= kRhoMax) {
+            B = most;
             break;
         }
     }
     if (!B) {
         upp = 1;
-        B = block_rows(st * (0.5 * d * (double)(kScanStep - 1)), pi.nz);
+        B = block_rows(st * (0.5 * d * (double)(kScanStep - 1)), pi.nz, most);
     }
     const long long need = B ? (long long)((units + upp - 1) / upp) * padded((pi.nz + B - 1) / B) : 0;
     const bool fits = B != 0 && need <= pi.blk_cap;
@@ -1155,6 +1191,7 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_panel_groups(int P, const P
     const int* cnt = counts + (size_t)p * kScanMax;
     const double lo = Row::lo(pi), hi = Row::hi(pi), st = Row::steepness(pi);
     const int M = pi.M, n = pi.n_scan, nb = (M + bis_item - 1) / bis_item;
+    const int most = most_rows(Row::span(pi));
     int ng = 0, used = 0;  // panels and records taken so far (warp-uniform)
     for (int k0 = 0; k0 < nb; k0 += kPlanItems) {
         const int m = min(kPlanItems, nb - k0);
@@ -1173,14 +1210,14 @@ __global__ void __launch_bounds__(kPlanWarps * 32) k_panel_groups(int P, const P
                 double b = xb[wid][i];
                 int e = i + 1;
                 auto wide = [&](double c) {
-                    return !(st * (0.5 * (c - a)) * (double)kPanelMaxBlk * (double)kPanelMaxBlk <= kRhoMax);
+                    return !(st * (0.5 * (c - a)) * (double)most * (double)most <= kRhoMax);
                 };
                 if (!wide(b))
                     while (e < m && !wide(fmax(b, xb[wid][e]))) b = fmax(b, xb[wid][e++]);
                 PanelDesc d;
                 d.xc = 0.5 * (a + b);
                 d.r = fmax(0.5 * (b - a), 1e-300);
-                d.blk = block_rows(st * d.r, pi.nz);
+                d.blk = block_rows(st * d.r, pi.nz, most);
                 d.problem = p;
                 d.rec = pi.blk_off + used;
                 const int need = d.blk ? padded((pi.nz + d.blk - 1) / d.blk) : 0;
@@ -1670,7 +1707,7 @@ struct VecChain {
     }
     __device__ __forceinline__ void rescale() {
         const int x = max(biased_exp(u), biased_exp(e)), sh = x - 1023;
-        if (x != 0 && (sh > 240 || sh < -240)) {  // products of two stay finite
+        if (x != 0 && (sh > kVecBits || sh < -240)) {  // products of two stay finite
             const double sc = pow2(-sh);
             u *= sc;
             e *= sc;

@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(256) k_wmod_build(const GroupDesc* __restrict_
     ProblemInfo* __restrict__ pinfo = G.pinfo;
     double2* __restrict__ rows = reinterpret_cast<double2*>(G.s);
     double* __restrict__ kz2 = G.kz2;
-    double cmin = 1e300, cmax = -1e300;
+    double cmin = 1e300, cmax = -1e300, c0min = 1e300;
     const int top = nz - (nz / 10);
     const int itop = top + 1 < nz ? top + 1 : nz - 1;
     if (i >= nz && i < nz_pad)
@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(256) k_wmod_build(const GroupDesc* __restrict_
         const double wc = spline_get(nk, zk, wck + (size_t)az * nk, wcc + (size_t)az * 4 * (nk - 1), z);
         const double ce = spline_get(nk, zk, ceffk + (size_t)az * nk, ceffc + (size_t)az * 4 * (nk - 1), z);
         cmin = cmax = ce;
+        c0min = c0;
         for (int f = f0; f < f1; ++f) {
             const int p = f * n_az + az;
             const double omega = pinfo[p].omega;
@@ -75,18 +76,21 @@ __global__ void __launch_bounds__(256) k_wmod_build(const GroupDesc* __restrict_
     for (int o = 16; o > 0; o >>= 1) {
         cmin = fmin(cmin, __shfl_xor_sync(0xffffffffu, cmin, o));
         cmax = fmax(cmax, __shfl_xor_sync(0xffffffffu, cmax, o));
+        c0min = fmin(c0min, __shfl_xor_sync(0xffffffffu, c0min, o));
     }
-    __shared__ double smin[8], smax[8];
+    __shared__ double smin[8], smax[8], s0min[8];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0) {
         smin[wid] = cmin;
         smax[wid] = cmax;
+        s0min[wid] = c0min;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int k = 1; k < 8; ++k) {
             cmin = fmin(cmin, smin[k]);
             cmax = fmax(cmax, smax[k]);
+            c0min = fmin(c0min, s0min[k]);
         }
         cmin = fmin(cmin, smin[0]);
         cmax = fmax(cmax, smax[0]);
@@ -95,6 +99,7 @@ __global__ void __launch_bounds__(256) k_wmod_build(const GroupDesc* __restrict_
                 const int p = f * n_az + az;
                 atomicMin(&pinfo[p].ceffmin_bits, (unsigned long long)__double_as_longlong(cmin));
                 atomicMax(&pinfo[p].ceffmax_bits, (unsigned long long)__double_as_longlong(cmax));
+                atomicMin(&pinfo[p].c0min_bits, (unsigned long long)__double_as_longlong(c0min));
             }
         }
     }
