@@ -880,8 +880,8 @@ void layout_panels(ncpa_modes* M, const std::vector<Group>& groups, const ncpa_e
                 const double n = std::max(n_it, n_s);
                 const double n_g = std::ceil(std::min(2.0 * R * B * B / rho + 2.0, n_it));
                 // a narrow window far above the band of most rows has short blocks for their
-                // growth (most_rows; |sigma| about (h k_max)^2 at most): two such panels
-                const double k = kh / c_lo, b_min = std::max(std::min(B, 60.0 / std::acosh(1.0 + 0.5 * k * k)), 8.0);
+                // growth (most_rows; lambda about h k_max at most): two such panels
+                const double b_min = std::max(std::min(B, 60.0 * c_lo / kh), 8.0);
                 const double blocks = std::min(2.0 * nz * R * B / rho, 2.0 * nz * std::sqrt(n * R / rho)) +
                                       2.0 * std::ceil(nz / b_min);
                 pi.grp_off = M->n_desc;

@@ -31,9 +31,14 @@
 // In a block, the solution that starts with u = 0 changes sign n2(x) times, and
 // any other solution n2 or n2 + 1 times (Sturm separation), so the parity of
 // the sign change between the block's ends decides.  n2 is counted at the
-// panel's centre; elsewhere in the panel it differs by at most one (the phase
-// over half a panel is at most sqrt(rho) ~ 3.2 rad), downwards in t, which the
-// sign of the entry T12 tells.
+// panel's centre.  Elsewhere it is less by the zeros of the entry T12 in between,
+// the levels of the block's rows with u = 0 at both ends: at even sigma they are
+// 29 / B^2 apart and half a panel is kRhoMax / B^2, so it differs by one at most,
+// which the sign of T12 tells; with sigma varying by V over the block they are
+// still 29 / B^2 - V apart.  Where V is above kFlat / B^2 the roots of T12 are
+// bounded from its coefficients, where these allow more than one the expansion
+// counts at the panel's ends too, and a block that differs there by more than one
+// (two wells with a barrier between them) is counted by its rows.
 //
 // Eigenvectors.  u runs up from the ground and b, the solution that meets the
 // upper boundary, runs down; they are joined at the twist row r where |u b| is
@@ -319,6 +324,64 @@ __device__ void plan_scan_panels(ProblemInfo& pi, int n) {
 // expansion
 // ---------------------------------------------------------------------------
 constexpr int kExpThreads = 64;
+constexpr double kFlat = 16.0;
+constexpr int kByRows = 1 << 20;  // (even) added to the n2 of a block that is counted by its rows
+static_assert(kRhoMax + kFlat < 27.0, "two levels of a block are further apart than half a panel");
+
+__device__ __forceinline__ unsigned neg(double v) { return static_cast<unsigned>(__double2hiint(v)) >> 31; }
+
+// the upper words of doubles as integers in the same order, and back
+__device__ __forceinline__ int order_word(double v) {
+    const int h = __double2hiint(v);
+    return h ^ ((h >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ double word_value(int k) { return __hiloint2double(k ^ ((k >> 31) & 0x7fffffff), 0); }
+
+// whether the sign changes over the rows [a, end) of the solution that starts with
+// u = 0 differ by more than one between t = 0, where they are n2, and t = -1 or 1
+template <class Row>
+__device__ __forceinline__ bool far_zeros(const Panel& P, int a, int end, int n2) {
+    double u[2] = {0.0, 0.0}, e[2] = {1.0, 1.0};
+    unsigned prev[2] = {0u, 0u};
+    int n[2] = {0, 0};
+    for (int i = a; i < end; ++i) {
+        const Quad q = Row::series(P.rows, i, P.xc, P.r);
+        const double even = Row::kQuad ? q.s0 + q.s2 : q.s0;
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            e[k] = fma(k ? even + q.s1 : even - q.s1, u[k], e[k]);
+            u[k] += e[k];
+            n[k] += static_cast<int>(neg(u[k]) ^ prev[k]);
+            prev[k] = neg(u[k]);
+        }
+    }
+    return n[0] > n2 + 1 || n[1] < n2 - 1;
+}
+
+// sign changes in the coefficients of a polynomial
+__device__ __forceinline__ int variations(const double (&c)[kPD + 1]) {
+    int n = 0;
+#pragma unroll
+    for (int k = 0; k < kPD; ++k) n += static_cast<int>(neg(c[k]) ^ neg(c[k + 1]));
+    return n;
+}
+// By Budan's theorem a polynomial has at most as many roots in (s, t] as its
+// Taylor coefficients lose sign changes from s to t: whether that leaves T12 (c)
+// more than one root on either side of 0 within [-1, 1]
+__device__ __forceinline__ bool may_have_pairs(const double (&c)[kPD + 1]) {
+    const int here = variations(c);
+    double p[kPD + 1], m[kPD + 1];
+#pragma unroll
+    for (int k = 0; k <= kPD; ++k) p[k] = m[k] = c[k];
+#pragma unroll
+    for (int i = 0; i < kPD; ++i)
+#pragma unroll
+        for (int j = kPD - 1; j >= i; --j) {
+            p[j] += p[j + 1];
+            m[j] -= m[j + 1];
+        }
+    return variations(m) - here > 1 || here - variations(p) > 1;
+}
 
 // One thread per (panel, block, column of the transfer matrix): it runs the
 // block's rows with the power series of u and e in t, and of their derivatives
@@ -346,10 +409,12 @@ __device__ __forceinline__ void expand_block(const Panel& P, int b, int col, con
     else e[0] = 1.0;
     const double r = P.r;
     unsigned prev = 0u;
-    int n2 = 0;
+    int n2 = 0, top = INT_MIN, bot = INT_MAX;
     for (int i = a; i < end; ++i) {
         const Quad sq = Row::series(P.rows, i, P.xc, r);
         const double sg = sq.s0, s1 = sq.s1;
+        top = max(top, order_word(sg));
+        bot = min(bot, order_word(sg));
         const double wi = NW > 0 ? -__ldg(wp + i) : 0.0;
         const double gi = NW > 1 ? (gp ? -__ldg(gp + i) : -1.0) : 0.0;
 #pragma unroll
@@ -391,6 +456,9 @@ __device__ __forceinline__ void expand_block(const Panel& P, int b, int col, con
         o[4 * k + 2] = e[k];
     }
     if (col == 1) {
+        const double hi = word_value(top), lo = word_value(bot);  // to 2^-20 of themselves
+        const bool flat = (hi - lo + 1e-6 * (fabs(hi) + fabs(lo))) * (double)P.blk * (double)P.blk <= kFlat;
+        if (!flat && may_have_pairs(u) && far_zeros<Row>(P, a, end, n2)) n2 += kByRows;
         T[rec * kRecT + kRecZeros] = __hiloint2double(0, n2);
         T[rec * kRecT + kRecMid] = Row::middle(P.rows, min(P.nz - 1, a + P.blk / 2), P.xc);
     }
@@ -500,13 +568,29 @@ __device__ __forceinline__ void ring_stream(PRing& R, int n, unsigned* err, Issu
     R.loads = base + n;
 }
 
-// t of a shift x in the blocks of a panel
-__device__ __forceinline__ unsigned neg(double v) { return static_cast<unsigned>(__double2hiint(v)) >> 31; }
+// n2 at a shift x where the panel's centre does not tell, by the rows of block b
+template <class Row>
+__device__ __forceinline__ int rows_zeros(const Panel& P, int b, double x) {
+    double u = 0.0, e = 1.0;
+    unsigned prev = 0u;
+    int n = 0;
+    const int end = min(P.nz, (b + 1) * P.blk);
+#pragma unroll 1
+    for (int i = b * P.blk; i < end; ++i) {
+        e = fma(-Row::sigma(P.rows, i, x), u, e);
+        u += e;
+        n += static_cast<int>(neg(u) ^ prev);
+        prev = neg(u);
+    }
+    return n;
+}
 
-// sign changes of a chain across a block: u before, un after, T12 at the
-// chain's t, n2 at the panel's centre
-__device__ __forceinline__ int block_zeros(double u, double un, double T12, double t, int n2) {
-    if (neg(T12) != static_cast<unsigned>(n2 & 1)) n2 += t > 0.0 ? -1 : 1;
+// n2 at t from that at the panel's centre and the sign of T12 there
+__device__ __forceinline__ int zeros_here(double T12, double t, int n2) {
+    return neg(T12) != static_cast<unsigned>(n2 & 1) ? n2 + (t > 0.0 ? -1 : 1) : n2;
+}
+// sign changes of a chain across a block: u before, un after
+__device__ __forceinline__ int block_zeros(double u, double un, int n2) {
     return n2 + static_cast<int>((neg(u) ^ neg(un)) ^ static_cast<unsigned>(n2 & 1));
 }
 
@@ -915,6 +999,22 @@ __device__ __noinline__ RowBoth<NC> rows_both(const Panel P, double xa, double x
     return out;
 }
 
+// the two columns of NC transfer matrices by a common factor
+template <int NC>
+__device__ __forceinline__ void rescale_columns(double (&u)[NC], double (&e)[NC], double (&v)[NC], double (&f)[NC]) {
+#pragma unroll
+    for (int n = 0; n < NC; ++n) {
+        const int s = rescale_shift(fmax(fabs(u[n]), fabs(v[n])), fmax(fabs(e[n]), fabs(f[n])));
+        if (s) {
+            const double sc = pow2(-s);
+            u[n] *= sc;
+            e[n] *= sc;
+            v[n] *= sc;
+            f[n] *= sc;
+        }
+    }
+}
+
 // The transfer matrix of the chunks [c0, c1) at NC shifts per lane (its two
 // columns u, e and v, f up to a common scale) and the sign changes of the
 // column that starts with u = 0 (v), by which those of any state that enters
@@ -958,23 +1058,52 @@ __device__ __forceinline__ void count_segment(const Panel& P, const double* __re
                         const double un = fma(m[0], u[n], m[1] * e[n]), vn = fma(m[0], v[n], m[1] * f[n]);
                         e[n] = fma(m[2], u[n], m[3] * e[n]);
                         f[n] = fma(m[2], v[n], m[3] * f[n]);
-                        zeros[n] += block_zeros(v[n], vn, m[1], t[b][n], n2);
+                        zeros[n] += block_zeros(v[n], vn, zeros_here(m[1], t[b][n], n2));
                         u[n] = un;
                         v[n] = vn;
                     }
                 }
             }
+            rescale_columns(u, e, v, f);
+        });
+    if (zeros[0] < kByRows) return;
+    // some block has its count from its rows: the sweep again, a block at a time
 #pragma unroll
-            for (int n = 0; n < NC; ++n) {
-                const int s = rescale_shift(fmax(fabs(u[n]), fabs(v[n])), fmax(fabs(e[n]), fabs(f[n])));
-                if (s) {
-                    const double sc = pow2(-s);
-                    u[n] *= sc;
-                    e[n] *= sc;
-                    v[n] *= sc;
-                    f[n] *= sc;
+    for (int n = 0; n < NC; ++n) {
+        u[n] = f[n] = 1.0;
+        e[n] = v[n] = 0.0;
+        zeros[n] = 0;
+    }
+    ring_stream(
+        R, c1 - c0, err,
+        [&](double* dst, uint64_t* bar, int o) {
+            mbar_expect_tx(bar, kTD * 8);
+            tma_load_1d(dst, src + (size_t)(c0 + o) * kTD, kTD * 8, bar);
+        },
+        [&](const double* buf, int o) {
+            const int b0 = (c0 + o) * kPanelChunk, nb = min(kPanelChunk, P.nblk - b0);
+#pragma unroll 1
+            for (int q = 0; q < nb; ++q) {
+                const double* rec = buf + q * kRecT;
+                const int n2 = __double2loint(rec[kRecZeros]);
+#pragma unroll
+                for (int n = 0; n < NC; ++n) {
+                    const double t = sh[n].at(rec);
+                    double m[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
+                    for (int k = kPD; k >= 0; --k)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) m[j] = fma(m[j], t, rec[4 * k + j]);
+                    const int z = n2 >= kByRows ? rows_zeros<Row>(P, b0 + q, x[n]) : zeros_here(m[1], t, n2);
+                    const double un = fma(m[0], u[n], m[1] * e[n]), vn = fma(m[0], v[n], m[1] * f[n]);
+                    e[n] = fma(m[2], u[n], m[3] * e[n]);
+                    f[n] = fma(m[2], v[n], m[3] * f[n]);
+                    zeros[n] += block_zeros(v[n], vn, z);
+                    u[n] = un;
+                    v[n] = vn;
                 }
             }
+            rescale_columns(u, e, v, f);
         });
 }
 
