@@ -168,14 +168,14 @@ int launch_panel_scan(cudaStream_t st, bool wide, int P, int nz_max, ProblemInfo
                       int slots, unsigned* done, unsigned* err);
 // c_lo, c_hi, M and off of every problem, the work items (at most bis_item
 // eigenvalues, their panel in WorkItem::pad or -1) and the panels; tot =
-// {items, items, modes, items without a panel}; kErrTooMany above
+// {items, items, modes, items without a panel, 0}; kErrTooMany above
 // max_modes or cap
 int launch_panel_items(cudaStream_t st, bool wide, int P, ProblemInfo* pinfo, const int* counts, int max_modes, int bis_item,
                        WorkItem* items, int cap, PanelDesc* desc, int* tot, unsigned* err, int order);
 // expansions of the work items' panels
 int launch_panel_expand(cudaStream_t st, bool wide, int n_desc, int nz_max, const ProblemInfo* pinfo, const PanelDesc* desc,
                         const double* s, const double* w, const double* g, double* T, double* W0, double* W1);
-constexpr int kCkVals = 4;  // doubles of a coarse row's checkpoint, at most
+constexpr int kCkVals = 5;  // doubles of a coarse row's checkpoint, at most
 // full vectors: the state of a chain before a coarse row, times 2^E
 struct VecState {
     double u, e;
@@ -213,6 +213,8 @@ struct ModesArgs {
     double* vfull;              // [row][mode] per problem at vfull_off
     const long long* vfull_off;
     int* sched;  // six item counters (zeroed) or null: round-robin
+    int2* redo;   // items and lanes for launch_twist_modes, and their number (zeroed)
+    int* n_redo;
     int num_sms;
     int min_items, max_items;  // (set by the launcher) a launch returns for other item counts
     unsigned* err;
@@ -227,7 +229,10 @@ int panel_ctas_per_sm();
 // the items without panels, which launch_panel_modes leaves out: the same grid and
 // arguments, on any stream
 int launch_rows_modes(cudaStream_t st, bool wide, int grid, const ModesArgs& a, int what);
-// checkpoint slots of both on that many CTAs
+// the modes whose twist the launches above found wanting, after them (grids with
+// a few rows to a mode; elsewhere there are none)
+int launch_twist_modes(cudaStream_t st, bool wide, int grid, const ModesArgs& a);
+// checkpoint slots of all on that many CTAs
 int panel_ck_slots(int grid, bool rows);
 
 // 1-D TL; m_max: at least the most modes of a problem; scratch of tl1d_scratch

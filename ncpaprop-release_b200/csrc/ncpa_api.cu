@@ -196,7 +196,7 @@ struct ncpa_profile {
     int has_z0 = 0;
     double z_lo = 0.0, z_hi = 0.0;
     std::vector<double> h_c0, h_u, h_v;  // host copies: bounds of c_eff size the panel expansions
-    double h_wind = 0.0;                 // the largest wind speed
+    double h_c0min = 0.0, h_wind = 0.0;  // the least c0 and the largest wind speed
     int plan_refs = 0;  // plans whose graphs read this profile's arrays
 };
 
@@ -213,6 +213,7 @@ struct ncpa_modes {
     long long n_blocks = 0;  // block records of the panel expansions
     int n_desc = 0;          // panels of the work items
     bool rows = false;       // some may have none
+    bool twist = false;      // some modes may live between two coarse rows
     int Mtot = 0;
     DevBuf d_pinfo, d_kr, d_ki, d_vs, d_vr, d_vg, d_vfull, d_vfull_off;
     mutable DevBuf tl_re, tl_im, tl_inc;  // 1-D TL kept in HBM
@@ -519,7 +520,7 @@ struct Tuning {
 // allocations of some hundred MB they cost the host 350 us a solve) unless
 // own_ck is set (a captured graph must keep its addresses for good).
 struct SolveBufs {
-    DevBuf counts, items, tot, mu, sched;
+    DevBuf counts, items, tot, mu, sched, redo;
     DevBuf desc;
     DevBuf ex, ck1, cke;  // own_ck: panel expansions and checkpoints (else the context's)
     double *T = nullptr, *W0 = nullptr, *W1 = nullptr;
@@ -545,7 +546,8 @@ void prepare_solve(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, int
     b.item_cap = P * ((cap_modes + min_bis_item - 1) / min_bis_item);
     b.desc.alloc((size_t)M->n_desc * sizeof(ncpa::PanelDesc), st);
     b.items.alloc((size_t)b.item_cap * sizeof(WorkItem), st);
-    b.tot.alloc(4 * sizeof(int), st);
+    b.tot.alloc(8 * sizeof(int), st);
+    if (M->twist) b.redo.alloc((size_t)b.item_cap * sizeof(int2), st);
     b.mu.alloc(mcap * 8, st);
     b.sched.alloc(8 * sizeof(int), st);
     const size_t nT = (size_t)M->n_blocks * ncpa::kRecT, nW = (size_t)M->n_blocks * ncpa::kRecW;
@@ -687,6 +689,8 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
     a.ck_stride = ncpa::coarse_slot_elems(M->nz_max);
     a.sched = ctx->bis_order ? b.sched.as<int>() : nullptr;
     a.num_sms = ctx->num_sms;
+    a.redo = b.redo.as<int2>();
+    a.n_redo = b.tot.as<int>() + 4;
     a.err = err;
     if (prm->want_vectors) {
         a.vstate = v.state.as<ncpa::VecState>();
@@ -707,6 +711,7 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
         }
         n += ncpa::launch_panel_modes(st, wide, grid, a, what);
         if (M->rows) CK(cudaStreamWaitEvent(st, ctx->joined, 0));
+        if (M->twist && (what & 2)) n += ncpa::launch_twist_modes(st, wide, grid, a);
         check_launch(ctx, n);
     };
     if (fuse) {
@@ -844,7 +849,7 @@ std::pair<double, double> ceff_bounds(const ncpa_profile* prof, int k) {
 void layout_panels(ncpa_modes* M, const std::vector<Group>& groups, const ncpa_ess_params* prm, double slack) {
     M->n_blocks = 0;
     M->n_desc = 0;
-    M->rows = false;
+    M->rows = M->twist = false;
     const double rho = ncpa::kRhoMax, B = ncpa::kPanelMaxBlk;
     const double n_s = ncpa::kScanMax / ncpa::kScanStep;  // scan panels
     std::map<std::pair<const ncpa_profile*, int>, std::pair<double, double>> seen;
@@ -873,6 +878,9 @@ void layout_panels(ncpa_modes* M, const std::vector<Group>& groups, const ncpa_e
                 // half the window times the steepness of sigma (1, or 3 kappa_max)
                 const double win = prm->method == NCPA_METHOD_WMOD ? 3.0 / c_lo * (1.0 / c_lo - 1.0 / c_hi) : dk;
                 const double R = std::min(1.05 * slack * 0.5 * kh * kh * win, 8.0);
+                // as twist_check, for the least c_eff of any azimuth and no upper bound
+                if (0.5 * ncpa::kCkRows * kh * std::sqrt(slack) > 10.0 * std::max(g.prof->h_c0min - g.prof->h_wind, 50.0))
+                    M->twist = true;
                 const double b = ncpa::panel_min_blk(pi.nz);
                 if (R * b * b > rho) M->rows = true;
                 // items of 16 modes, the smallest a plan tries
@@ -1300,6 +1308,7 @@ void fill_profile(ncpa_ctx* ctx, ncpa_profile* P, const ncpa_profile_desc* d) {
     for (int i = 0; i < n; ++i) P->h_c0[i] = d->c0 ? d->c0[i] : std::sqrt(1.4 * d->p[i] / d->rho[i]);
     P->h_u.assign(d->u, d->u + n);
     P->h_v.assign(d->v, d->v + n);
+    P->h_c0min = *std::min_element(P->h_c0.begin(), P->h_c0.end());
     P->h_wind = 0.0;
     for (int i = 0; i < n; ++i) P->h_wind = std::max(P->h_wind, std::sqrt(d->u[i] * d->u[i] + d->v[i] * d->v[i]));
     const std::pair<DevBuf*, const double*> cols[] = {{&P->z, d->z}, {&P->u, d->u}, {&P->v, d->v},

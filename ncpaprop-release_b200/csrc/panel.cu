@@ -1282,7 +1282,7 @@ __global__ void __launch_bounds__(kItemThreads) k_panel_items(int P, ProblemInfo
         tot[0] = min(base, cap);
         tot[1] = min(base, cap);
         tot[2] = base_m;
-        tot[3] = 0;
+        tot[3] = tot[4] = 0;
     }
 }
 
@@ -1784,6 +1784,21 @@ __device__ __forceinline__ void rows_down(const double* __restrict__ rows, int i
     }
 }
 
+// Grids so coarse that a mode can live between two coarse rows: beyond it a chain
+// picks up the growing solution, by e^g eps of the mode after a decay of e^-g.
+// The coarse twist leaves at most half of kCkRows for that; up to g = 10 it costs
+// 2e-12 of the mode's top.  Above, the twist is checked: z solves the rows but for
+// gamma at the twist, and |gamma| / |z| is about the eigenvalue's error over
+// z_r / |z|.  From kTwist on (the twist a factor of some 1e4 below the top, on
+// grids where modes live in a few rows any row at all) the mode is redone with the
+// best of all rows (k_twist_modes).
+constexpr double kTwist = 1e-9;
+__device__ __forceinline__ bool twist_check(const ProblemInfo& pi) {
+    const double c0 = __longlong_as_double((long long)pi.ceffmin_bits), c1 = __longlong_as_double((long long)pi.ceffmax_bits);
+    const double g = 0.5 * kCkRows * (pi.omega * pi.dz);
+    return g * g * (1.0 / (c0 * c0) - 1.0 / (c1 * c1)) > 100.0;
+}
+
 // v = m 2^E with |m| in [1, 2)
 __device__ __forceinline__ void normalize(double& v, int& E) {
     const int e = biased_exp(v);
@@ -1962,9 +1977,10 @@ __device__ __noinline__ RowVals rows_vector(const ModesArgs& A, const ProblemInf
         if (i % kCkRows) return;
         const double v = kDown ? um : u, e = kDown ? um - u : u - um;
         const size_t c = (size_t)(i / kCkRows);
-        double* o = ck + c * (1 + kN) * 32 + lane;
+        double* o = ck + c * (2 + kN) * 32 + lane;
         if (kPart != 2) {
             o[0] = v;
+            o[32 * (1 + kN)] = e;
             cke[c * 32 + lane] = E;
         }
         if (Q::norm) o[32] = sum[0];
@@ -2019,6 +2035,7 @@ __device__ __forceinline__ void vector_half(const ModesArgs& A, const ProblemInf
     constexpr int kN = kSums<Row, NW>;
     const int lane = threadIdx.x & 31;
     const int nz = P.nz, isrc = pi.isrc, ircv = pi.ircv;
+    const bool check = twist_check(pi);
     const double rinv = 1.0 / P.r;
     const typename Row::Shift sh(P, mu);
     VecChain<Row, NW, kPart> C;
@@ -2029,9 +2046,10 @@ __device__ __forceinline__ void vector_half(const ModesArgs& A, const ProblemInf
     auto keep = [&](int a, double sgn) {  // state before row a
         if (a % kCkRows) return;
         const size_t c = (size_t)(a / kCkRows);
-        double* o = ck + c * (1 + kN) * 32 + lane;
+        double* o = ck + c * (2 + kN) * 32 + lane;
         if (kPart != 2) {
             o[0] = C.u;
+            if (check) o[32 * (1 + kN)] = C.e;
             cke[c * 32 + lane] = C.E;
         }
         if (Q::norm) o[32] = C.sum(0, rinv, sgn);
@@ -2114,84 +2132,65 @@ struct TwistAt {
     int Eu, Eb, r;
 };
 
-// Full vectors on grids so coarse that a mode can live between two coarse
-// rows: beyond it a chain picks up the growing solution, by e^{g} eps of the
-// mode after a decay of g.  The coarse twist leaves at most half a chunk of
-// that; up to g = 10 it costs 2e-12 and the search below is left out.
-__device__ __forceinline__ bool fine_twist_needed(const ProblemInfo& pi) {
-    const double c0 = __longlong_as_double((long long)pi.ceffmin_bits), c1 = __longlong_as_double((long long)pi.ceffmax_bits);
-    const double kh = pi.omega * pi.dz, g = 0.5 * kCkRows * kh;
-    return g * g * (1.0 / (c0 * c0) - 1.0 / (c1 * c1)) > 100.0;
-}
+// where a mode's chains end at the source and receiver rows, from below and above
+struct ModeEnds {
+    double us, ur, bs, br;
+    int Eus, Eur, Ebs, Ebr;
+};
 
-// the row with the largest |u b| in the two chunks around coarse row c0 (the
-// lowest of equal ones), and the sums up to it.  vfull's rows hold b meanwhile.
-template <class Row, int NW>
-__device__ __noinline__ void fine_twist(const ModesArgs& A, const ProblemInfo& pi, const Panel& P, const WorkItem& w,
-                                        double mu, double* const (&cks)[2], int c0, const VecState* st,
-                                        TwistAt<kSums<Row, NW>>& W) {
+// the values of mode i from its chains; returns sum z^2 / z_r^2
+template <class Row, int NW, bool kV>
+__device__ __forceinline__ double finish_mode(const ModesArgs& A, const ProblemInfo& pi, int i, bool write, double mu,
+                                              const TwistAt<kSums<Row, NW>>& tw, const ModeEnds& v) {
     constexpr int kN = kSums<Row, NW>;
-    const int lane = threadIdx.x & 31, nz = P.nz, M = pi.M, nc = (nz + kCkRows - 1) / kCkRows;
-    double* tmp = A.vfull + A.vfull_off[w.problem] + w.j0 + lane;
-    const VecState* sd = st + (long long)nc * M;
-    TwistKey K{0.0, 0, 0};
-    for (int c = max(c0 - 1, 0); c <= c0; ++c) {
-        const int a = c * kCkRows, end = min(nz, a + kCkRows);
-        VecState v{0.0, -1.0, 0, 0};
-        if (c + 1 < nc) v = sd[(long long)(c + 1) * M];
-        double u = v.u, e = v.e;
-        for (int i = end - 1; i >= a; --i) {
-            u -= e;
-            e = fma(Row::sigma(P.rows, i, mu), u, e);
-            tmp[(long long)i * M] = u;
-        }
-        const VecState q = st[(long long)c * M];
-        u = q.u;
-        e = q.e;
-        for (int i = a; i < end; ++i) {
-            K.take(u, q.E, tmp[(long long)i * M], v.E, i);
-            e = fma(-Row::sigma(P.rows, i, mu), u, e);
-            u += e;
-        }
-    }
-    if (K.m == 0.0) return;
-    const int c = K.c / kCkRows, a = c * kCkRows, end = min(nz, a + kCkRows);
-    const double* wp = A.w + pi.w_off;
-    const double* gp = NW > 1 && A.g ? A.g + pi.s_off : nullptr;
-    auto add = [&](double (&s)[kN], int i, double x) {
-        const double x2 = x * x;
-        if (Row::kUnitNorm) s[0] += x2;
-        s[kN - NW] = fma(wp[i], x2, s[kN - NW]);
-        if (NW > 1) s[kN - 1] = fma(gp ? gp[i] : 1.0, x2, s[kN - 1]);
+    double ut = tw.u, bt = tw.b;
+    int Eut = tw.Eu, Ebt = tw.Eb;
+    normalize(ut, Eut);
+    normalize(bt, Ebt);
+    const int eut = Eut - tw.Eu, ebt = Ebt - tw.Eb;  // exponents of u and b themselves
+    const double iu2 = 1.0 / (ut * ut), ib2 = 1.0 / (bt * bt);
+    auto total = [&](int n) {  // sum over all rows in units of z_r^2
+        double x = tw.su[n], y = tw.sb[n];
+        int ex = 0, ey = 0;
+        normalize(x, ex);
+        normalize(y, ey);
+        // both sums were taken at the exponents of u and b at the twist
+        return x * iu2 * pow2(ex - 2 * eut) + y * ib2 * pow2(ey - 2 * ebt);
     };
-    W.r = K.c;
-    W.Eb = 0;
-#pragma unroll
-    for (int n = 0; n < kN; ++n) {
-        W.su[n] = cks[0][((size_t)c * (1 + kN) + 1 + n) * 32 + lane];
-        W.sb[n] = c + 1 < nc ? __ldcg(cks[1] + ((size_t)(c + 1) * (1 + kN) + 1 + n) * 32 + lane) : 0.0;
+    const int r = tw.r, isrc = pi.isrc, ircv = pi.ircv;
+    const int n1 = Row::kUnitNorm ? 0 : kN - 1, nw = kN - NW;
+    const double nrm = total(n1);
+    const double f2 = Row::kUnitNorm ? 1.0 : 1.0 / (1.0 + (mu / pi.dz) * (mu / pi.dz));
+    const double scale = Row::kUnitNorm ? 1.0 / sqrt(nrm * pi.dz) : sqrt(f2 / (nrm * pi.dz));
+    const double zs = (isrc <= r) ? (v.us / ut) * pow2(v.Eus - Eut) : (v.bs / bt) * pow2(v.Ebs - Ebt);
+    const double zr = (ircv <= r) ? (v.ur / ut) * pow2(v.Eur - Eut) : (v.br / bt) * pow2(v.Ebr - Ebt);
+    const double absorption = total(nw) / nrm * f2;
+    const double ks = Row::kUnitNorm ? sqrt(mu / (pi.dz * pi.dz)) : mu / pi.dz;
+    const auto kp = csqrt_principal(ks * ks, absorption);
+    if (write) {
+        A.kr[i] = kp.real();
+        A.ki[i] = kp.imag();
+        A.vs[i] = zs * scale;
+        A.vr[i] = zr * scale;
+        if (kV) A.vtwist[i] = VecTwist{mu, scale / ut, scale / bt, Eut, Ebt, r, 0};
+        if (Row::kUnitNorm && NW > 1) {
+            const double vph = pi.omega / kp.real();
+            A.vg[i] = 1.0 / (vph * (total(nw + 1) / nrm));
+        } else if (A.vg) {
+            A.vg[i] = 0.0;
+        }
     }
-    if (c + 1 < nc) W.Eb = sd[(long long)(c + 1) * M].E;
-    for (int i = end - 1; i >= W.r; --i) add(W.sb, i, W.b = tmp[(long long)i * M]);
-    const VecState q = st[(long long)c * M];
-    double u = q.u, e = q.e;
-    for (int i = a; i < W.r; ++i) {
-        add(W.su, i, u);
-        e = fma(-Row::sigma(P.rows, i, mu), u, e);
-        u += e;
-    }
-    W.u = u;
-    W.Eu = q.E;
+    return nrm;
 }
 
 template <class Row, int NW, bool kV, int W, bool kRows>
 __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemInfo& pi, const Panel& P,
-                                             const WorkItem& w, double mu, PRing& R, Team<W>& pr, bool split,
-                                             double* __restrict__ ck, int* __restrict__ cke) {
+                                             const WorkItem& w, int it, double mu, PRing& R, Team<W>& pr,
+                                             bool split, double* __restrict__ ck, int* __restrict__ cke) {
     constexpr int kN = kSums<Row, NW>;
     const int lane = threadIdx.x & 31, half = pr.half & 1;
     const int nc = (P.nz + kCkRows - 1) / kCkRows;
-    double* cks[2] = {ck, ck + A.ck_stride * (1 + kN)};
+    double* cks[2] = {ck, ck + A.ck_stride * (2 + kN)};
     int* ckes[2] = {cke, cke + A.ck_stride};
     double vs, vr;
     int Es, Er;
@@ -2250,7 +2249,7 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
     const int c0 = half ? nc / 2 : 0, c1 = half || W == 1 ? nc : nc / 2;
 #pragma unroll 4
     for (int c = c0; c < c1; ++c) {
-        const size_t o = (size_t)c * (1 + kN) * 32 + lane, i = (size_t)c * 32 + lane;
+        const size_t o = (size_t)c * (2 + kN) * 32 + lane, i = (size_t)c * 32 + lane;
         K.take(__ldcg(cks[0] + o), __ldcg(ckes[0] + i), __ldcg(cks[1] + o), __ldcg(ckes[1] + i), c);
     }
     if (half) {
@@ -2264,13 +2263,19 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
         const int E = __double2hiint(ec);
         if (m > 0.0 && (K.m == 0.0 || E > K.E || (E == K.E && m > K.m))) K.c = __double2loint(ec);
     }
-    const double us = vs, ur = vr, bs = W == 1 ? above.vs : X.v[tb][1][0][lane];
-    const double br = W == 1 ? above.vr : X.v[tb][1][1][lane];
+    ModeEnds ends;
+    ends.us = vs;
+    ends.ur = vr;
+    ends.Eus = Es;
+    ends.Eur = Er;
+    ends.bs = W == 1 ? above.vs : X.v[tb][1][0][lane];
+    ends.br = W == 1 ? above.vr : X.v[tb][1][1][lane];
     const double eb = W == 1 ? __hiloint2double(above.Es, above.Er) : X.v[tb][1][2][lane];
-    const int Eus = Es, Eur = Er, Ebs = __double2hiint(eb), Ebr = __double2loint(eb);
+    ends.Ebs = __double2hiint(eb);
+    ends.Ebr = __double2loint(eb);
     TwistAt<kN> tw;
     tw.r = K.c * kCkRows;
-    const size_t o = (size_t)K.c * (1 + kN) * 32 + lane;
+    const size_t o = (size_t)K.c * (2 + kN) * 32 + lane;
     tw.u = __ldcg(cks[0] + o);
     tw.b = __ldcg(cks[1] + o);
     tw.Eu = __ldcg(ckes[0] + (size_t)K.c * 32 + lane);
@@ -2280,47 +2285,11 @@ __device__ __forceinline__ void panel_vector(const ModesArgs& A, const ProblemIn
         tw.su[n] = __ldcg(cks[0] + o + 32 * (1 + n));
         tw.sb[n] = __ldcg(cks[1] + o + 32 * (1 + n));
     }
-    if (kV && fine_twist_needed(pi)) {
-        if (lane < w.m) fine_twist<Row, NW>(A, pi, P, w, mu, cks, K.c, st, tw);
-        __syncwarp();
-    }
-    double ut = tw.u, bt = tw.b;
-    int Eut = tw.Eu, Ebt = tw.Eb;
-    normalize(ut, Eut);
-    normalize(bt, Ebt);
-    const int eut = Eut - tw.Eu, ebt = Ebt - tw.Eb;  // exponents of u and b themselves
-    const double iu2 = 1.0 / (ut * ut), ib2 = 1.0 / (bt * bt);
-    auto total = [&](int n) {  // sum over all rows in units of z_r^2
-        double x = tw.su[n], y = tw.sb[n];
-        int ex = 0, ey = 0;
-        normalize(x, ex);
-        normalize(y, ey);
-        // both sums were taken at the exponents of u and b at the twist
-        return x * iu2 * pow2(ex - 2 * eut) + y * ib2 * pow2(ey - 2 * ebt);
-    };
-    const int r = tw.r, isrc = pi.isrc, ircv = pi.ircv;
-    const int n1 = Row::kUnitNorm ? 0 : kN - 1, nw = kN - NW;
-    const double nrm = total(n1);  // sum z^2 / z_r^2
-    const double f2 = Row::kUnitNorm ? 1.0 : 1.0 / (1.0 + (mu / pi.dz) * (mu / pi.dz));
-    const double scale = Row::kUnitNorm ? 1.0 / sqrt(nrm * pi.dz) : sqrt(f2 / (nrm * pi.dz));
-    const double zs = (isrc <= r) ? (us / ut) * pow2(Eus - Eut) : (bs / bt) * pow2(Ebs - Ebt);
-    const double zr = (ircv <= r) ? (ur / ut) * pow2(Eur - Eut) : (br / bt) * pow2(Ebr - Ebt);
-    const double absorption = total(nw) / nrm * f2;
-    const double ks = Row::kUnitNorm ? sqrt(mu / (pi.dz * pi.dz)) : mu / pi.dz;
-    const auto kp = csqrt_principal(ks * ks, absorption);
-    if (lane < w.m) {
-        const int i = pi.off + w.j0 + lane;
-        A.kr[i] = kp.real();
-        A.ki[i] = kp.imag();
-        A.vs[i] = zs * scale;
-        A.vr[i] = zr * scale;
-        if (kV) A.vtwist[i] = VecTwist{mu, scale / ut, scale / bt, Eut, Ebt, r, 0};
-        if (Row::kUnitNorm && NW > 1) {
-            const double vph = pi.omega / kp.real();
-            A.vg[i] = 1.0 / (vph * (total(nw + 1) / nrm));
-        } else if (A.vg) {
-            A.vg[i] = 0.0;
-        }
+    const double nrm = finish_mode<Row, NW, kV>(A, pi, pi.off + w.j0 + lane, lane < w.m, mu, tw, ends);
+    if (A.redo && twist_check(pi)) {
+        const double g = __ldcg(cks[1] + o + 32 * (1 + kN)) / tw.b - __ldcg(cks[0] + o + 32 * (1 + kN)) / tw.u;
+        const unsigned bad = __ballot_sync(0xffffffffu, lane < w.m && !(g * g <= kTwist * kTwist * nrm));
+        if (bad && lane == 0) A.redo[atomicAdd(A.n_redo, 1)] = make_int2(it, (int)bad);
     }
 }
 
@@ -2350,7 +2319,7 @@ __global__ void __launch_bounds__(kPWarps * 32, kPanelCtas) k_panel_modes(const 
     pr.area = reinterpret_cast<double*>(smem_raw) + (size_t)pr.id * W * pr.stride;
     pr.turn = 0;
     const long long gp = (long long)blockIdx.x * kTeams + pr.id;
-    double* ck = A.ck_u + gp * 2 * A.ck_stride * (1 + kSums<Row, NW>);
+    double* ck = A.ck_u + gp * 2 * A.ck_stride * (2 + kSums<Row, NW>);
     int* cke = A.ck_e + gp * 2 * A.ck_stride;
     // first items: one to the first team of as many CTAs as there are SMs (which
     // start on different ones), then to their second teams, then to the next
@@ -2382,7 +2351,7 @@ __global__ void __launch_bounds__(kPWarps * 32, kPanelCtas) k_panel_modes(const 
         } else if (lane < w.m) {
             x = A.mu[pi.off + w.j0 + lane];
         }
-        if (kDo & 2) panel_vector<Row, NW, kV, W, false>(A, pi, P, w, x, R, pr, n_items <= A.num_sms, ck, cke);
+        if (kDo & 2) panel_vector<Row, NW, kV, W, false>(A, pi, P, w, it, x, R, pr, n_items <= A.num_sms, ck, cke);
     }
 }
 
@@ -2411,7 +2380,7 @@ __global__ void __launch_bounds__(kPWarps * 32, W == 1 ? kRowsCtas : kPanelCtas)
     pr.area = reinterpret_cast<double*>(smem_raw) + (size_t)pr.id * W * pr.stride;
     pr.turn = 0;
     const long long slot = (long long)blockIdx.x * kTeams + pr.id;
-    double* ck = A.ck_u + slot * 2 * A.ck_stride * (1 + kSums<Row, NW>);
+    double* ck = A.ck_u + slot * 2 * A.ck_stride * (2 + kSums<Row, NW>);
     int* cke = A.ck_e + slot * 2 * A.ck_stride;
     const int n_teams = gridDim.x * kTeams;
     int next = pr.id * gridDim.x + blockIdx.x;  // first items on different SMs
@@ -2437,7 +2406,188 @@ __global__ void __launch_bounds__(kPWarps * 32, W == 1 ? kRowsCtas : kPanelCtas)
         } else if (lane < w.m) {
             x = A.mu[pi.off + w.j0 + lane];
         }
-        if (kDo & 2) panel_vector<Row, NW, kV, W, true>(A, pi, P, w, x, R, pr, false, ck, cke);
+        if (kDo & 2) panel_vector<Row, NW, kV, W, true>(A, pi, P, w, it, x, R, pr, false, ck, cke);
+    }
+}
+
+// a chain's state normalised: the larger of |u|, |e| in [1, 2)
+struct RowState {
+    double u, e;
+    int E;
+    __device__ __forceinline__ void normal() {
+        const int x = max(biased_exp(u), biased_exp(e));
+        if (x == 0 || x == 1023) return;
+        const double sc = pow2(1023 - x);
+        u *= sc;
+        e *= sc;
+        E += x - 1023;
+    }
+};
+
+// The modes whose coarse twist was not good enough (redo: item and lanes), a CTA
+// to an item: both chains by rows, on a warp each, then |u b| row by row, 32 rows
+// of b in shared memory at a time, and the values from the row where it is
+// largest.  Rows of the two chunks at the coarse twist while gamma is below 1e-7
+// of |z|; from there on the decay to the coarse rows may be past the chains'
+// rounding, where |u b| is level and its largest value tells nothing, and the
+// four warps go through all chunks.  A serial chain over the rows, some 30 cycles
+// each: 100 us for 2500 rows.
+template <class Row, int NW, bool kV>
+__global__ void __launch_bounds__(kPWarps * 32) k_twist_modes(const __grid_constant__ ModesArgs A) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    constexpr int kSl = kTD + NW * kWD, kN = kSums<Row, NW>, kSeg = 32, kSegs = kCkRows / kSeg;
+    static_assert(kSeg * 32 <= kPBuf * kSl, "a segment fits the ring");
+    __shared__ RowVals box[32];
+    __shared__ TwistKey keys[kPWarps][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int n = *A.n_redo;
+    if (blockIdx.x >= n) return;
+    PRing R = make_ring(smem_raw, wid, kSl);
+    double* cks[2];
+    int* ckes[2];
+    for (int h = 0; h < 2; ++h) {
+        cks[h] = A.ck_u + (2ll * blockIdx.x + h) * A.ck_stride * (2 + kN);
+        ckes[h] = A.ck_e + (2ll * blockIdx.x + h) * A.ck_stride;
+    }
+    for (int k = blockIdx.x; k < n; k += gridDim.x) {
+        const int2 job = A.redo[k];
+        const WorkItem w = A.items[job.x];
+        const ProblemInfo& pi = A.pinfo[w.problem];
+        PanelDesc d{};
+        d.xc = Row::lo(pi);
+        const Panel P = panel_of<Row>(pi, d, A.rows);
+        const int nz = P.nz, nc = (nz + kCkRows - 1) / kCkRows, i = pi.off + w.j0 + lane;
+        const bool mine = ((unsigned)job.y >> lane) & 1u;
+        const double mu = lane < w.m ? A.mu[i] : P.xc;
+        VecState* st = nullptr;
+        if (kV && mine) st = A.vstate + A.vstate_off[w.problem] + w.j0 + lane + (long long)(wid & 1) * nc * pi.M;
+        RowVals below{};
+        if (wid == 0) {
+            below = rows_vector<Row, NW, kV, 0, false>(A, pi, P, mu, st, R, cks[0], ckes[0]);
+            R.loads = below.loads;
+        } else if (wid == 1) {
+            box[lane] = rows_vector<Row, NW, kV, 0, true>(A, pi, P, mu, st, R, cks[1], ckes[1]);
+            R.loads = box[lane].loads;
+        }
+        __syncthreads();
+        auto at = [&](int h, int c) { return cks[h] + (size_t)c * (2 + kN) * 32 + lane; };
+        auto state = [&](int h, int c) {
+            const double* o = at(h, c);
+            return RowState{o[0], o[32 * (1 + kN)], ckes[h][(size_t)c * 32 + lane]};
+        };
+        auto up = [&](RowState& S, int row) {
+            S.e = fma(-Row::sigma(P.rows, row, mu), S.u, S.e);
+            S.u += S.e;
+        };
+        auto down = [&](RowState& S, int row) {
+            S.u -= S.e;
+            S.e = fma(Row::sigma(P.rows, row, mu), S.u, S.e);
+        };
+        TwistKey K{0.0, 0, 0};
+        for (int c = 0; c < nc; ++c) {
+            const RowState U = state(0, c), S = state(1, c);
+            K.take(U.u, U.E, S.u, S.E, c);
+        }
+        const int c0 = K.c;
+        bool all;
+        {
+            const RowState U = state(0, c0), S = state(1, c0);
+            const int q = Row::kUnitNorm ? 1 : kN;  // the norm
+            const double g = S.e / S.u - U.e / U.u;
+            const double nrm = at(0, c0)[32 * q] / (U.u * U.u) + at(1, c0)[32 * q] / (S.u * S.u);
+            all = __any_sync(0xffffffffu, mine && !(g * g <= 1e-14 * nrm));
+        }
+        double* buf = R.buf + lane;
+        K = TwistKey{0.0, 0, 0};
+        for (int q = wid; q < (all ? nc : 2); q += kPWarps) {
+            const int c = all ? q : max(c0 - 1, 0) + min(q, c0);
+            const int a = c * kCkRows, end = min(nz, a + kCkRows);
+            RowState S = c + 1 < nc ? state(1, c + 1) : RowState{0.0, -1.0, 0}, behind[kSegs];
+            S.normal();
+#pragma unroll
+            for (int s = kSegs - 1; s >= 0; --s) {  // b behind each segment
+                behind[s] = S;
+#pragma unroll 8
+                for (int row = min(end, a + (s + 1) * kSeg) - 1; row >= a + s * kSeg; --row) down(S, row);
+                S.normal();
+            }
+            RowState U = state(0, c);
+            U.normal();
+#pragma unroll
+            for (int s = 0; s < kSegs; ++s) {
+                const int lo = a + s * kSeg, hi = min(end, lo + kSeg);
+                S = behind[s];
+#pragma unroll 8
+                for (int row = hi - 1; row >= lo; --row) {
+                    down(S, row);
+                    buf[(row - lo) * 32] = S.u;
+                }
+#pragma unroll 4
+                for (int row = lo; row < hi; ++row) {
+                    K.take(U.u, U.E, buf[(row - lo) * 32], behind[s].E, row);
+                    up(U, row);
+                }
+                U.normal();
+            }
+        }
+        keys[wid][lane] = K;
+        __syncthreads();
+        if (wid == 0) {
+            for (int q = 1; q < kPWarps; ++q) {
+                const TwistKey& o = keys[q][lane];
+                if (o.m > 0.0 && (K.m == 0.0 || o.E > K.E || (o.E == K.E && (o.m > K.m || (o.m == K.m && o.c < K.c)))))
+                    K = o;
+            }
+        }
+        const RowVals above = box[lane];
+        __syncthreads();  // the box and the keys are free
+        if (wid == 0 && mine && K.m > 0.0) {
+            TwistAt<kN> tw;
+            const int c = K.c / kCkRows, a = c * kCkRows, end = min(nz, a + kCkRows);
+            const double* wp = A.w + pi.w_off;
+            const double* gp = NW > 1 && A.g ? A.g + pi.s_off : nullptr;
+            auto add = [&](double (&x)[kN], RowState& S, int row) {
+                const double z2 = S.u * S.u;
+                if (Row::kUnitNorm) x[0] += z2;
+                x[kN - NW] = fma(wp[row], z2, x[kN - NW]);
+                if (NW > 1) x[kN - 1] = fma(gp ? gp[row] : 1.0, z2, x[kN - 1]);
+            };
+            auto fold = [&](double (&x)[kN], RowState& S, int row) {  // the squares stay finite
+                const int big = max(biased_exp(S.u), biased_exp(S.e)) - 1023;
+                if ((row & 7) || big <= 100) return;
+                const double sc = pow2(-big);
+                S.u *= sc;
+                S.e *= sc;
+                S.E += big;
+                for (int q = 0; q < kN; ++q) x[q] *= sc * sc;
+            };
+            tw.r = K.c;
+            RowState S{0.0, -1.0, 0};
+            if (c + 1 < nc) S = state(1, c + 1);
+#pragma unroll
+            for (int q = 0; q < kN; ++q) {
+                tw.su[q] = cks[0][((size_t)c * (2 + kN) + 1 + q) * 32 + lane];
+                tw.sb[q] = c + 1 < nc ? cks[1][((size_t)(c + 1) * (2 + kN) + 1 + q) * 32 + lane] : 0.0;
+            }
+            for (int row = end - 1; row >= tw.r; --row) {
+                down(S, row);
+                add(tw.sb, S, row);
+                if (row > tw.r) fold(tw.sb, S, row);
+            }
+            tw.b = S.u;
+            tw.Eb = S.E;
+            S = state(0, c);
+            for (int row = a; row < tw.r; ++row) {
+                add(tw.su, S, row);
+                up(S, row);
+                fold(tw.su, S, row);
+            }
+            tw.u = S.u;
+            tw.Eu = S.E;
+            const ModeEnds ends{below.vs, below.vr, above.vs, above.vr, below.Es, below.Er, above.Es, above.Er};
+            finish_mode<Row, NW, kV>(A, pi, i, true, mu, tw, ends);
+        }
+        __syncthreads();  // and the checkpoints
     }
 }
 
@@ -2789,6 +2939,23 @@ int launch_panel_fill(cudaStream_t st, bool wide, int P, int nz_max, int m_max, 
         n += 2;
     }
     return n;
+}
+
+namespace {
+template <class Row, int NW, bool kV>
+int twist_run(cudaStream_t st, int grid, const ModesArgs& a) {
+    const size_t sm = kRingBytes<kTD + NW * kWD>;
+    auto* f = k_twist_modes<Row, NW, kV>;
+    cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    f<<<std::min(panel_slots(grid) / 2, a.item_cap), kPWarps * 32, sm, st>>>(a);
+    return 1;
+}
+}  // namespace
+
+int launch_twist_modes(cudaStream_t st, bool wide, int grid, const ModesArgs& a) {
+    if (wide) return a.vstate ? twist_run<WmodPanel, 2, true>(st, grid, a) : twist_run<WmodPanel, 2, false>(st, grid, a);
+    if (a.g) return a.vstate ? twist_run<EssPanel, 2, true>(st, grid, a) : twist_run<EssPanel, 2, false>(st, grid, a);
+    return a.vstate ? twist_run<EssPanel, 1, true>(st, grid, a) : twist_run<EssPanel, 1, false>(st, grid, a);
 }
 
 int launch_rows_modes(cudaStream_t st, bool wide, int grid, const ModesArgs& a, int what) {
