@@ -15,9 +15,9 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -46,11 +46,22 @@ public:
     }
 
     // Copies the parts after what the stream holds, and waits for all of it
-    // (the stream is idle on return).
+    // (the stream is idle on return, after errors and exceptions too: nothing
+    // writes to the caller's memory or the ring any more).
     cudaError_t run(int device, cudaStream_t st, const Part* parts, size_t n) {
+        struct Wait {
+            cudaStream_t st;
+            bool done = false;
+            cudaError_t now() {
+                done = true;
+                return cudaStreamSynchronize(st);
+            }
+            ~Wait() {
+                if (!done) cudaStreamSynchronize(st);
+            }
+        } wait{st};
         std::vector<Chunk> todo;
         std::vector<const void*> dev;
-        size_t total = 0;
         for (size_t i = 0; i < n; ++i) {
             const Part& p = parts[i];
             if (!p.bytes) continue;
@@ -66,7 +77,6 @@ public:
             for (size_t o = 0; o < p.bytes; o += kChunk)
                 todo.push_back({static_cast<char*>(p.dst) + o, static_cast<const char*>(p.src) + o,
                                 std::min(kChunk, p.bytes - o), nullptr});
-            total += p.bytes;
         }
         for (size_t i = 0; i < todo.size();) {
             // as many chunks as the ring holds; few small ones share one wait
@@ -83,7 +93,7 @@ public:
                                                  cudaMemcpyDeviceToHost, st);
                 if (rc == cudaSuccess && !shared) rc = event(k - i, &todo[k].ev);
                 if (rc == cudaSuccess && !shared) rc = cudaEventRecord(todo[k].ev, st);
-                if (rc != cudaSuccess) return drain(st, rc);
+                if (rc != cudaSuccess) return rc;
             }
             if (shared) {
                 const cudaError_t rc = cudaStreamSynchronize(st);
@@ -95,11 +105,11 @@ public:
                 job->chunks.assign(todo.begin() + i, todo.begin() + e);
                 finish(job);
                 const cudaError_t rc = static_cast<cudaError_t>(job->err.load());
-                if (rc != cudaSuccess) return drain(st, rc);
+                if (rc != cudaSuccess) return rc;
             }
             i = e;
         }
-        return cudaStreamSynchronize(st);
+        return wait.now();
     }
 
     // The same between host arrays.
@@ -164,10 +174,6 @@ private:
         *ev = ev_[i];
         return cudaSuccess;
     }
-    static cudaError_t drain(cudaStream_t st, cudaError_t rc) {
-        cudaStreamSynchronize(st);  // the ring is free for the next copy
-        return rc;
-    }
     // runs the job on this thread and the helpers
     void finish(const std::shared_ptr<Job>& job) {
         post(job);
@@ -179,7 +185,7 @@ private:
             const int n = std::min<int>(kHelpers, (int)std::thread::hardware_concurrency() - 1);
             try {
                 for (int i = 0; i < n; ++i) helpers_.emplace_back([this] { help(); });
-            } catch (const std::system_error&) {
+            } catch (const std::exception&) {
                 // fewer helpers, or none: the caller copies on its own
             }
         }
