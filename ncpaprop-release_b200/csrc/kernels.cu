@@ -562,7 +562,6 @@ __global__ void k_window(int P, ProblemInfo* __restrict__ pinfo, int wkb, int wv
     pinfo[p].hi = hi;
     pinfo[p].used_wkb = wkb ? 1 : 0;
     pinfo[p].n_scan = kScanDefault;
-    pinfo[p].n_scan_raw = kScanDefault;
     pinfo[p].m_est = -1.f;
 }
 

@@ -34,7 +34,6 @@ struct ProblemInfo {
     int used_wkb;
     int wkb_trial;         // first WKB trial that ends the walk (kWkbNone before it is taken)
     int n_scan;            // shifts of the isolation scan (<= kScanMax)
-    int n_scan_raw;        // the size estimated from the problem alone (before the batch-wide trim)
     float m_est;           // estimated mode count in [lo, hi] (-1: not estimated)
     int upp, sp_blk;       // the scan's panels (panel.cu): scan units per panel and rows per block (0: raw rows)
     int item0;             // first work item
@@ -81,7 +80,7 @@ struct PanelDesc {
 };
 
 constexpr int kScanMax = 512;      // count slots per problem of the isolation scan
-constexpr int kScanStep = 64;      // shifts per scan unit (one warp, two per lane)
+constexpr int kScanStep = 64;      // shifts per scan unit (four warps, each a quarter of the rows, two shifts per lane)
 constexpr int kScanDefault = 256;  // shifts per problem unless the scan sizes them (wide-angle rows)
 constexpr int kChunk = 1024;      // doubles per TMA chunk of the diagonal
 constexpr int kBlk = 16;          // rows between rescalings in k_eigvec
@@ -161,11 +160,10 @@ int launch_eigvec(cudaStream_t st, int grid, const EigvecArgs& a);
 // the wide-angle rows (mu = kappa = h k; W1 for a weight of ones).  T: block
 // transfer matrices (kRecT doubles a record), W0, W1: their derivatives for the
 // weights w and, for group speeds, g (kRecW doubles).
-// Isolation scan: sizes, batch-wide trim (slots: warp schedulers of the device,
-// 0 for none; done: a zeroed counter), expansions and Sturm counts at
-// pinfo[p].n_scan points, counts[p kScanMax + t]
+// Isolation scan: sizes, expansions and Sturm counts at pinfo[p].n_scan points,
+// counts[p kScanMax + t]
 int launch_panel_scan(cudaStream_t st, bool wide, int P, int nz_max, ProblemInfo* pinfo, const double* s, double* T, int* counts,
-                      int slots, unsigned* done, unsigned* err);
+                      unsigned* err);
 // c_lo, c_hi, M and off of every problem, the work items (at most bis_item
 // eigenvalues, their panel in WorkItem::pad or -1) and the panels; tot =
 // {items, items, modes, items without a panel, 0}; kErrTooMany above

@@ -138,9 +138,6 @@ struct ncpa_ctx {
     // modal sum of ncpa_tl_2d (the front ends' tloss_2d.nm): NCPA_SUM_FP64,
     // or NCPA_SUM_TC_GUARDED with NCPA_TL2D_SUM=3
     int tl2d_method = NCPA_SUM_FP64;
-    // isolation scan trimmed to a whole number of units per warp scheduler;
-    // NCPA_SCAN_TRIM=0 keeps every problem's own estimate
-    bool scan_trim = true;
     bool fuse_solve = true;        // fused bisection + eigenvector launch; NCPA_FUSE_SOLVE=0 turns it off
     double* h_pin = nullptr;       // small pinned host buffer for scalars read back per solve
     int* h_tot = nullptr;          // pinned: item and mode totals of a device-built solve, status word at [8]
@@ -571,9 +568,6 @@ void prepare_solve(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, int
     ce.alloc(need * 4, st);
 }
 
-// warp schedulers of the device for the scan trim (0: no trim)
-int scan_slots(const ncpa_ctx* ctx) { return ctx->scan_trim ? 4 * ctx->num_sms : 0; }
-
 // after the work items: a problem above max_modes is an error
 void check_mode_limit(ncpa_ctx* ctx, const ncpa_modes* M, unsigned err) {
     if (!(err & ncpa::kErrTooMany)) return;
@@ -646,10 +640,9 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
                                           prm->c_min, prm->c_max, err));
     tm.mark("window");
     // ---- isolation scan ----
-    // item counters of the launches below and the scan's block counter
+    // item counters of the launches below
     CK(cudaMemsetAsync(b.sched.p, 0, 8 * sizeof(int), st));
-    check_launch(ctx, ncpa::launch_panel_scan(st, wide, P, M->nz_max, d_pinfo, s, b.T, b.counts.as<int>(),
-                                              scan_slots(ctx), b.sched.as<unsigned>() + 7, err));
+    check_launch(ctx, ncpa::launch_panel_scan(st, wide, P, M->nz_max, d_pinfo, s, b.T, b.counts.as<int>(), err));
     tm.mark("scan");
     // one launch for eigenvalues and mode values, unless per-phase timing or
     // step counts ask for the two apart
@@ -1243,7 +1236,6 @@ ncpa_status ncpa_ctx_create(ncpa_ctx** out, const ncpa_ctx_opts* opts) {
         if (const char* fv = std::getenv("NCPA_FUSE_SOLVE")) ctx->fuse_solve = fv[0] != '0';
         if (const char* mv = std::getenv("NCPA_MS_TUNE")) ctx->ms_tune = mv[0] != '0';
         if (const char* ov = std::getenv("NCPA_BISECT_ORDER")) ctx->bis_order = ov[0] != '0';
-        if (const char* sv = std::getenv("NCPA_SCAN_TRIM")) ctx->scan_trim = sv[0] != '0';
         if (const char* tv2 = std::getenv("NCPA_TL2D_SUM"))
             ctx->tl2d_method = std::atoi(tv2) == NCPA_SUM_TC_GUARDED ? NCPA_SUM_TC_GUARDED : NCPA_SUM_FP64;
         // tuning override of the eigenvalues per bisection item (1..32)

@@ -2765,114 +2765,60 @@ int expand_launch(cudaStream_t st, int n_desc, int nz_max, const ProblemInfo* pi
     return n;
 }
 
-// Scan size of every problem, then (last block) the batch-wide trim and the
-// scan's panels.  The number of eigenvalues of S (diagonal s_i, unit
-// off-diagonals) below x is close to the sum over the rows of theta_i / pi with
-// cos theta_i = (s_i - x) / 2 clipped to [-1, 1] (each row's local band is [s_i
-// - 2, s_i + 2]); on the 20000-point grids of 0.002-0.5 Hz it gives the mode
-// count in [lo, hi] within one mode.  The scan takes about two shifts per mode
-// plus 32, in units of kScanStep.  Trim: with slots > 0 (the device's warp
-// schedulers) and U units in all, the batch drops U mod slots units when that is
-// at most a quarter of U, one each from the first problems that keep at least
-// 1.75 shifts per estimated mode.
+// Scan size of every problem and the scan's panels.  The number of eigenvalues
+// of S (diagonal s_i, unit off-diagonals) below x is close to the sum over the
+// rows of theta_i / pi with cos theta_i = (s_i - x) / 2 clipped to [-1, 1] (each
+// row's local band is [s_i - 2, s_i + 2]); on the 20000-point grids of 0.002-0.5
+// Hz it gives the mode count in [lo, hi] within one mode.  The scan takes about
+// two shifts per mode plus 32, in units of kScanStep: of the problem alone, so
+// that its modes do not depend on the batch to the last bit.  (Batches were once
+// trimmed to a multiple of the device's warp schedulers, for units of one warp
+// each; units have blocks of four: 45-azimuth sweep 6.86 ms trimmed, 6.69 not,
+// 256 frequencies 2.31 and 2.28.)
 // The sum over the rows is taken in 256 partial sums (single precision: their
 // order fixes the scan's size); 1024 threads evaluate its terms, 2048 rows at a
 // time, which the sums then take from shared memory (one problem of 20000 rows
 // 31 us with a thread to a partial sum, now 22; a 45-azimuth sweep 88 and 65).
 constexpr int kSizeThreads = 1024, kSizeSums = 256, kSizeRows = 2048;
 
-__device__ __forceinline__ bool scan_trimmable(int n_scan_raw, float m_est) {
-    const int u = n_scan_raw / kScanStep;
-    return u >= 2 && m_est >= 0.f && (float)((u - 1) * kScanStep) >= 1.75f * m_est;
-}
-
-__device__ int size_block_sum(int v, int* sh) {  // inclusive over the threads; sh[kSizeThreads] ints
-    const int t = threadIdx.x;
-    __syncthreads();
-    sh[t] = v;
-    __syncthreads();
-    for (int o = 1; o < kSizeThreads; o <<= 1) {
-        const int a = t >= o ? sh[t - o] : 0;
-        __syncthreads();
-        sh[t] += a;
-        __syncthreads();
-    }
-    return sh[t];
-}
-
 __global__ void __launch_bounds__(kSizeThreads) k_panel_size(int P, ProblemInfo* __restrict__ pinfo,
-                                                             const double* __restrict__ s, int slots,
-                                                             unsigned* __restrict__ done) {
+                                                             const double* __restrict__ s) {
     __shared__ float part[kSizeSums / 32], term[kSizeRows];
-    __shared__ int sh[kSizeThreads];
-    __shared__ bool last;
-    {
-        const int p = blockIdx.x;
-        const double lo = pinfo[p].lo, hi = pinfo[p].hi;
-        const double* __restrict__ row = s + pinfo[p].s_off;
-        const int nz = pinfo[p].nz;
-        float acc = 0.f;
-        for (int r0 = 0; r0 < nz; r0 += kSizeRows) {
+    const int p = blockIdx.x;
+    const double lo = pinfo[p].lo, hi = pinfo[p].hi;
+    const double* __restrict__ row = s + pinfo[p].s_off;
+    const int nz = pinfo[p].nz;
+    float acc = 0.f;
+    for (int r0 = 0; r0 < nz; r0 += kSizeRows) {
 #pragma unroll
-            for (int j = 0; j < kSizeRows / kSizeThreads; ++j) {
-                const int t = threadIdx.x + j * kSizeThreads, i = r0 + t;
-                float x = 0.f;
-                if (i < nz) {
-                    const double v = row[i];
-                    const float ch = fminf(fmaxf((float)((v - hi) * 0.5), -1.f), 1.f);
-                    const float cl = fminf(fmaxf((float)((v - lo) * 0.5), -1.f), 1.f);
-                    x = acosf(ch) - acosf(cl);
-                }
-                term[t] = x;
+        for (int j = 0; j < kSizeRows / kSizeThreads; ++j) {
+            const int t = threadIdx.x + j * kSizeThreads, i = r0 + t;
+            float x = 0.f;
+            if (i < nz) {
+                const double v = row[i];
+                const float ch = fminf(fmaxf((float)((v - hi) * 0.5), -1.f), 1.f);
+                const float cl = fminf(fmaxf((float)((v - lo) * 0.5), -1.f), 1.f);
+                x = acosf(ch) - acosf(cl);
             }
-            __syncthreads();
-            if (threadIdx.x < kSizeSums)
-                for (int j = 0; j < kSizeRows / kSizeSums; ++j) acc += term[threadIdx.x + j * kSizeSums];
-            __syncthreads();
+            term[t] = x;
         }
+        __syncthreads();
+        if (threadIdx.x < kSizeSums)
+            for (int j = 0; j < kSizeRows / kSizeSums; ++j) acc += term[threadIdx.x + j * kSizeSums];
+        __syncthreads();
+    }
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-        if ((threadIdx.x & 31) == 0 && threadIdx.x < kSizeSums) part[threadIdx.x >> 5] = acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float t = 0.f;
-            for (int w = 0; w < kSizeSums / 32; ++w) t += part[w];
-            const float m_est = fmaxf(t * (float)(1.0 / kPi), 0.f);
-            const int n = ((int)(2.f * m_est) + 32 + kScanStep - 1) / kScanStep * kScanStep;
-            pinfo[p].n_scan_raw = min(max(n, kScanStep), kScanMax);
-            pinfo[p].m_est = m_est;
-            __threadfence();
-            last = atomicAdd(done, 1u) == gridDim.x - 1;
-        }
-        __syncthreads();
-    }
-    if (!last) return;
-    __threadfence();
-    // the records are read past L1: other blocks wrote them
-    auto raw = [&](int p) { return __ldcg(&pinfo[p].n_scan_raw); };
-    auto trim = [&](int p) { return scan_trimmable(raw(p), __ldcg(&pinfo[p].m_est)) ? 1 : 0; };
-    int remove = 0;
-    if (slots > 0) {
-        int u = 0;
-        for (int p = threadIdx.x; p < P; p += kSizeThreads) u += raw(p) / kScanStep;
-        size_block_sum(u, sh);
-        const int U = sh[kSizeThreads - 1];
-        const int rem = U % slots;
-        if (U >= slots && 4 * rem <= U) remove = rem;
-    }
-    int trimmed = 0;
-    for (int p0 = 0; p0 < P; p0 += kSizeThreads) {
-        const int p = p0 + threadIdx.x;
-        const int tr = remove > 0 && p < P ? trim(p) : 0;
-        const int incl = remove > 0 ? size_block_sum(tr, sh) : 0;
-        if (p < P) {
-            int n = raw(p);
-            if (tr && trimmed + incl - 1 < remove) n -= kScanStep;
-            pinfo[p].n_scan = n;
-            plan_scan_panels<EssPanel>(pinfo[p], n);
-        }
-        if (remove > 0) trimmed += sh[kSizeThreads - 1];
-        __syncthreads();
+    for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if ((threadIdx.x & 31) == 0 && threadIdx.x < kSizeSums) part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float t = 0.f;
+        for (int w = 0; w < kSizeSums / 32; ++w) t += part[w];
+        const float m_est = fmaxf(t * (float)(1.0 / kPi), 0.f);
+        const int n = ((int)(2.f * m_est) + 32 + kScanStep - 1) / kScanStep * kScanStep;
+        pinfo[p].n_scan = min(max(n, kScanStep), kScanMax);
+        pinfo[p].m_est = m_est;
+        plan_scan_panels<EssPanel>(pinfo[p], pinfo[p].n_scan);
     }
 }
 
@@ -2901,12 +2847,12 @@ int scan_launch(cudaStream_t st, int P, int nz_max, const ProblemInfo* pinfo, co
 }  // namespace
 
 int launch_panel_scan(cudaStream_t st, bool wide, int P, int nz_max, ProblemInfo* pinfo, const double* rows, double* T,
-                      int* counts, int slots, unsigned* done, unsigned* err) {
+                      int* counts, unsigned* err) {
     if (wide) {
         k_panel_size_fixed<<<(P + 127) / 128, 128, 0, st>>>(P, pinfo);
         return 1 + scan_launch<WmodPanel>(st, P, nz_max, pinfo, rows, T, counts, err);
     }
-    k_panel_size<<<P, kSizeThreads, 0, st>>>(P, pinfo, rows, slots, done);
+    k_panel_size<<<P, kSizeThreads, 0, st>>>(P, pinfo, rows);
     return 1 + scan_launch<EssPanel>(st, P, nz_max, pinfo, rows, T, counts, err);
 }
 
