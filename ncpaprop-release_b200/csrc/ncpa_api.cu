@@ -723,10 +723,15 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
         check_launch(ctx, ncpa::launch_panel_fill(st, wide, P, M->nz_max, v.m_max, a));
         tm.mark("vectors");
     }
-    CK(cudaMemcpyAsync(tot_dst, b.tot.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(tot_dst, b.tot.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(info_dst, d_pinfo, P * sizeof(ProblemInfo), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(err_dst, err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
 }
+
+// After enqueue_solve and a wait: items by rows without a launch for them.  The
+// records are sized from bounds (layout_panels), which a plan's profiles may
+// leave between replays.
+bool lacks_rows(const ncpa_modes* M, const int* tot) { return tot[3] > 0 && !M->rows; }
 
 // After enqueue_solve: waits for the stream, reports a problem above
 // max_modes and device errors, records the mode total and fetches the modes
@@ -745,7 +750,8 @@ void finish_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const int* tot, 
 // Window, Sturm scan, work items, bisection and eigenvectors over all
 // problems of M (their matrices built; each problem's rows of s, w, g and kz2
 // at the offsets in its ProblemInfo).  h_info: P records, pinned or M->info.
-void solve_core(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_params* prm, bool wkb, DevBuf& s,
+// False: to be done again with M->rows.
+bool solve_core(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_params* prm, bool wkb, DevBuf& s,
                 DevBuf& w, DevBuf& g, DevBuf& kz2, ProblemInfo* h_info) {
     Tuning t;
     if (ctx->item_override > 0) t.bis_item = std::min(ctx->item_override, ncpa::kWItem);
@@ -755,8 +761,10 @@ void solve_core(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_par
     enqueue_solve(ctx, tm, M, prm, wkb, s.as<double>(), w.as<double>(), g.as<double>(), kz2.as<double>(), b, t,
                   ctx->stats && !ctx->stats_fused, ctx->h_tot, h_info, h_err);
     CK(cudaStreamSynchronize(ctx->stream));
+    if (lacks_rows(M, ctx->h_tot)) return false;
     if (h_info != M->info.data()) std::copy(h_info, h_info + M->P, M->info.begin());
     finish_solve(ctx, tm, M, ctx->h_tot, h_err);
+    return true;
 }
 
 void init_modes(ncpa_modes* M, ncpa_ctx* ctx, const ncpa_ess_params* prm, int P) {
@@ -917,27 +925,31 @@ void solve_groups(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, std:
     const bool wide = prm->method == NCPA_METHOD_WMOD;
     if (wide)
         for (Group& g : groups) wmod_geometry(g, prm);
-    long long s_tot = 0, w_tot = 0;
-    layout_groups(M, groups, s_tot, w_tot);
-    layout_panels(M, groups, prm, 1.0);
-    upload(M->d_pinfo, M->info, st);
     const bool wkb = wants_wkb(prm);
     DevBuf s, w, gs, kz2;
-    s.alloc((size_t)s_tot * (wide ? 16 : 8), st);
-    w.alloc((size_t)w_tot * 8, st);
-    if (wkb) kz2.alloc((size_t)s_tot * 8, st);
-    if (prm->want_group_speed && !wide) gs.alloc((size_t)s_tot * 8, st);
     static_assert(sizeof(ProblemInfo) % 8 == 0, "records behind the densities");
     // the records come back behind the densities; very many of them (4 MB and
     // up) straight to their place, at the driver's pace
     const bool stage = (size_t)M->P * sizeof(ProblemInfo) <= (4u << 20);
     double* rho_pairs = pinned(ctx, 2 * groups.size() + (stage ? (size_t)M->P * (sizeof(ProblemInfo) / 8) : 0));
     ProblemInfo* h_info = stage ? reinterpret_cast<ProblemInfo*>(rho_pairs + 2 * groups.size()) : M->info.data();
-    ProblemInfo* d_pinfo = M->d_pinfo.as<ProblemInfo>();
     GroupTable gt;
-    prepare_groups(ctx, prm, groups, d_pinfo, s.as<double>(), w.as<double>(), gs.as<double>(), kz2.as<double>(), gt);
-    enqueue_groups(ctx, tm, gt, rho_pairs);
-    solve_core(ctx, tm, M, prm, wkb, s, w, gs, kz2, h_info);
+    for (bool again = false;; again = true) {
+        long long s_tot = 0, w_tot = 0;
+        if (again) M->info.assign(M->P, ProblemInfo{});
+        layout_groups(M, groups, s_tot, w_tot);
+        layout_panels(M, groups, prm, 1.0);
+        if (again) M->rows = true;
+        upload(M->d_pinfo, M->info, st);
+        s.alloc((size_t)s_tot * (wide ? 16 : 8), st);
+        w.alloc((size_t)w_tot * 8, st);
+        if (wkb) kz2.alloc((size_t)s_tot * 8, st);
+        if (prm->want_group_speed && !wide) gs.alloc((size_t)s_tot * 8, st);
+        prepare_groups(ctx, prm, groups, M->d_pinfo.as<ProblemInfo>(), s.as<double>(), w.as<double>(), gs.as<double>(),
+                       kz2.as<double>(), gt);
+        enqueue_groups(ctx, tm, gt, rho_pairs);
+        if (solve_core(ctx, tm, M, prm, wkb, s, w, gs, kz2, h_info)) break;
+    }
     for (size_t gi = 0; gi < groups.size(); ++gi) {
         const Group& g = groups[gi];
         const int np = g.n_freq * g.n_az;
@@ -975,6 +987,7 @@ struct PlanData {
     cudaGraphExec_t exec = nullptr;
     long long kernels = 0;  // kernel launches in one replay
     double tuned_ms = 0.0;
+    int min_item = ncpa::kWItem;  // smallest item size its buffers are for
 };
 
 // The device sequence of a plan (captured into its graph).
@@ -1045,6 +1058,26 @@ void finish_plan(PlanData& pl) {
         }
     }
     pl.ran = true;
+}
+
+// One replay of the plan's graph, and its results.
+void run_plan(PlanData& pl) {
+    ncpa_ctx* ctx = pl.ctx;
+    ncpa_modes* M = pl.M.get();
+    for (;;) {
+        if (!pl.exec) throw ApiError(NCPA_ECUDA, "the plan was lost with an earlier error");
+        CK(cudaGraphLaunch(pl.exec, ctx->stream));
+        ctx->launches += pl.kernels;
+        CK(cudaStreamSynchronize(ctx->stream));
+        if (!lacks_rows(M, pl.h_tot)) break;
+        // with the launch of these items, and checkpoints for it: a new graph
+        M->rows = true;
+        cudaGraphExecDestroy(pl.exec);
+        pl.exec = nullptr;
+        prepare_solve(ctx, M, &pl.prm, pl.min_item, pl.sb);
+        pl.exec = capture_plan(pl, pl.tuning);
+    }
+    finish_plan(pl);
 }
 
 // Replays exec reps times (after one untimed replay) and returns ms per replay.
@@ -2356,7 +2389,8 @@ ncpa_status ncpa_ess_plan_create(ncpa_ctx* ctx, const ncpa_ess_job* jobs, int n_
                        pl.gs.as<double>(), pl.kz2.as<double>(), pl.gt);
         const int kMinItem = 16;  // smallest bisection item the tuner tries
         pl.sb.own_ck = true;
-        prepare_solve(ctx, M, &pl.prm, tune ? kMinItem : ncpa::kWItem, pl.sb);
+        if (tune) pl.min_item = kMinItem;
+        prepare_solve(ctx, M, &pl.prm, pl.min_item, pl.sb);
         if (tl) {
             pl.with_tl = true;
             pl.tp = *tl;
@@ -2412,7 +2446,10 @@ ncpa_status ncpa_ess_plan_create(ncpa_ctx* ctx, const ncpa_ess_job* jobs, int n_
             }
         }
         pl.exec = capture_plan(pl, pl.tuning);
-        if (tune) pl.tuned_ms = time_graph(pl, pl.exec, 3);
+        if (tune) {
+            run_plan(pl);
+            pl.tuned_ms = time_graph(pl, pl.exec, 3);
+        }
         *out = plan.release();
         return NCPA_OK;
     });
@@ -2423,9 +2460,7 @@ ncpa_status ncpa_ess_plan_run(ncpa_plan* plan) {
     PlanData& pl = plan->d;
     return guarded(pl.ctx, [&]() -> ncpa_status {
         CK(cudaSetDevice(pl.ctx->device));
-        CK(cudaGraphLaunch(pl.exec, pl.ctx->stream));
-        pl.ctx->launches += pl.kernels;
-        finish_plan(pl);
+        run_plan(pl);
         return NCPA_OK;
     });
 }
