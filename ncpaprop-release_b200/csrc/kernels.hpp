@@ -166,10 +166,11 @@ int launch_panel_scan(cudaStream_t st, bool wide, int P, int nz_max, ProblemInfo
                       unsigned* err);
 // c_lo, c_hi, M and off of every problem, the work items (at most bis_item
 // eigenvalues, their panel in WorkItem::pad or -1) and the panels; tot =
-// {items, items, modes, items without a panel, 0}; kErrTooMany above
-// max_modes or cap
+// {items, items, modes, items without a panel, 0, 0}, or after the first part of
+// a batch the modes and [5], the items without a panel, added to those of the
+// parts before; kErrTooMany above max_modes or cap
 int launch_panel_items(cudaStream_t st, bool wide, int P, ProblemInfo* pinfo, const int* counts, int max_modes, int bis_item,
-                       WorkItem* items, int cap, PanelDesc* desc, int* tot, unsigned* err, int order);
+                       WorkItem* items, int cap, PanelDesc* desc, int* tot, bool first, unsigned* err, int order);
 // expansions of the work items' panels
 int launch_panel_expand(cudaStream_t st, bool wide, int n_desc, int nz_max, const ProblemInfo* pinfo, const PanelDesc* desc,
                         const double* s, const double* w, const double* g, double* T, double* W0, double* W1);

@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <array>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -207,8 +208,14 @@ struct ncpa_modes {
     bool multi_job = false;                     // built by ncpa_ess_solve_jobs (one profile per job)
     bool plan_owned = false;                    // the arrays are a plan's graph buffers
     std::vector<ProblemInfo> info;
-    long long n_blocks = 0;  // block records of the panel expansions
-    int n_desc = 0;          // panels of the work items
+    // Problems [p0, p1) whose block records fit kRecordBytes, solved one part of
+    // a batch after the other in the same buffers; n_desc: panels of their items
+    struct Part {
+        int p0, p1, n_desc;
+    };
+    std::vector<Part> parts;
+    long long n_blocks = 0;  // block records of the panel expansions, and panels, the most of a part
+    int n_desc = 0;
     bool rows = false;       // some may have none
     bool twist = false;      // some modes may live between two coarse rows
     int Mtot = 0;
@@ -525,6 +532,12 @@ struct SolveBufs {
     int item_cap = 0;
 };
 
+// Bytes of block records at most (a problem that needs more gets them); a batch
+// above it is solved in parts.  At 2 Hz on 20000 rows that is some 1500 problems.
+// The last items of a part cost 0.9 ms: 1500 such problems in four parts of 8 GB
+// 101.3 ms, in one 98.6.
+constexpr size_t kRecordBytes = 32ull << 30;
+
 int modes_grid(const ncpa_ctx* ctx, int ctas_per_sm) {
     const int fit = ncpa::panel_ctas_per_sm();
     return ctx->num_sms * (ctas_per_sm > 0 ? std::min(ctas_per_sm, fit) : fit);
@@ -552,7 +565,7 @@ void prepare_solve(ncpa_ctx* ctx, ncpa_modes* M, const ncpa_ess_params* prm, int
     const bool two = prm->want_group_speed || prm->method == NCPA_METHOD_WMOD;  // weights of the expansions
     const size_t n_ex = (nT + (two ? 2 : 1) * nW) * 8;
     // a quarter more than asked when it grows: other atmospheres need a little more or less
-    if (ex.bytes < n_ex) ex.alloc(b.own_ck ? n_ex : n_ex + n_ex / 4, st);
+    if (ex.bytes < n_ex) ex.alloc(b.own_ck ? n_ex : std::max(n_ex, std::min(n_ex + n_ex / 4, kRecordBytes)), st);
     b.T = ex.as<double>();
     b.W0 = b.T + nT;
     b.W1 = two ? b.W0 + nW : nullptr;
@@ -639,91 +652,96 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
     check_launch(ctx, ncpa::launch_window(st, P, d_pinfo, wkb ? kz2 : nullptr, wkb ? 1 : 0, prm->wvnum_filter,
                                           prm->c_min, prm->c_max, err));
     tm.mark("window");
-    // ---- isolation scan ----
-    // item counters of the launches below
-    CK(cudaMemsetAsync(b.sched.p, 0, 8 * sizeof(int), st));
-    check_launch(ctx, ncpa::launch_panel_scan(st, wide, P, M->nz_max, d_pinfo, s, b.T, b.counts.as<int>(), err));
-    tm.mark("scan");
-    // one launch for eigenvalues and mode values, unless per-phase timing or
-    // step counts ask for the two apart
-    const bool fuse = ctx->fuse_solve && !ctx->timing && (!ctx->stats || ctx->stats_fused) && !count_steps;
-    check_launch(ctx, ncpa::launch_panel_items(st, wide, P, d_pinfo, b.counts.as<int>(), M->prm.max_modes, t.bis_item,
-                                               b.items.as<WorkItem>(), b.item_cap, desc, b.tot.as<int>(), err,
-                                               ctx->bis_order ? 1 : 0));
-    tm.mark("host-items");
     VecBufs v;
-    if (prm->want_vectors) prepare_vectors(ctx, M, b, v);
-    // ---- panel expansions ----
-    check_launch(ctx, ncpa::launch_panel_expand(st, wide, M->n_desc, M->nz_max, d_pinfo, desc, s, w, g, b.T,
-                                                b.W0, b.W1));
-    tm.mark("expand");
     ncpa::ModesArgs a{};
-    a.pinfo = d_pinfo;
-    a.rows = s;
-    a.w = w;
-    a.g = g;
-    a.T = b.T;
-    a.W0 = b.W0;
-    a.W1 = b.W1;
-    a.desc = desc;
-    a.counts = b.counts.as<int>();
-    a.items = b.items.as<WorkItem>();
-    a.n_items_dev = b.tot.as<int>();
-    a.item_cap = b.item_cap;
-    a.tol = wide ? kWmodTol : kBisectTol;
-    a.mu = b.mu.as<double>();
-    a.kr = M->d_kr.as<double>();
-    a.ki = M->d_ki.as<double>();
-    a.vs = M->d_vs.as<double>();
-    a.vr = M->d_vr.as<double>();
-    a.vg = M->d_vg.as<double>();
-    a.ck_u = (b.own_ck ? b.ck1 : ctx->ck1).as<double>();
-    a.ck_e = (b.own_ck ? b.cke : ctx->cke).as<int>();
-    a.ck_stride = ncpa::coarse_slot_elems(M->nz_max);
-    a.sched = ctx->bis_order ? b.sched.as<int>() : nullptr;
-    a.num_sms = ctx->num_sms;
-    a.redo = b.redo.as<int2>();
-    a.n_redo = b.tot.as<int>() + 4;
-    a.err = err;
-    if (prm->want_vectors) {
-        a.vstate = v.state.as<ncpa::VecState>();
-        a.vstate_off = v.off.as<long long>();
-        a.vtwist = v.twist.as<ncpa::VecTwist>();
-        a.vpeak = v.peak.as<unsigned long long>();
-        a.vfull = M->d_vfull.as<double>();
-        a.vfull_off = M->d_vfull_off.as<long long>();
-    }
-    auto modes = [&](int what) {
-        const int grid = modes_grid(ctx, t.bis_ctas);
-        int n = 0;
-        if (M->rows) {
-            CK(cudaEventRecord(ctx->forked, st));
-            CK(cudaStreamWaitEvent(ctx->side, ctx->forked, 0));
-            n = ncpa::launch_rows_modes(ctx->side, wide, grid, a, what);
-            CK(cudaEventRecord(ctx->joined, ctx->side));
+    for (const ncpa_modes::Part& part : M->parts) {
+        const int n_p = part.p1 - part.p0;
+        ProblemInfo* pinfo = d_pinfo + part.p0;
+        int* counts = b.counts.as<int>() + (size_t)part.p0 * ncpa::kScanMax;
+        // ---- isolation scan ----
+        // item counters of the launches below
+        CK(cudaMemsetAsync(b.sched.p, 0, 8 * sizeof(int), st));
+        check_launch(ctx, ncpa::launch_panel_scan(st, wide, n_p, M->nz_max, pinfo, s, b.T, counts, err));
+        tm.mark("scan");
+        // one launch for eigenvalues and mode values, unless per-phase timing or
+        // step counts ask for the two apart
+        const bool fuse = ctx->fuse_solve && !ctx->timing && (!ctx->stats || ctx->stats_fused) && !count_steps;
+        check_launch(ctx, ncpa::launch_panel_items(st, wide, n_p, pinfo, counts, M->prm.max_modes, t.bis_item,
+                                                   b.items.as<WorkItem>(), b.item_cap, desc, b.tot.as<int>(),
+                                                   part.p0 == 0, err, ctx->bis_order ? 1 : 0));
+        tm.mark("host-items");
+        if (prm->want_vectors) prepare_vectors(ctx, M, b, v);
+        // ---- panel expansions ----
+        check_launch(ctx, ncpa::launch_panel_expand(st, wide, part.n_desc, M->nz_max, pinfo, desc, s, w, g, b.T,
+                                                    b.W0, b.W1));
+        tm.mark("expand");
+        a.pinfo = pinfo;
+        a.rows = s;
+        a.w = w;
+        a.g = g;
+        a.T = b.T;
+        a.W0 = b.W0;
+        a.W1 = b.W1;
+        a.desc = desc;
+        a.counts = counts;
+        a.items = b.items.as<WorkItem>();
+        a.n_items_dev = b.tot.as<int>();
+        a.item_cap = b.item_cap;
+        a.tol = wide ? kWmodTol : kBisectTol;
+        a.mu = b.mu.as<double>();
+        a.kr = M->d_kr.as<double>();
+        a.ki = M->d_ki.as<double>();
+        a.vs = M->d_vs.as<double>();
+        a.vr = M->d_vr.as<double>();
+        a.vg = M->d_vg.as<double>();
+        a.ck_u = (b.own_ck ? b.ck1 : ctx->ck1).as<double>();
+        a.ck_e = (b.own_ck ? b.cke : ctx->cke).as<int>();
+        a.ck_stride = ncpa::coarse_slot_elems(M->nz_max);
+        a.sched = ctx->bis_order ? b.sched.as<int>() : nullptr;
+        a.num_sms = ctx->num_sms;
+        a.redo = b.redo.as<int2>();
+        a.n_redo = b.tot.as<int>() + 4;
+        a.err = err;
+        if (prm->want_vectors) {
+            a.vstate = v.state.as<ncpa::VecState>();
+            a.vstate_off = v.off.as<long long>();
+            a.vtwist = v.twist.as<ncpa::VecTwist>();
+            a.vpeak = v.peak.as<unsigned long long>();
+            a.vfull = M->d_vfull.as<double>();
+            a.vfull_off = M->d_vfull_off.as<long long>();
         }
-        n += ncpa::launch_panel_modes(st, wide, grid, a, what);
-        if (M->rows) CK(cudaStreamWaitEvent(st, ctx->joined, 0));
-        if (M->twist && (what & 2)) n += ncpa::launch_twist_modes(st, wide, grid, a);
-        check_launch(ctx, n);
-    };
-    if (fuse) {
-        modes(3);
-        tm.mark("bisect+eigvec");
-    } else {
-        a.steps = count_steps ? ctx->d_stats.as<unsigned long long>() : nullptr;
-        modes(1);
-        tm.mark("bisect");
-        a.steps = nullptr;
-        if (a.sched) ++a.sched;
-        modes(2);
-        tm.mark("eigvec");
+        auto modes = [&](int what) {
+            const int grid = modes_grid(ctx, t.bis_ctas);
+            int n = 0;
+            if (M->rows) {
+                CK(cudaEventRecord(ctx->forked, st));
+                CK(cudaStreamWaitEvent(ctx->side, ctx->forked, 0));
+                n = ncpa::launch_rows_modes(ctx->side, wide, grid, a, what);
+                CK(cudaEventRecord(ctx->joined, ctx->side));
+            }
+            n += ncpa::launch_panel_modes(st, wide, grid, a, what);
+            if (M->rows) CK(cudaStreamWaitEvent(st, ctx->joined, 0));
+            if (M->twist && (what & 2)) n += ncpa::launch_twist_modes(st, wide, grid, a);
+            check_launch(ctx, n);
+        };
+        if (fuse) {
+            modes(3);
+            tm.mark("bisect+eigvec");
+        } else {
+            a.steps = count_steps ? ctx->d_stats.as<unsigned long long>() : nullptr;
+            modes(1);
+            tm.mark("bisect");
+            a.steps = nullptr;
+            if (a.sched) ++a.sched;
+            modes(2);
+            tm.mark("eigvec");
+        }
     }
     if (prm->want_vectors) {
         check_launch(ctx, ncpa::launch_panel_fill(st, wide, P, M->nz_max, v.m_max, a));
         tm.mark("vectors");
     }
-    CK(cudaMemcpyAsync(tot_dst, b.tot.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(tot_dst, b.tot.p, 6 * sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(info_dst, d_pinfo, P * sizeof(ProblemInfo), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(err_dst, err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
 }
@@ -731,7 +749,7 @@ void enqueue_solve(ncpa_ctx* ctx, PhaseTimer& tm, ncpa_modes* M, const ncpa_ess_
 // After enqueue_solve and a wait: items by rows without a launch for them.  The
 // records are sized from bounds (layout_panels), which a plan's profiles may
 // leave between replays.
-bool lacks_rows(const ncpa_modes* M, const int* tot) { return tot[3] > 0 && !M->rows; }
+bool lacks_rows(const ncpa_modes* M, const int* tot) { return tot[3] + tot[5] > 0 && !M->rows; }
 
 // After enqueue_solve: waits for the stream, reports a problem above
 // max_modes and device errors, records the mode total and fetches the modes
@@ -846,7 +864,8 @@ std::pair<double, double> ceff_bounds(const ncpa_profile* prof, int k) {
 // itself wider than kRhoMax / (2 b)^2; over disjoint panels that makes at most
 // 2 nz R B / kRhoMax records, or 2 nz sqrt(n R / kRhoMax) for n items.  slack
 // widens R for plans, whose profiles may change between replays.  A problem
-// that needs more after all sweeps its raw rows.
+// that needs more after all sweeps its raw rows.  Then cuts the batch into parts
+// whose records fit kRecordBytes.
 void layout_panels(ncpa_modes* M, const std::vector<Group>& groups, const ncpa_ess_params* prm, double slack) {
     M->n_blocks = 0;
     M->n_desc = 0;
@@ -893,15 +912,32 @@ void layout_panels(ncpa_modes* M, const std::vector<Group>& groups, const ncpa_e
                 const double b_min = std::max(std::min(B, 60.0 * c_lo / kh), 8.0);
                 const double blocks = std::min(2.0 * nz * R * B / rho, 2.0 * nz * std::sqrt(n * R / rho)) +
                                       2.0 * std::ceil(nz / b_min);
-                pi.grp_off = M->n_desc;
                 pi.grp_cap = (int)n_g;
-                M->n_desc += pi.grp_cap;
-                pi.blk_off = M->n_blocks;
                 // every panel's records are padded to whole chunks
                 pi.blk_cap = (int)blocks + (int)(std::max(n_g, n_s) + 1.0) * ncpa::kPanelChunk;
-                M->n_blocks += pi.blk_cap;
             }
         }
+    // full vectors are larger than the records by far, and sized for the batch: no parts
+    const bool two = prm->want_group_speed || prm->method == NCPA_METHOD_WMOD;
+    const long long most =
+        prm->want_vectors ? LLONG_MAX : (long long)(kRecordBytes / (8 * (ncpa::kRecT + (two ? 2 : 1) * ncpa::kRecW)));
+    M->parts.clear();
+    long long n_blocks = 0;
+    for (int p = 0; p < M->P; ++p) {
+        ProblemInfo& pi = M->info[p];
+        if (p == 0 || n_blocks + pi.blk_cap > most) {
+            M->parts.push_back({p, p, 0});
+            n_blocks = 0;
+        }
+        ncpa_modes::Part& part = M->parts.back();
+        part.p1 = p + 1;
+        pi.grp_off = part.n_desc;
+        part.n_desc += pi.grp_cap;
+        pi.blk_off = n_blocks;
+        n_blocks += pi.blk_cap;
+        M->n_blocks = std::max(M->n_blocks, n_blocks);
+        M->n_desc = std::max(M->n_desc, part.n_desc);
+    }
 }
 
 // WMod (wide-angle): the matrix spacing of WModeSolver::solve, (maxheight - z_min) / Nz_grid
@@ -2382,7 +2418,7 @@ ncpa_status ncpa_ess_plan_create(ncpa_ctx* ctx, const ncpa_ess_job* jobs, int n_
         if (pl.wkb) pl.kz2.alloc((size_t)s_tot * 8, st);
         if (prm->want_group_speed) pl.gs.alloc((size_t)s_tot * 8, st);
         CK(cudaHostAlloc((void**)&pl.h_info, (size_t)P * sizeof(ProblemInfo), cudaHostAllocDefault));
-        CK(cudaHostAlloc((void**)&pl.h_tot, 4 * sizeof(int), cudaHostAllocDefault));
+        CK(cudaHostAlloc((void**)&pl.h_tot, 6 * sizeof(int), cudaHostAllocDefault));
         CK(cudaHostAlloc((void**)&pl.h_err, sizeof(unsigned), cudaHostAllocDefault));
         CK(cudaHostAlloc((void**)&pl.h_rho, 2 * pl.groups.size() * sizeof(double), cudaHostAllocDefault));
         prepare_groups(ctx, prm, pl.groups, M->d_pinfo.as<ProblemInfo>(), pl.s.as<double>(), pl.w.as<double>(),

@@ -1224,13 +1224,13 @@ constexpr int kRankMax = 4096;
 
 __global__ void __launch_bounds__(kItemThreads) k_panel_items(int P, ProblemInfo* __restrict__ pinfo,
                                                               const int* __restrict__ counts, int max_modes,
-                                                              int bis_item, int cap, int* __restrict__ tot,
+                                                              int bis_item, int cap, int* __restrict__ tot, bool first,
                                                               unsigned* __restrict__ err, int order) {
     __shared__ int sh[32];
     __shared__ float skey[kRankMax];
     __shared__ int sperm[kRankMax];
     const bool ranked = order != 0 && P <= kRankMax;
-    int base_m = 0;
+    int base_m = first ? 0 : tot[2];
     for (int p0 = 0; p0 < P; p0 += kItemThreads) {
         const int p = p0 + threadIdx.x;
         int M = 0;
@@ -1282,6 +1282,7 @@ __global__ void __launch_bounds__(kItemThreads) k_panel_items(int P, ProblemInfo
         tot[0] = min(base, cap);
         tot[1] = min(base, cap);
         tot[2] = base_m;
+        tot[5] = first ? 0 : tot[5] + tot[3];
         tot[3] = tot[4] = 0;
     }
 }
@@ -2857,9 +2858,10 @@ int launch_panel_scan(cudaStream_t st, bool wide, int P, int nz_max, ProblemInfo
 }
 
 int launch_panel_items(cudaStream_t st, bool wide, int P, ProblemInfo* pinfo, const int* counts, int max_modes,
-                       int bis_item, WorkItem* items, int cap, PanelDesc* desc, int* tot, unsigned* err, int order) {
+                       int bis_item, WorkItem* items, int cap, PanelDesc* desc, int* tot, bool first, unsigned* err,
+                       int order) {
     if (bis_item < 1 || bis_item > kWItem) return -1;
-    k_panel_items<<<1, kItemThreads, 0, st>>>(P, pinfo, counts, max_modes, bis_item, cap, tot, err, order);
+    k_panel_items<<<1, kItemThreads, 0, st>>>(P, pinfo, counts, max_modes, bis_item, cap, tot, first, err, order);
     auto* f = wide ? k_panel_groups<WmodPanel> : k_panel_groups<EssPanel>;
     f<<<(P + kPlanWarps - 1) / kPlanWarps, kPlanWarps * 32, 0, st>>>(P, pinfo, counts, bis_item, items, cap, desc, tot);
     return 2;
