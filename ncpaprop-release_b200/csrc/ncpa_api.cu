@@ -1369,9 +1369,13 @@ void fill_profile(ncpa_ctx* ctx, ncpa_profile* P, const ncpa_profile_desc* d) {
     for (int i = 0; i < n; ++i) P->h_c0[i] = d->c0 ? d->c0[i] : std::sqrt(1.4 * d->p[i] / d->rho[i]);
     P->h_u.assign(d->u, d->u + n);
     P->h_v.assign(d->v, d->v + n);
-    P->h_c0min = *std::min_element(P->h_c0.begin(), P->h_c0.end());
-    P->h_wind = 0.0;
-    for (int i = 0; i < n; ++i) P->h_wind = std::max(P->h_wind, std::sqrt(d->u[i] * d->u[i] + d->v[i] * d->v[i]));
+    double c_min = INFINITY, w2 = 0.0;
+    for (int i = 0; i < n; ++i) {
+        c_min = std::min(c_min, P->h_c0[i]);
+        w2 = std::max(w2, d->u[i] * d->u[i] + d->v[i] * d->v[i]);
+    }
+    P->h_c0min = c_min;
+    P->h_wind = std::sqrt(w2);
     const std::pair<DevBuf*, const double*> cols[] = {{&P->z, d->z}, {&P->u, d->u}, {&P->v, d->v},
                                                       {&P->t, d->t}, {&P->p, d->p}, {&P->rho, d->rho}};
     for (const auto& c : cols) CK(cudaMemcpyAsync(c.first->p, c.second, n * sizeof(double), cudaMemcpyHostToDevice, st));
