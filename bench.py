@@ -354,7 +354,8 @@ def run_ours(args):
         value = solves / (ms_dev / 1e3)
         e2e_value = solves / (ms_e2e / 1e3)
         # eigenvalue sweeps, row steps (one shift over one grid point) counted by
-        # the kernel.  At 128 rows a block: a count's four polynomials of degree
+        # the kernel, each at the flops of a row in blocks of 128: a lower bound, as
+        # rows in shorter blocks take more.  At 128 rows a block: a count's four polynomials of degree
         # 14 and two columns are 126 FP64 flops a block, 1.0 a row; a Laguerre
         # chain's, with first and second derivatives, 375, 2.9 a row
         flops = 1.0 * (sturm_steps - deriv_steps) + 2.9 * deriv_steps  # over the bis_n timed launches
@@ -390,8 +391,8 @@ def run_ours(args):
                          "traffic": None, "traffic_source": "not measured by this run (DRAM counters need ncu)",
                          "avg_launch_ms": round(bis_ms / max(bis_n, 1), 4),
                          "flops_per_launch": flops / bis_n if bis_n else None,
-                         "flops": "1.0 per count-chain row step, 2.9 per Laguerre-chain row step (blocks of 128 "
-                                  "rows)",
+                         "flops": "1.0 per count-chain row step, 2.9 per Laguerre-chain row step (as in blocks of 128 "
+                                  "rows, a lower bound: shorter ones take more)",
                          "chain_steps_per_launch": sturm_steps / bis_n if bis_n else None,
                          "laguerre_chain_steps_per_launch": deriv_steps / bis_n if bis_n else None,
                          "fused": {"kernel": "k_panel_modes (eigenvalues and mode values as in the timed steps)",

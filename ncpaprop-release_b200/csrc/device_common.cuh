@@ -44,15 +44,6 @@ __device__ __forceinline__ double spline_get(int n, const double* __restrict__ x
     return c[3] + t * (c[2] + t * (c[1] + t * c[0]));
 }
 
-__device__ __forceinline__ double spline_deriv(int n, const double* __restrict__ x,
-                                               const double* __restrict__ coef, double xq) {
-    if (xq > x[n - 1] || xq < x[0]) return 0.0;
-    int i = knot_search(n, x, xq);
-    const double* c = coef + 4 * i;
-    double t = xq - x[i];
-    return c[2] + t * (2.0 * c[1] + t * 3.0 * c[0]);
-}
-
 // shift t of an isolation scan of n points on an even grid of [lo, hi]
 __device__ __forceinline__ double scan_x(double lo, double hi, int t, int n) {
     if (t == 0) return lo;

@@ -4,8 +4,8 @@
 // to a page-locked ring of the context, and the calling thread and up to
 // kHelpers others copy the chunks on as they arrive (most of a large result's
 // time is the first touch of its pages).  Page-locked destinations are written
-// directly.  64 receivers x 20000 ranges (20 MB, 0.35 ms of it the sum): 5.0 -> 1.6 ms; one
-// problem of 0.05 Hz with 200 ranges (a few KB in eight parts): 500 -> 404 us a
+// directly.  64 receivers x 20000 ranges (20 MB, 0.35 ms of it the sum): 5.0 -> 1.1 ms; one
+// problem of 0.05 Hz with 200 ranges (a few KB in eight parts): 500 -> 336 us a
 // call.
 #pragma once
 

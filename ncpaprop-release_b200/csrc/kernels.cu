@@ -1535,8 +1535,6 @@ __global__ void __launch_bounds__(256) k_src_dft(int n, const double* __restrict
     }
 }
 
-// out[c][r] = in[r][c] for a rows x cols matrix of doubles, 32 x 32 tiles
-// staged in shared memory (both sides coalesced)
 // out[i] = (re[i], im[i])
 __global__ void __launch_bounds__(256) k_pairs(size_t n, const double* __restrict__ re, const double* __restrict__ im,
                                                double2* __restrict__ out) {
@@ -1549,6 +1547,8 @@ int launch_pairs(cudaStream_t st, size_t n, const double* re, const double* im, 
     return 1;
 }
 
+// out[c][r] = in[r][c] for a rows x cols matrix of doubles, 32 x 32 tiles
+// staged in shared memory (both sides coalesced)
 __global__ void __launch_bounds__(256) k_transpose(int rows, int cols, const double* __restrict__ in,
                                                    double* __restrict__ out) {
     __shared__ double t[32][33];

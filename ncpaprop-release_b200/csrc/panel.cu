@@ -23,9 +23,11 @@
 // segments of blocks can be taken apart.  0.1 Hz, 20000 rows: eigenvalues 750
 // -> 77 us, mode values 647 -> 86; 256 frequencies 3.28 -> 0.88 ms for both.
 // Accuracy: the rounding of a block perturbs sigma by about 1e-16 on one row
-// in B, and errors relative to u are harmless; eigenvalues agree with a
-// 128-bit evaluation of the row recurrence to 1e-18 (units of h^2 A; the row
-// recurrence itself: 1e-17), mode values to 1e-12.
+// in B, and errors relative to u are harmless.  What counts is that the shift is
+// taken as doubles see it (Shift: up to 1.1e-16) and that the iteration ends with
+// a correction below 1e-15: eigenvalues are within 1.1e-15 (median 6e-17, units
+// of h^2 A) of an evaluation of the rows in 80 bits (0.1 and 0.5 Hz, 5000 and
+// 20000 rows), mode values within 1e-12.
 //
 // Counts.  The number of negative pivots is nz minus the sign changes of u.
 // In a block, the solution that starts with u = 0 changes sign n2(x) times, and
@@ -139,10 +141,12 @@ struct EssPanel {
     // is s_i less x rounded to that grid where it lies above -2, and below,
     // where doubles are 2^-51 apart, s_i less the grid point under or over x as
     // s_i is even or odd: halfway, on average.  The block sweeps take their
-    // shifts there too (a block counts as below by its middle row), so they see
-    // the matrix that an evaluation of the rows sees to about 1e-18, and pairs
-    // of modes closer than 1e-8 or phases k r at 1000 km come out alike
-    // whichever way they are computed.
+    // shifts there too (a block counts as below by its middle row): no nearer to
+    // the exact eigenvalues, but nearer to those of an evaluation of the rows in
+    // doubles, so that pairs of modes closer than 1e-8 or phases k r at 1000 km
+    // come out alike whichever way they are computed.  (Where h k is above 1 the
+    // rows leave (-2, -1], their spacing is another, and the shift is merely
+    // rounded by as much.)
     struct Shift {
         double x, t0, t1;
         __device__ __forceinline__ Shift() {}
@@ -1218,8 +1222,8 @@ __device__ int block_scan(int v, int* sh, int* total) {
 // One CTA: per problem the mode number, the CSR offset and the place of its
 // items in the list.  With order set and P <= kRankMax the problems are listed
 // by the cost of an item, nz x m x (1 + M / 512) (m eigenvalues of a problem
-// with M: denser windows need more rounds), heaviest first; the item scheduler
-// then takes items from both ends.
+// with M: denser windows need more rounds), heaviest first, and
+// taken in that order as teams get free.
 constexpr int kRankMax = 4096;
 
 __global__ void __launch_bounds__(kItemThreads) k_panel_items(int P, ProblemInfo* __restrict__ pinfo,
@@ -2713,7 +2717,7 @@ void modes_run(cudaStream_t st, int grid, const ModesArgs& a) {
 // launch that it does not ask for returns at once; those beyond item_cap are
 // left out).  The arithmetic is the same.
 //  up to two an SM     teams of four, both stages in one launch: an item alone on
-//                      its SM has a scheduler for each warp (0.1 Hz: 77 + 102
+//                      its SM has a scheduler for each warp (0.1 Hz: 77 + 86
 //                      us as pairs 129 + 107; 32 requests 289 + 205 as pairs 543
 //                      + 207)
 //  up to 4 x the pairs teams of four for the eigenvalues, pairs for the mode
